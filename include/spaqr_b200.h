@@ -49,10 +49,10 @@ int spq_set_square(spq_tree* t, int s);
  * equal-norm ties by rounding noise): the pivot is the first column whose
  * partial norm is within rtol of the largest.  0 = first maximum. Default 1e-6. */
 int spq_set_pivot_rtol(spq_tree* t, double rtol);
-/* Tuning of the pivoted QR (no reference counterpart).  Each interface gets
- * the smallest thread-block cluster (1..16 CTAs) whose CTAs handle at most
- * max(elems, level total / (fill * SMs)) elements of the compression matrix
- * per pivot step.  elems >= 1024 (default 65536), 0 < fill <= 64 (default 2). */
+/* Tuning of the pivoted QR (no reference counterpart).   A level's
+ * interfaces get thread-block clusters (1..16 CTAs each) that together fill
+ * about fill / 2 CTAs per SM, with at least elems elements of the compression
+ * matrix a CTA.  elems >= 1024 (default 65536), 0 < fill <= 64 (default 2). */
 int spq_set_rrqr_work(spq_tree* t, double elems, double fill);
 /* Mixed precision (no reference counterpart; the reference is FP64 only):
  * bits = 32 stores the factor blocks and applies the preconditioner in float
@@ -85,6 +85,13 @@ int spq_tune_table(spq_tree* t, float* out);
  * stride byte offsets of the descriptors (bit 0 / 1: first GEMM A / B, bit 2 /
  * 3: second GEMM A / B). */
 int spq_debug_tc_probe(const float* C, const float* V, const float* W2, int m, int flags, float* out1, float* out2);
+/* Diagnostic of the pivoted QR's pivot selection (no reference counterpart):
+ * the pivots of the m x w host matrix C (column-major if cm, else row-major)
+ * on a cluster of cs CTAs (1, 2, 4, 8 or 16) holding at most smem_limit bytes
+ * of shared memory each (0: all there is).  Writes the kept rank and the
+ * columns in pivot order (colat holds min(m, w) entries). */
+int spq_debug_pivots(const double* C, int m, int w, int cm, int cs, long long smem_limit, double tol,
+                     double pivot_rtol, int* colat, int* rank);
 /* Reuse of descriptor lists across factorizations of one partition (no
  * reference counterpart; the reference rebuilds its task graph every time,
  * ptree.cpp:885-2123).  A level's lists depend only on its cluster sizes and on
@@ -250,9 +257,8 @@ int spq_level_flops(spq_tree* t, double* flops);
 /* Nominal FP64 flops of the last factorization (LAPACK Working Note 41 counts). */
 double spq_factor_flops(spq_tree* t);
 /* Bytes of compression-matrix data the pivoted QR of the last factorization
- * moves: the transposed gather (read + write), one pass for the column norms
- * and one per pivot step over the columns still active (the algorithmic
- * traffic of its roofline).  No reference counterpart. */
+ * cannot do without: the gather (read + write) and one pass for the column
+ * norms.  No reference counterpart. */
 double spq_rrqr_bytes(spq_tree* t);
 /* Bytes of device memory held by factor blocks. */
 double spq_pool_bytes(spq_tree* t);
@@ -284,9 +290,8 @@ int spq_set_rank_model(spq_tree* t, const float* params, const float* mean, cons
  * fallback rate near the quantile's complement. */
 int spq_set_rank_margin(spq_tree* t, float margin);
 /* Tuning of the learned path: the sketch's pivoted QR stops at
- * sketch_tol * tol (default 0.1); smem = 1 holds each CTA's block of the
- * sketch in shared memory when it fits (default 0: reads it from global memory,
- * measured faster on the 64^3 diffusion problem). */
+ * sketch_tol * tol (default 0.1); smem (0 or 1) is accepted
+ * and without effect: the pivot selection always works in shared memory. */
 int spq_set_sketch_tuning(spq_tree* t, double sketch_tol, int smem);
 /* out[0..2] = interfaces whose learned rank was accepted, interfaces that fell
  * back to the pivoted QR, and the sum of the sketch widths, since the model was set. */

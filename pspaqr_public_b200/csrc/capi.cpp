@@ -127,6 +127,45 @@ int spq_debug_tc_probe(const float* C, const float* V, const float* W2, int m, i
   return e ? -10 : (status ? -12 : 0);
 }
 
+int spq_debug_pivots(const double* C, int m, int w, int cm, int cs, long long smem_limit, double tol,
+                     double pivot_rtol, int* colat, int* rank) {
+  if (!C || !colat || !rank || m < 1 || w < 1 || cm < 0 || cm > 1 || cs < 1 || cs > 16 || (cs & (cs - 1))) return -1;
+  spq::PivotShape sh = spq::pivot_shape(m, w, cs, smem_limit > 0 ? (size_t)smem_limit : 227 * 1024);
+  if (!sh.ok || !spq::pivots_cluster_fit(cs, sh.smem, sh.big)) return -12;
+  const int kmin = m < w ? m : w, ldq = (m + 1) / 2 * 2;
+  const size_t nc = (size_t)m * w, nq = (size_t)ldq * kmin;
+  double* d = nullptr;
+  int* di = nullptr;
+  if (cudaMalloc(&d, sizeof(double) * (nc + nq + sh.panel + 64) + sizeof(spq::PivotTask)) != cudaSuccess) return -11;
+  if (cudaMalloc(&di, sizeof(int) * ((size_t)kmin + 1)) != cudaSuccess) {
+    cudaFree(d);
+    return -11;
+  }
+  // basis, panel, C, task: each a whole number of 16-byte units from the start
+  spq::PivotTask t{};
+  t.Q = d;
+  t.panel = d + (nq + 1) / 2 * 2;
+  double* dC = t.panel + (sh.panel + 1) / 2 * 2;
+  t.C = dC;
+  t.colat = di;
+  t.rank = di + kmin;
+  t.m = m;
+  t.w = w;
+  t.ldq = ldq;
+  t.ldc = cm ? m : w;
+  t.cm = cm;
+  auto* dt = reinterpret_cast<spq::PivotTask*>(dC + (nc + 1) / 2 * 2);
+  cudaError_t e = cudaMemcpy(dC, C, sizeof(double) * nc, cudaMemcpyHostToDevice);
+  if (!e) e = cudaMemcpy(dt, &t, sizeof(t), cudaMemcpyHostToDevice);
+  if (!e) e = spq::launch_pivots(dt, 1, cs, sh.smem, sh.big, tol, pivot_rtol, nullptr);
+  if (!e) e = cudaDeviceSynchronize();
+  if (!e) e = cudaMemcpy(rank, t.rank, sizeof(int), cudaMemcpyDeviceToHost);
+  if (!e) e = cudaMemcpy(colat, t.colat, sizeof(int) * (size_t)*rank, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  cudaFree(di);
+  return e ? -10 : 0;
+}
+
 int spq_set_tensor_cores(spq_tree* h, int mode) {
   if (!h || mode < 0 || mode > 2) return -1;
   h->t->tensor_cores = mode;

@@ -38,13 +38,7 @@ static int partition_small_left(std::vector<EdgeChunk>& v, bool fp32) {
   return (int)(mid - v.begin());
 }
 constexpr int kBigCluster = 8;    // CTAs per task for blocks of >= 8 panels
-constexpr int kRrqrMaxCols = 1024;  // own columns of C per CTA (four per thread)
-// shared memory of a CTA holding its block of C (the sketches of the learned
-// path): the block itself, the CTA's whole allotment, and the growth a
-// launch group's arrays may add when sized by its largest task
-constexpr size_t kRrqrSmemBlock = 120 * 1024;
-constexpr size_t kRrqrSmemBudget = 176 * 1024;
-constexpr size_t kRrqrSmemSlack = 48 * 1024;
+constexpr int kPivotMaxCols = 16384;  // columns of one compression matrix at most
 
 // SMs of the current device (queried once per process)
 int num_sms() {
@@ -730,7 +724,10 @@ int Tree::factorize() {
       }
       cudaEventRecord(ev[2], stream_);
       // compression matrices C (m x w) of the level's interfaces, gathered
-      // transposed into scratch by k_rrqr_assemble
+      // into scratch by k_rrqr_assemble: column-major for the pivot selection,
+      // which reads whole columns; row-major where the sketch and feature
+      // kernels, which stream rows, read them too
+      const bool c_cm = !rank_model_ && !rank_log_;
       const size_t nsp = Lv.spars_clusters.size();
       std::vector<RrqrSrc>& rs = P.rs;
       std::vector<int>& sp_w = P.sp_w;
@@ -744,7 +741,6 @@ int Tree::factorize() {
       std::vector<char> plain_qr(nsp, 1);            // interface ran the plain pivoted QR on C
       std::vector<std::array<double, 3>> sketch_qr;  // (m, ell, steps) of each sketch's pivoted QR
       int* d_stats = verbose >= 2 ? static_cast<int*>(scratch_.alloc(sizeof(int) * 8 * nsp + 8)) : nullptr;
-      double level_work = 0;
       for (size_t q = 0; q < nsp; ++q) {
         const int p = Lv.spars_clusters[q];
         const int mp = size_[p];
@@ -755,20 +751,19 @@ int Tree::factorize() {
           sp_w[q] = w;
         }
         const int w = sp_w[q];
-        sp_ldw[q] = (w + 3) / 4 * 4;
-        level_work += (double)mp * w;
-        double* Ct = scratch_.dalloc((size_t)std::max(mp, 1) * std::max(sp_ldw[q], 4));
+        sp_ldw[q] = c_cm ? std::max(mp, 1) : (w + 3) / 4 * 4;
+        double* Ct = scratch_.dalloc((size_t)std::max(mp, 1) * ((std::max(w, 1) + 3) / 4 * 4));
         if (!Ct) return fail(-11, "out of device memory (rrqr)");
         sp_C[q] = Ct;
         int c0 = 0;
         for (int k = Lv.sp_out_begin[q]; !hit && k < Lv.sp_out_end[q]; ++k) {
           const int e = Lv.sp_out[k];
-          if (rows_[e] > 0 && mp > 0) rs.push_back({ptr_[e], ld_[e], rows_[e], cols_[e], 1, Ct, sp_ldw[q], c0});
+          if (rows_[e] > 0 && mp > 0) rs.push_back({ptr_[e], ld_[e], rows_[e], cols_[e], 1, Ct, sp_ldw[q], c0, c_cm ? 1 : 0});
           c0 += rows_[e];
         }
         for (int k = Lv.sp_in_begin[q]; !hit && k < Lv.sp_in_end[q]; ++k) {
           const int e = Lv.sp_in[k];
-          if (cols_[e] > 0 && mp > 0) rs.push_back({ptr_[e], ld_[e], rows_[e], cols_[e], 0, Ct, sp_ldw[q], c0});
+          if (cols_[e] > 0 && mp > 0) rs.push_back({ptr_[e], ld_[e], rows_[e], cols_[e], 0, Ct, sp_ldw[q], c0, c_cm ? 1 : 0});
           c0 += cols_[e];
         }
         Qsp_[p] = arena_.dalloc((size_t)std::max(mp, 1) * std::max(mp, 1));
@@ -780,111 +775,103 @@ int Tree::factorize() {
         if (!spV[q] || !spT[q]) return fail(-11, "out of device memory (rrqr)");
         rr_dims.push_back({(double)mp, (double)w});
       }
-      // pivoted-QR launch groups: index 2 * log2(cluster size) + (the CTAs'
-      // blocks of C held in shared memory)
+      // pivoted-QR launch groups: pivot selections by 2 * log2(cluster size) +
+      // (rows too long for shared memory), then the QRs of the selected columns
+      // by cluster size
       struct RrqrGroups {
-        std::vector<RrqrTask> t[10];
-        int m[10], k[10], nl[10], rc[10];
-        size_t cd[10];  // largest block of C in shared memory (doubles)
-        RrqrGroups() {
-          for (int g = 0; g < 10; ++g) {
-            m[g] = k[g] = nl[g] = rc[g] = 1;
-            cd[g] = 0;
-          }
-        }
+        std::vector<PivotTask> t[10];
+        int m[10] = {};  // longest rows (error reports)
+        size_t smem[10] = {};
+        std::vector<RrqrTask> sel[3];
+        int sel_m[3] = {1, 1, 1}, sel_n[3] = {1, 1, 1};
       };
-      // A set of compression matrices of total work W is dealt so that about
-      // rrqr_fill CTAs per SM share it: each CTA holds at most
-      // max(floor, W / (rrqr_fill * SMs)) elements of C.
-      auto work_cap = [&](double W, double floor_elems) {
-        return std::max(floor_elems, W / (rrqr_fill * num_sms()));
-      };
-      // a pivoted QR of the row-major m x w matrix C (ld ldw) into V / T of
-      // interface p; rank to *rank; the orthonormal basis (m x min(m,w)) to Qc
-      // when given.  The cluster is the smallest whose CTAs each hold at most
-      // `cap` elements of C and kRrqrMaxCols columns.  With `smem` the
-      // smallest cluster whose CTAs' blocks of C fit in kRrqrSmemBlock bytes
-      // of shared memory keeps them there (when one exists).  Returns the
-      // cluster size, 0 on failure.
-      auto add_rrqr = [&](RrqrGroups& G, const double* C, int mp, int w, int ldw, int p, int* rank, double* Qc,
-                          int* stats, double cap, bool smem) -> int {
+      // a pivoted QR of the m x w matrix C (leading dimension ldc, column-major
+      // if cm) into V / T of interface p; rank to *rank; the orthonormal basis
+      // (m x min(m,w)) to Qc when given.  A set of ntasks matrices is dealt to
+      // clusters so that they fill about half of rrqr_fill CTAs per SM (one CTA
+      // of all of an SM's shared memory each where rows are long: a second wave
+      // of clusters would cost more than wider clusters save), with at least
+      // `floor` elements of C a CTA.  Returns the cluster size, 0 on failure.
+      auto add_rrqr = [&](RrqrGroups& G, const double* C, int mp, int w, int ldc, bool cm, int p, int* rank,
+                          double* Qc, int* stats, size_t ntasks, double floor) -> int {
         const double work = (double)mp * w;
         const int npan = (w + NB - 1) / NB;
         int lg = 0;
-        bool in_smem = false;
-        if (smem) {
-          for (int l2 = 0; l2 <= 4 && !in_smem; ++l2) {
-            const int c = 1 << l2;
-            if (c > 1 && (w + 1) / 2 < c) break;
-            const int nl = rrqr_cols_per_cta(w, c, true);
-            const size_t cdb = (size_t)mp * ((nl + 1) & ~1);
-            const size_t b = rrqr_smem(mp, std::min(mp, w), nl, (mp + c - 1) / c, cdb);
-            if (sizeof(double) * cdb <= kRrqrSmemBlock && b <= kRrqrSmemBudget &&
-                (c <= 8 || rrqr_cluster_fits(c, b + kRrqrSmemSlack, true))) {
-              lg = l2;
-              in_smem = true;
-            }
-          }
-        }
-        if (!in_smem) {
-          auto lc = [&](int c) { return rrqr_cols_per_cta(w, c, false); };
-          while (lg < 4 && (work > cap * (1 << lg) || lc(1 << lg) > kRrqrMaxCols) && npan >= (2 << lg)) ++lg;
-          if (lg == 4 && !rrqr_cluster_fits(16, rrqr_smem(std::max(G.m[8], mp), std::max(G.k[8], std::min(mp, w)),
-                                                          std::max(G.nl[8], lc(16)), std::max(G.rc[8], (mp + 15) / 16))))
-            lg = 3;
-        }
-        const int cs = 1 << lg;
-        const int nlc = rrqr_cols_per_cta(w, cs, in_smem);
-        if (nlc > kRrqrMaxCols) {
+        while (lg < 4 && (double)(ntasks << (lg + 1)) <= 0.5 * rrqr_fill * num_sms() && work > floor * (1 << lg) &&
+               npan >= (2 << lg))
+          ++lg;
+        PivotShape sh = pivot_shape(mp, w, 1 << lg);
+        if (lg == 4 && !pivots_cluster_fit(16, sh.smem, sh.big)) sh = pivot_shape(mp, w, 1 << --lg);
+        if (w > kPivotMaxCols || !sh.ok) {
           fail(-12, "interface too wide for the pivoted QR kernel");
           return 0;
         }
-        const int g = 2 * lg + (in_smem ? 1 : 0);
-        RrqrTask t{};
+        const int cs = 1 << lg, g = 2 * lg + (sh.big ? 1 : 0);
+        const int kmin = std::max(1, std::min(mp, w));
+        PivotTask t{};
         t.m = mp;
         t.w = w;
-        t.ldw = ldw;
-        t.ldq = std::max(1, std::min(mp, w));
+        t.ldc = ldc;
+        t.cm = cm ? 1 : 0;
+        t.ldq = (std::max(mp, 1) + 1) / 2 * 2;
         t.C = C;
-        t.Q = scratch_.dalloc((size_t)std::max(mp, 1) * t.ldq);
-        t.Qc = Qc ? Qc : scratch_.dalloc((size_t)std::max(mp, 1) * t.ldq);
-        t.F = scratch_.dalloc((size_t)std::max(w, 1) * t.ldq);
-        t.V = spV[sp_q[p]];
-        t.T = spT[sp_q[p]];
-        t.tau = scratch_.dalloc(std::max(mp, 1));
-        t.colat = static_cast<int*>(scratch_.alloc(sizeof(int) * std::max(w, 1)));
+        t.Q = scratch_.dalloc((size_t)t.ldq * kmin);
+        t.Qc = Qc;
+        t.panel = sh.panel ? scratch_.dalloc(sh.panel) : nullptr;
+        t.colat = static_cast<int*>(scratch_.alloc(sizeof(int) * kmin));
         t.rank = rank;
         t.stats = stats;
-        if (!t.Q || !t.Qc || !t.F || !t.tau || !t.colat) {
+        RrqrTask r{};
+        r.C = C;
+        r.V = spV[sp_q[p]];
+        r.T = spT[sp_q[p]];
+        r.tau = scratch_.dalloc(std::max(mp, 1));
+        r.colat = t.colat;
+        r.rank = rank;
+        r.m = mp;
+        r.w = w;
+        r.ldw = ldc;
+        r.cm = t.cm;
+        if (!t.Q || (sh.panel && !t.panel) || !t.colat || !r.tau) {
           fail(-11, "out of device memory (rrqr)");
           return 0;
         }
         G.t[g].push_back(t);
         G.m[g] = std::max(G.m[g], mp);
-        G.k[g] = std::max(G.k[g], std::min(mp, w));
-        G.nl[g] = std::max(G.nl[g], nlc);
-        G.rc[g] = std::max(G.rc[g], (mp + cs - 1) / cs);
-        if (in_smem) G.cd[g] = std::max(G.cd[g], (size_t)mp * ((nlc + 1) & ~1));
+        G.smem[g] = std::max(G.smem[g], sh.smem);
+        const int sc = cluster_for(kmin), sg = sc == 1 ? 0 : (sc == 4 ? 1 : 2);
+        G.sel[sg].push_back(r);
+        G.sel_m[sg] = std::max(G.sel_m[sg], mp);
+        G.sel_n[sg] = std::max(G.sel_n[sg], kmin);
         return cs;
       };
       auto up_any = [&](auto& v) { return upload(v.data(), sizeof(v[0]) * v.size()); };
+      auto run_selected = [&](std::vector<RrqrTask>* sel, const int* sel_m, const int* sel_n) -> int {
+        const int sel_cs[3] = {1, 4, kBigCluster};
+        for (int g = 0; g < 3; ++g) {
+          if (sel[g].empty()) continue;
+          auto* d = static_cast<RrqrTask*>(up_any(sel[g]));
+          if (!d) return fail(-11, "out of device memory (rrqr tasks)");
+          if (ck(launch_selected_qr(d, (int)sel[g].size(), sel_cs[g], sel_m[g], sel_n[g], stream_),
+                 "QR of the selected columns"))
+            return -10;
+        }
+        return 0;
+      };
       auto run_rrqr = [&](RrqrGroups& G, double tol) -> int {
         for (int g = 0; g < 10; ++g) {
           if (G.t[g].empty()) continue;
-          auto* d = static_cast<RrqrTask*>(up_any(G.t[g]));
+          auto* d = static_cast<PivotTask*>(up_any(G.t[g]));
           if (!d) return fail(-11, "out of device memory (rrqr tasks)");
           const int cs = 1 << (g / 2);
-          if (ck(launch_rrqr(d, (int)G.t[g].size(), cs, G.m[g], G.k[g], G.nl[g], G.rc[g], G.cd[g], tol, pivot_rtol,
-                             stream_),
-                 "rrqr kernel")) {
-            error += " [cluster " + std::to_string(cs) + ((g & 1) ? " (C in shared memory)" : "") + ", tasks " +
-                     std::to_string(G.t[g].size()) + ", rows " + std::to_string(G.m[g]) + ", steps " +
-                     std::to_string(G.k[g]) + ", columns/CTA " + std::to_string(G.nl[g]) + ", shared " +
-                     std::to_string(rrqr_smem(G.m[g], G.k[g], G.nl[g], G.rc[g], G.cd[g])) + " B]";
+          if (ck(launch_pivots(d, (int)G.t[g].size(), cs, G.smem[g], (g & 1) != 0, tol, pivot_rtol, stream_),
+                 "pivot selection")) {
+            error += " [cluster " + std::to_string(cs) + ", tasks " + std::to_string(G.t[g].size()) + ", rows " +
+                     std::to_string(G.m[g]) + ", shared " + std::to_string(G.smem[g]) + " B]";
             return -10;
           }
         }
-        return 0;
+        return run_selected(G.sel, G.sel_m, G.sel_n);
       };
       auto* d_rs = static_cast<RrqrSrc*>(up_vec(rs));
       if (!d_rs) return fail(-11, "out of device memory (sparsification)");
@@ -1014,8 +1001,8 @@ int Tree::factorize() {
         RrqrGroups G;
         for (size_t q = 0; q < nsp; ++q) {
           const int p = Lv.spars_clusters[q];
-          rr_cs[q] = add_rrqr(G, sp_C[q], size_[p], sp_w[q], sp_ldw[q], p, d_rank_ + p, nullptr,
-                              d_stats ? d_stats + 8 * q : nullptr, work_cap(level_work, rrqr_work), false);
+          rr_cs[q] = add_rrqr(G, sp_C[q], size_[p], sp_w[q], sp_ldw[q], c_cm, p, d_rank_ + p, nullptr,
+                              d_stats ? d_stats + 8 * q : nullptr, nsp, rrqr_work);
           if (!rr_cs[q]) return -12;
         }
         if (int rc = run_rrqr(G, tol)) return rc;
@@ -1041,13 +1028,8 @@ int Tree::factorize() {
         int sel_m[3] = {1, 1, 1}, sel_n[3] = {1, 1, 1};
         std::vector<int> pc_order[2];  // pivoted Cholesky: sketches of <= 64 columns, wider ones
         int pc_max[2] = {1, 1};
-        const int sel_cs[3] = {1, 4, kBigCluster};
         size_t mtot = 0;
-        double sketch_work = 0;
-        for (size_t q = 0; q < nsp; ++q) {
-          mtot += (size_t)ell[q] + 1;
-          sketch_work += (double)sk[q].m * std::max(1, ell[q]);
-        }
+        for (size_t q = 0; q < nsp; ++q) mtot += (size_t)ell[q] + 1;
         auto* d_M =
             static_cast<unsigned long long*>(scratch_.alloc(sizeof(unsigned long long) * std::max<size_t>(mtot, 1)));
         if (!d_M || ck(cudaMemsetAsync(d_M, 0, sizeof(unsigned long long) * mtot, stream_), "residuals"))
@@ -1099,8 +1081,8 @@ int Tree::factorize() {
             const int pg = ell[q] <= 64 ? 0 : 1;
             pc_order[pg].push_back((int)q);
             pc_max[pg] = std::max(pc_max[pg], ell[q]);
-          } else if (!add_rrqr(G, t.Y, t.m, ell[q], t.ldy, p, d_ell + q, Qc, d_stats ? d_stats + 8 * q : nullptr,
-                               work_cap(sketch_work, 4096), sketch_smem)) {
+          } else if (!add_rrqr(G, t.Y, t.m, ell[q], t.ldy, false, p, d_ell + q, Qc,
+                               d_stats ? d_stats + 8 * q : nullptr, nsp, 4096)) {
             return -12;
           }
         }
@@ -1124,14 +1106,7 @@ int Tree::factorize() {
                    "sketch pivots"))
               return -10;
           }
-          for (int g = 0; g < 3; ++g) {
-            if (sel[g].empty()) continue;
-            auto* d_sel = static_cast<RrqrTask*>(up_any(sel[g]));
-            if (!d_sel) return fail(-11, "out of device memory (sketch)");
-            if (ck(launch_selected_qr(d_sel, (int)sel[g].size(), sel_cs[g], sel_m[g], sel_n[g], stream_),
-                   "sketch QR"))
-              return -10;
-          }
+          if (int rc = run_selected(sel, sel_m, sel_n)) return rc;
         } else if (int rc = run_rrqr(G, stol)) {
           return rc;
         }
@@ -1146,9 +1121,8 @@ int Tree::factorize() {
             sync_timed("rank selection"))
           return -10;
         RrqrGroups Fb;
-        double fb_work = 0;
-        for (size_t q = 0; q < nsp; ++q)
-          if (fb[q]) fb_work += (double)sk[q].m * sk[q].w;
+        size_t nfb = 0;
+        for (int f : fb) nfb += f != 0;
         for (size_t q = 0; q < nsp; ++q) {
           const int p = Lv.spars_clusters[q];
           const SketchTask& t = sk[q];
@@ -1159,8 +1133,8 @@ int Tree::factorize() {
           plain_qr[q] = fb[q] ? 1 : 0;
           if (fb[q]) {
             ++learned_fallbacks_;
-            rr_cs[q] = add_rrqr(Fb, sp_C[q], t.m, t.w, t.ldw, p, d_rank_ + p, nullptr, nullptr,
-                                work_cap(fb_work, 16384), false);
+            rr_cs[q] = add_rrqr(Fb, sp_C[q], t.m, t.w, t.ldw, c_cm, p, d_rank_ + p, nullptr, nullptr,
+                                nfb, 16384);
             if (!rr_cs[q]) return -12;
           } else {
             ++learned_accepted_;
@@ -1172,24 +1146,23 @@ int Tree::factorize() {
           cudaEventSynchronize(le[5]);
           float ms[5];
           for (int k = 0; k < 5; ++k) cudaEventElapsedTime(&ms[k], le[k], le[k + 1]);
-          int nfb = 0;
-          for (int f : fb) nfb += f;
-          printf("learned level %d: plan %.2f sketch %.2f qr %.2f project %.2f fallback(%d) %.2f ms\n", lvl, ms[0], ms[1],
+          printf("learned level %d: plan %.2f sketch %.2f qr %.2f project %.2f fallback(%zu) %.2f ms\n", lvl, ms[0], ms[1],
                  ms[2], ms[3], nfb, ms[4]);
           if (d_stats && !gram) {
             std::vector<int> st(8 * nsp);
             cudaMemcpy(st.data(), d_stats, sizeof(int) * st.size(), cudaMemcpyDeviceToHost);
-            double steps = 0, recomp = 0, kc[6] = {0, 0, 0, 0, 0, 0}, ellsum = 0;
+            double steps = 0, rebuilds = 0, kc[3] = {0, 0, 0}, ellsum = 0;
             for (size_t q = 0; q < nsp; ++q) {
-              recomp += st[8 * q];
+              rebuilds += st[8 * q];
               steps += st[8 * q + 1];
-              for (int k = 0; k < 5; ++k) kc[k] += st[8 * q + 2 + k];
+              kc[0] += st[8 * q + 2];
+              kc[1] += st[8 * q + 3];
+              kc[2] += st[8 * q + 5];
               ellsum += ell[q];
             }
-            printf("  sketch QR: tasks %zu mean ell %.0f mean steps %.0f recomputes/task %.0f  kcycles/task pivot %.0f "
-                   "proj %.0f basis %.0f rowR %.0f finalQR %.0f\n",
-                   nsp, ellsum / nsp, steps / nsp, recomp / nsp, kc[0] / nsp, kc[1] / nsp, kc[2] / nsp, kc[3] / nsp,
-                   kc[4] / nsp);
+            printf("  sketch QR: tasks %zu mean ell %.0f mean steps %.0f rebuilds/task %.0f  kcycles/task norms %.0f "
+                   "rebuilds %.0f steps %.0f\n",
+                   nsp, ellsum / nsp, steps / nsp, rebuilds / nsp, kc[0] / nsp, kc[1] / nsp, kc[2] / nsp);
           }
         }
         for (auto& e : le) cudaEventDestroy(e);
@@ -1260,18 +1233,19 @@ int Tree::factorize() {
           return -10;
       }
       // nominal flops (LAPACK Working Note 41 geqp3 count) and the bytes of C
-      // the pivoted QR moves: the transposed gather (read + write), one pass
-      // for the norms, one per pivot step over the active columns
-      auto account = [&](double m, double w, double steps, double r) {
+      // the pivoted QR cannot do without: the gather (read + write) and one pass
+      // for the norms
+      auto account = [&](double m, double w, double r) {
         lt_[lvl].flops[4] += 4.0 * m * w * r - 2.0 * r * r * (m + w) + 4.0 * r * r * r / 3.0 + m * r * r;
-        rrqr_bytes_ += 8.0 * m * (3.0 * w + steps * w - steps * (steps + 1.0) / 2.0);
+        rrqr_bytes_ += 24.0 * m * w;
       };
-      for (const auto& e : sketch_qr) account(e[0], e[1], e[2], e[2]);
+      for (const auto& e : sketch_qr) account(e[0], e[1], e[2]);
       for (size_t q = 0; q < Lv.spars_clusters.size(); ++q) {
         const double m = rr_dims[q].first, w = rr_dims[q].second, r = size_[Lv.spars_clusters[q]];
-        if (plain_qr[q]) account(m, w, std::min(r + 1.0, std::min(m, w)), r);
+        if (plain_qr[q]) account(m, w, r);
         if (verbose >= 2)
-          printf("rrqr level %d m %d w %d rank %d cluster %d recomputed %d kcycles %d %d %d %d %d %d\n", lvl, (int)m,
+          printf("rrqr level %d m %d w %d rank %d cluster %d rebuilds %d kcycles norms %d rebuilds %d panel %d "
+                 "kcycles steps %d columns %d %d\n", lvl, (int)m,
                  (int)w, (int)r, rr_cs[q], stats[8 * q], stats[8 * q + 2], stats[8 * q + 3], stats[8 * q + 4],
                  stats[8 * q + 5], stats[8 * q + 6], stats[8 * q + 7]);
       }

@@ -112,10 +112,11 @@ class Tree {
   // largest (0 = LAPACK's first maximum).  Equal norms in exact arithmetic
   // (symmetric stencils) are otherwise resolved by rounding noise.
   double pivot_rtol = 1e-6;
-  // pivoted QR: elements of the compression matrix each CTA of a cluster
-  // handles per pivot step (sets the cluster size, 1..16 CTAs per interface)
+  // pivoted QR: a level's interfaces are dealt to clusters (1..16 CTAs each)
+  // that fill about half of rrqr_fill CTAs per SM, with at least rrqr_work
+  // elements of the compression matrix a CTA.  64^3 Laplacian, tolerance 1e-2:
+  // fill 2 / 4 / 8 give 104 / 102 / 108 ms of pivoted QR.
   double rrqr_work = 65536;
-  // ... and a level's compression work is spread over about rrqr_fill CTAs per SM
   double rrqr_fill = 2;
   // factor storage and preconditioner arithmetic: 64 (plain) or 32 (mixed
   // precision: float blocks and solve, double SpMV, Krylov loop and pivoted
@@ -153,8 +154,7 @@ class Tree {
   // learned ranks: the sketch's pivoted QR stops at sketch_tol * tol (the
   // kept rank is then chosen on C itself)
   double sketch_tol = 0.1;
-  // the sketch's pivoted QR holds each CTA's block of the sketch in shared
-  // memory when it fits
+  // accepted and without effect: the pivot selection always works in shared memory
   bool sketch_smem = false;
   // learned ranks: added to the predicted kept fraction before the sketch is
   // sized (an upper quantile of the predictor's error on its training pairs)

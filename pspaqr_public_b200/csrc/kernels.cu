@@ -820,41 +820,24 @@ __global__ void __launch_bounds__(kThreads) k_edge_right(const EdgeChunk* __rest
 // ------------------------------------------------------------ RRQR
 // Truncated column-pivoted QR of the compression matrix C (m x w) of one
 // interface: LAPACK geqp3 stopped at the first i >= 1 with
-// |R(i,i)| / |R(0,0)| < tol (ptree.cpp:373-439, util.cpp:830-851).
-//
-// The pivot sequence follows dlaqp2 step by step: the pivot is the first
-// POSITION (column order after dlaqp2's swaps) whose partial norm is within
-// pivot_rtol of the largest, partial norms are downdated with row i of R and
-// recomputed when the downdate loses accuracy (tol3z = sqrt(eps)).  C itself
-// is never rewritten: row i of R is q_i^T C, where q_i is column i of the
-// orthonormal factor, obtained by Gram-Schmidt with reorthogonalisation (CGS2)
-// of the pivot column against q_0..q_{i-1}; |R(i,i)| is the norm left after
-// the projection.  Each step therefore READS C once (one GEMV) instead of
-// reading and rewriting the trailing matrix.  With the pivots known, the
-// Householder reflectors are those of an unpivoted QR of the selected
-// columns in pivot order (the first k steps of a pivoted QR act on exactly
-// those columns), computed by dist_qr into V, tau and the panel factors T.
-//
-// A task runs on one thread-block cluster.  C is stored transposed (Ct, w x m)
-// so the GEMV is coalesced with one column per thread; columns are dealt to
-// the CTAs in contiguous ranges and rows of the basis in contiguous slices.
-// Five cluster barriers per step publish the two pivot reductions, the two
-// Gram-Schmidt projections and the new basis vector; every published value
-// is reduced over the CTAs in rank order, so all CTAs take identical
-// decisions.
+// |R(i,i)| / |R(0,0)| < tol (ptree.cpp:373-439, util.cpp:830-851).  pivot.cu
+// selects the pivots; the Householder reflectors are then those of an
+// unpivoted QR of the selected columns in pivot order (the first k steps of a
+// pivoted QR act on exactly those columns), computed by k_selected_qr.
 
-// Gathers the compression matrix of every task, transposed: C column c0 + jj
-// is row jj of an out-block A(n,p) or column jj of an in-block A(p,m).
+// Gathers the compression matrix of every task: C column c0 + jj is row jj of
+// an out-block A(n,p) or column jj of an in-block A(p,m).  Where the source's
+// contiguous index is not the destination's, 32 x 32 tiles turn in shared memory.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_rrqr_assemble(const RrqrSrc* __restrict__ srcs) {
   __shared__ double tile[32][33];
   const RrqrSrc s = srcs[blockIdx.x];
   const T* SA = as<T>(s.A);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double* dst = s.Ct + s.c0;
-  if (s.transpose) {
-    for (int r = warp; r < s.cols; r += kWarps)
-      for (int jj = lane; jj < s.rows; jj += 32) dst[(size_t)r * s.w + jj] = (double)SA[jj + (size_t)r * s.lda];
+  double* dst = s.C + (s.cm ? (size_t)s.c0 * s.ldc : (size_t)s.c0);
+  if ((s.transpose != 0) != (s.cm != 0)) {  // source columns are runs of the destination
+    for (int c = warp; c < s.cols; c += kWarps)
+      for (int r = lane; r < s.rows; r += 32) dst[(size_t)c * s.ldc + r] = (double)SA[r + (size_t)c * s.lda];
     return;
   }
   for (int j0 = 0; j0 < s.cols; j0 += 32)
@@ -866,521 +849,15 @@ __global__ void __launch_bounds__(kThreads) k_rrqr_assemble(const RrqrSrc* __res
       __syncthreads();
       for (int q = warp; q < 32; q += kWarps) {
         const int r = r0 + q, j = j0 + lane;
-        if (r < s.rows && j < s.cols) dst[(size_t)r * s.w + j] = tile[lane][q];
+        if (r < s.rows && j < s.cols) dst[(size_t)r * s.ldc + j] = tile[lane][q];
       }
       __syncthreads();
     }
 }
 
-// Column dots over the CTA's own columns [ja, ja + nloc) of C:
-// fin(jl, sum_r C(r, ja + jl) * x(r)) (kSq: x = the column itself) for every
-// jl with act(jl).  A lane reads two adjacent columns per 16-byte load, a warp
-// 64 consecutive columns (512 bytes of a row of Ct) per load instruction and
-// four such segments at once; the warps split into RG row groups (rows
-// r = rg mod RG, about 16 rows each) times kWarps / RG column groups.  The
-// loads of kRows rows are issued before their products, so every thread
-// keeps sixteen 16-byte loads in flight (64 KB per CTA).  Partial sums meet in `gp` (8 * kThreads doubles)
-// and are added in row-group order.
-constexpr int kRows = 4;  // rows of loads issued together in col_dots
-
-template <bool kSq, bool kShared, typename Act, typename Fin>
-__device__ __forceinline__ void col_dots(const double* __restrict__ Ct, int ldw, int m, int ja, int nloc,
-                                         const double* x, double* gp, Act act, Fin fin) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int RG = 1;
-  while (RG < kWarps && RG * 16 < m) RG <<= 1;
-  const int CG = kWarps / RG;
-  const int rg = warp % RG, cgp = warp / RG;
-  for (int base = 0; base < nloc; base += 256 * CG) {
-    const int cb = base + 256 * cgp + 2 * lane;
-    bool a[4][2], l[4];
-    double acc[4][2];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int jl = cb + 64 * u + e;
-        a[u][e] = jl < nloc && act(jl);
-        acc[u][e] = 0.0;
-      }
-      l[u] = a[u][0] || a[u][1];
-    }
-    const double* col = Ct + ja + cb;
-    for (int r0 = rg; r0 < m; r0 += kRows * RG) {
-      double2 v[kRows][4];
-#pragma unroll
-      for (int k = 0; k < kRows; ++k) {
-        const int r = r0 + k * RG;
-        const double2* row = reinterpret_cast<const double2*>(col + (size_t)r * ldw);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          v[k][u] = (r < m && l[u]) ? (kShared ? row[32 * u] : __ldg(row + 32 * u)) : make_double2(0.0, 0.0);
-      }
-#pragma unroll
-      for (int k = 0; k < kRows; ++k) {
-        const int r = r0 + k * RG;
-        const double xr = kSq ? 0.0 : (r < m ? x[r] : 0.0);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          acc[u][0] += kSq ? v[k][u].x * v[k][u].x : v[k][u].x * xr;
-          acc[u][1] += kSq ? v[k][u].y * v[k][u].y : v[k][u].y * xr;
-        }
-      }
-    }
-    if (RG > 1) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) gp[(size_t)((warp * 4 + u) * 2 + e) * 32 + lane] = acc[u][e];
-      __syncthreads();
-      if (rg == 0) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int e = 0; e < 2; ++e)
-            for (int q = 1; q < RG; ++q) acc[u][e] += gp[(size_t)(((warp + q) * 4 + u) * 2 + e) * 32 + lane];
-      }
-      __syncthreads();
-    }
-    if (rg == 0) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-          if (a[u][e]) fin(cb + 64 * u + e, acc[u][e]);
-    }
-  }
-  __syncthreads();
-}
-
-// Sum over the cluster's CTAs, in rank order, of the value at shared address
-// x in each CTA; the remote loads are issued together.
-__device__ __forceinline__ double cluster_sum(double* x, int cs) {
-  if (cs == 1) return *x;
-  cg::cluster_group cl = cg::this_cluster();
-  double v[16];
-#pragma unroll
-  for (int q = 0; q < 16; ++q) v[q] = q < cs ? *cl.map_shared_rank(x, q) : 0.0;
-  double sum = v[0];
-#pragma unroll
-  for (int q = 1; q < 16; ++q)
-    if (q < cs) sum += v[q];
-  return sum;
-}
-
-// (position, column) with the smallest position across the warp
-__device__ __forceinline__ void warp_min_pos(int& bp, int& bc) {
-  for (int o = 16; o > 0; o >>= 1) {
-    const int op = __shfl_xor_sync(0xffffffffu, bp, o);
-    const int oc = __shfl_xor_sync(0xffffffffu, bc, o);
-    if (op < bp || (op == bp && oc < bc)) {
-      bp = op;
-      bc = oc;
-    }
-  }
-}
-
-// Partial-sum scratch of k_rrqr; vn1, vn2 and it also hold the tiled-apply
-// scratch of the final QR (dev::kTileSmem doubles).
-__host__ __device__ constexpr int rrqr_gp_doubles(int nlmax) {
-  return 8 * kThreads > dev::kTileSmem - 2 * nlmax ? 8 * kThreads : dev::kTileSmem - 2 * nlmax;
-}
-
-// Shared-memory carve of k_rrqr (doubles, then ints); rrqr_smem mirrors it.
-struct RrqrSmem {
-  double *red, *tmp, *spa, *spb, *s1, *s2, *sq, *cv, *qf, *vn1, *vn2, *gp;
-  int *pos, *flg;
-  __device__ RrqrSmem(double* sm, int mmax, int kmax, int nlmax, int rcmax) {
-    red = sm;
-    tmp = red + kRed;
-    spa = tmp + kNB;
-    spb = spa + kmax + 1;
-    s1 = spb + kmax + 1;
-    s2 = s1 + kmax + 1;
-    sq = s2 + kmax + 1;
-    cv = sq + rcmax;
-    qf = cv + rcmax;
-    vn1 = qf + mmax;
-    vn2 = vn1 + nlmax;
-    gp = vn2 + nlmax;
-    pos = reinterpret_cast<int*>(gp + rrqr_gp_doubles(nlmax));
-    flg = pos + nlmax;
-  }
-};
-
-// First own active position (>= i) whose partial norm is >= thr: position,
-// global column and norm in s_k[0][0], s_k[1][0], s_xv[0] (INT_MAX, -1, -1 if none).
-__device__ __forceinline__ void own_first(const RrqrSmem& S, int nloc, int ja, int i, double thr, int (*s_k)[kWarps],
-                                          double* s_xv) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int bp = 0x7fffffff, bc = -1;
-  double bvn = -1.0;
-  for (int jl = threadIdx.x; jl < nloc; jl += kThreads) {
-    const int p = S.pos[jl];
-    if (p >= i && p < bp && S.vn1[jl] >= thr) {
-      bp = p;
-      bc = ja + jl;
-      bvn = S.vn1[jl];
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const int op = __shfl_xor_sync(0xffffffffu, bp, o);
-    const int oc = __shfl_xor_sync(0xffffffffu, bc, o);
-    const double ov = __shfl_xor_sync(0xffffffffu, bvn, o);
-    if (op < bp) {
-      bp = op;
-      bc = oc;
-      bvn = ov;
-    }
-  }
-  __syncthreads();  // s_k / s_xv free (an earlier reader may still hold them)
-  if (lane == 0) {
-    s_k[0][warp] = bp;
-    s_k[1][warp] = bc;
-    s_xv[warp] = bvn;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 1; q < kWarps; ++q)
-      if (s_k[0][q] < s_k[0][0]) {
-        s_k[0][0] = s_k[0][q];
-        s_k[1][0] = s_k[1][q];
-        s_xv[0] = s_xv[q];
-      }
-  }
-  __syncthreads();
-}
-
-template <bool kSmemC>
-__global__ void __launch_bounds__(kThreads, 2) k_rrqr(const RrqrTask* __restrict__ tasks, double tol,
-                                                      double pivot_rtol, int cs, int mmax, int kmax, int nlmax,
-                                                      int rcmax) {
-  extern __shared__ double sm[];
-  __shared__ double s_x[kWarps];
-  __shared__ int s_k[2][kWarps];
-  __shared__ double s_xv[kWarps];
-  // published by step parity: own largest partial norm M, the first own
-  // position P whose norm is within pivot_rtol of M, its column and norm;
-  // P2/C2 for the exact second round
-  __shared__ double s_pm[2], s_pv[2];
-  __shared__ int s_pp[2], s_pc[2], s_p2[2], s_c2[2];
-  __shared__ int s_piv[3];
-  __shared__ double s_thr;
-  __shared__ int s_nflag;
-  RrqrSmem S(sm, mmax, kmax, nlmax, rcmax);
-  const RrqrTask t = tasks[blockIdx.x / cs];
-  const int rank = crank(cs);
-  const int m = t.m, w = t.w, ldq = t.ldq;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const double* __restrict__ Ct = t.C;
-  const int ldw = t.ldw;
-  double* Qt = t.Q;
-
-  // own columns [ja, jb) and own rows [ra, rb)
-  const int wc = rrqr_cols_per_cta(w, cs, kSmemC);
-  const int ja = min(w, rank * wc), jb = min(w, ja + wc), nloc = jb - ja;
-  const int rc = (m + cs - 1) / cs;
-  const int ra = min(m, rank * rc), rb = min(m, ra + rc);
-  const int kmin = min(m, w);
-  // remote shared memory of cluster rank q (the CTA's own for cs == 1)
-  auto remote = [&](double* p, int q) -> double {
-    if (cs == 1) return *p;
-    return *cg::this_cluster().map_shared_rank(p, q);
-  };
-  auto remote_i = [&](int* p, int q) -> int {
-    if (cs == 1) return *p;
-    return *cg::this_cluster().map_shared_rank(p, q);
-  };
-  // initial norms, positions
-  // kSmemC: the CTA's column block of C (m x nlp, nlp = nloc rounded up to
-  // even, the pad column zero) is held in shared memory after S's arrays and
-  // every pivot step reads it there
-  const int nlp = (nloc + 1) & ~1;
-  double* sC = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(S.flg + nlmax) + 15) & ~(uintptr_t)15);
-  if (kSmemC) {
-    for (size_t e = threadIdx.x; e < (size_t)m * nlp; e += kThreads) {
-      const int r = (int)(e / nlp), jl = (int)(e % nlp);
-      sC[e] = jl < nloc ? __ldg(Ct + (size_t)r * ldw + ja + jl) : 0.0;
-    }
-    __syncthreads();
-  }
-  const double* Cb = kSmemC ? sC : Ct + ja;
-  const int ldb = kSmemC ? nlp : ldw;
-  col_dots<true, kSmemC>(Cb, ldb, m, 0, nloc, nullptr, S.gp, [](int) { return true; }, [&](int jl, double ss) {
-    const double v = sqrt(ss);
-    S.vn1[jl] = v;
-    S.vn2[jl] = v;
-    S.pos[jl] = ja + jl;
-    t.colat[ja + jl] = ja + jl;
-  });
-  __threadfence();
-  csync(cs);
-  const double tol3z = sqrt(1.1102230246251565e-16);
-  double r00 = 0.0;
-  int rk = kmin, nrecomp = 0;
-  long long ph[4] = {0, 0, 0, 0};  // cycles: pivot choice, projections, basis vector, row of R
-  long long tc = clock64();
-  auto lap = [&](int k) {
-    const long long now = clock64();
-    ph[k] += now - tc;
-    tc = now;
-  };
-  for (int i = 0; i < kmin; ++i) {
-    const int par = i & 1;
-    // (a) own largest partial norm M over active columns (position >= i)
-    double bv = -1.0;
-    for (int jl = threadIdx.x; jl < nloc; jl += kThreads)
-      if (S.pos[jl] >= i) bv = fmax(bv, S.vn1[jl]);
-    for (int o = 16; o > 0; o >>= 1) bv = fmax(bv, __shfl_xor_sync(0xffffffffu, bv, o));
-    if (lane == 0) s_x[warp] = bv;
-    __syncthreads();
-    double mloc = s_x[0];
-    for (int q = 1; q < kWarps; ++q) mloc = fmax(mloc, s_x[q]);
-    // (b) first own position within pivot_rtol of M, published with M
-    own_first(S, nloc, ja, i, mloc * (1.0 - pivot_rtol), s_k, s_xv);
-    if (threadIdx.x == 0) {
-      s_pm[par] = mloc;
-      s_pp[par] = s_k[0][0];
-      s_pc[par] = s_k[1][0];
-      s_pv[par] = s_xv[0];
-    }
-    csync(cs);
-    // the pivot: the first position within pivot_rtol of the cluster's largest
-    // norm.  A CTA's published position is exact unless its own maximum is
-    // within pivot_rtol of the largest but the published column is not: then
-    // a second round at the cluster's threshold decides.
-    if (warp == 0) {
-      double M = -1.0, V = -1.0;
-      int P = 0x7fffffff, Cc = -1;
-      if (lane < cs) {
-        M = remote(&s_pm[par], lane);
-        V = remote(&s_pv[par], lane);
-        P = remote_i(&s_pp[par], lane);
-        Cc = remote_i(&s_pc[par], lane);
-      }
-      double gm = M;
-      for (int o = 16; o > 0; o >>= 1) gm = fmax(gm, __shfl_xor_sync(0xffffffffu, gm, o));
-      const double thr = gm * (1.0 - pivot_rtol);
-      const bool amb = lane < cs && M >= thr && !(V >= thr);
-      int bp = (lane < cs && M >= thr && V >= thr) ? P : 0x7fffffff, bc = bp != 0x7fffffff ? Cc : -1;
-      warp_min_pos(bp, bc);
-      const bool any_amb = __any_sync(0xffffffffu, amb);
-      if (lane == 0) {
-        s_piv[0] = bp;
-        s_piv[1] = bc;
-        s_piv[2] = any_amb ? 1 : 0;
-        s_thr = thr;
-      }
-    }
-    __syncthreads();
-    int ppos = s_piv[0], pcol = s_piv[1];
-    if (s_piv[2]) {
-      own_first(S, nloc, ja, i, s_thr, s_k, s_xv);
-      if (threadIdx.x == 0) {
-        s_p2[par] = s_k[0][0];
-        s_c2[par] = s_k[1][0];
-      }
-      csync(cs);
-      if (warp == 0) {
-        int bp = 0x7fffffff, bc = -1;
-        if (lane < cs) {
-          bp = remote_i(&s_p2[par], lane);
-          bc = remote_i(&s_c2[par], lane);
-        }
-        warp_min_pos(bp, bc);
-        if (lane == 0) {
-          s_piv[0] = bp;
-          s_piv[1] = bc;
-        }
-      }
-      __syncthreads();
-      ppos = s_piv[0];
-      pcol = s_piv[1];
-    }
-    const int cur = __ldcg(t.colat + i);  // column now at position i
-    if (pcol < 0) {  // no finite maximum (NaN norms): keep the column at position i
-      ppos = i;
-      pcol = cur;
-    }
-    lap(0);
-    // (c) projection s = Q^T c of the pivot column on q_0..q_{i-1} and ||c||^2,
-    // partial sums over own rows published together
-    for (int r = ra + threadIdx.x; r < rb; r += kThreads) S.cv[r - ra] = __ldg(Ct + (size_t)r * ldw + pcol);
-    __syncthreads();
-    for (int l = threadIdx.x; l < i; l += kThreads) {
-      double acc = 0.0;
-      for (int r = ra; r < rb; ++r) acc += Qt[(size_t)r * ldq + l] * S.cv[r - ra];
-      S.spa[l] = acc;
-    }
-    {
-      double cc = 0.0;
-      for (int r = ra + threadIdx.x; r < rb; r += kThreads) cc += S.cv[r - ra] * S.cv[r - ra];
-      cc = dev::cta_sum(cc, S.red);
-      if (threadIdx.x == 0) S.spa[kmax] = cc;
-    }
-    csync(cs);
-    double ss = 0.0;
-    for (int l = threadIdx.x; l < i; l += kThreads) {
-      const double v = cluster_sum(S.spa + l, cs);
-      S.s1[l] = v;
-      ss += v * v;
-    }
-    ss = dev::cta_sum(ss, S.red);
-    const double cc = cluster_sum(S.spa + kmax, cs);
-    // |R(i,i)|^2 = ||c||^2 - ||s||^2 while that loses at most 1e-10 relative
-    // accuracy; otherwise a second, explicit projection pass (CGS2)
-    double nrm2 = cc - ss;
-    const double* proj = S.s1;
-    __syncthreads();
-    for (int r = ra + warp; r < rb; r += kWarps) {
-      const double* qr = Qt + (size_t)r * ldq;
-      double d = 0.0;
-      for (int l = lane; l < i; l += 32) d += qr[l] * S.s1[l];
-      d = dev::warp_sum(d);
-      if (lane == 0) S.cv[r - ra] -= d;
-    }
-    if (!(nrm2 >= 1e-6 * cc)) {
-      __syncthreads();
-      for (int l = threadIdx.x; l < i; l += kThreads) {
-        double acc = 0.0;
-        for (int r = ra; r < rb; ++r) acc += Qt[(size_t)r * ldq + l] * S.cv[r - ra];
-        S.spb[l] = acc;
-      }
-      {
-        double nn = 0.0;
-        for (int r = ra + threadIdx.x; r < rb; r += kThreads) nn += S.cv[r - ra] * S.cv[r - ra];
-        nn = dev::cta_sum(nn, S.red);
-        if (threadIdx.x == 0) S.spb[kmax] = nn;
-      }
-      csync(cs);
-      double s2s = 0.0;
-      for (int l = threadIdx.x; l < i; l += kThreads) {
-        const double v = cluster_sum(S.spb + l, cs);
-        S.s2[l] = v;
-        s2s += v * v;
-      }
-      s2s = dev::cta_sum(s2s, S.red);
-      nrm2 = cluster_sum(S.spb + kmax, cs) - s2s;
-      proj = S.s2;
-    }
-    const double nrm = sqrt(fmax(nrm2, 0.0));  // |R(i,i)|
-    lap(1);
-    if (i == 0) {
-      r00 = nrm;
-    } else if (!(nrm / r00 >= tol)) {
-      rk = i;
-      break;
-    }
-    // (d) every CTA has read colat[i]; book the swap, update own positions
-    if (pcol >= ja && pcol < jb && threadIdx.x == 0) {
-      t.colat[ppos] = cur;
-      t.colat[i] = pcol;
-      __threadfence();
-    }
-    for (int jl = threadIdx.x; jl < nloc; jl += kThreads) {
-      const int gc = ja + jl;
-      if (gc == pcol) S.pos[jl] = i;
-      else if (gc == cur) S.pos[jl] = ppos;
-    }
-    // q_i = (c - Q s [- Q s2]) / |R(i,i)| on own rows, then gathered whole
-    const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
-    const bool second = proj == S.s2;
-    for (int r = ra + warp; r < rb; r += kWarps) {
-      double* qr = Qt + (size_t)r * ldq;
-      double d = 0.0;
-      if (second)
-        for (int l = lane; l < i; l += 32) d += qr[l] * S.s2[l];
-      d = dev::warp_sum(d);
-      if (lane == 0) {
-        const double v = (S.cv[r - ra] - d) * inv;
-        S.sq[r - ra] = v;
-        qr[i] = v;
-        t.Qc[r + (size_t)i * m] = v;
-      }
-    }
-    __threadfence();
-    csync(cs);
-    for (int r = threadIdx.x; r < m; r += kThreads) {
-      const int q = r / rc;
-      S.qf[r] = remote(S.sq + (r - q * rc), q);
-    }
-    if (threadIdx.x == 0) s_nflag = 0;
-    __syncthreads();
-    lap(2);
-    // (e) row i of R over own active columns (kept in F for recomputations);
-    // dlaqp2 downdate of the partial norms
-    double* Fi = t.F + (size_t)i * w + ja;
-    col_dots<false, kSmemC>(Cb, ldb, m, 0, nloc, S.qf, S.gp, [&](int jl) { return S.pos[jl] > i; },
-                    [&](int jl, double rij) {
-                      Fi[jl] = rij;
-                      const double v1 = S.vn1[jl];
-                      if (v1 == 0.0) return;
-                      double temp = fabs(rij) / v1;
-                      temp = 1.0 - temp * temp;
-                      temp = temp < 0.0 ? 0.0 : temp;
-                      const double qq = v1 / S.vn2[jl];
-                      if (temp * qq * qq <= tol3z) S.flg[atomicAdd(&s_nflag, 1)] = jl;
-                      else S.vn1[jl] = v1 * sqrt(temp);
-                    });
-    // recomputed partial norms ||c_j - Q(:, 0:i) R(0:i, j)||, one warp per column
-    const int nf = s_nflag;
-    nrecomp += nf;
-    for (int f = warp; f < nf; f += kWarps) {
-      const int jl = S.flg[f], j = ja + jl;
-      double res = 0.0;
-      if (i + 1 < m) {
-        for (int r = lane; r < m; r += 32) {
-          double x[4] = {0.0, 0.0, 0.0, 0.0};
-          int l = 0;
-          for (; l + 8 <= i + 1; l += 8) {
-            double qv[8], fv[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              qv[u] = __ldcg(t.Qc + (size_t)(l + u) * m + r);
-              fv[u] = t.F[(size_t)(l + u) * w + j];
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) x[u & 3] += qv[u] * fv[u];
-          }
-          for (; l <= i; ++l) x[0] += __ldcg(t.Qc + (size_t)l * m + r) * t.F[(size_t)l * w + j];
-          const double e = __ldg(Ct + (size_t)r * ldw + j) - ((x[0] + x[1]) + (x[2] + x[3]));
-          res += e * e;
-        }
-        res = dev::warp_sum(res);
-      }
-      if (lane == 0) {
-        S.vn1[jl] = sqrt(res);
-        S.vn2[jl] = sqrt(res);
-      }
-    }
-    __syncthreads();
-    lap(3);
-  }
-  csync(cs);  // no CTA reads another's shared memory past this point
-  if (rank == 0 && threadIdx.x == 0 && t.stats) {
-    t.stats[0] = nrecomp;
-    t.stats[1] = rk;
-    for (int k = 0; k < 4; ++k) t.stats[2 + k] = (int)(ph[k] >> 10);
-    t.stats[7] = 0;
-  }
-  const long long tq = clock64();
-  // Householder QR of the selected columns C(:, colat[0:rk]) into V
-  for (int l = warp; l < rk; l += kWarps) {
-    if (!owns(l, rank, cs)) continue;
-    const int c = __ldcg(t.colat + l);
-    for (int r = lane; r < m; r += 32) t.V[r + (size_t)l * m] = __ldg(Ct + (size_t)r * ldw + c);
-  }
-  __syncthreads();
-  dist_qr<double>(t.V, m, nullptr, 0, m, rk, 1, t.T, t.tau, S.s1, S.qf, S.red, S.tmp, S.vn1, cs);
-  if (rank == 0 && threadIdx.x == 0) {
-    *t.rank = rk;
-    if (t.stats) t.stats[6] = (int)((clock64() - tq) >> 10);
-  }
-}
-
-// Householder QR of the selected columns C(:, colat[0:rank]) of a row-major C
-// (the pivot order fixed beforehand) into V / T / tau, then the orthonormal
-// basis Qc = C_sel R^{-1} (column-major, ld m) over the cluster's row blocks:
+// Householder QR of the selected columns C(:, colat[0:rank]) (the pivot order
+// fixed beforehand) into V / T / tau, then (where the task has a Qc) the
+// orthonormal basis Qc = C_sel R^{-1} (column-major, ld m) over the cluster's row blocks:
 // tiles of rt rows, 32-column blocks of R, a blocked update from the solved
 // columns and a triangular solve on the diagonal block.
 // kStage: the QR's panels are factored in shared memory (dist_qr's `pan`,
@@ -1405,11 +882,15 @@ __global__ void __launch_bounds__(kThreads, 2) k_selected_qr(const RrqrTask* __r
   for (int l = warp; l < rk; l += kWarps) {
     if (!owns(l, rank, cs)) continue;
     const int c = __ldg(t.colat + l);
-    for (int r = lane; r < m; r += 32) t.V[r + (size_t)l * m] = __ldg(C + (size_t)r * ldw + c);
+    if (t.cm)
+      for (int r = lane; r < m; r += 32) t.V[r + (size_t)l * m] = __ldg(C + (size_t)c * ldw + r);
+    else
+      for (int r = lane; r < m; r += 32) t.V[r + (size_t)l * m] = __ldg(C + (size_t)r * ldw + c);
   }
   __syncthreads();
   dist_qr<double>(t.V, m, nullptr, 0, m, rk, 1, t.T, t.tau, lt, vb, red, tmp, Qt, cs, nullptr,
                   kStage ? Qt : nullptr, mmax);
+  if (!t.Qc) return;
   // R(l, j) = V[l + j m] for l <= j, written by the owners of column j
   auto R = [&](int l, int j) { return __ldcg(t.V + l + (size_t)j * m); };
   const int rc = (m + cs - 1) / cs;
@@ -1418,7 +899,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_selected_qr(const RrqrTask* __r
     const int nr = min(rt, rb - r0);
     for (int e = threadIdx.x; e < nr * rk; e += kThreads) {
       const int rr = e / rk, l = e % rk;
-      Qt[rr * ldq + l] = __ldg(C + (size_t)(r0 + rr) * ldw + __ldg(t.colat + l));
+      const int c = __ldg(t.colat + l);
+      Qt[rr * ldq + l] = __ldg(C + (t.cm ? (size_t)c * ldw + r0 + rr : (size_t)(r0 + rr) * ldw + c));
     }
     __syncthreads();
     for (int j0 = 0; j0 < rk; j0 += 32) {
@@ -2138,46 +1620,6 @@ cudaError_t launch_tc_probe(const float* C, const float* V, const float* W2, int
   return last();
 }
 
-size_t rrqr_smem(int mmax, int kmax, int nlmax, int rcmax, size_t c_doubles) {
-  const size_t d = kRed + kNB + 4 * ((size_t)kmax + 1) + 2 * (size_t)rcmax + (size_t)std::max(mmax, 1) +
-                   2 * (size_t)nlmax + (size_t)rrqr_gp_doubles(nlmax);
-  size_t b = smem_bytes(d) + sizeof(int) * 2 * (size_t)nlmax;
-  if (c_doubles) b += 16 + smem_bytes(c_doubles);
-  return b;
-}
-
-template <bool kSmemC>
-bool rrqr_fits(int cs, size_t smem) {
-  if (smem > kSmemMax) return false;
-  if (cs <= 8) return true;
-  if (prep(k_rrqr<kSmemC>, smem)) return false;
-  if (cudaFuncSetAttribute(k_rrqr<kSmemC>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) {
-    cudaGetLastError();
-    return false;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)cs);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k_rrqr<kSmemC>, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return n > 0;
-}
-
-bool rrqr_cluster_fits(int cs, size_t smem, bool smem_c) {
-  return smem_c ? rrqr_fits<true>(cs, smem) : rrqr_fits<false>(cs, smem);
-}
-
 cudaError_t launch_rrqr_assemble(const RrqrSrc* s, int nsrc, cudaStream_t st) {
   if (cudaError_t pre = begin("launch_rrqr_assemble")) return pre;
   if (nsrc <= 0) return cudaSuccess;
@@ -2185,24 +1627,6 @@ cudaError_t launch_rrqr_assemble(const RrqrSrc* s, int nsrc, cudaStream_t st) {
   if (g_fp32) k_rrqr_assemble<float><<<nsrc, kThreads, 0, st>>>(s);
   else k_rrqr_assemble<double><<<nsrc, kThreads, 0, st>>>(s);
   return last();
-}
-
-template <bool kSmemC>
-cudaError_t launch_rrqr_t(const RrqrTask* t, int ntasks, int cs, int mmax, int kmax, int nlmax, int rcmax,
-                          size_t c_doubles, double tol, double pivot_rtol, cudaStream_t st) {
-  const size_t b = rrqr_smem(mmax, kmax, nlmax, rcmax, kSmemC ? c_doubles : 0);
-  cudaError_t e = prep(k_rrqr<kSmemC>, b);
-  if (!e && cs > 8) e = cudaFuncSetAttribute(k_rrqr<kSmemC>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e) return e;
-  return launch_clustered(k_rrqr<kSmemC>, ntasks, cs, b, st, t, tol, pivot_rtol, cs, mmax, kmax, nlmax, rcmax);
-}
-
-cudaError_t launch_rrqr(const RrqrTask* t, int ntasks, int cs, int mmax, int kmax, int nlmax, int rcmax,
-                        size_t c_doubles, double tol, double pivot_rtol, cudaStream_t st) {
-  if (cudaError_t pre = begin("launch_rrqr")) return pre;
-  if (ntasks <= 0) return cudaSuccess;
-  return c_doubles ? launch_rrqr_t<true>(t, ntasks, cs, mmax, kmax, nlmax, rcmax, c_doubles, tol, pivot_rtol, st)
-                   : launch_rrqr_t<false>(t, ntasks, cs, mmax, kmax, nlmax, rcmax, 0, tol, pivot_rtol, st);
 }
 
 int selected_qr_rows(int nmax) { return std::max(1, std::min(32, 12288 / (std::max(nmax, 1) + 1))); }

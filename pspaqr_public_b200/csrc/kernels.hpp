@@ -48,32 +48,25 @@ cudaError_t launch_update(const UpdTask* t, const UpdOp* o, int ntasks, cudaStre
 // kind 0: left apply on column chunks, 1: right triangular solve on row chunks,
 // 2: right apply on row chunks
 cudaError_t launch_edge(int kind, const EdgeChunk* t, int ntasks, cudaStream_t st);
-// Columns of C one CTA of a cs-CTA cluster owns in the pivoted QR: a
-// contiguous range, a multiple of 32 columns when C streams from global
-// memory (whole 256-byte row segments), of 2 when the CTA's block is held in
-// shared memory (16-byte loads).
-#if defined(__CUDACC__)
-__host__ __device__
-#endif
-inline int rrqr_cols_per_cta(int w, int cs, bool smem_c) {
-  const int a = smem_c ? 2 : 32;
-  return ((w + cs - 1) / cs + a - 1) / a * a;
-}
-// Shared memory of one pivoted-QR CTA for tasks of at most mmax rows, kmax
-// steps, nlmax own columns and rcmax own rows; c_doubles = the largest
-// m x (own columns rounded to even) of a task whose block of C is held in
-// shared memory (0: C streams from global memory).
-size_t rrqr_smem(int mmax, int kmax, int nlmax, int rcmax, size_t c_doubles = 0);
-// a cluster of cs CTAs with smem bytes each of the pivoted QR can be resident
-bool rrqr_cluster_fits(int cs, size_t smem, bool smem_c = false);
-// transposed gather of the compression matrices (one CTA per source block)
+// gather of the compression matrices (one CTA per source block)
 cudaError_t launch_rrqr_assemble(const RrqrSrc* s, int nsrc, cudaStream_t st);
-cudaError_t launch_rrqr(const RrqrTask* t, int ntasks, int cs, int mmax, int kmax, int nlmax, int rcmax,
-                        size_t c_doubles, double tol, double pivot_rtol, cudaStream_t st);
+// Pivot selection (pivot.cu) of an m x w matrix on a cs-CTA cluster: shared
+// memory per CTA (at most `limit`), whether the panel and the basis stay in
+// global memory (rows too long for shared memory) and the doubles of panel
+// scratch a task then needs; ok = 0 when the matrix is too wide.
+struct PivotShape {
+  size_t smem, panel;
+  bool big, ok;
+};
+PivotShape pivot_shape(int m, int w, int cs, size_t limit = 227 * 1024);
+// a cluster of cs CTAs with smem bytes each can be resident
+bool pivots_cluster_fit(int cs, size_t smem, bool big);
+cudaError_t launch_pivots(const PivotTask* t, int ntasks, int cs, size_t smem, bool big, double tol,
+                          double pivot_rtol, cudaStream_t st);
 // Householder QR of the columns C(:, colat[0:*rank]) (pivot order given) into
-// V / T / tau and the orthonormal basis Qc = C_sel R^{-1}; cs-CTA clusters,
-// tasks of at most mmax rows and nmax selected columns.  Uses C, Qc, V, T,
-// tau, colat, rank, m, ldw of the task.
+// V / T / tau and (where the task has a Qc) the orthonormal basis
+// Qc = C_sel R^{-1}; cs-CTA clusters, tasks of at most mmax rows and nmax
+// selected columns.
 // Shared memory of k_selected_qr; stage: with room for the QR's panels in
 // shared memory (0 when that does not fit).
 size_t selected_qr_smem(int mmax, int nmax, bool stage);

@@ -63,31 +63,39 @@ struct EdgeChunk {
   int lda, m, nc, ldv, k, lo, cnt;
 };
 
-// Truncated column-pivoted QR of the compression matrix of one interface
-// (ptree.cpp:373-439): C = [A(n,p)^T ... | A(p,m) ...], m = size of p.
-// C is assembled transposed (w x m, element (j, r) at Ct[r * w + j]) and stays
-// read-only while a thread-block cluster selects the pivots; the reflectors
-// are then computed from the selected columns.
-struct RrqrTask {
-  const double* C;  // Ct: element (j, r) at C[r * ldw + j], ldw >= w a multiple of 4
-  double* Q;        // m x ldq scratch: row r of the orthonormal basis at Q[r * ldq]
-  double* Qc;       // the same basis column-major (m x ldq, ld m)
-  double* F;        // ldq x w scratch: row i of R at F[i * w]
-  double* V;        // m x m output: reflector j below the diagonal of column j, R above (ld m)
-  double* T;        // kNB x m output block factors
-  double* tau;      // m
-  int* colat;       // w: column at each pivot position
+// Pivot selection of the truncated column-pivoted QR of a compression matrix C
+// (m x w, ptree.cpp:373-439) or of a sketch of it (pivot.cu).
+struct PivotTask {
+  const double* C;  // read-only: C(r, j) at C[r + j * ldc] (cm = 1) or C[r * ldc + j] (cm = 0)
+  double* Q;        // ldq x min(m, w) scratch: orthonormal basis, column i at Q + i * ldq, rows past m zero
+  double* Qc;       // the same basis with leading dimension m, or null
+  double* panel;    // global panel of the large-row variant (pivot_shape), or null
+  int* colat;       // output: columns in pivot order, [0, *rank)
   int* rank;        // output
-  int* stats;       // 8 ints or null: recomputations, rank, kilocycles of pivot choice,
-                    // projections, basis vector, row of R, final QR, whole selection
-  int m, w, ldq, ldw;
+  int* stats;       // 8 ints or null: panel rebuilds, rank, kilocycles of the norms, kilocycles of the rebuilds,
+                    // panel width, kilocycles of the steps, columns brought into the panel, 0
+  int m, w, ldq, ldc, cm;
+};
+// Householder QR of the selected columns C(:, colat[0:*rank]) (k_selected_qr).
+// C is assembled column-major (w columns of m) for the pivoted QR, row-major
+// (element (j, r) at C[r * ldw + j]) for the learned path's sketches.
+struct RrqrTask {
+  const double* C;
+  double* Qc;        // m x *rank output: the orthonormal basis C_sel R^{-1}, or null
+  double* V;         // m x m output: reflector j below the diagonal of column j, R above (ld m)
+  double* T;         // kNB x m output block factors
+  double* tau;       // m
+  const int* colat;  // column at each pivot position
+  int* rank;         // columns selected
+  int m, w, ldw, cm;
 };
 struct RrqrSrc {
   const double* A;
   int lda, rows, cols;
   int transpose;  // 1: out-block A(n,p) (rows x m) enters transposed
-  double* Ct;     // destination: columns [c0, c0 + width) of the task's C
-  int w, c0;      // w: leading dimension of Ct
+  double* C;      // destination: columns [c0, c0 + width) of the task's C
+  int ldc, c0;
+  int cm;         // C is column-major (else row-major), leading dimension ldc
 };
 
 // Merge of one child block into its parent block (ptree.cpp:289-340).

@@ -231,8 +231,8 @@ class ParTree:
         self._chk(lib().spq_set_pivot_rtol(self._h, r), "set_pivot_rtol")
 
     def set_rrqr_work(self, elems: float, fill: float = 2.0):
-        """Cluster sizing of the pivoted QR: elements of the compression matrix
-        per CTA and pivot step, and CTAs per SM a level's work is spread over."""
+        """Cluster sizing of the pivoted QR: least elements of the compression matrix
+        per CTA, and twice the CTAs per SM a level's interfaces are dealt to."""
         self._chk(lib().spq_set_rrqr_work(self._h, elems, fill), "set_rrqr_work")
 
     def set_precision(self, bits: int):
@@ -292,7 +292,7 @@ class ParTree:
         self._chk(lib().spq_set_rank_margin(self._h, float(model.get("margin", 0.0))), "set_rank_margin")
 
     def set_sketch_tuning(self, sketch_tol: float = 0.1, smem: bool = False):
-        """Stop of the sketch's pivoted QR (x tol) and its shared-memory mode."""
+        """Stop of the sketch's pivoted QR (x tol); ``smem`` is accepted and without effect."""
         self._chk(lib().spq_set_sketch_tuning(self._h, sketch_tol, int(smem)), "set_sketch_tuning")
 
     def learned_counts(self) -> dict:
@@ -463,7 +463,8 @@ class ParTree:
         return lib().spq_factor_flops(self._h)
 
     def rrqr_bytes(self) -> float:
-        """Compression-matrix bytes the pivoted QR read in the last factorize."""
+        """Compression-matrix bytes the pivoted QR of the last factorize cannot do without
+        (gather and one pass for the norms)."""
         return lib().spq_rrqr_bytes(self._h)
 
     def pool_bytes(self) -> float:
