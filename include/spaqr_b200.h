@@ -92,6 +92,11 @@ int spq_debug_tc_probe(const float* C, const float* V, const float* W2, int m, i
  * columns in pivot order (colat holds min(m, w) entries). */
 int spq_debug_pivots(const double* C, int m, int w, int cm, int cs, long long smem_limit, double tol,
                      double pivot_rtol, int* colat, int* rank);
+/* Diagnostic of the preconditioner apply (no reference counterpart): from the
+ * next factorize on, reflector panels of more than `rows` rows are read from
+ * global memory where they are used, as panels too long for shared memory are
+ * (0, the default: only those). */
+int spq_debug_sweep_rows(spq_tree* t, int rows);
 /* Reuse of descriptor lists across factorizations of one partition (no
  * reference counterpart; the reference rebuilds its task graph every time,
  * ptree.cpp:885-2123).  A level's lists depend only on its cluster sizes and on

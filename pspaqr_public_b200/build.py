@@ -17,8 +17,8 @@ LIB = os.path.join(HERE, "libspaqr_b200.so")
 DRIVER = os.path.join(HERE, "spaqr")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-SOURCES = ["structure.cpp", "engine.cu", "kernels.cu", "pivot.cu", "learned.cu", "noalloc.cu", "shard.cpp", "capi.cpp", "capi_learned.cpp"]
-HEADERS = ["structure.hpp", "engine.hpp", "tasks.hpp", "kernels.hpp", "dense.cuh", "tc_apply.cuh", "noalloc.hpp", "learned.hpp",
+SOURCES = ["structure.cpp", "engine.cu", "kernels.cu", "pivot.cu", "solve.cu", "learned.cu", "noalloc.cu", "shard.cpp", "capi.cpp", "capi_learned.cpp"]
+HEADERS = ["structure.hpp", "engine.hpp", "tasks.hpp", "kernels.hpp", "dense.cuh", "tc_apply.cuh", "noalloc.hpp", "learned.hpp", "solve.hpp",
            "capi_internal.hpp", "shard.hpp"]
 
 

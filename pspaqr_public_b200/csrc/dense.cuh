@@ -173,210 +173,6 @@ __device__ void panel_t_warp(const T* V, int ldv, int m, int kb, int unit, const
   }
 }
 
-// ---------------------------------------------------------------- applies
-// C (m x nc) <- (I - V T V^T)^T C for one block of k <= kNB reflectors,
-// V unit lower trapezoidal (m x k), T (k x k, ld ldt).  W: 2*k*nc doubles.
-template <typename T>
-__device__ void block_qt(const T* V, int ldv, const T* Tm, int ldt, int k, T* C, int ldc, int m, int nc,
-                         T* W) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T* W2 = W + (size_t)k * nc;
-  for (int p = warp; p < k * nc; p += kWarps) {
-    const int i = p % k, c = p / k;
-    const T* v = V + (size_t)i * ldv;
-    const T* x = C + (size_t)c * ldc;
-    T d = (lane == 0 && i < m) ? x[i] : 0.0;
-    for (int r = i + 1 + lane; r < m; r += 32) d += v[r] * x[r];
-    d = warp_sum(d);
-    if (lane == 0) W[i + (size_t)c * k] = d;
-  }
-  __syncthreads();
-  for (int p = threadIdx.x; p < k * nc; p += kThreads) {
-    const int i = p % k, c = p / k;
-    const T* t = Tm + (size_t)i * ldt;
-    T s = 0.0;
-    for (int l = 0; l <= i; ++l) s += t[l] * W[l + (size_t)c * k];
-    W2[i + (size_t)c * k] = s;
-  }
-  __syncthreads();
-  for (int p = threadIdx.x; p < m * nc; p += kThreads) {
-    const int r = p % m, c = p / m;
-    const int lim = r < k ? r : k;
-    T s = (r < k) ? W2[r + (size_t)c * k] : 0.0;
-    for (int i = 0; i < lim; ++i) s += V[r + (size_t)i * ldv] * W2[i + (size_t)c * k];
-    C[r + (size_t)c * ldc] -= s;
-  }
-  __syncthreads();
-}
-
-// C (m x nc) <- (I - V T V^T) C for one block (no transpose).
-template <typename T>
-__device__ void block_q(const T* V, int ldv, const T* Tm, int ldt, int k, T* C, int ldc, int m, int nc,
-                        T* W) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T* W2 = W + (size_t)k * nc;
-  for (int p = warp; p < k * nc; p += kWarps) {
-    const int i = p % k, c = p / k;
-    const T* v = V + (size_t)i * ldv;
-    const T* x = C + (size_t)c * ldc;
-    T d = (lane == 0 && i < m) ? x[i] : 0.0;
-    for (int r = i + 1 + lane; r < m; r += 32) d += v[r] * x[r];
-    d = warp_sum(d);
-    if (lane == 0) W[i + (size_t)c * k] = d;
-  }
-  __syncthreads();
-  // W2 = T W  (T upper: W2(i) = sum_{l>=i} T(i,l) W(l))
-  for (int p = threadIdx.x; p < k * nc; p += kThreads) {
-    const int i = p % k, c = p / k;
-    T s = 0.0;
-    for (int l = i; l < k; ++l) s += Tm[i + (size_t)l * ldt] * W[l + (size_t)c * k];
-    W2[i + (size_t)c * k] = s;
-  }
-  __syncthreads();
-  for (int p = threadIdx.x; p < m * nc; p += kThreads) {
-    const int r = p % m, c = p / m;
-    const int lim = r < k ? r : k;
-    T s = (r < k) ? W2[r + (size_t)c * k] : 0.0;
-    for (int i = 0; i < lim; ++i) s += V[r + (size_t)i * ldv] * W2[i + (size_t)c * k];
-    C[r + (size_t)c * ldc] -= s;
-  }
-  __syncthreads();
-}
-
-// [A (k x nc, rows of the panel); B (m x nc)] <- Q^T [A; B] for one pentagonal
-// block, Q = I - [I; V] T [I; V]^T with V full (m x k).
-template <typename T>
-__device__ void block_tpqt(const T* V, int ldv, const T* Tm, int ldt, int k, T* A, int lda, T* B,
-                           int ldb, int m, int nc, T* W) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T* W2 = W + (size_t)k * nc;
-  for (int p = warp; p < k * nc; p += kWarps) {
-    const int i = p % k, c = p / k;
-    const T* v = V + (size_t)i * ldv;
-    const T* x = B + (size_t)c * ldb;
-    T d = lane == 0 ? A[i + (size_t)c * lda] : 0.0;
-    for (int r = lane; r < m; r += 32) d += v[r] * x[r];
-    d = warp_sum(d);
-    if (lane == 0) W[i + (size_t)c * k] = d;
-  }
-  __syncthreads();
-  for (int p = threadIdx.x; p < k * nc; p += kThreads) {
-    const int i = p % k, c = p / k;
-    const T* t = Tm + (size_t)i * ldt;
-    T s = 0.0;
-    for (int l = 0; l <= i; ++l) s += t[l] * W[l + (size_t)c * k];
-    W2[i + (size_t)c * k] = s;
-  }
-  __syncthreads();
-  for (int p = threadIdx.x; p < k * nc; p += kThreads) {
-    const int i = p % k, c = p / k;
-    A[i + (size_t)c * lda] -= W2[i + (size_t)c * k];
-  }
-  for (int p = threadIdx.x; p < m * nc; p += kThreads) {
-    const int r = p % m, c = p / m;
-    T s = 0.0;
-    for (int i = 0; i < k; ++i) s += V[r + (size_t)i * ldv] * W2[i + (size_t)c * k];
-    B[r + (size_t)c * ldb] -= s;
-  }
-  __syncthreads();
-}
-
-// C (m x n) <- C (I - V T V^T) for one block, V unit lower trapezoidal (n x k).
-// W: 2*k*m doubles.
-template <typename T>
-__device__ void block_q_right(const T* V, int ldv, const T* Tm, int ldt, int k, T* C, int ldc, int m,
-                              int n, T* W) {
-  T* W2 = W + (size_t)k * m;
-  for (int p = threadIdx.x; p < k * m; p += kThreads) {
-    const int r = p % m, i = p / m;
-    const T* v = V + (size_t)i * ldv;
-    T s = C[r + (size_t)i * ldc];
-    for (int c = i + 1; c < n; ++c) s += C[r + (size_t)c * ldc] * v[c];
-    W[i + (size_t)r * k] = s;
-  }
-  __syncthreads();
-  for (int p = threadIdx.x; p < k * m; p += kThreads) {
-    const int r = p % m, i = p / m;
-    const T* t = Tm + (size_t)i * ldt;
-    T s = 0.0;
-    for (int l = 0; l <= i; ++l) s += W[l + (size_t)r * k] * t[l];
-    W2[i + (size_t)r * k] = s;
-  }
-  __syncthreads();
-  for (int p = threadIdx.x; p < m * n; p += kThreads) {
-    const int r = p % m, c = p / m;
-    T s = (c < k) ? W2[c + (size_t)r * k] : 0.0;
-    const int top = (c < k) ? c : k;
-    for (int i = 0; i < top; ++i) s += W2[i + (size_t)r * k] * V[c + (size_t)i * ldv];
-    C[r + (size_t)c * ldc] -= s;
-  }
-  __syncthreads();
-}
-
-// Panel-blocked applies over k reflectors (T in kNB x k layout).
-// Q^T C: panels in order; each acts on rows [j0, m).
-template <typename T>
-__device__ void apply_qt(const T* V, int ldv, const T* Tm, int k, T* C, int ldc, int m, int nc,
-                         T* W, int wcap) {
-  if (k <= 0 || nc <= 0 || m <= 0) return;
-  const int cmax = (wcap / (2 * kNB)) > 0 ? (wcap / (2 * kNB)) : 1;
-  for (int j0 = 0; j0 < k; j0 += kNB) {
-    const int kb = (k - j0) < kNB ? (k - j0) : kNB;
-    for (int c0 = 0; c0 < nc; c0 += cmax) {
-      const int cn = (nc - c0) < cmax ? (nc - c0) : cmax;
-      block_qt(V + j0 + (size_t)j0 * ldv, ldv, Tm + (size_t)j0 * kNB, kNB, kb, C + j0 + (size_t)c0 * ldc, ldc, m - j0,
-               cn, W);
-    }
-  }
-}
-// Q C: panels in reverse order.
-template <typename T>
-__device__ void apply_q(const T* V, int ldv, const T* Tm, int k, T* C, int ldc, int m, int nc, T* W,
-                        int wcap) {
-  if (k <= 0 || nc <= 0 || m <= 0) return;
-  const int cmax = (wcap / (2 * kNB)) > 0 ? (wcap / (2 * kNB)) : 1;
-  const int np = (k + kNB - 1) / kNB;
-  for (int p = np - 1; p >= 0; --p) {
-    const int j0 = p * kNB;
-    const int kb = (k - j0) < kNB ? (k - j0) : kNB;
-    for (int c0 = 0; c0 < nc; c0 += cmax) {
-      const int cn = (nc - c0) < cmax ? (nc - c0) : cmax;
-      block_q(V + j0 + (size_t)j0 * ldv, ldv, Tm + (size_t)j0 * kNB, kNB, kb, C + j0 + (size_t)c0 * ldc, ldc, m - j0,
-              cn, W);
-    }
-  }
-}
-// [A (k x nc); B (m x nc)] <- Q^T [A; B] for a pentagonal (tpqrt) factor.
-template <typename T>
-__device__ void apply_tpqt(const T* V, int ldv, const T* Tm, int k, T* A, int lda, T* B, int ldb,
-                           int m, int nc, T* W, int wcap) {
-  if (k <= 0 || nc <= 0) return;
-  const int cmax = (wcap / (2 * kNB)) > 0 ? (wcap / (2 * kNB)) : 1;
-  for (int j0 = 0; j0 < k; j0 += kNB) {
-    const int kb = (k - j0) < kNB ? (k - j0) : kNB;
-    for (int c0 = 0; c0 < nc; c0 += cmax) {
-      const int cn = (nc - c0) < cmax ? (nc - c0) : cmax;
-      block_tpqt(V + (size_t)j0 * ldv, ldv, Tm + (size_t)j0 * kNB, kNB, kb, A + j0 + (size_t)c0 * lda, lda,
-                 B + (size_t)c0 * ldb, ldb, m, cn, W);
-    }
-  }
-}
-// C (m x n) <- C Q, panels in order; each acts on columns [j0, n).
-template <typename T>
-__device__ void apply_q_right(const T* V, int ldv, const T* Tm, int k, T* C, int ldc, int m, int n,
-                              T* W, int wcap) {
-  if (k <= 0 || m <= 0 || n <= 0) return;
-  const int rmax = (wcap / (2 * kNB)) > 0 ? (wcap / (2 * kNB)) : 1;
-  for (int j0 = 0; j0 < k; j0 += kNB) {
-    const int kb = (k - j0) < kNB ? (k - j0) : kNB;
-    for (int r0 = 0; r0 < m; r0 += rmax) {
-      const int rn = (m - r0) < rmax ? (m - r0) : rmax;
-      block_q_right(V + j0 + (size_t)j0 * ldv, ldv, Tm + (size_t)j0 * kNB, kNB, kb, C + r0 + (size_t)j0 * ldc, ldc, rn,
-                    n - j0, W);
-    }
-  }
-}
-
 
 // ---------------------------------------------------------------- tiled matrix applies
 // Register-tiled block reflector applies on matrices: rows are streamed
@@ -797,244 +593,6 @@ __device__ void mat_apply_q_right(const T* V, int ldv, const T* Tm, int k, T* C,
   }
 }
 
-
-// ---------------------------------------------------------------- single-vector applies
-// Shared scratch of vec_panel (elements): partial sums and W2.
-constexpr int kVecRed = (kWarps + 1) * 32;
-
-// One panel of kb <= kNB reflectors on a vector in shared memory:
-//   unit = 1: x (m) <- (I - V T V^T)^T x (trans) or (I - V T V^T) x, V unit
-//             lower trapezoidal from the panel's diagonal;
-//   unit = 0: [a (kb); x (m)] <- Q^T [a; x], Q = I - [I; V] T [I; V]^T, V full.
-// Every thread takes rows t, t + kThreads, ... and issues the kb loads of a row
-// together; the kb partial sums are reduce-scattered across each warp (lane i
-// ends with reflector i's sum) and across the warps through `red`.
-template <typename T>
-__device__ void vec_panel(const T* V, int ldv, const T* Tm, int ldt, int kb, int unit, bool trans, T* a, T* x,
-                          int m, T* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // warp 0: column `lane` (trans) or row `lane` of T, loaded now and used
-  // after the rows' products, so that its latency overlaps them
-  T tv[kNB];
-  if (warp == 0) {
-#pragma unroll
-    for (int l = 0; l < kNB; ++l) {
-      const bool ok = l < kb && lane < kb && (trans ? l <= lane : l >= lane);
-      tv[l] = ok ? (trans ? Tm[l + (size_t)lane * ldt] : Tm[lane + (size_t)l * ldt]) : (T)0.0;
-    }
-  }
-  T acc[kNB];
-#pragma unroll
-  for (int i = 0; i < kNB; ++i) acc[i] = 0.0;
-  for (int r = threadIdx.x; r < m; r += kThreads) {
-    const T xr = x[r];
-#pragma unroll
-    for (int i = 0; i < kNB; ++i) {
-      T v = 0.0;
-      if (i < kb) v = unit ? (r == i ? (T)1.0 : (r < i ? (T)0.0 : V[r + (size_t)i * ldv])) : V[r + (size_t)i * ldv];
-      acc[i] += v * xr;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int q = 0; q < o; ++q) {
-      const T send = up ? acc[q] : acc[q + o];
-      const T keep = up ? acc[q + o] : acc[q];
-      acc[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  red[warp * 32 + lane] = acc[0];
-  __syncthreads();
-  T* w2 = red + kWarps * 32;
-  if (warp == 0) {
-    T w = 0.0;
-    for (int q = 0; q < kWarps; ++q) w += red[q * 32 + lane];
-    if (!unit && lane < kb) w += a[lane];
-    T s = 0.0;
-#pragma unroll
-    for (int l = 0; l < kNB; ++l) s += tv[l] * __shfl_sync(0xffffffffu, w, l);
-    w2[lane] = lane < kb ? s : (T)0.0;
-    if (!unit && lane < kb) a[lane] -= s;
-  }
-  __syncthreads();
-  for (int r = threadIdx.x; r < m; r += kThreads) {
-    T s = 0.0;
-#pragma unroll
-    for (int i = 0; i < kNB; ++i) {
-      T v = 0.0;
-      if (i < kb) v = unit ? (r == i ? (T)1.0 : (r < i ? (T)0.0 : V[r + (size_t)i * ldv])) : V[r + (size_t)i * ldv];
-      s += v * w2[i];
-    }
-    x[r] -= s;
-  }
-  __syncthreads();
-}
-
-// [a (k); x (m)] <- Q^T [a; x] for a pentagonal (tpqrt) factor, V full (m x k).
-template <typename T>
-__device__ void vec_apply_tpqt(const T* V, int ldv, const T* Tm, int k, T* a, T* x, int m, T* red) {
-  for (int j0 = 0; j0 < k; j0 += kNB) {
-    const int kb = (k - j0) < kNB ? (k - j0) : kNB;
-    vec_panel<T>(V + (size_t)j0 * ldv, ldv, Tm + (size_t)j0 * kNB, kNB, kb, 0, true, a + j0, x, m, red);
-  }
-}
-
-// ---------------------------------------------------------------- staged single-vector applies
-// Asynchronous global -> shared copies (cp.async): 16-byte chunks where the
-// source is 16-byte aligned, single elements at the unaligned head and tail.
-__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
-}
-template <typename T>
-__device__ __forceinline__ void cp_async_elem(T* sdst, const T* gsrc) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
-  if (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-// Elements of a 16-byte chunk, and the shift that gives a shared copy of
-// g[0, len) the same 16-byte phase as g.
-template <typename T>
-constexpr int kE16 = 16 / (int)sizeof(T);
-template <typename T>
-__device__ __forceinline__ int phase_of(const T* g) {
-  return (int)(((uintptr_t)g & 15u) / sizeof(T));
-}
-
-// One warp copies g[0, len) to d[0, len); d must have g's 16-byte phase.
-template <typename T>
-__device__ __forceinline__ void warp_copy_async(T* d, const T* g, int len, int lane) {
-  int h = (kE16<T> - phase_of(g)) % kE16<T>;
-  if (h > len) h = len;
-  for (int e = lane; e < h; e += 32) cp_async_elem(d + e, g + e);
-  const int nc = (len - h) / kE16<T>;
-  for (int c = lane; c < nc; c += 32) cp_async16(d + h + c * kE16<T>, g + h + c * kE16<T>);
-  for (int e = h + nc * kE16<T> + lane; e < len; e += 32) cp_async_elem(d + e, g + e);
-}
-
-// Shared memory (elements) of vec_apply_staged for m rows: two panel buffers
-// of kNB columns (column stride staged_ld), two T blocks (each with room for
-// a 16-byte phase shift), W and W2.
-template <typename T>
-__host__ __device__ constexpr int staged_ld(int m) {
-  return (m + 2 * kE16<T> - 1) / kE16<T> * kE16<T>;
-}
-template <typename T>
-__host__ __device__ constexpr int staged_tld() {
-  return kNB * kNB + kE16<T>;
-}
-template <typename T>
-__host__ __device__ constexpr size_t staged_elems(int m) {
-  return 2 * (size_t)kNB * staged_ld<T>(m) + 2 * (size_t)staged_tld<T>() + 2 * kNB;
-}
-
-// x (m) <- Q^T x (trans) or Q x for k unit lower trapezoidal reflectors (T in
-// kNB x k layout) with the panels streamed through shared memory: while panel
-// p is applied from one buffer, panel p + 1 (its rows from its diagonal down,
-// and its T block) is copied into the other with cp.async, so a whole panel
-// of loads is in flight instead of a few per thread.  Per panel:
-//   W = V^T x   (a warp per reflector, lanes over rows);
-//   W2 = T^T W (trans) or T W, by warp 0;
-//   x -= V W2   (a thread per row).
-// With `a` (pentagonal, trans only): [a (k); x (m)] <- Q^T [a; x] for
-// Q = I - [I; V] T [I; V]^T with V full (m x k), as in vec_apply_tpqt: every
-// panel covers all m rows, W adds a, and a -= W2.
-// x (and a) in shared memory; buf: staged_elems<T>(m) elements, 16-byte
-// aligned.  All threads of the CTA call it; it synchronises internally.
-template <typename T>
-__device__ void vec_apply_staged(const T* V, int ldv, const T* Tm, int k, T* x, int m, bool trans, T* buf,
-                                 T* a = nullptr) {
-  if (k <= 0 || m <= 0) return;
-  __shared__ int s_off[2][kNB];  // element (r, i) of the staged panel at pb[.][s_off[.][i] + r]
-  __shared__ int s_toff[2];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int lds = staged_ld<T>(m);
-  T* const pb0 = buf;
-  T* const tb0 = buf + 2 * (size_t)kNB * lds;
-  T* const W = tb0 + 2 * staged_tld<T>();
-  T* const W2 = W + kNB;
-  const int np = (k + kNB - 1) / kNB;
-  auto j0_of = [&](int s) { return (trans ? s : np - 1 - s) * kNB; };
-  auto stage = [&](int s, int b) {
-    const int j0 = j0_of(s);
-    const int kb = (k - j0) < kNB ? (k - j0) : kNB;
-    const int rs = a ? 0 : j0;  // first staged row
-    T* pb = pb0 + (size_t)b * kNB * lds;
-    for (int i = warp; i < kb; i += kWarps) {
-      const T* g = V + (size_t)(j0 + i) * ldv + rs;
-      const int ph = phase_of(g);
-      warp_copy_async(pb + (size_t)i * lds + ph, g, m - rs, lane);
-      if (lane == 0) s_off[b][i] = i * lds + ph - rs;
-    }
-    if (warp == kWarps - 1) {
-      const T* g = Tm + (size_t)j0 * kNB;
-      const int ph = phase_of(g);
-      warp_copy_async(tb0 + (size_t)b * staged_tld<T>() + ph, g, kNB * kb, lane);
-      if (lane == 0) s_toff[b] = b * staged_tld<T>() + ph;
-    }
-    cp_async_commit();
-  };
-  stage(0, 0);
-  for (int s = 0; s < np; ++s) {
-    const int b = s & 1;
-    const int j0 = j0_of(s);
-    const int kb = (k - j0) < kNB ? (k - j0) : kNB;
-    if (s + 1 < np) {
-      stage(s + 1, b ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const T* pb = pb0 + (size_t)b * kNB * lds;
-    const T* tp = tb0 + s_toff[b];
-    // W(i) = x(j0 + i) + sum_{r > j0 + i} V(r, i) x(r), or a(j0 + i) + sum_r V(r, i) x(r)
-    for (int i = warp; i < kb; i += kWarps) {
-      const T* col = pb + s_off[b][i];
-      T d = 0.0;
-      for (int r = (a ? 0 : j0 + i + 1) + lane; r < m; r += 32) d += col[r] * x[r];
-      d = warp_sum(d);
-      if (lane == 0) W[i] = d + (a ? a[j0 + i] : x[j0 + i]);
-    }
-    __syncthreads();
-    if (warp == 0) {
-      T acc = 0.0;
-      if (lane < kb) {
-        if (trans)
-          for (int l = 0; l <= lane; ++l) acc += tp[l + lane * kNB] * W[l];
-        else
-          for (int l = lane; l < kb; ++l) acc += tp[lane + l * kNB] * W[l];
-        if (a) a[j0 + lane] -= acc;
-      }
-      W2[lane] = acc;
-    }
-    __syncthreads();
-    if (a) {
-      for (int r = threadIdx.x; r < m; r += kThreads) {
-        T acc = 0.0;
-#pragma unroll 8
-        for (int i = 0; i < kb; ++i) acc += pb[s_off[b][i] + r] * W2[i];
-        x[r] -= acc;
-      }
-    } else {
-      for (int r = j0 + threadIdx.x; r < m; r += kThreads) {
-        const int lim = (r - j0) < kb ? (r - j0) : kb;
-        T acc = (r - j0) < kb ? W2[r - j0] : (T)0.0;
-#pragma unroll 8
-        for (int i = 0; i < lim; ++i) acc += pb[s_off[b][i] + r] * W2[i];
-        x[r] -= acc;
-      }
-    }
-    __syncthreads();
-  }
-}
-
 // C (m <= kNC rows x n) <- C R^{-1}, R upper triangular (n x n), blocked by 32
 // columns: C(:, J) -= C(:, 0:j0) R(0:j0, J) through shared-memory tiles, then
 // the 32 x 32 diagonal block is solved one row per thread.
@@ -1134,63 +692,16 @@ __device__ void tile_trsm_right_upper(const T* R, int ldr, T* C, int ldc, int m,
   }
 }
 
-// C (m x n) <- C R^{-1}, R upper triangular (n x n).  One thread per row.
+// ---------------------------------------------------------------- asynchronous copies
 template <typename T>
-__device__ void trsm_right_upper(const T* R, int ldr, T* C, int ldc, int m, int n) {
-  for (int r = threadIdx.x; r < m; r += kThreads) {
-    for (int j = 0; j < n; ++j) {
-      T s = C[r + (size_t)j * ldc];
-      const T* rj = R + (size_t)j * ldr;
-      for (int i = 0; i < j; ++i) s -= C[r + (size_t)i * ldc] * rj[i];
-      C[r + (size_t)j * ldc] = s / rj[j];
-    }
-  }
-  __syncthreads();
+__device__ __forceinline__ void cp_async_elem(T* sdst, const T* gsrc) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
+  if (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
-
-// Upper triangular solve x <- R^{-1} x (n x n), blocked by 32, bottom block
-// first.  Warp 0 holds the diagonal block in registers (lane i: row i's part
-// on and above the diagonal), loaded while the CTA updates the rows above the
-// previous block, and solves it with shuffles; the CTA then updates the rows
-// above with the solved block.
-template <typename T>
-__device__ void trsv_upper(const T* R, int ldr, T* x, int n, T* xs /*shared >= 32*/) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T rv[32];
-  auto fetch = [&](int lo, int bs) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      rv[j] = (j < bs && lane <= j) ? R[(lo + lane) + (size_t)(lo + j) * ldr] : (T)0.0;
-  };
-  if (warp == 0 && n > 0) fetch(n > 32 ? n - 32 : 0, n > 32 ? 32 : n);
-  for (int hi = n; hi > 0; hi -= 32) {
-    const int lo = hi > 32 ? hi - 32 : 0;
-    const int bs = hi - lo;
-    if (warp == 0) {
-      T xv = lane < bs ? x[lo + lane] : 0.0;
-#pragma unroll
-      for (int j = 31; j >= 0; --j) {
-        if (j < bs) {
-          if (lane == j) xv = xv / rv[j];
-          const T xj = __shfl_sync(0xffffffffu, xv, j);
-          if (lane < j) xv -= rv[j] * xj;
-        }
-      }
-      if (lane < bs) {
-        x[lo + lane] = xv;
-        xs[lane] = xv;
-      }
-      if (lo > 0) fetch(lo > 32 ? lo - 32 : 0, lo > 32 ? 32 : lo);
-    }
-    __syncthreads();
-    for (int r = threadIdx.x; r < lo; r += kThreads) {
-      T s = 0.0;
-      for (int j = 0; j < bs; ++j) s += R[r + (size_t)(lo + j) * ldr] * xs[j];
-      x[r] -= s;
-    }
-    __syncthreads();
-  }
-}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 }  // namespace dev
 }  // namespace spq

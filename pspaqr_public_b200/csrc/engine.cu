@@ -127,7 +127,6 @@ Tree::~Tree() {
   cudaFree(d_val_);
   cudaFree(d_xw_);
   cudaFree(d_turn_);
-  cudaFree(d_tickets_);
   cudaFree(d_status_);
   cudaFree(d_tmp_);
   cudaFree(d_dst_);
@@ -1443,86 +1442,112 @@ int Tree::alloc_level_blocks(const std::vector<int>& edges) {
   return 0;
 }
 
-// Cluster vectors: level-0 clusters at their permuted columns [0, n); every
-// later cluster gets its own segment of its level size.
-// Descriptors of one vector's preconditioner apply: per level the forward
-// elimination / sparsification tasks, the backward ones and the merge index
-// maps, all addressing the cluster vectors of the workspace xw (turn counters
-// in turn).  Uploaded into the block pool.
-int Tree::plan_solve(double* xw, int* turn, std::vector<SolvePlan>& ls) {
-  const int L = st_.nlevels;
-  ls.assign(L, SolvePlan());
-  auto up = [&](const void* h, size_t bytes) -> void* {
-    void* d = arena_.alloc(std::max<size_t>(bytes, 1));
-    if (d && bytes && h) cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, stream_);
-    return d;
+// Levels with at most this many interiors, some of them with more than kPipeRows
+// rows, run their forward elimination as a pipeline of one CTA per chain step:
+// more interiors fill the GPU by themselves, and a pipeline of one or two panels
+// hands on later than one CTA gets there.
+constexpr size_t kPipeInteriors = 256;
+constexpr int kPipeRows = 64;
+
+// Descriptors of the panel-chain sweeps (offsets into any workspace): packed into
+// one upload.  Also inverts the diagonal blocks of every triangular solve.
+int Tree::plan_sweep() {
+  const int L = st_.nlevels, NB = dev_nb();
+  sweep_.assign(L, SweepLevel());
+  sweep_wide_ok_ = true;
+  nprog_ = ndone_ = 0;
+  std::vector<char> buf;
+  std::vector<std::pair<void**, size_t>> fix;  // pointer to set, offset in buf
+  auto pack = [&](auto*& dst, const auto& v) {
+    buf.resize((buf.size() + 255) / 256 * 256);
+    fix.push_back({reinterpret_cast<void**>(&dst), buf.size()});
+    const char* b = reinterpret_cast<const char*>(v.data());
+    buf.insert(buf.end(), b, b + sizeof(v[0]) * v.size());
+  };
+  std::vector<InvTask> inv;
+  InvTask* d_inv = nullptr;
+  auto inverses = [&](const double* R, int n) {
+    double* out = arena_.dalloc((size_t)NB * NB * std::max(1, (n + NB - 1) / NB));
+    for (int b = 0; b * NB < n; ++b) inv.push_back({R, out, n, b});
+    return out;
   };
   for (int lvl = 0; lvl < L; ++lvl) {
     const Level& Lv = st_.levels[lvl];
-    SolvePlan& S = ls[lvl];
-    // turn order per neighbour: interiors ascending
-    std::vector<int> seen(Lv.count, 0);
-    std::vector<FwdElimTask> fe;
-    std::vector<FwdOut> fo;
+    SweepLevel& S = sweep_[lvl];
+    int longest = 0;
+    for (int c : Lv.interiors) longest = std::max(longest, size_[c]);
+    S.pipe = Lv.interiors.size() <= kPipeInteriors && longest > kPipeRows;
+    std::vector<int> seen(Lv.count, 0);  // turn order per neighbour: interiors ascending
+    std::vector<FwdItem> fw;
+    std::vector<FwdEdge> fe;
+    std::vector<BwdItem> bw;
+    std::vector<BwdEdge> be;
     for (size_t ii = 0; ii < Lv.interiors.size(); ++ii) {
-      const int c = Lv.interiors[ii];
-      FwdElimTask t;
+      const int c = Lv.interiors[ii], n = size_[c];
+      FwdItem t{};
       t.S = ptr_[Lv.self_edge_of[c - Lv.first]];
       t.T = T_[c];
-      t.x = elem(xw, xoff_[c]);
-      t.n = size_[c];
-      t.out_begin = (int)fo.size();
+      t.x = xoff_[c];
+      t.n = n;
+      t.own = 1;
+      t.out_begin = t.out_end = (int)fe.size();
+      t.pin = t.pout = -1;
+      const int nout = Lv.out_end[ii] - Lv.out_begin[ii];
       for (int q = Lv.out_begin[ii]; q < Lv.out_end[ii]; ++q) {
-        const int e = Lv.out_edges[q];
-        const int nb = st_.edges[e].n2;
-        FwdOut o;
-        o.V = ptr_[e];
-        o.T = tsqrtT_[e];
-        o.xn = elem(xw, xoff_[nb]);
-        o.turn = turn + nb;
-        o.m = rows_[e];
-        o.my_turn = seen[nb - Lv.first]++;
-        fo.push_back(o);
-        S.fe_mmax = std::max(S.fe_mmax, o.m);
+        const int e = Lv.out_edges[q], nb = st_.edges[e].n2;
+        fe.push_back({ptr_[e], tsqrtT_[e], xoff_[nb], nb, rows_[e], seen[nb - Lv.first]++});
+        S.fe_mmax = std::max(S.fe_mmax, rows_[e]);
       }
-      t.out_end = (int)fo.size();
-      fe.push_back(t);
-      S.fe_nmax = std::max(S.fe_nmax, t.n);
+      S.fe_nmax = std::max(S.fe_nmax, n);
+      if (S.pipe) {
+        for (int k = 0; k <= nout; ++k) {  // own reflectors, then one item per edge
+          FwdItem u = t;
+          u.own = k == 0;
+          u.out_begin = t.out_begin + std::max(0, k - 1);
+          u.out_end = t.out_begin + k;
+          u.pin = k == 0 ? -1 : nprog_ - 1;
+          u.pout = k < nout ? nprog_++ : -1;
+          fw.push_back(u);
+        }
+      } else {
+        t.out_end = (int)fe.size();
+        fw.push_back(t);
+      }
+      BwdItem b{};
+      b.S = t.S;
+      b.inv = inverses(t.S, n);
+      if (!b.inv) return fail(-11, "out of device memory (triangular inverses)");
+      b.x = xoff_[c];
+      b.n = n;
+      b.in_begin = (int)be.size();
+      for (int q = Lv.in_begin[ii]; q < Lv.in_end[ii]; ++q) {
+        const int e = Lv.in_edges[q];
+        if (cols_[e] > 0) be.push_back({ptr_[e], xoff_[st_.edges[e].n1], ld_[e], cols_[e]});
+      }
+      b.in_end = (int)be.size();
+      const int step = sweep_bwd_rows();
+      b.chunks = b.in_end > b.in_begin ? std::max(1, (n + step - 1) / step) : 1;
+      b.done = b.chunks > 1 ? ndone_++ : 0;
+      for (int k = 0; k < b.chunks; ++k) {
+        b.row0 = k * step;
+        bw.push_back(b);
+      }
+      S.be_nmax = std::max(S.be_nmax, n);
     }
-    std::vector<FwdSparsTask> fs;
+    std::vector<SparsItem> sp;
     for (int p : Lv.spars_clusters) {
-      FwdSparsTask t;
+      SparsItem t{};
       t.Qs = ptr_[Lv.self_edge_of[p - Lv.first]];
       t.Ts = Ts_[p];
       t.V = Qsp_[p];
       t.T = Tsp_[p];
       t.rank = d_rank_ + p;
-      t.x = elem(xw, xoff_[p]);
+      t.x = xoff_[p];
       t.n = size_org_[p];
-      fs.push_back(t);
-      S.fs_nmax = std::max(S.fs_nmax, t.n);
-    }
-    std::vector<BwdElimTask> be;
-    std::vector<BwdIn> bi;
-    for (size_t ii = 0; ii < Lv.interiors.size(); ++ii) {
-      const int c = Lv.interiors[ii];
-      BwdElimTask t;
-      t.S = ptr_[Lv.self_edge_of[c - Lv.first]];
-      t.x = elem(xw, xoff_[c]);
-      t.n = size_[c];
-      t.in_begin = (int)bi.size();
-      for (int q = Lv.in_begin[ii]; q < Lv.in_end[ii]; ++q) {
-        const int e = Lv.in_edges[q];
-        BwdIn b;
-        b.R = ptr_[e];
-        b.ldr = ld_[e];
-        b.s = cols_[e];
-        b.xm = elem(xw, xoff_[st_.edges[e].n1]);
-        bi.push_back(b);
-      }
-      t.in_end = (int)bi.size();
-      be.push_back(t);
-      S.be_nmax = std::max(S.be_nmax, t.n);
+      t.inv = inverses(t.Qs, t.n);
+      if (!t.inv) return fail(-11, "out of device memory (triangular inverses)");
+      sp.push_back(t);
+      S.sp_nmax = std::max(S.sp_nmax, t.n);
     }
     std::vector<int> gs, gd;
     if (lvl + 1 < L) {
@@ -1530,63 +1555,72 @@ int Tree::plan_solve(double* xw, int* turn, std::vector<SolvePlan>& ls) {
       for (int P = N.first; P < N.first + N.count; ++P) {
         const Cluster& C = st_.clusters[P];
         for (int k = C.child_begin; k < C.child_end; ++k) {
-          const int ch = st_.children[k];
-          for (int i = 0; i < size_[ch]; ++i) {
-            gs.push_back((int)(xoff_[ch] + i));
-            gd.push_back((int)(xoff_[P] + rpos_[ch] + i));
+          const int chd = st_.children[k];
+          for (int i = 0; i < size_[chd]; ++i) {
+            gs.push_back((int)(xoff_[chd] + i));
+            gd.push_back((int)(xoff_[P] + rpos_[chd] + i));
           }
         }
       }
     }
-    S.nfe = (int)fe.size();
-    S.nfs = (int)fs.size();
-    if (fp32_)
-      S.nfs_small = (int)(std::stable_partition(fs.begin(), fs.end(),
-                                                [](const FwdSparsTask& t) { return spars_small(t.n); }) -
-                          fs.begin());
-    S.nbe = (int)be.size();
+    S.nfwd = (int)fw.size();
+    S.nsp = (int)sp.size();
+    S.nbwd = (int)bw.size();
     S.ng = (int)gs.size();
-    S.fe = static_cast<FwdElimTask*>(up(fe.data(), sizeof(FwdElimTask) * fe.size()));
-    S.fo = static_cast<FwdOut*>(up(fo.data(), sizeof(FwdOut) * fo.size()));
-    S.fs = static_cast<FwdSparsTask*>(up(fs.data(), sizeof(FwdSparsTask) * fs.size()));
-    S.be = static_cast<BwdElimTask*>(up(be.data(), sizeof(BwdElimTask) * be.size()));
-    S.bi = static_cast<BwdIn*>(up(bi.data(), sizeof(BwdIn) * bi.size()));
-    S.gsrc = static_cast<int*>(up(gs.data(), sizeof(int) * gs.size()));
-    S.gdst = static_cast<int*>(up(gd.data(), sizeof(int) * gd.size()));
-    if (!S.fe || !S.fo || !S.fs || !S.be || !S.bi || !S.gsrc || !S.gdst)
-      return fail(-11, "out of device memory (solve descriptors)");
+    pack(S.fwd, fw);
+    pack(S.fe, fe);
+    pack(S.sp, sp);
+    pack(S.bwd, bw);
+    pack(S.be, be);
+    pack(S.gsrc, gs);
+    pack(S.gdst, gd);
+    const int fr = std::max(S.fe_nmax, S.fe_mmax);
+    sweep_wide_ok_ = sweep_wide_ok_ && sweep_wide_fits(fr, S.fe_nmax) && sweep_wide_fits(S.sp_nmax, 0) &&
+                     sweep_wide_fits(S.be_nmax, 0);
   }
+  pack(d_inv, inv);
+  char* d = static_cast<char*>(arena_.alloc(std::max<size_t>(buf.size(), 1)));
+  if (!d) return fail(-11, "out of device memory (solve descriptors)");
+  stage_reset();  // factorize ended with a stream synchronisation
+  const void* src = buf.data();
+  if (void* h = stage(buf.size())) src = std::memcpy(h, buf.data(), buf.size());
+  if (check_cuda(cudaMemcpyAsync(d, src, buf.size(), cudaMemcpyHostToDevice, stream_), "solve descriptors")) return -10;
+  for (auto& f : fix) *f.first = d + f.second;
+  if (check_cuda(launch_diag_inverse(d_inv, (int)inv.size(), stream_), "triangular inverses")) return -10;
   return check_cuda(cudaStreamSynchronize(stream_), "solve descriptors");
 }
 
-// Captures one vector's sweep (forward levels, then backward levels) into *g.
-int Tree::capture_solve(const std::vector<SolvePlan>& ls, double* xw, int* turn, int* tickets, cudaGraph_t* g,
-                        long long* kernels) {
+size_t Tree::sweep_counters() const { return st_.clusters.size() + st_.nlevels + (size_t)nprog_ + (size_t)ndone_; }
+
+// Captures the sweeps of one group of right-hand sides; counters: sweep_counters() ints.
+int Tree::capture_sweep(SweepRun run, int* counters, cudaGraph_t* g, long long* kernels) {
   const int L = st_.nlevels;
-  const int ncl = (int)st_.clusters.size();
+  run.turn = counters;
+  int* tickets = counters + st_.clusters.size();
+  run.prog = tickets + L;
+  run.done = run.prog + nprog_;
+  run.status = d_status_;
+  run.spin_limit = spin_limit;
+  run.rows_limit = sweep_rows;
   if (check_cuda(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture")) return -10;
-  const long long launches_before = kernel_launches();
-  cudaError_t cerr = cudaSuccess;
-  cudaMemsetAsync(turn, 0, sizeof(int) * ncl, stream_);
-  cudaMemsetAsync(tickets, 0, sizeof(int) * L, stream_);
+  const long long before = kernel_launches();
+  cudaError_t e = cudaMemsetAsync(counters, 0, sizeof(int) * sweep_counters(), stream_);
   for (int lvl = 0; lvl < L; ++lvl) {
-    const SolvePlan& S = ls[lvl];
-    cerr = cerr ? cerr : launch_fwd_elim(S.fe, S.fo, S.nfe, S.fe_nmax, S.fe_mmax, tickets + lvl, d_status_, spin_limit, stream_);
-    cerr = cerr ? cerr : launch_spars_small(true, S.fs, S.nfs_small, stream_);
-    cerr = cerr ? cerr : launch_fwd_spars(S.fs + S.nfs_small, S.nfs - S.nfs_small, S.fs_nmax, stream_);
-    cerr = cerr ? cerr : launch_copy_idx(S.ng, S.gsrc, S.gdst, xw, stream_);
+    const SweepLevel& S = sweep_[lvl];
+    e = e ? e : launch_sweep_fwd(S.fwd, S.fe, S.nfwd, S.pipe, S.fe_nmax, S.fe_mmax, tickets + lvl, run, stream_);
+    e = e ? e : launch_sweep_spars(true, S.sp, S.nsp, S.sp_nmax, run, stream_);
+    e = e ? e : launch_sweep_copy(S.ng, S.gsrc, S.gdst, run, stream_);
   }
   for (int lvl = L - 1; lvl >= 0; --lvl) {
-    const SolvePlan& S = ls[lvl];
-    cerr = cerr ? cerr : launch_spars_small(false, S.fs, S.nfs_small, stream_);
-    cerr = cerr ? cerr : launch_bwd_spars(S.fs + S.nfs_small, S.nfs - S.nfs_small, S.fs_nmax, stream_);
-    cerr = cerr ? cerr : launch_bwd_elim(S.be, S.bi, S.nbe, S.be_nmax, stream_);
-    if (lvl > 0) cerr = cerr ? cerr : launch_copy_idx(ls[lvl - 1].ng, ls[lvl - 1].gdst, ls[lvl - 1].gsrc, xw, stream_);
+    const SweepLevel& S = sweep_[lvl];
+    e = e ? e : launch_sweep_spars(false, S.sp, S.nsp, S.sp_nmax, run, stream_);
+    e = e ? e : launch_sweep_bwd(S.bwd, S.be, S.nbwd, S.be_nmax, run, stream_);
+    if (lvl > 0) e = e ? e : launch_sweep_copy(sweep_[lvl - 1].ng, sweep_[lvl - 1].gdst, sweep_[lvl - 1].gsrc, run, stream_);
   }
-  *kernels = kernel_launches() - launches_before;
+  *kernels = kernel_launches() - before;
   add_kernel_launches(-*kernels);  // captured, not executed
-  cudaError_t ce = cudaStreamEndCapture(stream_, g);
-  if (check_cuda(cerr, "solve kernel launch") || check_cuda(ce, "end capture")) return -10;
+  const cudaError_t ce = cudaStreamEndCapture(stream_, g);
+  if (check_cuda(e, "solve kernel launch") || check_cuda(ce, "end capture")) return -10;
   return 0;
 }
 
@@ -1603,23 +1637,36 @@ int Tree::build_solve_graph() {
     off += size_org_[o];
   }
   xw_size_ = off;
-  cudaFree(d_xw_);
-  cudaFree(d_turn_);
-  cudaFree(d_tickets_);
-  d_xw_ = nullptr, d_turn_ = nullptr, d_tickets_ = nullptr;
   release_block_solve();
-  if (check_cuda(cudaMalloc(&d_xw_, sizeof(double) * std::max<int64_t>(xw_size_, 1)), "malloc") ||
-      check_cuda(cudaMalloc(&d_turn_, sizeof(int) * ncl), "malloc") ||
-      check_cuda(cudaMalloc(&d_tickets_, sizeof(int) * L), "malloc"))
-    return -10;
-  std::vector<SolvePlan> ls;
-  if (int rc = plan_solve(d_xw_, d_turn_, ls)) return rc;
   if (solve_exec_) {
     cudaGraphExecDestroy(solve_exec_);
     cudaGraphDestroy(solve_graph_);
     solve_exec_ = nullptr;
+    solve_graph_ = nullptr;
   }
-  if (int rc = capture_solve(ls, d_xw_, d_turn_, d_tickets_, &solve_graph_, &solve_graph_kernels_)) return rc;
+  if (int rc = plan_sweep()) return rc;
+  // the workspace and the counters only grow: freeing them would wait for the
+  // whole device at every factorization
+  const size_t nx = (size_t)std::max<int64_t>(xw_size_, 1);
+  const size_t nc = sweep_counters();
+  if (nx > xw_cap_) {
+    cudaFree(d_xw_);
+    d_xw_ = nullptr;
+    xw_cap_ = 0;
+    if (check_cuda(cudaMalloc(&d_xw_, sizeof(double) * nx), "malloc")) return -10;
+    xw_cap_ = nx;
+  }
+  if (nc > counter_cap_) {
+    cudaFree(d_turn_);
+    d_turn_ = nullptr;
+    counter_cap_ = 0;
+    if (check_cuda(cudaMalloc(&d_turn_, sizeof(int) * nc), "malloc")) return -10;
+    counter_cap_ = nc;
+  }
+  SweepRun run{};
+  run.xw = d_xw_;
+  run.nrhs = 1;
+  if (int rc = capture_sweep(run, d_turn_, &solve_graph_, &solve_graph_kernels_)) return rc;
   if (check_cuda(cudaGraphInstantiate(&solve_exec_, solve_graph_, 0), "instantiate")) return -10;
   return 0;
 }
@@ -1631,39 +1678,44 @@ void Tree::release_block_solve() {
   block_graph_ = nullptr;
   cudaFree(d_xwb_);
   cudaFree(d_turnb_);
-  cudaFree(d_ticketsb_);
-  d_xwb_ = nullptr, d_turnb_ = nullptr, d_ticketsb_ = nullptr;
+  d_xwb_ = nullptr, d_turnb_ = nullptr;
   block_nrhs_ = 0;
   block_graph_kernels_ = 0;
 }
 
-// The preconditioner apply of nrhs vectors as one graph: nrhs independent
-// sweeps (own workspace, turn counters and tickets each) as parallel branches,
-// so that the GPU runs them concurrently.  Built on first use per factorization
-// and nrhs (it allocates), reused after.
+// The preconditioner apply of nrhs vectors as one graph: groups of right-hand
+// sides that share their sweeps, as parallel branches with a workspace and
+// counters each, so that the GPU runs the groups concurrently.  Built on first
+// use per factorization and nrhs (it allocates), reused after.
 int Tree::build_block_solve(int nrhs) {
   if (block_exec_ && block_nrhs_ == nrhs) return 0;
   release_block_solve();
-  const int L = st_.nlevels;
-  const int ncl = (int)st_.clusters.size();
+  const int width = sweep_wide_ok_ ? kSweepWide : 1;
+  const int groups = (nrhs + width - 1) / width;
+  const size_t nc = sweep_counters();
   if (check_cuda(cudaMalloc(&d_xwb_, sizeof(double) * (size_t)std::max<int64_t>(xw_size_, 1) * nrhs), "malloc") ||
-      check_cuda(cudaMalloc(&d_turnb_, sizeof(int) * (size_t)ncl * nrhs), "malloc") ||
-      check_cuda(cudaMalloc(&d_ticketsb_, sizeof(int) * (size_t)L * nrhs), "malloc"))
+      check_cuda(cudaMalloc(&d_turnb_, sizeof(int) * nc * groups), "malloc"))
     return -11;
   if (check_cuda(cudaGraphCreate(&block_graph_, 0), "graph")) return -10;
   set_factor_fp32(fp32_);
-  for (int r = 0; r < nrhs; ++r) {
+  for (int q = 0, r = 0; q < groups; ++q) {
+    const int here = (nrhs - r + groups - q - 1) / (groups - q);  // as even as possible
     double* xw = elem(d_xwb_, (size_t)r * xw_size_);
-    std::vector<SolvePlan> ls;
-    if (int rc = plan_solve(xw, d_turnb_ + (size_t)r * ncl, ls)) return rc;
+    int* counters = d_turnb_ + nc * q;
     cudaGraph_t g = nullptr;
     long long nk = 0;
-    if (int rc = capture_solve(ls, xw, d_turnb_ + (size_t)r * ncl, d_ticketsb_ + (size_t)r * L, &g, &nk)) return rc;
+    SweepRun run{};
+    run.xw = xw;
+    run.stride = xw_size_;
+    run.nrhs = here;
+    run.wide = here > 1;
+    if (int rc = capture_sweep(run, counters, &g, &nk)) return rc;
     cudaGraphNode_t node;
     const cudaError_t e = cudaGraphAddChildGraphNode(&node, block_graph_, nullptr, 0, g);
     cudaGraphDestroy(g);  // the child node holds a copy
     if (check_cuda(e, "block solve graph")) return -10;
     block_graph_kernels_ += nk;
+    r += here;
   }
   if (check_cuda(cudaGraphInstantiate(&block_exec_, block_graph_, 0), "instantiate block solve")) return -10;
   block_nrhs_ = nrhs;

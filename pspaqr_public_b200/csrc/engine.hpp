@@ -14,6 +14,7 @@
 #include <string>
 #include <vector>
 
+#include "solve.hpp"
 #include "structure.hpp"
 #include "tasks.hpp"
 
@@ -136,6 +137,9 @@ class Tree {
   // forward sweep (takes effect at the next factorize, which captures the
   // apply); a wait that runs out fails the apply with status -12
   long long spin_limit = 2000000000LL;
+  // panels of more rows than this stay in global memory during the apply (0: as
+  // shared memory allows; tests); takes effect at the next factorize
+  int sweep_rows = 0;
   // host-side checks of the trailing-update, compression and merge
   // descriptors before each upload: every block address lies in the block
   // pool (failure: status -5, nothing launched)
@@ -249,24 +253,29 @@ class Tree {
   void* stage(size_t bytes);
   void stage_reset() { pin_cur_ = 0, pin_off_ = 0; }
   int build_solve_graph();
-  // one vector's apply: descriptors for workspace xw / turn counters, and its capture
-  struct SolvePlan {
-    FwdElimTask* fe = nullptr;
-    FwdOut* fo = nullptr;
-    int nfe = 0, fe_nmax = 1, fe_mmax = 1;
-    FwdSparsTask* fs = nullptr;
-    int nfs = 0, fs_nmax = 1;
-    int nfs_small = 0;  // FP32: the first nfs_small tasks take the warp-per-interface kernels
-    BwdElimTask* be = nullptr;
-    BwdIn* bi = nullptr;
-    int nbe = 0, be_nmax = 1;
-    int* gsrc = nullptr;
-    int* gdst = nullptr;
+  // the apply by panel chains (solve.cu): descriptors for any workspace, built
+  // once per factorization
+  struct SweepLevel {
+    FwdItem* fwd = nullptr;
+    FwdEdge* fe = nullptr;
+    int nfwd = 0, fe_nmax = 0, fe_mmax = 0;
+    bool pipe = false;
+    SparsItem* sp = nullptr;
+    int nsp = 0, sp_nmax = 0;
+    BwdItem* bwd = nullptr;
+    BwdEdge* be = nullptr;
+    int nbwd = 0, be_nmax = 0;
+    int *gsrc = nullptr, *gdst = nullptr;
     int ng = 0;
   };
-  int plan_solve(double* xw, int* turn, std::vector<SolvePlan>& ls);
-  int capture_solve(const std::vector<SolvePlan>& ls, double* xw, int* turn, int* tickets, cudaGraph_t* g,
-                    long long* kernels);
+  std::vector<SweepLevel> sweep_;
+  bool sweep_wide_ok_ = false;  // kSweepWide right-hand sides fit the kernels at every level
+  int nprog_ = 0, ndone_ = 0;  // pipeline progress and completion counters of one apply
+  int plan_sweep();
+  // counters of one apply: turns, tickets, progress, completions
+  size_t sweep_counters() const;
+  int capture_sweep(SweepRun run, int* counters, cudaGraph_t* g, long long* kernels);
+  size_t xw_cap_ = 0, counter_cap_ = 0;  // allocated elements of d_xw_ / d_turn_
   int build_block_solve(int nrhs);
   void release_block_solve();
   int solve_block_cols(const std::vector<double*>& cols);
@@ -311,8 +320,7 @@ class Tree {
   bool asm_valid_ = false;
   double* d_xw_ = nullptr;     // solve workspace (all cluster vectors)
   int64_t xw_size_ = 0;
-  int* d_turn_ = nullptr;      // per cluster turn counters
-  int* d_tickets_ = nullptr;   // per level
+  int* d_turn_ = nullptr;      // per cluster turn counters, per level tickets, pipeline counters
   int* d_status_ = nullptr;
   cudaGraphExec_t solve_exec_ = nullptr;
   cudaGraph_t solve_graph_ = nullptr;
@@ -324,7 +332,6 @@ class Tree {
   int block_nrhs_ = 0;
   double* d_xwb_ = nullptr;
   int* d_turnb_ = nullptr;
-  int* d_ticketsb_ = nullptr;
   double* d_tmp_ = nullptr;    // 2 vectors for host-pointer entry points
   // Krylov workspace kept across GMRES calls
   double* d_krylov_ = nullptr;

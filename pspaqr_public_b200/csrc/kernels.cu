@@ -970,310 +970,11 @@ __global__ void k_merge(const MergeTask* __restrict__ tasks) {
   }
 }
 
-// ------------------------------------------------------------ solve
-__device__ __forceinline__ int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release(int* p, int v) {
-  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Forward elimination sweep of one level.  Interiors are taken in ascending
-// order through a ticket; a chain step on neighbour n waits (bounded) until
-// every interior ordered before this one in n's transform order has applied
-// its step, so the order matches the factorization (order_of_trans).  Waits
-// only target lower tickets, which are held by running CTAs, so the sweep
-// cannot deadlock; a wait that exceeds `spin_limit` cycles sets *status = 2.
-// kStaged: the interior's own reflectors stream through shared memory
-// (dev::vec_apply_staged), for levels with large interiors.
-template <typename T, bool kStaged>
-__global__ void __launch_bounds__(kThreads, 2) k_fwd_elim(const FwdElimTask* __restrict__ tasks,
-                                                       const FwdOut* __restrict__ outs, int ntasks, int* ticket,
-                                                       int* status, long long spin_limit, int nmax, int mmax) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* sm = reinterpret_cast<T*>(smraw);
-  __shared__ int s_task, s_abort;
-  if (threadIdx.x == 0) {
-    s_task = atomicAdd(ticket, 1);
-    s_abort = 0;
-  }
-  __syncthreads();
-  const int ti = s_task;
-  if (ti >= ntasks) return;
-  const FwdElimTask t = tasks[ti];
-  T* red = sm + (kStaged ? dev::staged_elems<T>(max(nmax, mmax)) : 0);
-  T* xc = red + dev::kVecRed;
-  T* xn = xc + (nmax > 0 ? nmax : 1);
-  for (int i = threadIdx.x; i < t.n; i += kThreads) xc[i] = __ldcg(as<T>(t.x) + i);
-  __syncthreads();
-  if (kStaged) dev::vec_apply_staged<T>(as<T>(t.S), t.n, as<T>(t.T), t.n, xc, t.n, true, sm);
-  else dev::apply_qt<T>(as<T>(t.S), t.n, as<T>(t.T), t.n, xc, t.n, t.n, 1, red, 2 * kNB);
-  for (int o = t.out_begin; o < t.out_end; ++o) {
-    const FwdOut e = outs[o];
-    if (threadIdx.x == 0) {
-      const long long t0 = clock64();
-      for (;;) {
-        const int v = ld_acquire(e.turn);
-        if (v == e.my_turn) break;
-        if (ld_acquire(status) != 0) {
-          s_abort = 1;
-          break;
-        }
-        if (clock64() - t0 > spin_limit) {
-          atomicExch(status, 2);
-          s_abort = 1;
-          break;
-        }
-        __nanosleep(64);
-      }
-      __threadfence();
-    }
-    __syncthreads();
-    if (s_abort) return;
-    for (int i = threadIdx.x; i < e.m; i += kThreads) xn[i] = __ldcg(as<T>(e.xn) + i);
-    __syncthreads();
-    if (kStaged) dev::vec_apply_staged<T>(as<T>(e.V), e.m, as<T>(e.T), t.n, xn, e.m, true, sm, xc);
-    else dev::vec_apply_tpqt<T>(as<T>(e.V), e.m, as<T>(e.T), t.n, xc, xn, e.m, red);
-    for (int i = threadIdx.x; i < e.m; i += kThreads) __stcg(as<T>(e.xn) + i, xn[i]);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      st_release(e.turn, e.my_turn + 1);
-    }
-  }
-  for (int i = threadIdx.x; i < t.n; i += kThreads) __stcg(as<T>(t.x) + i, xc[i]);
-}
-
-// kStaged: the reflector panels stream through shared memory
-// (dev::vec_apply_staged), for levels with large interfaces.
-template <typename T, bool kStaged>
-__global__ void __launch_bounds__(kThreads) k_fwd_spars(const FwdSparsTask* __restrict__ tasks) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* sm = reinterpret_cast<T*>(smraw);
-  const FwdSparsTask t = tasks[blockIdx.x];
-  T* red = sm + (kStaged ? dev::staged_elems<T>(t.n) : 0);
-  T* x = red + 2 * kNB;
-  for (int i = threadIdx.x; i < t.n; i += kThreads) x[i] = as<T>(t.x)[i];
-  __syncthreads();
-  if (kStaged) {
-    dev::vec_apply_staged<T>(as<T>(t.Qs), t.n, as<T>(t.Ts), t.n, x, t.n, true, sm);
-    dev::vec_apply_staged<T>(as<T>(t.V), t.n, as<T>(t.T), *t.rank, x, t.n, true, sm);
-  } else {
-    dev::apply_qt<T>(as<T>(t.Qs), t.n, as<T>(t.Ts), t.n, x, t.n, t.n, 1, red, 2 * kNB);
-    dev::apply_qt<T>(as<T>(t.V), t.n, as<T>(t.T), *t.rank, x, t.n, t.n, 1, red, 2 * kNB);
-  }
-  for (int i = threadIdx.x; i < t.n; i += kThreads) as<T>(t.x)[i] = x[i];
-}
-
-template <typename T, bool kStaged>
-__global__ void __launch_bounds__(kThreads) k_bwd_spars(const FwdSparsTask* __restrict__ tasks) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* sm = reinterpret_cast<T*>(smraw);
-  const FwdSparsTask t = tasks[blockIdx.x];
-  T* red = sm + (kStaged ? dev::staged_elems<T>(t.n) : 0);
-  T* xs = red + 2 * kNB;
-  T* x = xs + 32;
-  for (int i = threadIdx.x; i < t.n; i += kThreads) x[i] = as<T>(t.x)[i];
-  __syncthreads();
-  if (kStaged) dev::vec_apply_staged<T>(as<T>(t.V), t.n, as<T>(t.T), *t.rank, x, t.n, false, sm);
-  else dev::apply_q<T>(as<T>(t.V), t.n, as<T>(t.T), *t.rank, x, t.n, t.n, 1, red, 2 * kNB);
-  dev::trsv_upper<T>(as<T>(t.Qs), t.n, x, t.n, xs);
-  for (int i = threadIdx.x; i < t.n; i += kThreads) as<T>(t.x)[i] = x[i];
-}
-
-// Forward / backward scaling + sparsification steps of small interfaces (FP32,
-// n <= 32), one warp per interface: lane r holds x(r); each reflector block
-// (a single panel) and its T are staged in the warp's shared memory and the
-// sums run over shuffles.  The CTA kernels spend a 256-thread CTA and three
-// CTA barriers per panel on vectors of this size.
-constexpr int kSpLd = 33;
-constexpr size_t kSparsSmallSmem = (size_t)kWarps * 2 * 32 * kSpLd * sizeof(float);
-
-// Returns lane r's entry of Q^T x (trans) or Q x, Q = I - V T V^T for k <= 32
-// unit lower reflectors of n <= 32 rows (T in kNB x k layout).
-__device__ __forceinline__ float warp_apply_unit(const float* V, int ldv, const float* Tm, int k, float xr, int n,
-                                                 bool trans, float* sV, float* sT, int lane) {
-  for (int i = 0; i < 32; ++i) {
-    float v = 0.0f;
-    if (i < k && lane < n) v = lane == i ? 1.0f : (lane < i ? 0.0f : V[lane + (size_t)i * ldv]);
-    sV[lane * kSpLd + i] = v;                                                         // V(lane, i)
-    sT[lane * kSpLd + i] = (lane <= i && i < k) ? Tm[lane + (size_t)i * kNB] : 0.0f;  // T(lane, i)
-  }
-  __syncwarp();
-  float w = 0.0f;  // W(lane) = sum_r V(r, lane) x(r)
-  for (int r = 0; r < 32; ++r) {
-    const float xb = __shfl_sync(0xffffffffu, xr, r);
-    if (r < n) w += sV[r * kSpLd + lane] * xb;
-  }
-  float w2 = 0.0f;  // W2 = T^T W (trans) or T W
-  for (int l = 0; l < 32; ++l) {
-    const float wl = __shfl_sync(0xffffffffu, w, l);
-    if (trans ? l <= lane : l >= lane) w2 += (trans ? sT[l * kSpLd + lane] : sT[lane * kSpLd + l]) * wl;
-  }
-  if (lane >= k) w2 = 0.0f;
-  float acc = 0.0f;  // (V W2)(lane)
-  for (int i = 0; i < 32; ++i) {
-    const float wi = __shfl_sync(0xffffffffu, w2, i);
-    acc += sV[lane * kSpLd + i] * wi;
-  }
-  __syncwarp();  // the next block overwrites sV / sT
-  return xr - acc;
-}
-
-__global__ void __launch_bounds__(kThreads) k_fwd_spars_small(const FwdSparsTask* __restrict__ tasks, int ntasks) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ti = blockIdx.x * kWarps + warp;
-  if (ti >= ntasks) return;
-  const FwdSparsTask t = tasks[ti];
-  float* sV = reinterpret_cast<float*>(smraw) + (size_t)warp * 2 * 32 * kSpLd;
-  float* sT = sV + 32 * kSpLd;
-  float* x = as<float>(t.x);
-  const int n = t.n;
-  float xr = lane < n ? x[lane] : 0.0f;
-  xr = warp_apply_unit(as<float>(t.Qs), n, as<float>(t.Ts), n, xr, n, true, sV, sT, lane);
-  xr = warp_apply_unit(as<float>(t.V), n, as<float>(t.T), *t.rank, xr, n, true, sV, sT, lane);
-  if (lane < n) x[lane] = xr;
-}
-
-__global__ void __launch_bounds__(kThreads) k_bwd_spars_small(const FwdSparsTask* __restrict__ tasks, int ntasks) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ti = blockIdx.x * kWarps + warp;
-  if (ti >= ntasks) return;
-  const FwdSparsTask t = tasks[ti];
-  float* sV = reinterpret_cast<float*>(smraw) + (size_t)warp * 2 * 32 * kSpLd;
-  float* sT = sV + 32 * kSpLd;
-  float* x = as<float>(t.x);
-  const int n = t.n;
-  float xr = lane < n ? x[lane] : 0.0f;
-  xr = warp_apply_unit(as<float>(t.V), n, as<float>(t.T), *t.rank, xr, n, false, sV, sT, lane);
-  // x <- R^{-1} x, R the upper triangle of Qs: the diagonal-block solve of trsv_upper
-  const float* R = as<float>(t.Qs);
-  for (int j = 0; j < 32; ++j) sV[lane * kSpLd + j] = (lane < n && j < n && j >= lane) ? R[lane + (size_t)j * n] : 0.0f;
-  __syncwarp();
-  for (int j = 31; j >= 0; --j) {
-    if (j < n) {
-      if (lane == j) xr = xr / sV[j * kSpLd + j];
-      const float xj = __shfl_sync(0xffffffffu, xr, j);
-      if (lane < j) xr -= sV[lane * kSpLd + j] * xj;
-    }
-  }
-  if (lane < n) x[lane] = xr;
-}
-
-// kBwdRows: rows per lane of the backward GEMV (interiors of <= 32 kBwdRows
-// rows); 0: one thread per row.
-template <typename T, int kBwdRows>
-__global__ void __launch_bounds__(kThreads) k_bwd_elim(const BwdElimTask* __restrict__ tasks,
-                                                       const BwdIn* __restrict__ ins, int nmax) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* sm = reinterpret_cast<T*>(smraw);
-  const BwdElimTask t = tasks[blockIdx.x];
-  T* xs = sm;
-  T* x = sm + 32;
-  T* part = x + nmax;  // kWarps x nmax partial sums (kBwdRows > 0)
-  for (int i = threadIdx.x; i < t.n; i += kThreads) x[i] = as<T>(t.x)[i];
-  if (kBwdRows > 0) {
-    // x -= sum over in-edges of R_e x_e: warp w streams the columns j = w mod
-    // kWarps (lanes over rows, coalesced), two columns' loads in flight, into
-    // a partial vector held in registers; the warps' partials meet in `part`
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nrs = (t.n + 31) / 32;
-    constexpr int kR = kBwdRows > 0 ? kBwdRows : 1;
-    T y[kR];
-#pragma unroll
-    for (int u = 0; u < kR; ++u) y[u] = 0.0;
-    for (int q = t.in_begin; q < t.in_end; ++q) {
-      const BwdIn e = ins[q];
-      const T* R = as<T>(e.R);
-      const T* xm = as<T>(e.xm);
-      int j = warp;
-      if (kR <= 12)  // four columns' loads in flight while the registers allow it
-        for (; j + 3 * kWarps < e.s; j += 4 * kWarps) {
-          const T* c0 = R + (size_t)j * e.ldr;
-          const T* c1 = c0 + (size_t)kWarps * e.ldr;
-          const T* c2 = c1 + (size_t)kWarps * e.ldr;
-          const T* c3 = c2 + (size_t)kWarps * e.ldr;
-          T v0[kR], v1[kR], v2[kR], v3[kR];
-#pragma unroll
-          for (int u = 0; u < kR; ++u) {
-            const int r = lane + 32 * u;
-            const bool ok = u < nrs && r < t.n;
-            v0[u] = ok ? c0[r] : (T)0.0;
-            v1[u] = ok ? c1[r] : (T)0.0;
-            v2[u] = ok ? c2[r] : (T)0.0;
-            v3[u] = ok ? c3[r] : (T)0.0;
-          }
-          const T x0 = xm[j], x1 = xm[j + kWarps], x2 = xm[j + 2 * kWarps], x3 = xm[j + 3 * kWarps];
-#pragma unroll
-          for (int u = 0; u < kR; ++u) y[u] += (v0[u] * x0 + v1[u] * x1) + (v2[u] * x2 + v3[u] * x3);
-        }
-      for (; j + kWarps < e.s; j += 2 * kWarps) {
-        const T* c0 = R + (size_t)j * e.ldr;
-        const T* c1 = c0 + (size_t)kWarps * e.ldr;
-        T v0[kR], v1[kR];
-#pragma unroll
-        for (int u = 0; u < kR; ++u) {
-          const int r = lane + 32 * u;
-          const bool ok = u < nrs && r < t.n;
-          v0[u] = ok ? c0[r] : (T)0.0;
-          v1[u] = ok ? c1[r] : (T)0.0;
-        }
-        const T x0 = xm[j], x1 = xm[j + kWarps];
-#pragma unroll
-        for (int u = 0; u < kR; ++u) y[u] += v0[u] * x0 + v1[u] * x1;
-      }
-      if (j < e.s) {
-        const T* c0 = R + (size_t)j * e.ldr;
-        const T x0 = xm[j];
-#pragma unroll
-        for (int u = 0; u < kR; ++u) {
-          const int r = lane + 32 * u;
-          if (u < nrs && r < t.n) y[u] += c0[r] * x0;
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kR; ++u) {
-      const int r = lane + 32 * u;
-      if (u < nrs && r < t.n) part[warp * nmax + r] = y[u];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < t.n; i += kThreads) {
-      T s = 0.0;
-      for (int w = 0; w < kWarps; ++w) s += part[w * nmax + i];
-      x[i] -= s;
-    }
-  } else {
-    __syncthreads();
-    for (int q = t.in_begin; q < t.in_end; ++q) {
-      const BwdIn e = ins[q];
-      for (int i = threadIdx.x; i < t.n; i += kThreads) {
-        T s = 0.0;
-        for (int j = 0; j < e.s; ++j) s += as<T>(e.R)[i + (size_t)j * e.ldr] * as<T>(e.xm)[j];
-        x[i] -= s;
-      }
-    }
-  }
-  __syncthreads();
-  dev::trsv_upper<T>(as<T>(t.S), t.n, x, t.n, xs);
-  for (int i = threadIdx.x; i < t.n; i += kThreads) as<T>(t.x)[i] = x[i];
-}
-
+// ------------------------------------------------------------ vectors
 __global__ void k_permute(int n, const int* __restrict__ perm, const double* __restrict__ src, double* dst) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[perm[i]] = src[i];
 }
 
-template <typename T>
-__global__ void k_copy_idx(int n, const int* __restrict__ src, const int* __restrict__ dst, double* xd) {
-  T* x = as<T>(xd);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[dst[i]] = x[src[i]];
-}
-
-// ------------------------------------------------------------ sparse + Krylov
 __global__ void k_spmv(int n, const int* __restrict__ rowptr, const int* __restrict__ col,
                        const double* __restrict__ val, const double* __restrict__ x, double* __restrict__ y) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
@@ -1660,133 +1361,6 @@ cudaError_t launch_merge(const MergeTask* t, int ntasks, cudaStream_t st) {
   counted();
   if (g_fp32) k_merge<float><<<ntasks, 256, 0, st>>>(t);
   else k_merge<double><<<ntasks, 256, 0, st>>>(t);
-  return last();
-}
-
-// The staged sweep kernels (reflector panels streamed through shared memory)
-// serve levels whose largest block has at least kStagedMin rows and whose
-// buffers fit; smaller blocks keep more CTAs per SM with the direct loads.
-constexpr int kStagedMin = 256;
-template <typename T>
-bool use_staged(int nmax, size_t other_bytes) {
-  // 1 KB left for the kernels' static shared memory
-  return nmax >= kStagedMin && dev::staged_elems<T>(nmax) * sizeof(T) + other_bytes + 1024 <= kSmemMax;
-}
-
-cudaError_t launch_fwd_elim(const FwdElimTask* t, const FwdOut* o, int ntasks, int nmax, int mmax, int* ticket,
-                            int* status, long long spin_limit, cudaStream_t st) {
-  if (cudaError_t pre = begin("launch_fwd_elim")) return pre;
-  if (ntasks <= 0) return cudaSuccess;
-  nmax = std::max(nmax, 1);
-  mmax = std::max(mmax, 1);
-  const size_t b = smem_bytes(dev::kVecRed + (size_t)nmax + (size_t)mmax);
-  const int srows = std::max(nmax, mmax);  // rows of a staged panel: the interior's or a neighbour's
-  counted();
-  auto go = [&](auto kern, size_t bytes) -> cudaError_t {
-    if (cudaError_t e = prep(kern, bytes)) return e;
-    kern<<<ntasks, kThreads, bytes, st>>>(t, o, ntasks, ticket, status, spin_limit, nmax, mmax);
-    return cudaSuccess;
-  };
-  cudaError_t e;
-  // staged where the interiors themselves are large (the top levels, few
-  // CTAs); large neighbours of small interiors alone do not pay for it
-  const bool big = nmax >= kStagedMin;
-  if (g_fp32)
-    e = big && use_staged<float>(srows, b)
-            ? go(k_fwd_elim<float, true>, dev::staged_elems<float>(srows) * sizeof(float) + b)
-            : go(k_fwd_elim<float, false>, b);
-  else
-    e = big && use_staged<double>(srows, b)
-            ? go(k_fwd_elim<double, true>, dev::staged_elems<double>(srows) * sizeof(double) + b)
-            : go(k_fwd_elim<double, false>, b);
-  if (e) return e;
-  return last();
-}
-
-// k_fwd_spars / k_bwd_spars over ntasks interfaces of at most nmax rows
-template <bool kFwd>
-cudaError_t launch_spars(const FwdSparsTask* t, int ntasks, int nmax, cudaStream_t st) {
-  const size_t b = smem_bytes(2 * kNB + 32 + (size_t)std::max(nmax, 1));
-  counted();
-  auto go = [&](auto kern, size_t bytes) -> cudaError_t {
-    if (cudaError_t e = prep(kern, bytes)) return e;
-    kern<<<ntasks, kThreads, bytes, st>>>(t);
-    return cudaSuccess;
-  };
-  cudaError_t e;
-  if (g_fp32) {
-    const size_t bs = dev::staged_elems<float>(nmax) * sizeof(float) + b;
-    if (use_staged<float>(nmax, b)) e = kFwd ? go(k_fwd_spars<float, true>, bs) : go(k_bwd_spars<float, true>, bs);
-    else e = kFwd ? go(k_fwd_spars<float, false>, b) : go(k_bwd_spars<float, false>, b);
-  } else {
-    const size_t bs = dev::staged_elems<double>(nmax) * sizeof(double) + b;
-    if (use_staged<double>(nmax, b)) e = kFwd ? go(k_fwd_spars<double, true>, bs) : go(k_bwd_spars<double, true>, bs);
-    else e = kFwd ? go(k_fwd_spars<double, false>, b) : go(k_bwd_spars<double, false>, b);
-  }
-  if (e) return e;
-  return last();
-}
-
-// The warp-per-interface forms (FP32, n <= 32): kFwd chooses the forward step.
-cudaError_t launch_spars_small(bool fwd, const FwdSparsTask* t, int ntasks, cudaStream_t st) {
-  if (cudaError_t pre = begin("launch_spars_small")) return pre;
-  if (ntasks <= 0) return cudaSuccess;
-  if (!g_fp32) return cudaErrorInvalidValue;  // FP32 factors only
-  counted();
-  const int grid = (ntasks + kWarps - 1) / kWarps;
-  if (fwd) {
-    if (cudaError_t e = prep(k_fwd_spars_small, kSparsSmallSmem)) return e;
-    k_fwd_spars_small<<<grid, kThreads, kSparsSmallSmem, st>>>(t, ntasks);
-  } else {
-    if (cudaError_t e = prep(k_bwd_spars_small, kSparsSmallSmem)) return e;
-    k_bwd_spars_small<<<grid, kThreads, kSparsSmallSmem, st>>>(t, ntasks);
-  }
-  return last();
-}
-
-bool spars_small(int n) { return n <= 32; }
-
-cudaError_t launch_fwd_spars(const FwdSparsTask* t, int ntasks, int nmax, cudaStream_t st) {
-  if (cudaError_t pre = begin("launch_fwd_spars")) return pre;
-  if (ntasks <= 0) return cudaSuccess;
-  return launch_spars<true>(t, ntasks, nmax, st);
-}
-
-cudaError_t launch_bwd_spars(const FwdSparsTask* t, int ntasks, int nmax, cudaStream_t st) {
-  if (cudaError_t pre = begin("launch_bwd_spars")) return pre;
-  if (ntasks <= 0) return cudaSuccess;
-  return launch_spars<false>(t, ntasks, nmax, st);
-}
-
-cudaError_t launch_bwd_elim(const BwdElimTask* t, const BwdIn* in, int ntasks, int nmax, cudaStream_t st) {
-  if (cudaError_t pre = begin("launch_bwd_elim")) return pre;
-  if (ntasks <= 0) return cudaSuccess;
-  nmax = std::max(nmax, 1);
-  const int rows = nmax <= 128 ? 4 : nmax <= 384 ? 12 : nmax <= 1024 ? 32 : 0;
-  const size_t b = smem_bytes(32 + (size_t)nmax + (rows ? (size_t)kWarps * nmax : 0));
-  counted();
-  auto go = [&](auto kern) -> cudaError_t {
-    if (cudaError_t e = prep(kern, b)) return e;
-    kern<<<ntasks, kThreads, b, st>>>(t, in, nmax);
-    return cudaSuccess;
-  };
-  cudaError_t e;
-  if (g_fp32)
-    e = rows == 4 ? go(k_bwd_elim<float, 4>) : rows == 12 ? go(k_bwd_elim<float, 12>)
-        : rows == 32 ? go(k_bwd_elim<float, 32>) : go(k_bwd_elim<float, 0>);
-  else
-    e = rows == 4 ? go(k_bwd_elim<double, 4>) : rows == 12 ? go(k_bwd_elim<double, 12>)
-        : rows == 32 ? go(k_bwd_elim<double, 32>) : go(k_bwd_elim<double, 0>);
-  if (e) return e;
-  return last();
-}
-
-cudaError_t launch_copy_idx(int n, const int* src, const int* dst, double* x, cudaStream_t st) {
-  if (cudaError_t pre = begin("launch_copy_idx")) return pre;
-  if (n <= 0) return cudaSuccess;
-  counted();
-  if (g_fp32) k_copy_idx<float><<<grid_for(n), 256, 0, st>>>(n, src, dst, x);
-  else k_copy_idx<double><<<grid_for(n), 256, 0, st>>>(n, src, dst, x);
   return last();
 }
 

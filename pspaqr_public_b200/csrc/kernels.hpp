@@ -88,18 +88,6 @@ cudaError_t launch_edge_right_small(const EdgeChunk* t, int ntasks, cudaStream_t
 // per task.
 cudaError_t launch_update_small(const UpdTask* t, const UpdOp* o, int ntasks, cudaStream_t st);
 bool update_op_small(int k, int m);
-// Forward (fwd) or backward scaling + sparsification steps of FP32 interfaces
-// with spars_small(n) (at most 32 rows), one warp per interface.
-cudaError_t launch_spars_small(bool fwd, const FwdSparsTask* t, int ntasks, cudaStream_t st);
-bool spars_small(int n);
-
-cudaError_t launch_fwd_elim(const FwdElimTask* t, const FwdOut* o, int ntasks, int nmax, int mmax, int* ticket,
-                            int* status, long long spin_limit, cudaStream_t st);
-cudaError_t launch_fwd_spars(const FwdSparsTask* t, int ntasks, int nmax, cudaStream_t st);
-cudaError_t launch_bwd_spars(const FwdSparsTask* t, int ntasks, int nmax, cudaStream_t st);
-cudaError_t launch_bwd_elim(const BwdElimTask* t, const BwdIn* in, int ntasks, int nmax, cudaStream_t st);
-cudaError_t launch_copy_idx(int n, const int* src, const int* dst, double* x, cudaStream_t st);
-
 cudaError_t launch_spmv(int n, const int* rowptr, const int* col, const double* val, const double* x, double* y,
                         cudaStream_t st);
 int mgs_grid(int n);

@@ -107,46 +107,6 @@ struct MergeTask {
   int c0;        // first column of this slab of the child block (large blocks are split)
 };
 
-// ----------------------------------------------------------------- solve
-// Forward elimination sweep of one interior (ptree.cpp:2160-2187, 2840-2939).
-struct FwdElimTask {
-  const double* S;  // n x n (V below diagonal)
-  const double* T;
-  double* x;        // n
-  int n;
-  int out_begin, out_end;  // range in FwdOut
-};
-struct FwdOut {
-  const double* V;  // m x n reflector tails
-  const double* T;
-  double* xn;       // neighbour's vector (m)
-  int* turn;        // neighbour's turn counter
-  int m;
-  int my_turn;      // position of this interior in the neighbour's order
-};
-// Forward scaling + sparsification of one interface (ptree.cpp:2950-2981).
-struct FwdSparsTask {
-  const double* Qs;  // n x n
-  const double* Ts;
-  const double* V;   // n x rank
-  const double* T;
-  const int* rank;
-  double* x;
-  int n;
-};
-// Backward substitution of one interior (ptree.cpp:3060-3089, 3140-3174).
-struct BwdElimTask {
-  const double* S;
-  double* x;
-  int n;
-  int in_begin, in_end;  // range in BwdIn
-};
-struct BwdIn {
-  const double* R;  // n_c x s block A(c, m), ld = ldr
-  const double* xm;
-  int ldr, s;
-};
-
 // Conversion of one double array to float (mixed-precision factorization).
 struct ConvTask {
   const double* src;
