@@ -58,7 +58,11 @@ __device__ __forceinline__ T house(T alpha, T sumsq, T* beta, T* scal) {
     *scal = 0.0;
     return 0.0;
   }
-  T b = -copysign(hypot(alpha, sqrt(sumsq)), alpha);
+  // the square is safe but for extreme values (hypot costs twice as much, on
+  // the serial path of every reflector)
+  const T sq = alpha * alpha + sumsq;
+  const T lo = sizeof(T) == 8 ? (T)1e-280 : (T)1e-30, hi = sizeof(T) == 8 ? (T)1e280 : (T)1e30;
+  T b = -copysign(sq > lo && sq < hi ? sqrt(sq) : hypot(alpha, sqrt(sumsq)), alpha);
   *beta = b;
   *scal = 1.0 / (alpha - b);
   return (b - alpha) / b;
@@ -200,8 +204,8 @@ __device__ __forceinline__ T ld_v(const T* p) {
 // (geqrt / RRQR reflectors), A unused; unit = 0: pentagonal tpqrt panel,
 // [A (kb x nc); C] <- Q^T [A; C] with V full (m x kb).  Column c of A and C
 // is column c + (c / kNB) * cgap of the arrays (cgap > 0: the column panels
-// a CTA owns in a cluster-distributed factorization).  kCg: V and T are read
-// through L2.
+// a CTA owns in a cluster-distributed factorization).  kCg: V, T and A are
+// read through L2 (other CTAs write them).
 template <typename T, bool kCg = false>
 __device__ void tile_left_qt(const T* V, int ldv, const T* Tm, int ldt, int kb, int unit, T* A, int lda,
                              T* C, int ldc, int m, int nc, T* sm, int cgap = 0) {
@@ -267,7 +271,7 @@ __device__ void tile_left_qt(const T* V, int ldv, const T* Tm, int ldt, int kb, 
 #pragma unroll
   for (int q = 0; q < kSA; ++q) {
     const int idx = t + q * kThreads, i = idx & (kNB - 1), c = idx / kNB;
-    ra[q] = (!unit && i < kb && c < nc) ? A[i + col(c) * lda] : (T)0.0;
+    ra[q] = (!unit && i < kb && c < nc) ? ld_v<kCg>(A + i + col(c) * lda) : (T)0.0;
   }
   // ---- W = V^T C.  A thread accumulates W(i0:i0+kIW, c0:c0+4); the kSets
   // row sets of kTPO threads each take kRows consecutive rows of every tile

@@ -25,6 +25,7 @@ constexpr size_t kAlign = 256;
 constexpr size_t kArenaChunk = size_t(1) << 30;
 // bounded wait of the forward sweep: ~1 s at 2 GHz
 constexpr int kChunk = 64;        // columns (rows) per CTA of the chunked applies
+constexpr size_t kElimPipeInteriors = 256;  // levels with at most this many interiors pipeline their chains
 constexpr int kUpdSmallMinTasks = 4096;  // small update tasks needed for the team-per-task kernel
 constexpr float kTuneMargin = 0.95f;      // tensor cores chosen where at least 5 % faster
 
@@ -497,13 +498,47 @@ int Tree::factorize() {
     }
     // the chains run while the host builds the update lists
     {
-      auto* d_eo = static_cast<ElimOut*>(upload(eo.data(), sizeof(ElimOut) * eo.size()));
-      for (int g = 0; g < 3; ++g) {
-        if (et[g].empty()) continue;
-        auto* d_et = static_cast<ElimTask*>(upload(et[g].data(), sizeof(ElimTask) * et[g].size()));
-        if (!d_et || !d_eo) return fail(-11, "out of device memory (elimination descriptors)");
-        if (ck(launch_elim(d_et, d_eo, (int)et[g].size(), csz[g], nmax[g], vmax[g], stream_), "elimination kernel"))
+      // few interiors: a pipeline of one cluster per chain step, in clusters as
+      // wide as the steps leave SMs for
+      const bool pipe = Lv.interiors.size() <= kElimPipeInteriors && !eo.empty();
+      if (pipe) {
+        std::vector<ElimStep> st;
+        int nprog = 0, nm = 1, vm = 1;
+        for (int g = 0; g < 3; ++g) {
+          nm = std::max(nm, nmax[g]);
+          vm = std::max(vm, vmax[g]);
+        }
+        // interiors in their level's order, whatever their group
+        std::vector<const ElimTask*> all;
+        for (int g = 0; g < 3; ++g)
+          for (const ElimTask& t : et[g]) all.push_back(&t);
+        std::sort(all.begin(), all.end(), [](const ElimTask* x, const ElimTask* y) { return x->out_begin < y->out_begin; });
+        for (const ElimTask* t : all) {
+          const int nout = t->out_end - t->out_begin;
+          st.push_back({t->S, nullptr, t->T, t->tau, t->n, t->n, -1, nout ? nprog++ : -1});
+          for (int k = 0; k < nout; ++k) {
+            const ElimOut& o = eo[t->out_begin + k];
+            const int in = nprog - 1;
+            st.push_back({t->S, o.B, o.T, t->tau, t->n, o.m, in, k + 1 < nout ? nprog++ : -1});
+          }
+        }
+        int cs = cluster_for(nm);
+        while (cs > 1 && st.size() * cs > (size_t)num_sms()) cs = cs == kBigCluster ? 4 : 1;
+        auto* d_st = static_cast<ElimStep*>(upload(st.data(), sizeof(ElimStep) * st.size()));
+        auto* d_cnt = static_cast<int*>(scratch_.alloc(sizeof(int) * (size_t)(nprog + 1)));
+        if (!d_st || !d_cnt) return fail(-11, "out of device memory (elimination descriptors)");
+        if (ck(cudaMemsetAsync(d_cnt, 0, sizeof(int) * (size_t)(nprog + 1), stream_), "elimination counters") ||
+            ck(launch_elim_pipe(d_st, (int)st.size(), cs, nm, vm, d_cnt, d_cnt + 1, stream_), "elimination kernel"))
           return -10;
+      } else {
+        auto* d_eo = static_cast<ElimOut*>(upload(eo.data(), sizeof(ElimOut) * eo.size()));
+        for (int g = 0; g < 3; ++g) {
+          if (et[g].empty()) continue;
+          auto* d_et = static_cast<ElimTask*>(upload(et[g].data(), sizeof(ElimTask) * et[g].size()));
+          if (!d_et || !d_eo) return fail(-11, "out of device memory (elimination descriptors)");
+          if (ck(launch_elim(d_et, d_eo, (int)et[g].size(), csz[g], nmax[g], vmax[g], stream_), "elimination kernel"))
+            return -10;
+        }
       }
       cudaEventRecord(fe[0], stream_);
     }
@@ -1342,6 +1377,7 @@ int Tree::factorize() {
     if (ck(cudaStreamSynchronize(stream_), "factorize level")) return -10;
     if (const int ds = h_status ? *h_status : device_status()) {
       clear_status();
+      if (ds & 16) return fail(-12, "elimination pipeline wait timed out on the device at level " + std::to_string(lvl));
       if (ds & 2) return fail(-12, "tensor-core MMA wait timed out on the device at level " + std::to_string(lvl));
       return fail(-13, std::string(ds & 4 ? "non-finite" : "zero") + " pivot in the QR factorizations of level " +
                            std::to_string(lvl));

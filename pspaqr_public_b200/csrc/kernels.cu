@@ -73,20 +73,54 @@ __global__ void k_scatter(int nnz, const double* __restrict__ val, double* const
 // (two of its panels per pass).  `lt` holds the owner's tau values, `tg`
 // the global copy, `vb` a reflector tail, `tile` dev::kTileSmem elements.
 //
+// Steps of a chain on the same R (a tpqrt per out-edge, after the geqrt of R
+// itself) can run as a pipeline of CTAs: panel p of a step needs the rows of
+// panel p of R as the step before has left them and nothing else of R, so
+// `chain` holds the counter of panels that the step before has finished and the
+// one to publish this step's.
+//
 // With `pan` (ldp >= the panel's rows; ldp * kNB + kPanExtra elements, may
 // alias `tile`), the owner copies the panel into shared memory, runs the kb
 // reflector steps and the T factor there (one barrier per reflector, T by
 // one warp) and writes the panel back once.
+struct ChainLink {
+  const int* in = nullptr;  // panels of R finished by the step before
+  int* out = nullptr;       // panels finished here
+};
+// Cycle limit of a pipeline's waits (about a second); a wait that runs out sets
+// the status word's bit 4 (value 16) and the step goes on without waiting.
+constexpr long long kChainSpin = 2000000000LL;
+__device__ __forceinline__ int chain_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void chain_wait(const int* p, int v, int* status) {
+  const long long t0 = clock64();
+  while (chain_acquire(p) < v) {
+    if (chain_acquire(status) & 16) break;
+    if (clock64() - t0 > kChainSpin) {
+      atomicOr(status, 16);
+      break;
+    }
+  }
+  __threadfence();
+}
+
 template <typename T>
 __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T* Tout, T* tg,
                         T* lt, T* vb, T* red, T* tmp, T* tile, int cs, int* status = nullptr, T* pan = nullptr,
-                        int ldp = 0) {
+                        int ldp = 0, ChainLink chain = ChainLink()) {
   const int rank = crank(cs);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gap = (cs - 1) * kNB;  // columns between two panels of one CTA
   for (int j0 = 0; j0 < n; j0 += kNB) {
     const int kb = (n - j0) < kNB ? (n - j0) : kNB;
     const int pend = j0 + kb;
+    if (chain.in) {
+      if (threadIdx.x == 0) chain_wait(chain.in, j0 / kNB + 1, status);
+      __syncthreads();
+    }
     if (owns(j0, rank, cs) && pan) {
       // panel rows: [j0, m) of R's columns (geqrt) or B's m rows (tpqrt)
       const int pm = unit ? m - j0 : m;
@@ -140,21 +174,57 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
           // R(j, j) = 0 or not finite: the triangular solves would break down
           if (status && !(isfinite(beta) && beta != (T)0)) atomicOr(status, isfinite(beta) ? 8 : 4);
         }
-        for (int k = j + 1 + warp; k < pend; k += kWarps) {
-          const int kk = k - j0;
-          T* rjk = unit ? (pan + jj + (size_t)kk * ldp) : (pr + jj + kk * kNB);
-          T* tk = unit ? (pan + (jj + 1) + (size_t)kk * ldp) : (pan + (size_t)kk * ldp);
-          if (tj != 0.0) {
-            T d = lane == 0 ? *rjk : 0.0;
-            for (int i = lane; i < vlen; i += 32) d += (tail[i] * scal) * tk[i];
-            d = dev::warp_sum(d) * tj;
-            if (lane == 0) *rjk -= d;
-            for (int i = lane; i < vlen; i += 32) tk[i] -= (tail[i] * scal) * d;
+        // the warp's (at most four) columns together: their loads and the
+        // shuffles of their sums overlap
+        constexpr int kC = kNB / kWarps;
+        const int nk = pend - j - 1 > warp ? (pend - j - 2 - warp) / kWarps + 1 : 0;
+        if (nk > 0) {
+          T* rjk[kC];
+          T* tk[kC];
+          T d[kC];
+#pragma unroll
+          for (int u = 0; u < kC; ++u) {
+            const int kk = jj + 1 + warp + (u < nk ? u : 0) * kWarps;
+            rjk[u] = unit ? (pan + jj + (size_t)kk * ldp) : (pr + jj + kk * kNB);
+            tk[u] = unit ? (pan + (jj + 1) + (size_t)kk * ldp) : (pan + (size_t)kk * ldp);
+            d[u] = 0.0;
           }
-          if (k == j + 1) {  // reflector j + 1's tail: rows below its diagonal
-            T sq = 0.0;
+          const bool next = warp == 0;  // column j + 1: also its new tail's norm
+          T sq = 0.0;
+          if (tj != 0.0) {
+#pragma unroll
+            for (int u = 0; u < kC; ++u) d[u] = lane == 0 ? *rjk[u] : (T)0.0;
+#pragma unroll 2
+            for (int i = lane; i < vlen; i += 32) {
+              const T v = tail[i] * scal;
+#pragma unroll
+              for (int u = 0; u < kC; ++u) d[u] += v * tk[u][i];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+              for (int u = 0; u < kC; ++u) d[u] += __shfl_xor_sync(0xffffffffu, d[u], o);
+#pragma unroll
+            for (int u = 0; u < kC; ++u) {
+              d[u] *= tj;
+              if (lane == 0 && u < nk) *rjk[u] -= d[u];
+            }
+#pragma unroll 2
+            for (int i = lane; i < vlen; i += 32) {
+              const T v = tail[i] * scal;
+              T x[kC];
+#pragma unroll
+              for (int u = 0; u < kC; ++u) x[u] = tk[u][i] - v * d[u];
+#pragma unroll
+              for (int u = 0; u < kC; ++u)
+                if (u < nk) tk[u][i] = x[u];
+              if (!unit || i > 0) sq += x[0] * x[0];
+            }
+          } else if (next) {
             for (int i = lane; i < vlen; i += 32)
-              if (!unit || i > 0) sq += tk[i] * tk[i];
+              if (!unit || i > 0) sq += tk[0][i] * tk[0][i];
+          }
+          if (next) {  // reflector j + 1's tail: rows below its diagonal
             sq = dev::warp_sum(sq);
             if (lane == 0) s_nrm2[(j + 1) & 1] = sq;
           }
@@ -241,6 +311,13 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
         dev::tile_left_qt<T, true>(B + (size_t)j0 * ldb, ldb, Tm, kNB, kb, 0, R + j0 + (size_t)q0 * ldr, ldr,
                                    B + (size_t)q0 * ldb, ldb, m, nc, tile, gap);
     }
+    if (chain.out) {
+      csync(cs);
+      if (rank == 0 && threadIdx.x == 0) {
+        __threadfence();
+        asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(chain.out), "r"(j0 / kNB + 1) : "memory");
+      }
+    }
   }
   csync(cs);
 }
@@ -266,6 +343,36 @@ __global__ void __launch_bounds__(kThreads, 2) k_elim(const ElimTask* __restrict
     dist_qr<T>(as<T>(t.S), t.n, as<T>(e.B), e.m, e.m, t.n, 0, as<T>(e.T), as<T>(t.tau), lt, vb, red, tmp, tile,
                cs, status, pan, vmax);
   }
+}
+
+// The chains as pipelines: one cluster per step, taken in order by ticket, so
+// that the step a cluster waits for is held by a running one.
+template <typename T, bool kStage>
+__global__ void __launch_bounds__(kThreads, 2) k_elim_pipe(const ElimStep* __restrict__ steps, int cs, int nmax,
+                                                        int vmax, int* ticket, int* prog, int* status) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ int s_step;
+  T* sm = reinterpret_cast<T*>(smraw);
+  if (threadIdx.x == 0 && crank(cs) == 0) s_step = atomicAdd(ticket, 1);
+  csync(cs);
+  if (cs > 1) {
+    const int v = *cg::this_cluster().map_shared_rank(&s_step, 0);
+    csync(cs);
+    if (threadIdx.x == 0) s_step = v;
+    __syncthreads();
+  }
+  const ElimStep t = steps[s_step];
+  T* red = sm;
+  T* tmp = red + kRed;
+  T* lt = tmp + kNB;
+  T* vb = lt + nmax;
+  T* tile = vb + vmax;
+  ChainLink link;
+  if (t.in >= 0) link.in = prog + t.in;
+  if (t.out >= 0) link.out = prog + t.out;
+  T* B = as<T>(t.B);
+  dist_qr<T>(as<T>(t.S), t.n, B, t.m, B ? t.m : t.n, t.n, B ? 0 : 1, as<T>(t.T), as<T>(t.tau), lt, vb, red, tmp, tile,
+             cs, status, kStage ? tile : nullptr, vmax, link);
 }
 
 // kStage: panels factored in shared memory (nmax rows), as in k_elim.
@@ -1189,6 +1296,21 @@ cudaError_t launch_elim(const ElimTask* t, const ElimOut* o, int ntasks, int cs,
   }
   if (cudaError_t e = prep(k_elim<double, false>, head + smem_bytes(kWcap))) return e;
   return launch_clustered(k_elim<double, false>, ntasks, cs, head + smem_bytes(kWcap), st, t, o, cs, vmax, g_status);
+}
+
+cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, int vmax, int* ticket, int* prog,
+                             cudaStream_t st) {
+  if (cudaError_t pre = begin("launch_elim_pipe")) return pre;
+  if (nsteps <= 0) return cudaSuccess;
+  vmax = std::max(vmax, 1);
+  const size_t head = smem_bytes(kRed + kNB + (size_t)nmax + (size_t)vmax);
+  auto go = [&](auto kern, size_t b) {
+    if (cudaError_t e = prep(kern, b)) return e;
+    return launch_clustered(kern, nsteps, cs, b, st, t, cs, nmax, vmax, ticket, prog, g_status);
+  };
+  const size_t bs = g_fp32 ? staged_panel_bytes<float>(head, vmax) : staged_panel_bytes<double>(head, vmax);
+  if (g_fp32) return bs ? go(k_elim_pipe<float, true>, bs) : go(k_elim_pipe<float, false>, head + smem_bytes(kWcap));
+  return bs ? go(k_elim_pipe<double, true>, bs) : go(k_elim_pipe<double, false>, head + smem_bytes(kWcap));
 }
 
 cudaError_t launch_scale(const ScaleTask* t, int ntasks, int cs, int nmax, cudaStream_t st) {

@@ -27,6 +27,16 @@ struct ElimOut {
   int m;
 };
 
+// One step of such a chain: the geqrt of S (B null) or the tsqrt of [S; B].
+// in / out: progress counters of the step before and of this one (-1: none).
+struct ElimStep {
+  double* S;
+  double* B;
+  double* T;
+  double* tau;
+  int n, m, in, out;
+};
+
 // Trailing update of columns [col0, col0+ncols) of one column cluster
 // (ptree.cpp:216-266): the ops of the cluster applied in order; kind 0 =
 // larfb of an interior's diagonal reflectors on A(c, m), kind 1 = tpmqrt of
