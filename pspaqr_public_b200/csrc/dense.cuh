@@ -127,33 +127,57 @@ __device__ void panel_t(const T* V, int ldv, int m, int kb, int unit, const T* t
   larft_from_gram(Tm, ldt, kb, tau, tmp);
 }
 
+// D (8 x 8) += A (8 x 4) B (4 x 8) in FP64, one warp.  Lane = 4 n + k holds
+// A(n, k) and B(k, n), and D(n, 2 k), D(n, 2 k + 1).
+__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
 // panel_t for a panel in shared memory, with T built by one warp: the Gram
-// V^T V of the panel's reflectors goes to sG (kNB x (kNB + 1), shared), then
-// lane i holds row i of T in registers and forms column j as
-//   T(i, j) = -tau_j sum_{l=i}^{j-1} T(i, l) G(l, j),  T(j, j) = tau_j,
-// the sums of larft_from_gram in the same order, without its two barriers
-// and global round trips per column.  Tm is written by warp 0; the caller
-// synchronises before T is read.
+// matrix goes to sG (kNB x (kNB + 1), shared); lane i of warp 0 then holds row
+// i of T and forms T(i, j) = -tau_j sum_{l=i}^{j-1} T(i, l) G(l, j), T(j, j) =
+// tau_j, without barriers.  Tm is written by warp 0; the caller synchronises
+// before T is read.  The Gram matrix is the
+// panel's transpose times itself: ten 8 x 8 tiles on and above the diagonal, one
+// or two a warp, as FP64 mma products (the A and the B fragment of a column
+// block are the same registers).  Dot products by warps and shuffles took as
+// long as half of the panel's reflectors.
 template <typename T>
 __device__ void panel_t_warp(const T* V, int ldv, int m, int kb, int unit, const T* tau, T* Tm, int ldt, T* sG) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kLG = kNB + 1;
-  const int npairs = kb * (kb - 1) / 2;
-  for (int p = warp; p < npairs; p += kWarps) {
-    int l, j;
-    pair_of(p, &l, &j);
-    const T* vl = V + (size_t)l * ldv;
-    const T* vj = V + (size_t)j * ldv;
-    T d = 0.0;
-    if (unit) {
-      d = lane == 0 ? vl[j] : 0.0;
-      for (int i = j + 1 + lane; i < m; i += 32) d += vl[i] * vj[i];
-    } else {
-      for (int i = lane; i < m; i += 32) d += vl[i] * vj[i];
+  const int fn = lane >> 2, fk = lane & 3;
+  const int nt = (kb + 7) / 8;
+  int tile = 0;
+  for (int bi = 0; bi < nt; ++bi)
+    for (int bj = bi; bj < nt; ++bj, ++tile) {
+      if (tile % kWarps != warp) continue;
+      const int ci = 8 * bi + fn, cj = 8 * bj + fn;
+      const T* vi = V + (size_t)(ci < kb ? ci : 0) * ldv;
+      const T* vj = V + (size_t)(cj < kb ? cj : 0) * ldv;
+      auto el = [&](const T* v, int c, int r) -> double {
+        if (r >= m || c >= kb) return 0.0;
+        if (unit && r <= c) return r == c ? 1.0 : 0.0;
+        return (double)v[r];
+      };
+      double d[2][2] = {};
+      int r = 0;
+      for (; r < kNB; r += 8) {  // rows with the unit triangle
+        dmma(d[0][0], d[0][1], el(vi, ci, r + fk), el(vj, cj, r + fk));
+        dmma(d[1][0], d[1][1], el(vi, ci, r + 4 + fk), el(vj, cj, r + 4 + fk));
+      }
+      const double zi = ci < kb ? 1.0 : 0.0, zj = cj < kb ? 1.0 : 0.0;
+      for (; r + 8 <= m; r += 8) {
+        const double a0 = vi[r + fk], b0 = vj[r + fk], a1 = vi[r + 4 + fk], b1 = vj[r + 4 + fk];
+        dmma(d[0][0], d[0][1], a0 * zi, b0 * zj);
+        dmma(d[1][0], d[1][1], a1 * zi, b1 * zj);
+      }
+      for (; r < m; r += 4) dmma(d[0][0], d[0][1], el(vi, ci, r + fk), el(vj, cj, r + fk));
+#pragma unroll
+      for (int e = 0; e < 2; ++e) sG[(8 * bi + fn) * kLG + 8 * bj + 2 * fk + e] = (T)(d[0][e] + d[1][e]);
     }
-    d = warp_sum(d);
-    if (lane == 0) sG[l * kLG + j] = d;
-  }
   __syncthreads();
   if (warp == 0) {
     T t[kNB];
@@ -162,12 +186,12 @@ __device__ void panel_t_warp(const T* V, int ldv, int m, int kb, int unit, const
 #pragma unroll
     for (int j = 0; j < kNB; ++j) {
       if (j < kb) {
-        T s = 0.0;
+        T s[4] = {};
 #pragma unroll
         for (int l = 0; l < kNB; ++l)
-          if (l < j && l >= lane) s += t[l] * sG[l * kLG + j];
+          if (l < j && l >= lane) s[l & 3] += t[l] * sG[l * kLG + j];
         const T tj = tau[j];
-        t[j] = lane < j ? -tj * s : (lane == j ? tj : (T)0.0);
+        t[j] = lane < j ? -tj * ((s[0] + s[1]) + (s[2] + s[3])) : (lane == j ? tj : (T)0.0);
       }
     }
     if (lane < kb)

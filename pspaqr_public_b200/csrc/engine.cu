@@ -25,7 +25,13 @@ constexpr size_t kAlign = 256;
 constexpr size_t kArenaChunk = size_t(1) << 30;
 // bounded wait of the forward sweep: ~1 s at 2 GHz
 constexpr int kChunk = 64;        // columns (rows) per CTA of the chunked applies
-constexpr size_t kElimPipeInteriors = 256;  // levels with at most this many interiors pipeline their chains
+// Levels with at most kElimPipe interiors pipeline their chains: about 1.6 times
+// the work of a chain on one CTA (waits, no reuse between steps), so that it pays
+// while whole chains would leave a third of the GPU idle (64^3 FP64: 256 interiors
+// 2.7 ms whole, 4.3 ms pipelined; 128 interiors 10.4 and 5.3 ms).  With up to
+// kElimPipeMixed interiors of different cluster sizes, which as whole chains run
+// one size after the other, it pays too (1024 leaves of 384^2: 15.5 and 9.8 ms).
+constexpr size_t kElimPipe = 160, kElimPipeMixed = 1024;
 constexpr int kUpdSmallMinTasks = 4096;  // small update tasks needed for the team-per-task kernel
 constexpr float kTuneMargin = 0.95f;      // tensor cores chosen where at least 5 % faster
 
@@ -500,7 +506,8 @@ int Tree::factorize() {
     {
       // few interiors: a pipeline of one cluster per chain step, in clusters as
       // wide as the steps leave SMs for
-      const bool pipe = Lv.interiors.size() <= kElimPipeInteriors && !eo.empty();
+      const size_t ni = Lv.interiors.size(), sizes = !et[0].empty() + !et[1].empty() + !et[2].empty();
+      const bool pipe = !eo.empty() && (ni <= kElimPipe || (sizes > 1 && ni <= kElimPipeMixed));
       if (pipe) {
         std::vector<ElimStep> st;
         int nprog = 0, nm = 1, vm = 1;
@@ -1478,12 +1485,11 @@ int Tree::alloc_level_blocks(const std::vector<int>& edges) {
   return 0;
 }
 
-// Levels with at most this many interiors, some of them with more than kPipeRows
-// rows, run their forward elimination as a pipeline of one CTA per chain step:
-// more interiors fill the GPU by themselves, and a pipeline of one or two panels
-// hands on later than one CTA gets there.
+// Levels with at most this many interiors run the apply's forward elimination as a
+// pipeline of one CTA per chain step; more interiors fill the GPU by themselves
+// (384^2 float, 1024 leaves: 0.98 ms an apply at 256, 1.19 ms with the leaves
+// pipelined).
 constexpr size_t kPipeInteriors = 256;
-constexpr int kPipeRows = 64;
 
 // Descriptors of the panel-chain sweeps (offsets into any workspace): packed into
 // one upload.  Also inverts the diagonal blocks of every triangular solve.
@@ -1510,9 +1516,7 @@ int Tree::plan_sweep() {
   for (int lvl = 0; lvl < L; ++lvl) {
     const Level& Lv = st_.levels[lvl];
     SweepLevel& S = sweep_[lvl];
-    int longest = 0;
-    for (int c : Lv.interiors) longest = std::max(longest, size_[c]);
-    S.pipe = Lv.interiors.size() <= kPipeInteriors && longest > kPipeRows;
+    S.pipe = Lv.interiors.size() <= kPipeInteriors;
     std::vector<int> seen(Lv.count, 0);  // turn order per neighbour: interiors ascending
     std::vector<FwdItem> fw;
     std::vector<FwdEdge> fe;

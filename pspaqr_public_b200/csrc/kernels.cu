@@ -79,7 +79,8 @@ __global__ void k_scatter(int nnz, const double* __restrict__ val, double* const
 // `chain` holds the counter of panels that the step before has finished and the
 // one to publish this step's.
 //
-// With `pan` (ldp >= the panel's rows; ldp * kNB + kPanExtra elements, may
+// With `pan` (ldp >= the panel's rows; ldp * pw + kPanExtra elements, pw = 32
+// columns or 16 or 8 where a whole panel does not fit; may
 // alias `tile`), the owner copies the panel into shared memory, runs the kb
 // reflector steps and the T factor there (one barrier per reflector, T by
 // one warp) and writes the panel back once.
@@ -110,7 +111,7 @@ __device__ __forceinline__ void chain_wait(const int* p, int v, int* status) {
 template <typename T>
 __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T* Tout, T* tg,
                         T* lt, T* vb, T* red, T* tmp, T* tile, int cs, int* status = nullptr, T* pan = nullptr,
-                        int ldp = 0, ChainLink chain = ChainLink()) {
+                        int ldp = 0, int pw = kNB, ChainLink chain = ChainLink()) {
   const int rank = crank(cs);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gap = (cs - 1) * kNB;  // columns between two panels of one CTA
@@ -122,9 +123,12 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
       __syncthreads();
     }
     if (owns(j0, rank, cs) && pan) {
+     const int pstart = j0, pkb = kb, plast = pend;
+     for (int j0 = pstart; j0 < plast; j0 += pw) {  // the whole panel, or parts of pw columns where it does not fit
+      const int kb = min(pw, plast - j0), pend = j0 + kb;
       // panel rows: [j0, m) of R's columns (geqrt) or B's m rows (tpqrt)
       const int pm = unit ? m - j0 : m;
-      T* pr = pan + (size_t)ldp * kNB;  // tpqrt: R(j0:pend, j0:pend), ld kNB
+      T* pr = pan + (size_t)ldp * pw;  // tpqrt: R(j0:pend, j0:pend), ld kNB
       T* sG = pr + kNB * kNB;           // the panel's Gram matrix (panel_t_warp)
       __syncthreads();                  // `pan` may alias the tiled apply's scratch
       for (int c = warp; c < kb; c += kWarps) {
@@ -241,7 +245,7 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
         for (int i = threadIdx.x; i < prev_vlen; i += kThreads) prev_tail[i] *= prev_scal;
       if (threadIdx.x == 0 && prev_ajj) *prev_ajj = prev_beta;
       __syncthreads();
-      dev::panel_t_warp(pan, ldp, pm, kb, unit, lt + j0, Tout + (size_t)j0 * kNB, kNB, sG);
+      dev::panel_t_warp(pan, ldp, pm, kb, unit, lt + j0, Tout + (size_t)j0 * kNB + (j0 - pstart), kNB, sG);
       for (int c = warp; c < kb; c += kWarps) {
         T* dst = unit ? (R + j0 + (size_t)(j0 + c) * ldr) : (B + (size_t)(j0 + c) * ldb);
         for (int i = lane; i < pm; i += 32) dst[i] = pan[i + (size_t)c * ldp];
@@ -253,6 +257,25 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
         }
       __threadfence();
       __syncthreads();
+      if (pend < plast) {  // the part's block reflector on the rest of the panel
+        const T* Tm = Tout + (size_t)j0 * kNB + (j0 - pstart);
+        if (unit)
+          dev::tile_left_qt<T, true>(R + j0 + (size_t)j0 * ldr, ldr, Tm, kNB, kb, 1, nullptr, 0,
+                                     R + j0 + (size_t)pend * ldr, ldr, m - j0, plast - pend, tile, 0);
+        else
+          dev::tile_left_qt<T, true>(B + (size_t)j0 * ldb, ldb, Tm, kNB, kb, 0, R + j0 + (size_t)pend * ldr, ldr,
+                                     B + (size_t)pend * ldb, ldb, m, plast - pend, tile, 0);
+      }
+     }
+     if (pw < pkb) {  // T of the whole panel: the blocks between the parts
+      if (unit)
+        dev::panel_t(R + pstart + (size_t)pstart * ldr, ldr, m - pstart, pkb, 1, lt + pstart,
+                     Tout + (size_t)pstart * kNB, kNB, tmp);
+      else
+        dev::panel_t(B + (size_t)pstart * ldb, ldb, m, pkb, 0, lt + pstart, Tout + (size_t)pstart * kNB, kNB, tmp);
+      __threadfence();
+      __syncthreads();
+     }
     } else if (owns(j0, rank, cs)) {
       for (int j = j0; j < pend; ++j) {
         const int vlen = unit ? (m - j - 1) : m;
@@ -326,7 +349,7 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
 // tiled apply's scratch; vmax rows).
 template <typename T, bool kStage>
 __global__ void __launch_bounds__(kThreads, 2) k_elim(const ElimTask* __restrict__ tasks, const ElimOut* __restrict__ outs,
-                                                   int cs, int vmax, int* status) {
+                                                   int cs, int vmax, int pw, int* status) {
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);
   const ElimTask t = tasks[blockIdx.x / cs];
@@ -337,11 +360,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_elim(const ElimTask* __restrict
   T* tile = vb + vmax;
   T* pan = kStage ? tile : nullptr;
   dist_qr<T>(as<T>(t.S), t.n, nullptr, 0, t.n, t.n, 1, as<T>(t.T), as<T>(t.tau), lt, vb, red, tmp, tile, cs, status,
-             pan, vmax);
+             pan, vmax, pw);
   for (int o = t.out_begin; o < t.out_end; ++o) {
     const ElimOut e = outs[o];
     dist_qr<T>(as<T>(t.S), t.n, as<T>(e.B), e.m, e.m, t.n, 0, as<T>(e.T), as<T>(t.tau), lt, vb, red, tmp, tile,
-               cs, status, pan, vmax);
+               cs, status, pan, vmax, pw);
   }
 }
 
@@ -349,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_elim(const ElimTask* __restrict
 // that the step a cluster waits for is held by a running one.
 template <typename T, bool kStage>
 __global__ void __launch_bounds__(kThreads, 2) k_elim_pipe(const ElimStep* __restrict__ steps, int cs, int nmax,
-                                                        int vmax, int* ticket, int* prog, int* status) {
+                                                        int vmax, int pw, int* ticket, int* prog, int* status) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int s_step;
   T* sm = reinterpret_cast<T*>(smraw);
@@ -372,13 +395,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_elim_pipe(const ElimStep* __res
   if (t.out >= 0) link.out = prog + t.out;
   T* B = as<T>(t.B);
   dist_qr<T>(as<T>(t.S), t.n, B, t.m, B ? t.m : t.n, t.n, B ? 0 : 1, as<T>(t.T), as<T>(t.tau), lt, vb, red, tmp, tile,
-             cs, status, kStage ? tile : nullptr, vmax, link);
+             cs, status, kStage ? tile : nullptr, vmax, pw, link);
 }
 
 // kStage: panels factored in shared memory (nmax rows), as in k_elim.
 template <typename T, bool kStage>
 __global__ void __launch_bounds__(kThreads, 2) k_scale(const ScaleTask* __restrict__ tasks, int cs, int nmax,
-                                                    int* status) {
+                                                    int pw, int* status) {
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);
   const ScaleTask t = tasks[blockIdx.x / cs];
@@ -388,7 +411,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_scale(const ScaleTask* __restri
   T* vb = lt + nmax;
   T* tile = vb + nmax;
   dist_qr<T>(as<T>(t.S), t.n, nullptr, 0, t.n, t.n, 1, as<T>(t.T), as<T>(t.tau), lt, vb, red, tmp, tile, cs,
-             status, kStage ? tile : nullptr, nmax);
+             status, kStage ? tile : nullptr, nmax, pw);
 }
 
 // ------------------------------------------------------------ chunked applies
@@ -971,7 +994,7 @@ __global__ void __launch_bounds__(kThreads) k_rrqr_assemble(const RrqrSrc* __res
 // aliasing the basis tiles; mmax rows).
 template <bool kStage>
 __global__ void __launch_bounds__(kThreads, 2) k_selected_qr(const RrqrTask* __restrict__ tasks, int cs, int mmax,
-                                                          int nmax, int rt) {
+                                                          int nmax, int rt, int pw) {
   extern __shared__ double sm[];
   const RrqrTask t = tasks[blockIdx.x / cs];
   const int rank = crank(cs);
@@ -996,7 +1019,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_selected_qr(const RrqrTask* __r
   }
   __syncthreads();
   dist_qr<double>(t.V, m, nullptr, 0, m, rk, 1, t.T, t.tau, lt, vb, red, tmp, Qt, cs, nullptr,
-                  kStage ? Qt : nullptr, mmax);
+                  kStage ? Qt : nullptr, mmax, pw);
   if (!t.Qc) return;
   // R(l, j) = V[l + j m] for l <= j, written by the owners of column j
   auto R = [&](int l, int j) { return __ldcg(t.V + l + (size_t)j * m); };
@@ -1264,13 +1287,21 @@ cudaError_t launch_permute(int n, const int* perm, const double* src, double* ds
 
 // Shared memory of a dist_qr kernel whose panels are factored in shared
 // memory: `head` bytes, then one region that serves as the tiled apply's
-// scratch and as the panel buffer (rows x kNB plus a kNB x kNB block); 0
-// when that does not fit (the kernel then factors panels in global memory).
+// scratch and as the panel buffer (rows x pw plus kPanExtra), for the widest
+// parts of a panel that fit (32, 16 or 8 columns).  0 bytes when not even 8
+// columns fit (the kernel then factors panels in global memory).
+struct StagePlan {
+  size_t bytes = 0;
+  int pw = kNB;
+};
 template <typename T>
-size_t staged_panel_bytes(size_t head, int rows) {
-  const size_t panel = ((size_t)rows * kNB + kPanExtra) * sizeof(T);
-  const size_t region = std::max(smem_bytes(kWcap), panel);
-  return head + region + 1024 <= kSmemMax ? head + region : 0;
+StagePlan staged_panel(size_t head, int rows, size_t other_bytes = 0) {
+  for (int pw = kNB; pw >= 8; pw /= 2) {
+    const size_t panel = ((size_t)rows * pw + kPanExtra) * sizeof(T);
+    const size_t region = std::max(std::max(smem_bytes(kWcap), panel), other_bytes);
+    if (head + region + 1024 <= kSmemMax) return {head + region, pw};
+  }
+  return {};
 }
 
 cudaError_t launch_elim(const ElimTask* t, const ElimOut* o, int ntasks, int cs, int nmax, int vmax,
@@ -1279,23 +1310,14 @@ cudaError_t launch_elim(const ElimTask* t, const ElimOut* o, int ntasks, int cs,
   if (ntasks <= 0) return cudaSuccess;
   vmax = std::max(vmax, 1);
   const size_t head = smem_bytes(kRed + kNB + (size_t)nmax + (size_t)vmax);
-  if (g_fp32) {
-    const size_t bs = staged_panel_bytes<float>(head, vmax);
-    if (bs) {
-      if (cudaError_t e = prep(k_elim<float, true>, bs)) return e;
-      return launch_clustered(k_elim<float, true>, ntasks, cs, bs, st, t, o, cs, vmax, g_status);
-    }
-    if (cudaError_t e = prep(k_elim<float, false>, head + smem_bytes(kWcap))) return e;
-    return launch_clustered(k_elim<float, false>, ntasks, cs, head + smem_bytes(kWcap), st, t, o, cs, vmax,
-                            g_status);
-  }
-  const size_t bs = staged_panel_bytes<double>(head, vmax);
-  if (bs) {
-    if (cudaError_t e = prep(k_elim<double, true>, bs)) return e;
-    return launch_clustered(k_elim<double, true>, ntasks, cs, bs, st, t, o, cs, vmax, g_status);
-  }
-  if (cudaError_t e = prep(k_elim<double, false>, head + smem_bytes(kWcap))) return e;
-  return launch_clustered(k_elim<double, false>, ntasks, cs, head + smem_bytes(kWcap), st, t, o, cs, vmax, g_status);
+  const StagePlan p = g_fp32 ? staged_panel<float>(head, vmax) : staged_panel<double>(head, vmax);
+  const size_t b = p.bytes ? p.bytes : head + smem_bytes(kWcap);
+  auto go = [&](auto kern) {
+    if (cudaError_t e = prep(kern, b)) return e;
+    return launch_clustered(kern, ntasks, cs, b, st, t, o, cs, vmax, p.pw, g_status);
+  };
+  if (g_fp32) return p.bytes ? go(k_elim<float, true>) : go(k_elim<float, false>);
+  return p.bytes ? go(k_elim<double, true>) : go(k_elim<double, false>);
 }
 
 cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, int vmax, int* ticket, int* prog,
@@ -1304,13 +1326,14 @@ cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, in
   if (nsteps <= 0) return cudaSuccess;
   vmax = std::max(vmax, 1);
   const size_t head = smem_bytes(kRed + kNB + (size_t)nmax + (size_t)vmax);
-  auto go = [&](auto kern, size_t b) {
+  const StagePlan p = g_fp32 ? staged_panel<float>(head, vmax) : staged_panel<double>(head, vmax);
+  const size_t b = p.bytes ? p.bytes : head + smem_bytes(kWcap);
+  auto go = [&](auto kern) {
     if (cudaError_t e = prep(kern, b)) return e;
-    return launch_clustered(kern, nsteps, cs, b, st, t, cs, nmax, vmax, ticket, prog, g_status);
+    return launch_clustered(kern, nsteps, cs, b, st, t, cs, nmax, vmax, p.pw, ticket, prog, g_status);
   };
-  const size_t bs = g_fp32 ? staged_panel_bytes<float>(head, vmax) : staged_panel_bytes<double>(head, vmax);
-  if (g_fp32) return bs ? go(k_elim_pipe<float, true>, bs) : go(k_elim_pipe<float, false>, head + smem_bytes(kWcap));
-  return bs ? go(k_elim_pipe<double, true>, bs) : go(k_elim_pipe<double, false>, head + smem_bytes(kWcap));
+  if (g_fp32) return p.bytes ? go(k_elim_pipe<float, true>) : go(k_elim_pipe<float, false>);
+  return p.bytes ? go(k_elim_pipe<double, true>) : go(k_elim_pipe<double, false>);
 }
 
 cudaError_t launch_scale(const ScaleTask* t, int ntasks, int cs, int nmax, cudaStream_t st) {
@@ -1318,22 +1341,14 @@ cudaError_t launch_scale(const ScaleTask* t, int ntasks, int cs, int nmax, cudaS
   if (ntasks <= 0) return cudaSuccess;
   nmax = std::max(nmax, 1);
   const size_t head = smem_bytes(kRed + kNB + 2 * (size_t)nmax);
-  if (g_fp32) {
-    const size_t bs = staged_panel_bytes<float>(head, nmax);
-    if (bs) {
-      if (cudaError_t e = prep(k_scale<float, true>, bs)) return e;
-      return launch_clustered(k_scale<float, true>, ntasks, cs, bs, st, t, cs, nmax, g_status);
-    }
-    if (cudaError_t e = prep(k_scale<float, false>, head + smem_bytes(kWcap))) return e;
-    return launch_clustered(k_scale<float, false>, ntasks, cs, head + smem_bytes(kWcap), st, t, cs, nmax, g_status);
-  }
-  const size_t bs = staged_panel_bytes<double>(head, nmax);
-  if (bs) {
-    if (cudaError_t e = prep(k_scale<double, true>, bs)) return e;
-    return launch_clustered(k_scale<double, true>, ntasks, cs, bs, st, t, cs, nmax, g_status);
-  }
-  if (cudaError_t e = prep(k_scale<double, false>, head + smem_bytes(kWcap))) return e;
-  return launch_clustered(k_scale<double, false>, ntasks, cs, head + smem_bytes(kWcap), st, t, cs, nmax, g_status);
+  const StagePlan p = g_fp32 ? staged_panel<float>(head, nmax) : staged_panel<double>(head, nmax);
+  const size_t b = p.bytes ? p.bytes : head + smem_bytes(kWcap);
+  auto go = [&](auto kern) {
+    if (cudaError_t e = prep(kern, b)) return e;
+    return launch_clustered(kern, ntasks, cs, b, st, t, cs, nmax, p.pw, g_status);
+  };
+  if (g_fp32) return p.bytes ? go(k_scale<float, true>) : go(k_scale<float, false>);
+  return p.bytes ? go(k_scale<double, true>) : go(k_scale<double, false>);
 }
 
 cudaError_t launch_update(const UpdTask* t, const UpdOp* o, int ntasks, cudaStream_t st) {
@@ -1454,27 +1469,19 @@ cudaError_t launch_rrqr_assemble(const RrqrSrc* s, int nsrc, cudaStream_t st) {
 
 int selected_qr_rows(int nmax) { return std::max(1, std::min(32, 12288 / (std::max(nmax, 1) + 1))); }
 
-// stage: with room for the QR's staged panel (0 when that does not fit)
-size_t selected_qr_smem(int mmax, int nmax, bool stage) {
-  const int rt = selected_qr_rows(nmax);
-  mmax = std::max(mmax, 1);
-  size_t region = std::max((size_t)rt * (std::max(nmax, 1) + 1) + 32 * 33, (size_t)kWcap);
-  if (stage) region = std::max(region, (size_t)mmax * kNB + kPanExtra);
-  const size_t b = smem_bytes(kRed + kNB + (size_t)std::max(nmax, 1) + (size_t)mmax + region);
-  return !stage || b + 1024 <= kSmemMax ? b : 0;
-}
-
 cudaError_t launch_selected_qr(const RrqrTask* t, int ntasks, int cs, int mmax, int nmax, cudaStream_t st) {
   if (cudaError_t pre = begin("launch_selected_qr")) return pre;
   if (ntasks <= 0) return cudaSuccess;
   const int mm = std::max(mmax, 1), nn = std::max(nmax, 1), rt = selected_qr_rows(nmax);
-  if (const size_t bs = selected_qr_smem(mmax, nmax, true)) {
-    if (cudaError_t e = prep(k_selected_qr<true>, bs)) return e;
-    return launch_clustered(k_selected_qr<true>, ntasks, cs, bs, st, t, cs, mm, nn, rt);
-  }
-  const size_t b = selected_qr_smem(mmax, nmax, false);
-  if (cudaError_t e = prep(k_selected_qr<false>, b)) return e;
-  return launch_clustered(k_selected_qr<false>, ntasks, cs, b, st, t, cs, mm, nn, rt);
+  const size_t head = smem_bytes(kRed + kNB + (size_t)nn + (size_t)mm);
+  const size_t basis = smem_bytes((size_t)rt * (nn + 1) + 32 * 33);
+  const StagePlan p = staged_panel<double>(head, mm, basis);
+  const size_t b = p.bytes ? p.bytes : head + std::max(basis, smem_bytes(kWcap));
+  auto go = [&](auto kern) {
+    if (cudaError_t e = prep(kern, b)) return e;
+    return launch_clustered(kern, ntasks, cs, b, st, t, cs, mm, nn, rt, p.pw);
+  };
+  return p.bytes ? go(k_selected_qr<true>) : go(k_selected_qr<false>);
 }
 
 cudaError_t launch_merge(const MergeTask* t, int ntasks, cudaStream_t st) {

@@ -72,9 +72,6 @@ cudaError_t launch_pivots(const PivotTask* t, int ntasks, int cs, size_t smem, b
 // V / T / tau and (where the task has a Qc) the orthonormal basis
 // Qc = C_sel R^{-1}; cs-CTA clusters, tasks of at most mmax rows and nmax
 // selected columns.
-// Shared memory of k_selected_qr; stage: with room for the QR's panels in
-// shared memory (0 when that does not fit).
-size_t selected_qr_smem(int mmax, int nmax, bool stage);
 cudaError_t launch_selected_qr(const RrqrTask* t, int ntasks, int cs, int mmax, int nmax, cudaStream_t st);
 cudaError_t launch_merge(const MergeTask* t, int ntasks, cudaStream_t st);
 // Row scaling / left compression (launch_edge kind 0) of FP32 chunks whose
