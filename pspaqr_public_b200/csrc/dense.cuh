@@ -203,421 +203,246 @@ __device__ void panel_t_warp(const T* V, int ldv, int m, int kb, int unit, const
 
 
 // ---------------------------------------------------------------- tiled matrix applies
-// Register-tiled block reflector applies on matrices: rows are streamed
-// through shared memory in tiles of kRT; the left apply keeps two tiles in
-// flight (the next tile's global loads are issued before the current tile's
-// products).  `sm` holds kTileSmem elements (2 kTileSmem for T = float).
 constexpr int kNC = 64;   // columns (rows for right applies) per pass
 constexpr int kRT = 32;   // rows (columns) per shared-memory tile
-// Row strides of the V and C tiles of the left apply: 16-byte aligned rows
-// whose starts fall on distinct 16-byte bank groups for 8 consecutive rows.
-template <typename T>
-__host__ __device__ constexpr int tile_lv() { return kNB + (sizeof(T) == 4 ? 4 : 2); }
-template <typename T>
-__host__ __device__ constexpr int tile_lc() { return kNC + (sizeof(T) == 4 ? 4 : 2); }
-constexpr int kTileSmem = 2 * kRT * tile_lv<float>() + 2 * kRT * tile_lc<float>() + kNB * kNC;
+constexpr int kLdV = 40;  // column stride of the V, T and left C tiles (8 mod 16: 16-byte fragment
+                          // loads of two columns a quarter-warp fall on distinct banks)
+constexpr int kLdR = 66;  // row stride of the right C tiles (2 mod 8: 8-byte fragments, likewise)
+constexpr int kTileV = kNB * kLdV, kTileC = kNC * kLdV;
+static_assert(kRT * kLdR <= kTileC, "right tiles");
+// Shared memory (doubles) of mma_apply with `stages` tiles of V and C.
+__host__ __device__ constexpr int tile_smem(int stages) { return stages * (kTileV + kTileC) + kTileV + 2; }
+constexpr int kTileSmem = tile_smem(2);
 
-// Load through L2 (kCg: data written by another CTA of the cluster) or as is.
+// Load through L2 (kCg: data written by another CTA) or as is.
 template <bool kCg, typename T>
 __device__ __forceinline__ T ld_v(const T* p) {
   if (kCg) return __ldcg(p);
   return *p;
 }
 
-// C (m x nc <= kNC) <- Q^T C with one panel: unit = 1: V unit lower trapezoidal
-// (geqrt / RRQR reflectors), A unused; unit = 0: pentagonal tpqrt panel,
-// [A (kb x nc); C] <- Q^T [A; C] with V full (m x kb).  Column c of A and C
-// is column c + (c / kNB) * cgap of the arrays (cgap > 0: the column panels
-// a CTA owns in a cluster-distributed factorization).  kCg: V, T and A are
-// read through L2 (other CTAs write them).
-template <typename T, bool kCg = false>
-__device__ void tile_left_qt(const T* V, int ldv, const T* Tm, int ldt, int kb, int unit, T* A, int lda,
-                             T* C, int ldc, int m, int nc, T* sm, int cgap = 0) {
+// One panel of k <= 32 reflectors on a block of kNC vectors of length m:
+//   left  (kRight = false): the vectors are columns of C, C <- Q^T C;
+//   right (kRight = true):  the vectors are rows of C,    C <- C Q.
+// Both are w = c V (+ a), w <- w T, c -= w V^T (a -= w) for every vector c.
+// unit = 1: V unit lower trapezoidal (geqrt / RRQR reflectors), A unused;
+// unit = 0 (left only): pentagonal tpqrt panel, [A (kb x nc); C] <- Q^T [A; C]
+// with V full (m x kb).  Column c of A and C is column c + (c / kNB) * cgap of
+// the arrays (cgap > 0: the column panels a CTA owns in a cluster-distributed
+// factorization).  kCg: V, T and A are read through L2 (other CTAs write them).
+//
+// All three products run on FP64 mma (float blocks are widened when they are
+// staged and rounded once when they are stored: more accurate than FP32 sums,
+// and faster than the FP32 pipes ran here).  Warp w owns vectors 8 w .. 8 w + 7
+// from start to end, so that w never leaves its registers: the accumulators of
+// one product are the A fragments of the next when fragment lane fn of the B
+// operand takes column (fn >> 1) + 4 (fn & 1) (`perm`), which makes accumulator
+// 2 fk + e column fk + 4 e.  Only tiles of V (and C) are shared, one barrier a
+// tile, `stages` tiles in shared memory; the second pass runs backwards, over the
+// tiles that are still there first.  Before, with W, the partial sums of the row
+// sets, T and W2 exchanged through shared memory on the FP64 (FP32) pipes, a
+// panel reached 7 % of the FP64 peak (64^3 FP64, trailing updates).
+template <typename T, bool kCg, bool kRight>
+__device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int unit, T* A, int lda, T* C, int ldc,
+                          int m, int nc, double* sm, int stages, int cgap) {
   static_assert(kThreads == 256 && kNB == 32 && kNC == 64 && kRT == 32, "tile shapes");
-  constexpr int kLV = tile_lv<T>(), kLC = tile_lc<T>();
-  // FP32 callers pass 2 kTileSmem elements (kTileSmem doubles): the partial
-  // sums and W2 then go past the tile buffers
-  constexpr bool kKeep = sizeof(T) == 4;
-  static_assert(!kKeep || 3 * kNB * kNC + kNB * kNC <= kTileSmem, "FP32 park and W2 areas");
-  constexpr int kVS = kRT * kLV, kCS = kRT * kLC;
-  T* sV0 = sm;               // two [kRT][kLV] tiles of V
-  T* sC0 = sV0 + 2 * kVS;    // two [kRT][kLC] tiles of C
-  T* sW = sC0 + 2 * kCS;     // [kNB][kNC]: W, then the partial sums' landing area is sV0..sC0
-  const int t = threadIdx.x;
+  // 16-byte fragments; a float caller's scratch starts on any 4 bytes
+  sm = reinterpret_cast<double*>((reinterpret_cast<size_t>(sm) + 15) & ~(size_t)15);
+  double* sT = sm;
+  double* sV0 = sT + kTileV;
+  double* sC0 = sV0 + stages * kTileV;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int fn = lane >> 2, fk = lane & 3, perm = (fn >> 1) + 4 * (fn & 1);
   auto col = [&](int c) { return (size_t)(c + (c / kNB) * cgap); };
-  // global loads of one tile: lane = row (a warp reads 32 consecutive rows of
-  // one column: coalesced), warp w = columns kSV w .. (V) and kSC w .. (C), so
-  // that a thread stashes one row segment with 16-byte stores
-  constexpr int kSV = kRT * kNB / kThreads, kSC = kRT * kNC / kThreads;
-  const int lr = t & (kRT - 1), lw = t / kRT;
+  // staging: V by (row = lane, four columns a warp); left C by (row = lane, the
+  // warp's eight columns), right C by (vector = t % 64, columns t / 64 + 4 q): a
+  // warp reads runs of 32 elements
+  constexpr int kSV = kNB / kWarps, kSC = kRT * kNC / kThreads;
   T rv[kSV], rc[kSC];
-  auto vload = [&](int r0) {
-    const int gr = r0 + lr;
+  const int cv = t % kNC, cr = t / kNC;
+  auto load = [&](int tt) {
+    const int gr = tt * kRT + lane;
 #pragma unroll
     for (int q = 0; q < kSV; ++q) {
-      const int i = lw * kSV + q;
-      T v = 0.0;
+      const int i = warp * kSV + q;
+      T v = 0;
       if (gr < m && i < kb)
-        v = unit ? (gr == i ? (T)1.0 : (gr < i ? (T)0.0 : ld_v<kCg>(V + gr + (size_t)i * ldv)))
-                 : ld_v<kCg>(V + gr + (size_t)i * ldv);
+        v = unit && gr <= i ? (gr == i ? (T)1 : (T)0) : ld_v<kCg>(V + gr + (size_t)i * ldv);
       rv[q] = v;
     }
-  };
-  auto vstash = [&](int b) {
-    T* d = sV0 + b * kVS + lr * kLV + lw * kSV;
-#pragma unroll
-    for (int q = 0; q < kSV; ++q) d[q] = rv[q];
-  };
-  auto cload = [&](int r0) {
-    const int gr = r0 + lr;
 #pragma unroll
     for (int q = 0; q < kSC; ++q) {
-      const int c = lw * kSC + q;
-      rc[q] = (gr < m && c < nc) ? C[gr + col(c) * ldc] : (T)0.0;
+      if (kRight) {
+        const int r = tt * kRT + cr + 4 * q;
+        rc[q] = r < m && cv < nc ? C[cv + (size_t)r * ldc] : (T)0;
+      } else {
+        const int c = warp * kSC + q;
+        rc[q] = gr < m && c < nc ? C[gr + col(c) * ldc] : (T)0;
+      }
     }
   };
-  auto cstash = [&](int b) {
-    T* d = sC0 + b * kCS + lr * kLC + lw * kSC;
+  auto stash = [&](int tt) {
+    double* dv = sV0 + (tt % stages) * kTileV;
+    double* dc = sC0 + (tt % stages) * kTileC;
 #pragma unroll
-    for (int q = 0; q < kSC; ++q) d[q] = rc[q];
+    for (int q = 0; q < kSV; ++q) dv[(warp * kSV + q) * kLdV + lane] = (double)rv[q];
+#pragma unroll
+    for (int q = 0; q < kSC; ++q) {
+      if (kRight) dc[(cr + 4 * q) * kLdR + cv] = (double)rc[q];
+      else dc[(warp * kSC + q) * kLdV + lane] = (double)rc[q];
+    }
   };
   const int ntile = (m + kRT - 1) / kRT;
-  // T (and the top block A of a pentagonal panel) are read now, used after
-  // the products: element idx = t + kThreads q, T(l = idx & 31, i = idx >> 5)
-  // and A(i = idx & 31, c = idx >> 5)
-  constexpr int kST = kNB * kNB / kThreads, kSA = kNB * kNC / kThreads;
-  T rt[kST], ra[kSA];
-#pragma unroll
-  for (int q = 0; q < kST; ++q) {
-    const int idx = t + q * kThreads, l = idx & (kNB - 1), i = idx / kNB;
-    rt[q] = (l <= i && i < kb) ? ld_v<kCg>(Tm + l + (size_t)i * ldt) : (T)0.0;
-  }
-#pragma unroll
-  for (int q = 0; q < kSA; ++q) {
-    const int idx = t + q * kThreads, i = idx & (kNB - 1), c = idx / kNB;
-    ra[q] = (!unit && i < kb && c < nc) ? ld_v<kCg>(A + i + col(c) * lda) : (T)0.0;
-  }
-  // ---- W = V^T C.  A thread accumulates W(i0:i0+kIW, c0:c0+4); the kSets
-  // row sets of kTPO threads each take kRows consecutive rows of every tile
+  const int c = 8 * warp + fn;  // own vector
+  const bool have = c < nc;
+  if (ntile > 0) load(0);
+  // T, zero below its diagonal and past kb; the top block A
   {
-    constexpr int kIW = sizeof(T) == 4 ? 8 : 4;           // reflectors per thread
-    constexpr int kTPO = (kNB / kIW) * (kNC / 4);          // threads per set
-    constexpr int kSets = kThreads / kTPO, kRows = kRT / kSets;
-    const int set = t / kTPO, i0 = ((t % kTPO) / (kNC / 4)) * kIW, c0 = (t % (kNC / 4)) * 4;
-    T acc[kIW][4];
+    T rt[kNB * kNB / kThreads];
 #pragma unroll
-    for (int a = 0; a < kIW; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-    vload(0);
-    cload(0);
-    vstash(0);
-    cstash(0);
-    __syncthreads();
-    for (int tt = 0; tt < ntile; ++tt) {
-      const int b = tt & 1;
-      const bool more = tt + 1 < ntile;
-      if (more) {
-        vload((tt + 1) * kRT);
-        cload((tt + 1) * kRT);
-      }
-      const T* sV = sV0 + b * kVS + (set * kRows) * kLV + i0;
-      const T* sC = sC0 + b * kCS + (set * kRows) * kLC + c0;
-#pragma unroll 8
-      for (int r = 0; r < kRows; ++r) {
-        T v[kIW], c[4];
-#pragma unroll
-        for (int a = 0; a < kIW; ++a) v[a] = sV[r * kLV + a];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) c[q] = sC[r * kLC + q];
-#pragma unroll
-        for (int a = 0; a < kIW; ++a)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[a][q] += v[a] * c[q];
-      }
-      if (more) {
-        vstash(b ^ 1);
-        cstash(b ^ 1);
-      }
-      __syncthreads();
+    for (int q = 0; q < kNB * kNB / kThreads; ++q) {
+      const int l = lane, j = warp + q * kWarps;
+      rt[q] = l <= j && j < kb ? ld_v<kCg>(Tm + l + (size_t)j * ldt) : (T)0;
     }
-    // sets 1.. park their partial sums in the tile buffers (FP32: past them,
-    // so that a single tile stays staged for the update), set 0 adds them in
-    // set order
-    static_assert((kSets - 1) * kNB * kNC <= 2 * kVS + 2 * kCS, "park area");
-    T* park = kKeep ? sm + kTileSmem : sV0;
-    if (set > 0)
 #pragma unroll
-      for (int a = 0; a < kIW; ++a)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) park[(set - 1) * kNB * kNC + (i0 + a) * kNC + c0 + q] = acc[a][q];
-    __syncthreads();
-    if (set == 0)
-#pragma unroll
-      for (int a = 0; a < kIW; ++a)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int i = i0 + a, c = c0 + q;
-          T w = acc[a][q];
-#pragma unroll
-          for (int p = 0; p < kSets - 1; ++p) w += park[p * kNB * kNC + i * kNC + c];
-          sW[i * kNC + c] = w;
-        }
+    for (int q = 0; q < kNB * kNB / kThreads; ++q) sT[(warp + q * kWarps) * kLdV + lane] = (double)rt[q];
   }
-  __syncthreads();
-  // T to shared memory (the tail of the tile buffers), A into W
-  T* sT = sV0 + 2 * kVS + 2 * kCS - kNB * (kNB + 1);  // sT[l * (kNB+1) + i] = T(l, i)
+  double w[4][2], a[4][2];
 #pragma unroll
-  for (int q = 0; q < kST; ++q) {
-    const int idx = t + q * kThreads;
-    sT[(idx & (kNB - 1)) * (kNB + 1) + idx / kNB] = rt[q];
-  }
-  if (!unit)
+  for (int b = 0; b < 4; ++b)
 #pragma unroll
-    for (int q = 0; q < kSA; ++q) {
-      const int idx = t + q * kThreads;
-      sW[(idx & (kNB - 1)) * kNC + idx / kNB] += ra[q];
+    for (int e = 0; e < 2; ++e) {
+      const int i = 8 * b + fk + 4 * e;
+      a[b][e] = !unit && i < kb && have ? (double)ld_v<kCg>(A + i + col(c) * lda) : 0.0;
+      w[b][e] = a[b][e];
     }
+  // ---- w = c V (+ a)
+  if (ntile > 0) stash(0);
   __syncthreads();
-  // ---- W2 = T^T W (T upper triangular: W2(i) = sum_{l <= i} T(l, i) W(l))
-  T* sW2 = kKeep ? sm + kTileSmem + (kThreads / ((kNB / 8) * (kNC / 4)) - 1) * kNB * kNC : sV0;
-  static_assert(kNB * kNC <= 2 * kVS + 2 * kCS - kNB * (kNB + 1), "W2 and T areas");
-  for (int idx = t; idx < kNB * kNC; idx += kThreads) {
-    const int i = idx / kNC, c = idx % kNC;
-    T s = 0.0;
-    if (i < kb)
-      for (int l = 0; l <= i; ++l) s += sT[l * (kNB + 1) + i] * sW[l * kNC + c];
-    sW2[i * kNC + c] = s;
-  }
-  __syncthreads();
-  if (!unit)
-    for (int idx = t; idx < kb * nc; idx += kThreads) {
-      const int i = idx % kb, c = idx / kb;
-      A[i + col(c) * lda] -= sW2[i * kNC + c];
-    }
-  // ---- C -= V W2.  A thread keeps W2(:, its kCW columns) in registers and
-  // owns kRW rows of each tile (a warp shares its rows: V rows are broadcast)
-  constexpr int kCW = sizeof(T) == 4 ? 2 : 1;     // columns per thread
-  constexpr int kRW = kRT * kNC / kThreads / kCW;  // rows per thread
-  const int cq = (t % (kNC / kCW)) * kCW, rq = (t / (kNC / kCW)) * kRW;
-  T w2[kNB][kCW];
-#pragma unroll
-  for (int i = 0; i < kNB; ++i)
-#pragma unroll
-    for (int q = 0; q < kCW; ++q) w2[i][q] = sW2[i * kNC + cq + q];
-  __syncthreads();
-  if (!(kKeep && ntile == 1)) {  // a single FP32 tile is still staged in buffer 0
-    vload(0);
-    cload(0);
-    vstash(0);
-    cstash(0);
-    __syncthreads();
-  }
   for (int tt = 0; tt < ntile; ++tt) {
-    const int b = tt & 1, r0 = tt * kRT;
     const bool more = tt + 1 < ntile;
-    if (more) {
-      vload(r0 + kRT);
-      cload(r0 + kRT);
-    }
-    const T* sV = sV0 + b * kVS;
-    T* sC = sC0 + b * kCS;
+    if (more) load(tt + 1);
+    const double* sV = sV0 + (tt % stages) * kTileV;
+    const double* sC = sC0 + (tt % stages) * kTileC;
 #pragma unroll
-    for (int r = 0; r < kRW; ++r) {
-      const T* vr = sV + (rq + r) * kLV;
-      T u[kCW];
-#pragma unroll
-      for (int q = 0; q < kCW; ++q) u[q] = 0.0;
-#pragma unroll
-      for (int i = 0; i < kNB; ++i) {
-        const T a = vr[i];
-#pragma unroll
-        for (int q = 0; q < kCW; ++q) u[q] += a * w2[i][q];
+    for (int rr = 0; rr < kRT; rr += 8) {
+      double2 x;
+      if (kRight) {
+        x.x = sC[(rr + 2 * fk) * kLdR + c];
+        x.y = sC[(rr + 2 * fk + 1) * kLdR + c];
+      } else {
+        x = *reinterpret_cast<const double2*>(sC + c * kLdV + rr + 2 * fk);
       }
+      double2 v[4];
 #pragma unroll
-      for (int q = 0; q < kCW; ++q) sC[(rq + r) * kLC + cq + q] -= u[q];
+      for (int b = 0; b < 4; ++b) v[b] = *reinterpret_cast<const double2*>(sV + (8 * b + perm) * kLdV + rr + 2 * fk);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], x.x, v[b].x);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], x.y, v[b].y);
     }
+    // with two or more stages the next tile's buffer was last read a barrier ago
+    if (more) stash(tt + 1);
     __syncthreads();
-    // the updated tile back to global memory, coalesced
-    if (r0 + lr < m)
+  }
+  // ---- w <- w T (upper triangular)
+  double w2[4][2];
 #pragma unroll
-      for (int q = 0; q < kSC; ++q) {
-        const int c = lw * kSC + q;
-        if (c < nc) C[(r0 + lr) + col(c) * ldc] = sC[lr * kLC + c];
+  for (int j = 0; j < 4; ++j) {
+    w2[j][0] = w2[j][1] = 0.0;
+#pragma unroll
+    for (int b = 0; b <= j; ++b)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) dmma(w2[j][0], w2[j][1], w[b][e], sT[(8 * j + perm) * kLdV + 8 * b + fk + 4 * e]);
+  }
+  if (!unit)
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int i = 8 * b + fk + 4 * e;
+        if (i < kb && have) A[i + col(c) * lda] = (T)(a[b][e] - w2[b][e]);
       }
-    if (more) {
-      vstash(b ^ 1);
-      cstash(b ^ 1);
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) w2[b][e] = -w2[b][e];
+  // ---- c -= w V^T, last tiles first
+  const int resident = max(0, ntile - stages);  // tiles from here on are still staged
+  for (int tt = ntile - 1; tt >= 0; --tt) {
+    // the tile `stages` before the one just done takes its place
+    const int in = tt + 1 - stages;
+    const bool more = tt + 1 < ntile && in >= 0 && in < resident;
+    if (more) load(in);
+    const double* sV = sV0 + (tt % stages) * kTileV;
+    const double* sC = sC0 + (tt % stages) * kTileC;
+    double x[4][2];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (kRight) {
+        x[u][0] = sC[(8 * u + 2 * fk) * kLdR + c];
+        x[u][1] = sC[(8 * u + 2 * fk + 1) * kLdR + c];
+      } else {
+        const double2 y = *reinterpret_cast<const double2*>(sC + c * kLdV + 8 * u + 2 * fk);
+        x[u][0] = y.x;
+        x[u][1] = y.y;
+      }
     }
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          dmma(x[u][0], x[u][1], w2[b][e], sV[(8 * b + fk + 4 * e) * kLdV + 8 * u + fn]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = tt * kRT + 8 * u + 2 * fk + e;
+        if (r < m && have) C[kRight ? c + (size_t)r * ldc : r + col(c) * ldc] = (T)x[u][e];
+      }
+    if (more) stash(in);
     __syncthreads();
   }
 }
 
-// C (m <= kNC rows x n) <- C (I - V T V^T) with one panel, V unit lower
-// trapezoidal (n x kb).  Column tiles of kRT stream through two shared
-// buffers: the next tile's global loads are issued before the current tile's
-// products.
-template <typename T>
-__device__ void tile_right_q(const T* V, int ldv, const T* Tm, int ldt, int kb, T* C, int ldc, int m,
-                             int n, T* sm) {
-  constexpr int kVS = kRT * (kNB + 1), kCS = kNC * (kRT + 1);
-  static_assert(2 * kVS + 2 * kCS + kNC * kNB <= kTileSmem, "right apply scratch");
-  T* sV0 = sm;               // two [kRT][kNB+1] tiles: V rows c0..c0+31
-  T* sC0 = sV0 + 2 * kVS;    // two [kNC][kRT+1] tiles: C(r, c0+c)
-  T* sW = sC0 + 2 * kCS;     // [kNC][kNB] W(r, i)
-  const int t = threadIdx.x;
-  constexpr int kSV = kRT * kNB / kThreads, kSC = kNC * kRT / kThreads;
-  T rv[kSV], rc[kSC];
-  auto vload = [&](int c0) {
-#pragma unroll
-    for (int q = 0; q < kSV; ++q) {
-      const int idx = t + q * kThreads, c = idx % kRT, i = idx / kRT, gc = c0 + c;
-      T v = 0.0;
-      if (gc < n && i < kb) v = gc == i ? (T)1.0 : (gc < i ? (T)0.0 : V[gc + (size_t)i * ldv]);
-      rv[q] = v;
-    }
-  };
-  auto vstash = [&](int b) {
-#pragma unroll
-    for (int q = 0; q < kSV; ++q) {
-      const int idx = t + q * kThreads;
-      sV0[b * kVS + (idx % kRT) * (kNB + 1) + idx / kRT] = rv[q];
-    }
-  };
-  auto cload = [&](int c0) {
-#pragma unroll
-    for (int q = 0; q < kSC; ++q) {
-      const int idx = t + q * kThreads, r = idx % kNC, c = idx / kNC;
-      rc[q] = (r < m && c0 + c < n) ? C[r + (size_t)(c0 + c) * ldc] : (T)0.0;
-    }
-  };
-  auto cstash = [&](int b) {
-#pragma unroll
-    for (int q = 0; q < kSC; ++q) {
-      const int idx = t + q * kThreads;
-      sC0[b * kCS + (idx % kNC) * (kRT + 1) + idx / kNC] = rc[q];
-    }
-  };
-  const int ntile = (n + kRT - 1) / kRT;
-  const int ti = t & 7, tr = t >> 3;  // i = ti*4..+3, r = tr*2..+1
-  T acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-  vload(0);
-  cload(0);
-  vstash(0);
-  cstash(0);
-  __syncthreads();
-  for (int tt = 0; tt < ntile; ++tt) {
-    const int b = tt & 1;
-    const bool more = tt + 1 < ntile;
-    if (more) {
-      vload((tt + 1) * kRT);
-      cload((tt + 1) * kRT);
-    }
-    const T* sV = sV0 + b * kVS;
-    const T* sC = sC0 + b * kCS;
-#pragma unroll 8
-    for (int c = 0; c < kRT; ++c) {
-      const T a0 = sC[(tr * 2) * (kRT + 1) + c], a1 = sC[(tr * 2 + 1) * (kRT + 1) + c];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const T v = sV[c * (kNB + 1) + ti * 4 + q];
-        acc[0][q] += a0 * v;
-        acc[1][q] += a1 * v;
-      }
-    }
-    if (more) {
-      vstash(b ^ 1);
-      cstash(b ^ 1);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int p = 0; p < 2; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) sW[(tr * 2 + p) * kNB + ti * 4 + q] = acc[p][q];
-  __syncthreads();
-  // W2 = W T (W2(r,i) = sum_{l <= i} W(r,l) T(l,i)), T staged in shared memory
-  T* sT = sC0;                 // [kNB][kNB+1]
-  T* sW2 = sC0 + kNB * (kNB + 1);  // [kNC][kNB]
-  for (int idx = t; idx < kNB * kNB; idx += kThreads) {
-    const int l = idx % kNB, i = idx / kNB;
-    sT[l * (kNB + 1) + i] = (l <= i && i < kb) ? Tm[l + (size_t)i * ldt] : (T)0.0;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int p = 0; p < 2; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = tr * 2 + p, i = ti * 4 + q;
-      T s = 0.0;
-      if (i < kb)
-        for (int l = 0; l <= i; ++l) s += sW[r * kNB + l] * sT[l * (kNB + 1) + i];
-      sW2[r * kNB + i] = s;
-    }
-  __syncthreads();
-  // C(r, c) -= sum_i W2(r, i) V(c, i): thread rows rr, rr+32, columns cc*4..+3
-  // of each tile; the next tile's V is loaded before the current products
-  const int rr = t & 31, cc = t >> 5;
-  vload(0);
-  vstash(0);
-  __syncthreads();
-  for (int tt = 0; tt < ntile; ++tt) {
-    const int b = tt & 1, c0 = tt * kRT;
-    const bool more = tt + 1 < ntile;
-    if (more) vload(c0 + kRT);
-    const T* sV = sV0 + b * kVS;
-    T u[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-#pragma unroll 8
-    for (int i = 0; i < kNB; ++i) {
-      const T w0 = sW2[rr * kNB + i], w1 = sW2[(rr + 32) * kNB + i];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const T v = sV[(cc * 4 + q) * (kNB + 1) + i];
-        u[0][q] += w0 * v;
-        u[1][q] += w1 * v;
-      }
-    }
-#pragma unroll
-    for (int p = 0; p < 2; ++p)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int r = rr + 32 * p, c = cc * 4 + q;
-        if (r < m && c0 + c < n) C[r + (size_t)(c0 + c) * ldc] -= u[p][q];
-      }
-    if (more) vstash(b ^ 1);
-    __syncthreads();
-  }
+// C (m x nc <= kNC) <- Q^T C with one panel (see mma_apply).
+template <typename T, bool kCg = false>
+__device__ void tile_left_qt(const T* V, int ldv, const T* Tm, int ldt, int kb, int unit, T* A, int lda, T* C, int ldc,
+                             int m, int nc, T* sm, int cgap = 0, int stages = 2) {
+  mma_apply<T, kCg, false>(V, ldv, Tm, ldt, kb, unit, A, lda, C, ldc, m, nc, reinterpret_cast<double*>(sm), stages, cgap);
 }
 
-// Panel loops of the tiled applies over k reflectors (T in kNB x k layout).
 template <typename T>
 __device__ void mat_apply_qt(const T* V, int ldv, const T* Tm, int k, T* C, int ldc, int m, int nc,
-                             T* sm) {
+                             T* sm, int stages) {
   for (int j0 = 0; j0 < k; j0 += kNB) {
     const int kb = (k - j0) < kNB ? (k - j0) : kNB;
     for (int c0 = 0; c0 < nc; c0 += kNC)
       tile_left_qt<T>(V + j0 + (size_t)j0 * ldv, ldv, Tm + (size_t)j0 * kNB, kNB, kb, 1, nullptr, 0,
-                   C + j0 + (size_t)c0 * ldc, ldc, m - j0, (nc - c0) < kNC ? (nc - c0) : kNC, sm);
+                   C + j0 + (size_t)c0 * ldc, ldc, m - j0, (nc - c0) < kNC ? (nc - c0) : kNC, sm, 0, stages);
   }
 }
 template <typename T>
 __device__ void mat_apply_tpqt(const T* V, int ldv, const T* Tm, int k, T* A, int lda, T* B,
-                               int ldb, int m, int nc, T* sm) {
+                               int ldb, int m, int nc, T* sm, int stages) {
   for (int j0 = 0; j0 < k; j0 += kNB) {
     const int kb = (k - j0) < kNB ? (k - j0) : kNB;
     for (int c0 = 0; c0 < nc; c0 += kNC)
       tile_left_qt(V + (size_t)j0 * ldv, ldv, Tm + (size_t)j0 * kNB, kNB, kb, 0, A + j0 + (size_t)c0 * lda, lda,
-                   B + (size_t)c0 * ldb, ldb, m, (nc - c0) < kNC ? (nc - c0) : kNC, sm);
+                   B + (size_t)c0 * ldb, ldb, m, (nc - c0) < kNC ? (nc - c0) : kNC, sm, 0, stages);
   }
 }
 template <typename T>
 __device__ void mat_apply_q_right(const T* V, int ldv, const T* Tm, int k, T* C, int ldc, int m, int n,
-                                  T* sm) {
+                                  T* sm, int stages) {
   for (int j0 = 0; j0 < k; j0 += kNB) {
     const int kb = (k - j0) < kNB ? (k - j0) : kNB;
     for (int r0 = 0; r0 < m; r0 += kNC)
-      tile_right_q(V + j0 + (size_t)j0 * ldv, ldv, Tm + (size_t)j0 * kNB, kNB, kb, C + r0 + (size_t)j0 * ldc, ldc,
-                   (m - r0) < kNC ? (m - r0) : kNC, n - j0, sm);
+      mma_apply<T, false, true>(V + j0 + (size_t)j0 * ldv, ldv, Tm + (size_t)j0 * kNB, kNB, kb, 1, nullptr, 0,
+                                C + r0 + (size_t)j0 * ldc, ldc, n - j0, (m - r0) < kNC ? (m - r0) : kNC,
+                                reinterpret_cast<double*>(sm), stages, 0);
   }
 }
 

@@ -36,7 +36,9 @@ constexpr int kRed = 16;     // reduction scratch (doubles)
 // dist_qr's staged panel beyond its rows x kNB: the tpqrt's R block (kNB x
 // kNB) and the panel's Gram matrix (kNB x (kNB + 1))
 constexpr int kPanExtra = kNB * kNB + kNB * (kNB + 1);
-constexpr int kWcap = dev::kTileSmem;  // shared scratch (doubles) of the tiled block applies
+constexpr int kWcap = dev::kTileSmem;  // shared scratch (doubles) of the tiled block applies of dist_qr
+constexpr int kApplyStages = 3;        // tiles staged by the chunked applies (two CTAs on an SM)
+constexpr int kApplySmem = dev::tile_smem(kApplyStages);
 
 __device__ __forceinline__ void csync(int cs) {
   if (cs > 1) cg::this_cluster().sync();
@@ -424,10 +426,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_update(const UpdTask* __restric
     const UpdOp op = ops[o];
     if (op.kind == 0)
       dev::mat_apply_qt<T>(as<T>(op.V), op.ldv, as<T>(op.T), op.k, as<T>(op.A) + (size_t)t.col0 * op.lda, op.lda, op.m,
-                           t.ncols, sm);
+                           t.ncols, sm, kApplyStages);
     else
       dev::mat_apply_tpqt<T>(as<T>(op.V), op.ldv, as<T>(op.T), op.k, as<T>(op.A) + (size_t)t.col0 * op.lda, op.lda,
-                             as<T>(op.B) + (size_t)t.col0 * op.ldb, op.ldb, op.m, t.ncols, sm);
+                             as<T>(op.B) + (size_t)t.col0 * op.ldb, op.ldb, op.m, t.ncols, sm, kApplyStages);
   }
 }
 
@@ -444,7 +446,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_edge_left(const EdgeChunk* __re
     if (t.lo >= lim) return;
     cnt = min(cnt, lim - t.lo);
   }
-  dev::mat_apply_qt<T>(as<T>(t.V), t.ldv, as<T>(t.T), k, as<T>(t.A) + (size_t)t.lo * t.lda, t.lda, t.m, cnt, sm);
+  dev::mat_apply_qt<T>(as<T>(t.V), t.ldv, as<T>(t.T), k, as<T>(t.A) + (size_t)t.lo * t.lda, t.lda, t.m, cnt, sm,
+                       kApplyStages);
 }
 
 // Row scaling / left compression of small blocks, one warp per chunk: m <= 32
@@ -944,7 +947,8 @@ __global__ void __launch_bounds__(kThreads) k_edge_right(const EdgeChunk* __rest
   T* sm = reinterpret_cast<T*>(smraw);
   const EdgeChunk t = tasks[blockIdx.x];
   const int k = t.kdev ? *t.kdev : t.k;
-  dev::mat_apply_q_right<T>(as<T>(t.V), t.ldv, as<T>(t.T), k, as<T>(t.A) + t.lo, t.lda, t.cnt, t.nc, sm);
+  dev::mat_apply_q_right<T>(as<T>(t.V), t.ldv, as<T>(t.T), k, as<T>(t.A) + t.lo, t.lda, t.cnt, t.nc, sm,
+                            kApplyStages);
 }
 
 // ------------------------------------------------------------ RRQR
@@ -1354,7 +1358,7 @@ cudaError_t launch_scale(const ScaleTask* t, int ntasks, int cs, int nmax, cudaS
 cudaError_t launch_update(const UpdTask* t, const UpdOp* o, int ntasks, cudaStream_t st) {
   if (cudaError_t pre = begin("launch_update")) return pre;
   if (ntasks <= 0) return cudaSuccess;
-  const size_t b = smem_bytes(kWcap);
+  const size_t b = smem_bytes(kApplySmem);
   counted();
   if (g_fp32 && g_tc) {
     if (cudaError_t e = prep(k_update_tc, tc::kSmemBytes)) return e;
@@ -1372,7 +1376,7 @@ cudaError_t launch_update(const UpdTask* t, const UpdOp* o, int ntasks, cudaStre
 cudaError_t launch_edge(int kind, const EdgeChunk* t, int ntasks, cudaStream_t st) {
   if (cudaError_t pre = begin("launch_edge")) return pre;
   if (ntasks <= 0) return cudaSuccess;
-  const size_t b = smem_bytes(kWcap);
+  const size_t b = smem_bytes(kApplySmem);
   cudaError_t e = cudaSuccess;
   counted();
   auto go = [&](auto* left, auto* trsm, auto* right) -> cudaError_t {
