@@ -446,102 +446,98 @@ __device__ void mat_apply_q_right(const T* V, int ldv, const T* Tm, int k, T* C,
   }
 }
 
-// C (m <= kNC rows x n) <- C R^{-1}, R upper triangular (n x n), blocked by 32
-// columns: C(:, J) -= C(:, 0:j0) R(0:j0, J) through shared-memory tiles, then
-// the 32 x 32 diagonal block is solved one row per thread.
+// C (m <= kNC rows x n) <- C R^{-1}, R upper triangular (n x n), left-looking by
+// blocks of 32 columns: X_J = (C_J - X(:, 0:j0) R(0:j0, J)) R_JJ^{-1} with the
+// inverses of R's diagonal blocks given (block b at Inv + 32 * 32 b, column-major,
+// FP64).  Both products on FP64 mma as in mma_apply: warp w owns rows 8 w ..
+// 8 w + 7, tiles of X and R are shared.  (Substitution inside the diagonal blocks,
+// one thread a row, took longer than the products.)
 template <typename T>
-__device__ void tile_trsm_right_upper(const T* R, int ldr, T* C, int ldc, int m, int n, T* sm) {
-  constexpr int kRS = kRT * (kNB + 1), kCS = kNC * (kRT + 1);
-  static_assert(2 * kRS + 2 * kCS <= kTileSmem, "right solve scratch");
-  T* sR0 = sm;                 // two [kRT][kNB+1] tiles: R(l0+l, j0+j)
-  T* sC0 = sR0 + 2 * kRS;      // two [kNC][kRT+1] tiles: C(r, l0+l)
-  T* sR = sR0;                 // the diagonal block, after the products
-  T* sC = sC0;                 // the block being solved
-  const int t = threadIdx.x;
-  const int tj = t & 7, tr = t >> 3;    // cols tj*4..+3, rows tr*2..+1
-  constexpr int kSR = kRT * kNB / kThreads, kSC = kNC * kRT / kThreads;
-  T rr[kSR], rc[kSC];
-  // tiles of the already solved columns, the next one loaded before the
-  // current one's products
-  auto load = [&](int l0, int j0, int jb) {
-#pragma unroll
-    for (int q = 0; q < kSR; ++q) {
-      const int idx = t + q * kThreads, l = idx % kRT, j = idx / kRT;
-      rr[q] = (j < jb) ? R[(l0 + l) + (size_t)(j0 + j) * ldr] : (T)0.0;
-    }
-#pragma unroll
-    for (int q = 0; q < kSC; ++q) {
-      const int idx = t + q * kThreads, r = idx % kNC, l = idx / kNC;
-      rc[q] = (r < m) ? C[r + (size_t)(l0 + l) * ldc] : (T)0.0;
-    }
-  };
-  auto stash = [&](int b) {
-#pragma unroll
-    for (int q = 0; q < kSR; ++q) {
-      const int idx = t + q * kThreads;
-      sR0[b * kRS + (idx % kRT) * (kNB + 1) + idx / kRT] = rr[q];
-    }
-#pragma unroll
-    for (int q = 0; q < kSC; ++q) {
-      const int idx = t + q * kThreads;
-      sC0[b * kCS + (idx % kNC) * (kRT + 1) + idx / kNC] = rc[q];
-    }
-  };
+__device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int ldc, int m, int n, double* sm,
+                               int stages) {
+  sm = reinterpret_cast<double*>((reinterpret_cast<size_t>(sm) + 15) & ~(size_t)15);
+  double* sT = sm;
+  double* sV0 = sT + kTileV;
+  double* sC0 = sV0 + stages * kTileV;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int fn = lane >> 2, fk = lane & 3, perm = (fn >> 1) + 4 * (fn & 1);
+  constexpr int kSV = kNB / kWarps, kSC = kRT * kNC / kThreads;
+  T rv[kSV], rc[kSC];
+  const int cv = t % kNC, cr = t / kNC, c = 8 * warp + fn;
+  const bool have = c < m;
   for (int j0 = 0; j0 < n; j0 += kNB) {
-    const int jb = (n - j0) < kNB ? (n - j0) : kNB;
-    T acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-    const int nl = (j0 + kRT - 1) / kRT;
-    if (nl > 0) {
-      load(0, j0, jb);
-      stash(0);
+    const int jb = min(kNB, n - j0), ntile = j0 / kRT;
+    auto load = [&](int tt) {
+#pragma unroll
+      for (int q = 0; q < kSV; ++q) {
+        const int i = warp * kSV + q;
+        rv[q] = i < jb ? R[tt * kRT + lane + (size_t)(j0 + i) * ldr] : (T)0;
+      }
+#pragma unroll
+      for (int q = 0; q < kSC; ++q) rc[q] = cv < m ? C[cv + (size_t)(tt * kRT + cr + 4 * q) * ldc] : (T)0;
+    };
+    auto stash = [&](int tt) {
+      double* dv = sV0 + (tt % stages) * kTileV;
+      double* dc = sC0 + (tt % stages) * kTileC;
+#pragma unroll
+      for (int q = 0; q < kSV; ++q) dv[(warp * kSV + q) * kLdV + lane] = (double)rv[q];
+#pragma unroll
+      for (int q = 0; q < kSC; ++q) dc[(cr + 4 * q) * kLdR + cv] = (double)rc[q];
+    };
+    if (ntile > 0) load(0);
+    double w[4][2], x[4][2];
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int j = 8 * b + fk + 4 * e;
+        x[b][e] = j < jb && have ? (double)C[c + (size_t)(j0 + j) * ldc] : 0.0;
+        w[b][e] = 0.0;
+      }
+#pragma unroll
+    for (int q = 0; q < kNB * kNB / kThreads; ++q) {
+      const int j = warp + q * kWarps;
+      sT[j * kLdV + lane] = lane <= j && j < jb ? Inv[lane + (size_t)(j0 + j) * kNB] : 0.0;
+    }
+    if (ntile > 0) stash(0);
+    __syncthreads();
+    for (int tt = 0; tt < ntile; ++tt) {
+      const bool more = tt + 1 < ntile;
+      if (more) load(tt + 1);
+      const double* sV = sV0 + (tt % stages) * kTileV;
+      const double* sC = sC0 + (tt % stages) * kTileC;
+#pragma unroll
+      for (int rr = 0; rr < kRT; rr += 8) {
+        const double a0 = sC[(rr + 2 * fk) * kLdR + c], a1 = sC[(rr + 2 * fk + 1) * kLdR + c];
+        double2 v[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) v[b] = *reinterpret_cast<const double2*>(sV + (8 * b + perm) * kLdV + rr + 2 * fk);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], a0, v[b].x);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], a1, v[b].y);
+      }
+      if (more) stash(tt + 1);
       __syncthreads();
     }
-    for (int it = 0; it < nl; ++it) {
-      const int b = it & 1;
-      const bool more = it + 1 < nl;
-      if (more) load((it + 1) * kRT, j0, jb);
-      const T* tR = sR0 + b * kRS;
-      const T* tC = sC0 + b * kCS;
-#pragma unroll 4
-      for (int l = 0; l < kRT; ++l) {
-        const T a0 = tC[(tr * 2) * (kRT + 1) + l], a1 = tC[(tr * 2 + 1) * (kRT + 1) + l];
+    double y[4][2];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const T rv = tR[l * (kNB + 1) + tj * 4 + q];
-          acc[0][q] += a0 * rv;
-          acc[1][q] += a1 * rv;
-        }
-      }
-      if (more) stash(b ^ 1);
-      __syncthreads();
-    }
-    // subtract into the block, stage it in shared memory with the diagonal R block
-    for (int idx = t; idx < kNB * kNB; idx += kThreads) {
-      const int l = idx % kNB, j = idx / kNB;
-      sR[l * (kNB + 1) + j] = (l < jb && j < jb) ? R[(j0 + l) + (size_t)(j0 + j) * ldr] : 0.0;
+    for (int j = 0; j < 4; ++j) {
+      y[j][0] = y[j][1] = 0.0;
+#pragma unroll
+      for (int b = 0; b <= j; ++b)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          dmma(y[j][0], y[j][1], x[b][e] - w[b][e], sT[(8 * j + perm) * kLdV + 8 * b + fk + 4 * e]);
     }
 #pragma unroll
-    for (int p = 0; p < 2; ++p)
+    for (int b = 0; b < 4; ++b)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int r = tr * 2 + p, j = tj * 4 + q;
-        sC[r * (kRT + 1) + j] = (r < m && j < jb) ? C[r + (size_t)(j0 + j) * ldc] - acc[p][q] : 0.0;
+      for (int e = 0; e < 2; ++e) {
+        const int j = 8 * b + fk + 4 * e;
+        if (j < jb && have) C[c + (size_t)(j0 + j) * ldc] = (T)y[b][e];
       }
-    __syncthreads();
-    for (int r = t; r < m; r += kThreads) {
-      T* cr = sC + r * (kRT + 1);
-      for (int j = 0; j < jb; ++j) {
-        T s = cr[j];
-        for (int l = 0; l < j; ++l) s -= cr[l] * sR[l * (kNB + 1) + j];
-        cr[j] = s / sR[j * (kNB + 1) + j];
-      }
-    }
-    __syncthreads();
-    for (int idx = t; idx < kNC * kNB; idx += kThreads) {
-      const int r = idx % kNC, j = idx / kNC;
-      if (r < m && j < jb) C[r + (size_t)(j0 + j) * ldc] = sC[r * (kRT + 1) + j];
-    }
-    __syncthreads();
+    __syncthreads();  // X_J before it is read, T before it is overwritten
   }
 }
 

@@ -286,6 +286,7 @@ int Tree::assemble() {
   rpos_.assign(ncl, 0);
   T_.assign(ncl, nullptr);
   Ts_.assign(ncl, nullptr);
+  Rinv_.assign(ncl, nullptr);
   Qsp_.assign(ncl, nullptr);
   Tsp_.assign(ncl, nullptr);
   ptr_.assign(ned, nullptr);
@@ -675,6 +676,8 @@ int Tree::factorize() {
     const bool spars = !Lv.spars_clusters.empty();
     if (spars) {
       std::vector<ScaleTask> sc[3];
+      std::vector<InvTask> inv;  // of the scaling R's diagonal blocks, for the column scaling and the apply
+      std::vector<double*> inv64(st_.clusters.size(), nullptr);
       int smax[3] = {1, 1, 1};
       for (int p : Lv.spars_clusters) {
         const int np = size_[p];
@@ -684,7 +687,11 @@ int Tree::factorize() {
         t.T = Ts_[p];
         t.tau = scratch_.dalloc(std::max(np, 1));
         t.n = np;
-        if (!t.T || !t.tau) return fail(-11, "out of device memory (scaling)");
+        const size_t ninv = (size_t)NB * NB * std::max(1, (np + NB - 1) / NB);
+        Rinv_[p] = arena_.dalloc(ninv);
+        inv64[p] = fp32_ ? scratch_.dalloc(ninv) : Rinv_[p];
+        if (!t.T || !t.tau || !Rinv_[p] || !inv64[p]) return fail(-11, "out of device memory (scaling)");
+        for (int b = 0; b * NB < np; ++b) inv.push_back({t.S, Rinv_[p], fp32_ ? inv64[p] : nullptr, np, b});
         const int cs = cluster_for(np);
         const int g = cs == 1 ? 0 : (cs == 4 ? 1 : 2);
         sc[g].push_back(t);
@@ -705,6 +712,10 @@ int Tree::factorize() {
         if (sc[g].empty()) continue;
         auto* d = static_cast<ScaleTask*>(up_vec(sc[g]));
         if (!d || ck(launch_scale(d, (int)sc[g].size(), csz[g], smax[g], stream_), "scaling kernel")) return -10;
+      }
+      {
+        auto* d = static_cast<InvTask*>(up_vec(inv));
+        if (!d || ck(launch_diag_inverse(d, (int)inv.size(), stream_), "scaling inverses")) return -10;
       }
       cudaEventRecord(fe[1], stream_);
       std::vector<EdgeChunk>& rows_scale = P.rows_scale;
@@ -732,7 +743,7 @@ int Tree::factorize() {
         }
         if (c) {
           t.V = ptr_[Lv.self_edge_of[E.n1 - Lv.first]];
-          t.T = nullptr;
+          t.T = inv64[E.n1];
           t.ldv = size_[E.n1];
           for (int r0 = 0; r0 < t.m; r0 += kChunk) {
             t.lo = r0;
@@ -1510,7 +1521,7 @@ int Tree::plan_sweep() {
   InvTask* d_inv = nullptr;
   auto inverses = [&](const double* R, int n) {
     double* out = arena_.dalloc((size_t)NB * NB * std::max(1, (n + NB - 1) / NB));
-    for (int b = 0; b * NB < n; ++b) inv.push_back({R, out, n, b});
+    for (int b = 0; b * NB < n; ++b) inv.push_back({R, out, nullptr, n, b});
     return out;
   };
   for (int lvl = 0; lvl < L; ++lvl) {
@@ -1584,8 +1595,7 @@ int Tree::plan_sweep() {
       t.rank = d_rank_ + p;
       t.x = xoff_[p];
       t.n = size_org_[p];
-      t.inv = inverses(t.Qs, t.n);
-      if (!t.inv) return fail(-11, "out of device memory (triangular inverses)");
+      t.inv = Rinv_[p];
       sp.push_back(t);
       S.sp_nmax = std::max(S.sp_nmax, t.n);
     }

@@ -298,6 +298,7 @@ class Tree {
   // per cluster
   std::vector<int> size_, size_org_, rpos_;
   std::vector<double*> T_, Ts_, Qsp_, Tsp_;
+  std::vector<double*> Rinv_;  // inverses of the scaling R's diagonal blocks (null: no interface)
   std::vector<int64_t> xoff_;
   int* d_rank_ = nullptr;
   // per edge

@@ -822,7 +822,8 @@ __global__ void __launch_bounds__(kThreads) k_edge_trsm(const EdgeChunk* __restr
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);
   const EdgeChunk t = tasks[blockIdx.x];
-  dev::tile_trsm_right_upper<T>(as<T>(t.V), t.ldv, as<T>(t.A) + t.lo, t.lda, t.cnt, t.nc, sm);
+  dev::mma_trsm_right<T>(as<T>(t.V), t.ldv, t.T, as<T>(t.A) + t.lo, t.lda, t.cnt, t.nc, reinterpret_cast<double*>(sm),
+                         kApplyStages);
 }
 
 // Column scaling of small blocks (FP32, at most 32 columns, chunks of at most

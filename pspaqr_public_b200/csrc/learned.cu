@@ -378,122 +378,151 @@ __global__ void k_mlp_adam(float* P, const float* __restrict__ g, float* m1, flo
 }
 
 // ---------------------------------------------------------------- sketch / projection GEMMs
-// 64 x 64 output tile per CTA, k-steps of 32, each thread a 4 x 4 block of
-// outputs at rows ty + 16 a (the sketch: rows 4 ty + a), columns tx + 16 b.
-// In the sketch the next
-// k-step's C tile is copied into the other half of a double buffer with
-// cp.async while the current one is multiplied (the projection loads each
-// step's tiles directly: its two tiles in a double buffer would halve the
-// CTAs per SM); every output sums its k terms in ascending order.
-__global__ void __launch_bounds__(kT) k_sketch(const SketchTask* __restrict__ tasks,
-                                               const GemmTile* __restrict__ tiles) {
-  // C(r0 + rr, j0 + jj) at As[.][jj][rr]: a thread's four consecutive rows are
-  // two 16-byte loads (rows of kTile + 2 doubles keep them 16-byte aligned)
-  __shared__ __align__(16) double As[2][kKStep][kTile + 2];
-  __shared__ unsigned long long Ws[2][kKStep];  // signs of Omega(j0 + jj, c0 .. c0 + 63)
+// 64 x 64 output tile per CTA, k-steps of 32, FP64 mma: warp w computes rows
+// 16 (w % 4) .. + 15 and columns 32 (w / 4) .. + 31.  A tiles are stored with k
+// contiguous (16-byte fragments, two k of one row), B tiles of the projection as
+// rows of C (8-byte fragments); the next k-step's elements are loaded into
+// registers while the current one is multiplied.  (On the FP64 pipes with 4 x 4
+// outputs a thread: 11 - 13 TFLOP/s.)
+constexpr int kLdA = 40;  // 8 mod 16 doubles: two rows of a quarter-warp on distinct banks
+constexpr int kLdB = 66;  // 2 mod 8 doubles: likewise for 8-byte fragments of four k rows
+static_assert(kTile == 64 && kKStep == 32 && kT == 256, "tile shapes");
+
+__global__ void __launch_bounds__(kT, 2) k_sketch(const SketchTask* __restrict__ tasks,
+                                                  const GemmTile* __restrict__ tiles) {
+  __shared__ __align__(16) double As[2][kTile * kLdA];  // C(r0 + rr, j0 + jj) at rr * kLdA + jj
+  __shared__ __align__(16) unsigned long long Ws[2][kKStep];  // signs of Omega(j0 + jj, c0 .. c0 + 63)
   const GemmTile g = tiles[blockIdx.x];
   const SketchTask t = tasks[g.task];
   const int ell = *t.ell;
   if (g.c0 >= ell) return;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fn = lane >> 2, fk = lane & 3;
   const int nsteps = (t.w + kKStep - 1) / kKStep;
-  auto load = [&](int s, int b) {
-    const int j0 = s * kKStep;
-    for (int e = threadIdx.x; e < kTile * kKStep; e += kT) {
-      const int rr = e / kKStep, jj = e % kKStep;
-      const int r = g.r0 + rr, j = j0 + jj;
-      if (r < t.m && j < t.w) dev::cp_async_elem(&As[b][jj][rr], t.C + (size_t)r * t.ldw + j);
-      else As[b][jj][rr] = 0.0;
+  constexpr int kE = kTile * kKStep / kT;  // elements a thread
+  double ra[kE];
+  unsigned long long rw = 0;
+  auto load = [&](int s) {
+    const int j = s * kKStep + lane;
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+      const int r = g.r0 + warp + 8 * q;
+      ra[q] = r < t.m && j < t.w ? __ldg(t.C + (size_t)r * t.ldw + j) : 0.0;
     }
-    if (threadIdx.x < kKStep) Ws[b][threadIdx.x] = omega_bits(t.seed, j0 + threadIdx.x, g.c0 >> 6);
-    dev::cp_async_commit();
+    if (threadIdx.x < kKStep) rw = omega_bits(t.seed, s * kKStep + threadIdx.x, g.c0 >> 6);
   };
-  double acc[4][4] = {};
-  if (nsteps > 0) load(0, 0);
+  auto stash = [&](int b) {
+#pragma unroll
+    for (int q = 0; q < kE; ++q) As[b][(warp + 8 * q) * kLdA + lane] = ra[q];
+    if (threadIdx.x < kKStep) Ws[b][threadIdx.x] = rw;
+  };
+  double acc[2][4][2] = {};
+  const int wr = 16 * (warp & 3), wc = 32 * (warp >> 2);
+  if (nsteps > 0) {
+    load(0);
+    stash(0);
+  }
+  __syncthreads();
   for (int s = 0; s < nsteps; ++s) {
     const int b = s & 1;
-    if (s + 1 < nsteps) {
-      load(s + 1, b ^ 1);
-      dev::cp_async_wait<1>();
-    } else {
-      dev::cp_async_wait<0>();
+    if (s + 1 < nsteps) load(s + 1);
+#pragma unroll
+    for (int kk = 0; kk < kKStep; kk += 8) {
+      double2 a[2];
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+        a[p] = *reinterpret_cast<const double2*>(&As[b][(wr + 8 * p + fn) * kLdA + kk + 2 * fk]);
+      const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&Ws[b][kk + 2 * fk]);
+      const unsigned w0 = (unsigned)(w.x >> wc), w1 = (unsigned)(w.y >> wc);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double b0 = (w0 >> (8 * q + fn)) & 1u ? 1.0 : -1.0, b1 = (w1 >> (8 * q + fn)) & 1u ? 1.0 : -1.0;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) dev::dmma(acc[p][q][0], acc[p][q][1], a[p].x, b0);
+#pragma unroll
+        for (int p = 0; p < 2; ++p) dev::dmma(acc[p][q][0], acc[p][q][1], a[p].y, b1);
+      }
     }
-    __syncthreads();
-#pragma unroll 8
-    for (int jj = 0; jj < kKStep; ++jj) {
-      const unsigned long long w = Ws[b][jj];
-      const double2 a01 = *reinterpret_cast<const double2*>(&As[b][jj][4 * ty]);
-      const double2 a23 = *reinterpret_cast<const double2*>(&As[b][jj][4 * ty + 2]);
-      const double a[4] = {a01.x, a01.y, a23.x, a23.y};
-      double bq[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) bq[q] = ((w >> (tx + 16 * q)) & 1ull) ? 1.0 : -1.0;
-#pragma unroll
-      for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[p][q] += a[p] * bq[q];
-    }
+    if (s + 1 < nsteps) stash(b ^ 1);
     __syncthreads();
   }
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int r = g.r0 + 4 * ty + p;
+  for (int p = 0; p < 2; ++p) {
+    const int r = g.r0 + wr + 8 * p + fn;
     if (r >= t.m) continue;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = g.c0 + tx + 16 * q;
-      if (c < ell) t.Y[(size_t)r * t.ldy + c] = acc[p][q];
-    }
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = g.c0 + wc + 8 * q + 2 * fk + e;
+        if (c < ell) t.Y[(size_t)r * t.ldy + c] = acc[p][q][e];
+      }
   }
 }
 
 // B(l, j) = sum_r Q(r, l) C(r, j); tile rows l (basis vectors), columns j
-__global__ void __launch_bounds__(kT) k_project(const SketchTask* __restrict__ tasks,
-                                                const GemmTile* __restrict__ tiles) {
-  __shared__ double As[kKStep][kTile + 1];  // Q(r0 + rr, l0 + ll) at As[rr][ll]
-  __shared__ double Bs[kKStep][kTile + 1];  // C(r0 + rr, j0 + jj) at Bs[rr][jj]
+__global__ void __launch_bounds__(kT, 2) k_project(const SketchTask* __restrict__ tasks,
+                                                   const GemmTile* __restrict__ tiles) {
+  __shared__ __align__(16) double As[kTile * kLdA];  // Q(r0 + rr, l0 + ll) at ll * kLdA + rr
+  __shared__ __align__(16) double Bs[kKStep * kLdB];  // C(r0 + rr, j0 + jj) at rr * kLdB + jj
   const GemmTile g = tiles[blockIdx.x];
   const SketchTask t = tasks[g.task];
   const int ell = *t.ell;
   if (g.r0 >= ell) return;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[4][4] = {};
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fn = lane >> 2, fk = lane & 3;
+  constexpr int kE = kTile * kKStep / kT;
+  double ra[kE], rb[kE];
+  const int bj = threadIdx.x % kTile, br = threadIdx.x / kTile;
+  auto load = [&](int k0) {
+    const int r = k0 + lane;
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+      const int l = g.r0 + warp + 8 * q;
+      ra[q] = l < ell && r < t.m ? __ldg(t.Qc + (size_t)l * t.m + r) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+      const int rr = k0 + br + 4 * q, j = g.c0 + bj;
+      rb[q] = rr < t.m && j < t.w ? __ldg(t.C + (size_t)rr * t.ldw + j) : 0.0;
+    }
+  };
+  double acc[2][4][2] = {};
+  const int wr = 16 * (warp & 3), wc = 32 * (warp >> 2);
+  load(0);
   for (int k0 = 0; k0 < t.m; k0 += kKStep) {
-    for (int e = threadIdx.x; e < kTile * kKStep; e += kT) {
-      const int ll = e / kKStep, rr = e % kKStep;
-      const int l = g.r0 + ll, r = k0 + rr;
-      As[rr][ll] = (l < ell && r < t.m) ? __ldg(t.Qc + (size_t)l * t.m + r) : 0.0;
-    }
-    for (int e = threadIdx.x; e < kTile * kKStep; e += kT) {
-      const int rr = e / kTile, jj = e % kTile;
-      const int r = k0 + rr, j = g.c0 + jj;
-      Bs[rr][jj] = (r < t.m && j < t.w) ? __ldg(t.C + (size_t)r * t.ldw + j) : 0.0;
-    }
+#pragma unroll
+    for (int q = 0; q < kE; ++q) As[(warp + 8 * q) * kLdA + lane] = ra[q];
+#pragma unroll
+    for (int q = 0; q < kE; ++q) Bs[(br + 4 * q) * kLdB + bj] = rb[q];
     __syncthreads();
-#pragma unroll 8
-    for (int rr = 0; rr < kKStep; ++rr) {
-      double a[4], b[4];
+    if (k0 + kKStep < t.m) load(k0 + kKStep);
+#pragma unroll
+    for (int kk = 0; kk < kKStep; kk += 8) {
+      double2 a[2];
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+        a[p] = *reinterpret_cast<const double2*>(&As[(wr + 8 * p + fn) * kLdA + kk + 2 * fk]);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        a[q] = As[rr][ty + 16 * q];
-        b[q] = Bs[rr][tx + 16 * q];
+        const double b0 = Bs[(kk + 2 * fk) * kLdB + wc + 8 * q + fn], b1 = Bs[(kk + 2 * fk + 1) * kLdB + wc + 8 * q + fn];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) dev::dmma(acc[p][q][0], acc[p][q][1], a[p].x, b0);
+#pragma unroll
+        for (int p = 0; p < 2; ++p) dev::dmma(acc[p][q][0], acc[p][q][1], a[p].y, b1);
       }
-#pragma unroll
-      for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[p][q] += a[p] * b[q];
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int l = g.r0 + ty + 16 * p;
+  for (int p = 0; p < 2; ++p) {
+    const int l = g.r0 + wr + 8 * p + fn;
     if (l >= ell) continue;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int j = g.c0 + tx + 16 * q;
-      if (j < t.w) t.B[(size_t)l * t.w + j] = acc[p][q];
-    }
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int j = g.c0 + wc + 8 * q + 2 * fk + e;
+        if (j < t.w) t.B[(size_t)l * t.w + j] = acc[p][q][e];
+      }
   }
 }
 

@@ -655,30 +655,33 @@ __global__ void k_sweep_copy(int n, const int* __restrict__ src, const int* __re
 // A warp inverts one 32 x 32 diagonal block, lane j column j by back substitution.
 template <typename T>
 __global__ void __launch_bounds__(128) k_diag_inverse(const InvTask* __restrict__ tasks, int ntasks) {
-  __shared__ T sR[4][kNB * (kNB + 1)];
+  __shared__ double sR[4][kNB * (kNB + 1)];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ti = blockIdx.x * 4 + warp;
   if (ti >= ntasks) return;
   const InvTask t = tasks[ti];
   const int c = t.block * kNB, kb = min(kNB, t.n - c);
   const T* R = as<T>(t.R) + c + (size_t)c * t.n;
-  T* s = sR[warp];
+  double* s = sR[warp];
   for (int j = 0; j < kb; ++j)
-    if (lane <= j) s[lane * (kNB + 1) + j] = R[lane + (size_t)j * t.n];
+    if (lane <= j) s[lane * (kNB + 1) + j] = (double)R[lane + (size_t)j * t.n];
   __syncwarp();
-  T x[kNB];
+  double x[kNB];
 #pragma unroll
   for (int l = kNB - 1; l >= 0; --l) {
-    T v = l == lane ? (T)1 : (T)0;
+    double v = l == lane ? 1.0 : 0.0;
 #pragma unroll
     for (int q = l + 1; q < kNB; ++q)
       if (q <= lane && q < kb) v -= s[l * (kNB + 1) + q] * x[q];
-    x[l] = l <= lane && lane < kb ? v / s[l * (kNB + 1) + l] : (T)0;
+    x[l] = l <= lane && lane < kb ? v / s[l * (kNB + 1) + l] : 0.0;
   }
   T* out = reinterpret_cast<T*>(t.out) + (size_t)t.block * kNB * kNB;
   if (lane < kb)
 #pragma unroll
-    for (int l = 0; l < kNB; ++l) out[l + lane * kNB] = x[l];
+    for (int l = 0; l < kNB; ++l) out[l + lane * kNB] = (T)x[l];
+  if (t.out64 && lane < kb)
+#pragma unroll
+    for (int l = 0; l < kNB; ++l) t.out64[(size_t)t.block * kNB * kNB + l + lane * kNB] = x[l];
 }
 
 // ---------------------------------------------------------------- launchers

@@ -45,10 +45,12 @@ struct BwdEdge {
   int ldr, s;
 };
 // Inverses of the 32 x 32 diagonal blocks of an upper-triangular R (n x n, ld n),
-// block b at out + 32 * 32 * b (column-major, ld 32).
+// block b at out + 32 * 32 * b (column-major, ld 32), computed in FP64 and stored
+// in the factors' precision; out64: also unrounded, or null.
 struct InvTask {
   const double* R;
   double* out;
+  double* out64;
   int n, block;
 };
 

@@ -67,7 +67,7 @@ struct ScaleTask {
 struct EdgeChunk {
   double* A;
   const double* V;     // reflectors (or the upper-triangular R for column scaling)
-  const double* T;     // block factors (kNB x k)
+  const double* T;     // block factors (kNB x k); column scaling: FP64 inverses of R's diagonal blocks
   const int* kdev;     // number of reflectors read on the device (rank), or null: use k
   const int* limdev;   // left compression: only columns < *limdev exist, or null
   int lda, m, nc, ldv, k, lo, cnt;
