@@ -117,6 +117,13 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
   const int rank = crank(cs);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gap = (cs - 1) * kNB;  // columns between two panels of one CTA
+  // one panel's (or part's) block reflector on nc columns: Rc their rows of R from
+  // j0 on, Bc their columns of B
+  auto apply = [&](T* Rc, T* Bc, const T* Tm, int j0, int kb, int nc, int cgap) {
+    dev::tile_left_qt<T, true>(unit ? R + j0 + (size_t)j0 * ldr : B + (size_t)j0 * ldb, unit ? ldr : ldb, Tm, kNB, kb,
+                               unit, unit ? nullptr : Rc, ldr, unit ? Rc : Bc, unit ? ldr : ldb, unit ? m - j0 : m, nc,
+                               tile, cgap);
+  };
   for (int j0 = 0; j0 < n; j0 += kNB) {
     const int kb = (n - j0) < kNB ? (n - j0) : kNB;
     const int pend = j0 + kb;
@@ -260,13 +267,8 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
       __threadfence();
       __syncthreads();
       if (pend < plast) {  // the part's block reflector on the rest of the panel
-        const T* Tm = Tout + (size_t)j0 * kNB + (j0 - pstart);
-        if (unit)
-          dev::tile_left_qt<T, true>(R + j0 + (size_t)j0 * ldr, ldr, Tm, kNB, kb, 1, nullptr, 0,
-                                     R + j0 + (size_t)pend * ldr, ldr, m - j0, plast - pend, tile, 0);
-        else
-          dev::tile_left_qt<T, true>(B + (size_t)j0 * ldb, ldb, Tm, kNB, kb, 0, R + j0 + (size_t)pend * ldr, ldr,
-                                     B + (size_t)pend * ldb, ldb, m, plast - pend, tile, 0);
+        apply(R + j0 + (size_t)pend * ldr, B + (size_t)pend * ldb, Tout + (size_t)j0 * kNB + (j0 - pstart), j0, kb,
+              plast - pend, 0);
       }
      }
      if (pw < pkb) {  // T of the whole panel: the blocks between the parts
@@ -329,12 +331,7 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
     for (; q0 < n; q0 += 2 * cs * kNB) {
       const int second = q0 + cs * kNB;
       const int nc = (q0 + kNB < n ? kNB : n - q0) + (second < n ? ((second + kNB < n ? kNB : n - second)) : 0);
-      if (unit)
-        dev::tile_left_qt<T, true>(R + j0 + (size_t)j0 * ldr, ldr, Tm, kNB, kb, 1, nullptr, 0,
-                                   R + j0 + (size_t)q0 * ldr, ldr, m - j0, nc, tile, gap);
-      else
-        dev::tile_left_qt<T, true>(B + (size_t)j0 * ldb, ldb, Tm, kNB, kb, 0, R + j0 + (size_t)q0 * ldr, ldr,
-                                   B + (size_t)q0 * ldb, ldb, m, nc, tile, gap);
+      apply(R + j0 + (size_t)q0 * ldr, B + (size_t)q0 * ldb, Tm, j0, kb, nc, gap);
     }
     if (chain.out) {
       csync(cs);
