@@ -92,6 +92,13 @@ int spq_debug_tc_probe(const float* C, const float* V, const float* W2, int m, i
  * columns in pivot order (colat holds min(m, w) entries). */
 int spq_debug_pivots(const double* C, int m, int w, int cm, int cs, long long smem_limit, double tol,
                      double pivot_rtol, int* colat, int* rank);
+
+/* One elimination chain on its own, for tests: the geqrt of S (n x n, column-major) and a tsqrt of [S; B_i] for
+ * each of nout blocks (rows[i] x n, column-major, one after the other in B), in clusters of cs CTAs, as one cluster
+ * or as a pipeline with a cluster per step.  In place: S holds R and the geqrt's reflectors below its diagonal, B the
+ * reflector tails; T (32 x n for each of the nout + 1 steps) the panels' block factors.  bits 64 or 32: the factors'
+ * type. */
+int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int cs, int pipe, int bits, double* T);
 /* Diagnostic of the preconditioner apply (no reference counterpart): from the
  * next factorize on, reflector panels of more than `rows` rows are read from
  * global memory where they are used, as panels too long for shared memory are

@@ -172,6 +172,90 @@ int spq_debug_pivots(const double* C, int m, int w, int cm, int cs, long long sm
   return e ? -10 : 0;
 }
 
+int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int cs, int pipe, int bits, double* T) {
+  if (!S || !T || n < 1 || nout < 0 || (nout && (!B || !rows)) || cs < 1 || cs > 8 || (cs & (cs - 1)) || pipe < 0 ||
+      pipe > 1 || (bits != 64 && bits != 32))
+    return -1;
+  // arrays on 64-element boundaries, as the engine's pools place them: S, the blocks, T of each step, tau
+  auto pad = [](size_t k) { return (k + 63) / 64 * 64; };
+  std::vector<size_t> ob(nout), ot(nout + 1);
+  size_t tot = pad((size_t)n * n);
+  int vm = n;
+  for (int i = 0; i < nout; ++i) {
+    if (rows[i] < 1) return -1;
+    vm = std::max(vm, rows[i]);
+    ob[i] = tot;
+    tot += pad((size_t)rows[i] * n);
+  }
+  const size_t nt = (size_t)32 * n;
+  for (int i = 0; i <= nout; ++i) {
+    ot[i] = tot;
+    tot += pad(nt);
+  }
+  const size_t otau = tot;
+  tot += pad(n);
+  const bool f32 = bits == 32;
+  const size_t es = f32 ? 4 : 8;
+  const size_t nd = sizeof(spq::ElimStep) * (nout + 1) + sizeof(spq::ElimTask) + sizeof(spq::ElimOut) * nout;
+  const size_t cnt = (size_t)nout + 2;  // ticket, status, progress
+  char* d = nullptr;
+  if (cudaMalloc(&d, tot * es + nd + sizeof(int) * cnt) != cudaSuccess) return -11;
+  auto at = [&](size_t i) { return reinterpret_cast<double*>(d + i * es); };
+  std::vector<float> hf(f32 ? tot : 0);
+  std::vector<double> hd(f32 ? 0 : tot);
+  auto put = [&](size_t at, const double* x, size_t k) {
+    for (size_t i = 0; i < k; ++i)
+      if (f32) hf[at + i] = (float)x[i];
+      else hd[at + i] = x[i];
+  };
+  auto get = [&](size_t at, double* x, size_t k) {
+    for (size_t i = 0; i < k; ++i) x[i] = f32 ? (double)hf[at + i] : hd[at + i];
+  };
+  std::vector<spq::ElimStep> st;
+  std::vector<spq::ElimOut> eo;
+  const spq::ElimTask et{at(0), at(ot[0]), at(otau), n, 0, nout};
+  st.push_back({at(0), nullptr, at(ot[0]), at(otau), n, n, -1, nout ? 0 : -1});
+  put(0, S, (size_t)n * n);
+  const double* src = B;
+  for (int i = 0; i < nout; ++i) {
+    st.push_back({at(0), at(ob[i]), at(ot[i + 1]), at(otau), n, rows[i], i, i + 1 < nout ? i + 1 : -1});
+    eo.push_back({at(ob[i]), at(ot[i + 1]), rows[i]});
+    put(ob[i], src, (size_t)rows[i] * n);
+    src += (size_t)rows[i] * n;
+  }
+  void* hv = f32 ? (void*)hf.data() : (void*)hd.data();
+  auto* d_st = reinterpret_cast<spq::ElimStep*>(d + tot * es);
+  auto* d_eo = reinterpret_cast<spq::ElimOut*>(d_st + st.size());
+  auto* d_et = reinterpret_cast<spq::ElimTask*>(d_eo + nout);
+  auto* d_cnt = reinterpret_cast<int*>(d_et + 1);
+  cudaError_t e = cudaMemcpy(d, hv, tot * es, cudaMemcpyHostToDevice);
+  if (!e) e = cudaMemcpy(d_st, st.data(), sizeof(st[0]) * st.size(), cudaMemcpyHostToDevice);
+  if (!e && nout) e = cudaMemcpy(d_eo, eo.data(), sizeof(eo[0]) * eo.size(), cudaMemcpyHostToDevice);
+  if (!e) e = cudaMemcpy(d_et, &et, sizeof(et), cudaMemcpyHostToDevice);
+  if (!e) e = cudaMemset(d_cnt, 0, sizeof(int) * cnt);
+  const bool was = spq::factor_fp32();
+  spq::set_factor_fp32(f32);
+  spq::set_status_word(d_cnt + 1);
+  if (!e)
+    e = pipe ? spq::launch_elim_pipe(d_st, nout + 1, cs, n, vm, d_cnt, d_cnt + 2, nullptr)
+             : spq::launch_elim(d_et, d_eo, 1, cs, n, vm, nullptr);
+  spq::set_factor_fp32(was);
+  spq::set_status_word(nullptr);  // a factorization sets its own
+  if (!e) e = cudaDeviceSynchronize();
+  int status = 0;
+  if (!e) e = cudaMemcpy(&status, d_cnt + 1, sizeof(int), cudaMemcpyDeviceToHost);
+  if (!e) e = cudaMemcpy(hv, d, tot * es, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e || status & 16) return e ? -10 : -12;
+  get(0, S, (size_t)n * n);
+  for (int i = 0; i < nout; ++i) {
+    get(ob[i], B, (size_t)rows[i] * n);
+    B += (size_t)rows[i] * n;
+  }
+  for (int i = 0; i <= nout; ++i) get(ot[i], T + nt * i, nt);
+  return 0;
+}
+
 int spq_set_tensor_cores(spq_tree* h, int mode) {
   if (!h || mode < 0 || mode > 2) return -1;
   h->t->tensor_cores = mode;

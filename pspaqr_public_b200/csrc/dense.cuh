@@ -135,69 +135,203 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-// panel_t for a panel in shared memory, with T built by one warp: the Gram
-// matrix goes to sG (kNB x (kNB + 1), shared); lane i of warp 0 then holds row
-// i of T and forms T(i, j) = -tau_j sum_{l=i}^{j-1} T(i, l) G(l, j), T(j, j) =
-// tau_j, without barriers.  Tm is written by warp 0; the caller synchronises
-// before T is read.  The Gram matrix is the
-// panel's transpose times itself: ten 8 x 8 tiles on and above the diagonal, one
-// or two a warp, as FP64 mma products (the A and the B fragment of a column
-// block are the same registers).  Dot products by warps and shuffles took as
-// long as half of the panel's reflectors.
+// Householder QR of one panel of kb <= 32 columns in shared memory: a geqrt of
+// pan (pm rows, column-major, ld ldp; pr = null) or the tpqrt of [pr; pan] (pr kb x
+// kb upper triangular, ld kNB).  Writes the reflectors and R in place, tau to
+// lt[0:kb] and tg[0:kb], T (kNB x kb layout) to global Tout.
+//
+// A panel is latency: 32 reflectors one after the other.  Reflectors are built and
+// applied within parts of eight columns, one column a warp and one barrier a
+// reflector; a part's block reflector is then applied to the rest of the panel by
+// FP64 mma, in the same pass that multiplies the part with the reflectors before
+// it, which gives T block by block (T(0:b, b) = -T(0:b, 0:b) (V(0:b)^T V_b) T_b).
+// Each warp works on its own rows; the partial products meet in `sc` (kPanelScratch
+// doubles).  With reflectors applied to all 31 columns a reflector took 4.6k cycles
+// at 400 rows, and T another third of the panel.  Before -> now: chains of a 64^3
+// FP64 factorization 50 -> 38.9 ms, scaling QRs 32 -> 28.8; at 25^3 5.6 -> 4.8 and
+// 3.4 -> 2.6 ms.
+constexpr int kPanelScratch = kWarps * 256 + 2 * 256 + kNB * (kNB + 1);
 template <typename T>
-__device__ void panel_t_warp(const T* V, int ldv, int m, int kb, int unit, const T* tau, T* Tm, int ldt, T* sG) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kLG = kNB + 1;
-  const int fn = lane >> 2, fk = lane & 3;
-  const int nt = (kb + 7) / 8;
-  int tile = 0;
-  for (int bi = 0; bi < nt; ++bi)
-    for (int bj = bi; bj < nt; ++bj, ++tile) {
-      if (tile % kWarps != warp) continue;
-      const int ci = 8 * bi + fn, cj = 8 * bj + fn;
-      const T* vi = V + (size_t)(ci < kb ? ci : 0) * ldv;
-      const T* vj = V + (size_t)(cj < kb ? cj : 0) * ldv;
-      auto el = [&](const T* v, int c, int r) -> double {
-        if (r >= m || c >= kb) return 0.0;
-        if (unit && r <= c) return r == c ? 1.0 : 0.0;
-        return (double)v[r];
-      };
-      double d[2][2] = {};
-      int r = 0;
-      for (; r < kNB; r += 8) {  // rows with the unit triangle
-        dmma(d[0][0], d[0][1], el(vi, ci, r + fk), el(vj, cj, r + fk));
-        dmma(d[1][0], d[1][1], el(vi, ci, r + 4 + fk), el(vj, cj, r + 4 + fk));
-      }
-      const double zi = ci < kb ? 1.0 : 0.0, zj = cj < kb ? 1.0 : 0.0;
-      for (; r + 8 <= m; r += 8) {
-        const double a0 = vi[r + fk], b0 = vj[r + fk], a1 = vi[r + 4 + fk], b1 = vj[r + 4 + fk];
-        dmma(d[0][0], d[0][1], a0 * zi, b0 * zj);
-        dmma(d[1][0], d[1][1], a1 * zi, b1 * zj);
-      }
-      for (; r < m; r += 4) dmma(d[0][0], d[0][1], el(vi, ci, r + fk), el(vj, cj, r + fk));
-#pragma unroll
-      for (int e = 0; e < 2; ++e) sG[(8 * bi + fn) * kLG + 8 * bj + 2 * fk + e] = (T)(d[0][e] + d[1][e]);
+__device__ void panel_qr(T* pan, int ldp, int pm, T* pr, int kb, T* lt, T* tg, double* sc, T* red, int* status,
+                         T* Tout) {
+  __shared__ T s_nrm2[2];
+  constexpr int kL = kNB + 1;
+  const bool unit = pr == nullptr;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, fn = lane >> 2, fk = lane & 3;
+  double* part = sc;               // kWarps x 4 blocks of 8 x 8
+  double* sD = part + kWarps * 256;  // block k: V_b^T times columns 8 k .. of the panel
+  double* sW = sD + 256;           // T_b^T sD
+  double* sT = sW + 256;           // T, ld kL
+  for (int b0 = 0; b0 < kb; b0 += 8) {
+    const int nb = min(8, kb - b0), b = b0 / 8;
+    // ---- the part's reflectors.  Every thread forms reflector jj from its alpha
+    // and the squared norm of its tail; warp w applies it to column jj + 1 + w with
+    // v = tail * scal formed on the fly, and warp 0 also sums that column's new tail
+    // for the next reflector.  The scaled tail and beta are stored one step later,
+    // when no warp reads them.
+    T nrm2;
+    {
+      const T* c = pan + (size_t)b0 * ldp;
+      T sq = 0;
+      for (int i = (unit ? b0 + 1 : 0) + t; i < pm; i += kThreads) sq += c[i] * c[i];
+      nrm2 = cta_sum(sq, red);
     }
-  __syncthreads();
-  if (warp == 0) {
-    T t[kNB];
+    T* prev_tail = nullptr;
+    T* prev_ajj = nullptr;
+    T prev_scal = 0, prev_beta = 0;
+    int prev_vlen = 0;
+    for (int jj = b0; jj < b0 + nb; ++jj) {
+      const int vlen = unit ? pm - jj - 1 : pm, first = unit ? jj + 1 : 0;
+      T* tail = pan + first + (size_t)jj * ldp;
+      T* ajj = unit ? pan + jj + (size_t)jj * ldp : pr + jj + jj * kNB;
+      T beta, scal;
+      const T tj = house(*ajj, nrm2, &beta, &scal);
+      if (prev_tail)
+        for (int i = t; i < prev_vlen; i += kThreads) prev_tail[i] *= prev_scal;
+      if (t == 0) {
+        if (prev_ajj) *prev_ajj = prev_beta;
+        lt[jj] = tj;
+        tg[jj] = tj;
+        // R(j, j) = 0 or not finite: the triangular solves would break down
+        if (status && !(isfinite(beta) && beta != (T)0)) atomicOr(status, isfinite(beta) ? 8 : 4);
+      }
+      const int kk = jj + 1 + warp;
+      if (kk < b0 + nb) {
+        T* rjk = unit ? pan + jj + (size_t)kk * ldp : pr + jj + kk * kNB;
+        T* tk = pan + first + (size_t)kk * ldp;
+        T sq = 0;
+        if (tj != (T)0) {
+          T d[2] = {lane == 0 ? *rjk : (T)0, 0};
+          int i = lane;
+          for (; i + 32 < vlen; i += 64) {
+            d[0] += (tail[i] * scal) * tk[i];
+            d[1] += (tail[i + 32] * scal) * tk[i + 32];
+          }
+          if (i < vlen) d[0] += (tail[i] * scal) * tk[i];
+          const T f = warp_sum(d[0] + d[1]) * tj;
+          if (lane == 0) *rjk -= f;
+#pragma unroll 4
+          for (int i = lane; i < vlen; i += 32) {
+            const T x = tk[i] - (tail[i] * scal) * f;
+            tk[i] = x;
+            if (!unit || i > 0) sq += x * x;
+          }
+        } else if (warp == 0) {
+          for (int i = lane; i < vlen; i += 32)
+            if (!unit || i > 0) sq += tk[i] * tk[i];
+        }
+        if (warp == 0) {  // the next reflector's tail: rows below its diagonal
+          sq = warp_sum(sq);
+          if (lane == 0) s_nrm2[(jj + 1) & 1] = sq;
+        }
+      }
+      prev_tail = tj != (T)0 ? tail : nullptr;
+      prev_scal = scal;
+      prev_vlen = vlen;
+      prev_ajj = ajj;
+      prev_beta = beta;
+      __syncthreads();
+      nrm2 = s_nrm2[(jj + 1) & 1];
+    }
+    if (prev_tail)
+      for (int i = t; i < prev_vlen; i += kThreads) prev_tail[i] *= prev_scal;
+    if (t == 0 && prev_ajj) *prev_ajj = prev_beta;
+    __syncthreads();
+    // ---- V_b^T times every block of the panel (reflectors before, V_b, the rest)
+    const int rs = unit ? b0 : 0, ch = (pm - rs + 8 * kWarps - 1) / (8 * kWarps) * 8;
+    const int r0 = rs + warp * ch, r1 = min(pm, r0 + ch);
+    auto vb = [&](int i, int r) -> double {  // V_b(r, i)
+      if (i >= nb || r >= pm) return 0.0;
+      if (unit && r - b0 <= i) return r - b0 == i ? 1.0 : 0.0;
+      return (double)pan[(size_t)(b0 + i) * ldp + r];
+    };
+    {
+      double acc[4][2] = {};
+#pragma unroll 2
+      for (int r = r0; r < r1; r += 4) {
+        const int rr = r + fk;
+        const double a = vb(fn, rr);
 #pragma unroll
-    for (int j = 0; j < kNB; ++j) t[j] = 0.0;
+        for (int k = 0; k < 4; ++k)
+          if (8 * k < kb) {
+            const int col = 8 * k + fn;
+            const double x = k == b ? a : col < kb && rr < pm ? (double)pan[(size_t)col * ldp + rr] : 0.0;
+            dmma(acc[k][0], acc[k][1], a, x);
+          }
+      }
 #pragma unroll
-    for (int j = 0; j < kNB; ++j) {
-      if (j < kb) {
-        T s[4] = {};
+      for (int k = 0; k < 4; ++k)
 #pragma unroll
-        for (int l = 0; l < kNB; ++l)
-          if (l < j && l >= lane) s[l & 3] += t[l] * sG[l * kLG + j];
-        const T tj = tau[j];
-        t[j] = lane < j ? -tj * ((s[0] + s[1]) + (s[2] + s[3])) : (lane == j ? tj : (T)0.0);
+        for (int e = 0; e < 2; ++e) part[(warp * 4 + k) * 64 + fn * 8 + 2 * fk + e] = acc[k][e];
+    }
+    __syncthreads();
+    const int ek = t >> 6, ei = (t >> 3) & 7, ec = t & 7;  // entry (ei, ec) of block ek
+    {
+      double s = 0.0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) s += part[w * 256 + t];
+      if (!unit && ek > b && ei < nb && 8 * ek + ec < kb) s += (double)pr[b0 + ei + (8 * ek + ec) * kNB];
+      sD[t] = s;
+    }
+    __syncthreads();
+    if (warp == 0) {  // T_b: lane i holds row i
+      double ti[8] = {};
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j < nb) {
+          double s = 0.0;
+#pragma unroll
+          for (int l = 0; l < j; ++l)
+            if (l >= lane) s += ti[l] * sD[b * 64 + l * 8 + j];
+          const double tj = (double)lt[b0 + j];
+          ti[j] = lane < j ? -tj * s : lane == j ? tj : 0.0;
+          if (lane < nb) sT[b0 + lane + (b0 + j) * kL] = ti[j];
+        }
+    }
+    __syncthreads();
+    {
+      double s = 0.0;
+      if (ek != b && ei < nb)
+        for (int l = 0; l <= ei; ++l) s += sT[b0 + l + (b0 + ei) * kL] * sD[ek * 64 + l * 8 + ec];
+      sW[t] = s;
+      if (!unit && ek > b && ei < nb && 8 * ek + ec < kb) pr[b0 + ei + (8 * ek + ec) * kNB] -= (T)s;
+    }
+    __syncthreads();
+    if (t < b0 * nb) {  // T(0:b0, b0:b0+nb)
+      const int i = t % b0, j = t / b0;
+      double s = 0.0;
+      for (int q = i; q < b0; ++q) s += sT[i + q * kL] * sW[(q >> 3) * 64 + j * 8 + (q & 7)];
+      sT[i + (b0 + j) * kL] = -s;
+    }
+    if (b0 + 8 < kb) {  // the rest of the panel -= V_b sW
+      double w[4][2];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) w[k][e] = k > b ? -sW[k * 64 + (fk + 4 * e) * 8 + fn] : 0.0;
+#pragma unroll 2
+      for (int r = r0; r < r1; r += 8) {
+        const double v0 = vb(fk, r + fn), v1 = vb(fk + 4, r + fn);
+        const int ra = r + 2 * fk;
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+          if (k > b && 8 * k < kb) {
+            const int col = 8 * k + fn;
+            T* c = pan + (size_t)(col < kb ? col : 8 * k) * ldp;
+            double x0 = ra < pm ? (double)c[ra] : 0.0, x1 = ra + 1 < pm ? (double)c[ra + 1] : 0.0;
+            dmma(x0, x1, w[k][0], v0);
+            dmma(x0, x1, w[k][1], v1);
+            __syncwarp();  // lanes of an absent column have read the column they stand on
+            if (col < kb && ra < pm) c[ra] = (T)x0;
+            if (col < kb && ra + 1 < pm) c[ra + 1] = (T)x1;
+          }
       }
     }
-    if (lane < kb)
-#pragma unroll
-      for (int j = 0; j < kNB; ++j)
-        if (j < kb) Tm[lane + (size_t)j * ldt] = t[j];
+    __syncthreads();
+  }
+  for (int e = t; e < kb * kb; e += kThreads) {
+    const int l = e % kb, j = e / kb;
+    if (l <= j) Tout[l + (size_t)j * kNB] = (T)sT[l + j * kL];
   }
 }
 

@@ -33,9 +33,15 @@ using dev::kThreads;
 using dev::kWarps;
 
 constexpr int kRed = 16;     // reduction scratch (doubles)
-// dist_qr's staged panel beyond its rows x kNB: the tpqrt's R block (kNB x
-// kNB) and the panel's Gram matrix (kNB x (kNB + 1))
-constexpr int kPanExtra = kNB * kNB + kNB * (kNB + 1);
+// dist_qr's staged panel beyond its rows x columns: the tpqrt's R block (kNB x
+// kNB) and panel_qr's scratch
+template <typename T>
+constexpr size_t pan_extra_bytes() {
+  return sizeof(T) * kNB * kNB + sizeof(double) * dev::kPanelScratch + 8;
+}
+// Rows of a staged panel: 4 mod 16, so that the four rows x eight columns of an
+// mma fragment fall on distinct banks.
+inline int panel_rows(int m) { return (m + 11) / 16 * 16 + 4; }
 constexpr int kWcap = dev::kTileSmem;  // shared scratch (doubles) of the tiled block applies of dist_qr
 constexpr int kApplyStages = 3;        // tiles staged by the chunked applies (two CTAs on an SM)
 constexpr int kApplySmem = dev::tile_smem(kApplyStages);
@@ -81,11 +87,10 @@ __global__ void k_scatter(int nnz, const double* __restrict__ val, double* const
 // `chain` holds the counter of panels that the step before has finished and the
 // one to publish this step's.
 //
-// With `pan` (ldp >= the panel's rows; ldp * pw + kPanExtra elements, pw = 32
-// columns or 16 or 8 where a whole panel does not fit; may
-// alias `tile`), the owner copies the panel into shared memory, runs the kb
-// reflector steps and the T factor there (one barrier per reflector, T by
-// one warp) and writes the panel back once.
+// With `pan` (ldp >= the panel's rows; ldp * pw elements and pan_extra_bytes, pw =
+// 32 columns or 16 or 8 where a whole panel does not fit; may alias `tile`), the
+// owner copies the panel into shared memory, factors it there (dev::panel_qr) and
+// writes it back once.
 struct ChainLink {
   const int* in = nullptr;  // panels of R finished by the step before
   int* out = nullptr;       // panels finished here
@@ -138,7 +143,7 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
       // panel rows: [j0, m) of R's columns (geqrt) or B's m rows (tpqrt)
       const int pm = unit ? m - j0 : m;
       T* pr = pan + (size_t)ldp * pw;  // tpqrt: R(j0:pend, j0:pend), ld kNB
-      T* sG = pr + kNB * kNB;           // the panel's Gram matrix (panel_t_warp)
+      double* sc = reinterpret_cast<double*>((reinterpret_cast<size_t>(pr + kNB * kNB) + 7) & ~(size_t)7);
       __syncthreads();                  // `pan` may alias the tiled apply's scratch
       for (int c = warp; c < kb; c += kWarps) {
         const T* src = unit ? (R + j0 + (size_t)(j0 + c) * ldr) : (B + (size_t)(j0 + c) * ldb);
@@ -150,111 +155,8 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
           if (r <= c) pr[r + c * kNB] = __ldcg(R + (j0 + r) + (size_t)(j0 + c) * ldr);
         }
       __syncthreads();
-      // One barrier per reflector.  Every thread forms reflector j from its
-      // alpha and the squared norm of its tail; warp w applies it to columns
-      // j + 1 + w, ... with v = tail * scal formed on the fly, and the warp of
-      // column j + 1 also sums that column's new tail for reflector j + 1.
-      // The scaled tail and beta are stored one step later, when no warp
-      // reads them.
-      __shared__ T s_nrm2[2];
-      T nrm2;
-      {
-        const int vlen = unit ? m - j0 - 1 : m;
-        const T* tail = unit ? pan + 1 : pan;
-        T sq = 0.0;
-        for (int i = threadIdx.x; i < vlen; i += kThreads) sq += tail[i] * tail[i];
-        nrm2 = dev::cta_sum(sq, red);
-      }
-      T* prev_tail = nullptr;
-      T prev_scal = 0.0;
-      int prev_vlen = 0;
-      T* prev_ajj = nullptr;
-      T prev_beta = 0.0;
-      for (int j = j0; j < pend; ++j) {
-        const int jj = j - j0;
-        const int vlen = unit ? (m - j - 1) : m;
-        T* tail = unit ? (pan + (jj + 1) + (size_t)jj * ldp) : (pan + (size_t)jj * ldp);
-        T* ajj = unit ? (pan + jj + (size_t)jj * ldp) : (pr + jj + jj * kNB);
-        const T alpha = *ajj;
-        T beta, scal;
-        const T tj = dev::house(alpha, nrm2, &beta, &scal);
-        if (prev_tail)
-          for (int i = threadIdx.x; i < prev_vlen; i += kThreads) prev_tail[i] *= prev_scal;
-        if (threadIdx.x == 0) {
-          if (prev_ajj) *prev_ajj = prev_beta;
-          lt[j] = tj;
-          tg[j] = tj;
-          // R(j, j) = 0 or not finite: the triangular solves would break down
-          if (status && !(isfinite(beta) && beta != (T)0)) atomicOr(status, isfinite(beta) ? 8 : 4);
-        }
-        // the warp's (at most four) columns together: their loads and the
-        // shuffles of their sums overlap
-        constexpr int kC = kNB / kWarps;
-        const int nk = pend - j - 1 > warp ? (pend - j - 2 - warp) / kWarps + 1 : 0;
-        if (nk > 0) {
-          T* rjk[kC];
-          T* tk[kC];
-          T d[kC];
-#pragma unroll
-          for (int u = 0; u < kC; ++u) {
-            const int kk = jj + 1 + warp + (u < nk ? u : 0) * kWarps;
-            rjk[u] = unit ? (pan + jj + (size_t)kk * ldp) : (pr + jj + kk * kNB);
-            tk[u] = unit ? (pan + (jj + 1) + (size_t)kk * ldp) : (pan + (size_t)kk * ldp);
-            d[u] = 0.0;
-          }
-          const bool next = warp == 0;  // column j + 1: also its new tail's norm
-          T sq = 0.0;
-          if (tj != 0.0) {
-#pragma unroll
-            for (int u = 0; u < kC; ++u) d[u] = lane == 0 ? *rjk[u] : (T)0.0;
-#pragma unroll 2
-            for (int i = lane; i < vlen; i += 32) {
-              const T v = tail[i] * scal;
-#pragma unroll
-              for (int u = 0; u < kC; ++u) d[u] += v * tk[u][i];
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-              for (int u = 0; u < kC; ++u) d[u] += __shfl_xor_sync(0xffffffffu, d[u], o);
-#pragma unroll
-            for (int u = 0; u < kC; ++u) {
-              d[u] *= tj;
-              if (lane == 0 && u < nk) *rjk[u] -= d[u];
-            }
-#pragma unroll 2
-            for (int i = lane; i < vlen; i += 32) {
-              const T v = tail[i] * scal;
-              T x[kC];
-#pragma unroll
-              for (int u = 0; u < kC; ++u) x[u] = tk[u][i] - v * d[u];
-#pragma unroll
-              for (int u = 0; u < kC; ++u)
-                if (u < nk) tk[u][i] = x[u];
-              if (!unit || i > 0) sq += x[0] * x[0];
-            }
-          } else if (next) {
-            for (int i = lane; i < vlen; i += 32)
-              if (!unit || i > 0) sq += tk[0][i] * tk[0][i];
-          }
-          if (next) {  // reflector j + 1's tail: rows below its diagonal
-            sq = dev::warp_sum(sq);
-            if (lane == 0) s_nrm2[(j + 1) & 1] = sq;
-          }
-        }
-        prev_tail = tj != 0.0 ? tail : nullptr;
-        prev_scal = scal;
-        prev_vlen = vlen;
-        prev_ajj = ajj;
-        prev_beta = beta;
-        __syncthreads();
-        nrm2 = s_nrm2[(j + 1) & 1];
-      }
-      if (prev_tail)
-        for (int i = threadIdx.x; i < prev_vlen; i += kThreads) prev_tail[i] *= prev_scal;
-      if (threadIdx.x == 0 && prev_ajj) *prev_ajj = prev_beta;
-      __syncthreads();
-      dev::panel_t_warp(pan, ldp, pm, kb, unit, lt + j0, Tout + (size_t)j0 * kNB + (j0 - pstart), kNB, sG);
+      dev::panel_qr(pan, ldp, pm, unit ? nullptr : pr, kb, lt + j0, tg + j0, sc, red, status,
+                    Tout + (size_t)j0 * kNB + (j0 - pstart));
       for (int c = warp; c < kb; c += kWarps) {
         T* dst = unit ? (R + j0 + (size_t)(j0 + c) * ldr) : (B + (size_t)(j0 + c) * ldb);
         for (int i = lane; i < pm; i += 32) dst[i] = pan[i + (size_t)c * ldp];
@@ -1289,7 +1191,7 @@ cudaError_t launch_permute(int n, const int* perm, const double* src, double* ds
 
 // Shared memory of a dist_qr kernel whose panels are factored in shared
 // memory: `head` bytes, then one region that serves as the tiled apply's
-// scratch and as the panel buffer (rows x pw plus kPanExtra), for the widest
+// scratch and as the panel buffer (rows x pw plus pan_extra_bytes), for the widest
 // parts of a panel that fit (32, 16 or 8 columns).  0 bytes when not even 8
 // columns fit (the kernel then factors panels in global memory).
 struct StagePlan {
@@ -1299,7 +1201,7 @@ struct StagePlan {
 template <typename T>
 StagePlan staged_panel(size_t head, int rows, size_t other_bytes = 0) {
   for (int pw = kNB; pw >= 8; pw /= 2) {
-    const size_t panel = ((size_t)rows * pw + kPanExtra) * sizeof(T);
+    const size_t panel = (size_t)rows * pw * sizeof(T) + pan_extra_bytes<T>();
     const size_t region = std::max(std::max(smem_bytes(kWcap), panel), other_bytes);
     if (head + region + 1024 <= kSmemMax) return {head + region, pw};
   }
@@ -1310,7 +1212,7 @@ cudaError_t launch_elim(const ElimTask* t, const ElimOut* o, int ntasks, int cs,
                         cudaStream_t st) {
   if (cudaError_t pre = begin("launch_elim")) return pre;
   if (ntasks <= 0) return cudaSuccess;
-  vmax = std::max(vmax, 1);
+  vmax = panel_rows(std::max(vmax, 1));
   const size_t head = smem_bytes(kRed + kNB + (size_t)nmax + (size_t)vmax);
   const StagePlan p = g_fp32 ? staged_panel<float>(head, vmax) : staged_panel<double>(head, vmax);
   const size_t b = p.bytes ? p.bytes : head + smem_bytes(kWcap);
@@ -1326,7 +1228,8 @@ cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, in
                              cudaStream_t st) {
   if (cudaError_t pre = begin("launch_elim_pipe")) return pre;
   if (nsteps <= 0) return cudaSuccess;
-  vmax = std::max(vmax, 1);
+  if (!g_status) return cudaErrorInvalidValue;  // its waits read and set the status word
+  vmax = panel_rows(std::max(vmax, 1));
   const size_t head = smem_bytes(kRed + kNB + (size_t)nmax + (size_t)vmax);
   const StagePlan p = g_fp32 ? staged_panel<float>(head, vmax) : staged_panel<double>(head, vmax);
   const size_t b = p.bytes ? p.bytes : head + smem_bytes(kWcap);
@@ -1341,7 +1244,7 @@ cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, in
 cudaError_t launch_scale(const ScaleTask* t, int ntasks, int cs, int nmax, cudaStream_t st) {
   if (cudaError_t pre = begin("launch_scale")) return pre;
   if (ntasks <= 0) return cudaSuccess;
-  nmax = std::max(nmax, 1);
+  nmax = panel_rows(std::max(nmax, 1));
   const size_t head = smem_bytes(kRed + kNB + 2 * (size_t)nmax);
   const StagePlan p = g_fp32 ? staged_panel<float>(head, nmax) : staged_panel<double>(head, nmax);
   const size_t b = p.bytes ? p.bytes : head + smem_bytes(kWcap);
@@ -1474,7 +1377,7 @@ int selected_qr_rows(int nmax) { return std::max(1, std::min(32, 12288 / (std::m
 cudaError_t launch_selected_qr(const RrqrTask* t, int ntasks, int cs, int mmax, int nmax, cudaStream_t st) {
   if (cudaError_t pre = begin("launch_selected_qr")) return pre;
   if (ntasks <= 0) return cudaSuccess;
-  const int mm = std::max(mmax, 1), nn = std::max(nmax, 1), rt = selected_qr_rows(nmax);
+  const int mm = panel_rows(std::max(mmax, 1)), nn = std::max(nmax, 1), rt = selected_qr_rows(nmax);
   const size_t head = smem_bytes(kRed + kNB + (size_t)nn + (size_t)mm);
   const size_t basis = smem_bytes((size_t)rt * (nn + 1) + 32 * 33);
   const StagePlan p = staged_panel<double>(head, mm, basis);
