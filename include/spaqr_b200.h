@@ -104,6 +104,10 @@ int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int 
  * global memory where they are used, as panels too long for shared memory are
  * (0, the default: only those). */
 int spq_debug_sweep_rows(spq_tree* t, int rows);
+
+/* For tests: levels with at most `tasks` update tasks run their trailing updates as a pipeline of ops (negative:
+ * the library's own rule).  The results are the same bit for bit. */
+int spq_debug_update_pipe(spq_tree* t, int tasks);
 /* Reuse of descriptor lists across factorizations of one partition (no
  * reference counterpart; the reference rebuilds its task graph every time,
  * ptree.cpp:885-2123).  A level's lists depend only on its cluster sizes and on

@@ -89,6 +89,12 @@ int spq_set_spin_limit(spq_tree* h, long long cycles) {
   return 0;
 }
 
+int spq_debug_update_pipe(spq_tree* h, int tasks) {
+  if (!h) return -1;
+  h->t->update_pipe = tasks;
+  return 0;
+}
+
 int spq_debug_sweep_rows(spq_tree* h, int rows) {
   if (!h || rows < 0) return -1;
   h->t->sweep_rows = rows;

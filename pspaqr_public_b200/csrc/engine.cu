@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <numeric>
+#include <unordered_map>
 
 #include "kernels.hpp"
 #include "learned.hpp"
@@ -32,6 +33,12 @@ constexpr int kChunk = 64;        // columns (rows) per CTA of the chunked appli
 // kElimPipeMixed interiors of different cluster sizes, which as whole chains run
 // one size after the other, it pays too (1024 leaves of 384^2: 15.5 and 9.8 ms).
 constexpr size_t kElimPipe = 160, kElimPipeMixed = 1024;
+// Levels with at most kUpdPipe update tasks run the ops of a task as a pipeline of
+// CTAs.  64^3 FP64, tasks whole / pipelined: 1372 tasks 11.5 / 9.2 ms, 794 13.2 / 9.1,
+// 427 14.0 / 6.1, 251 13.7 / 6.4, 48 5.8 / 2.3; 2117 6.2 / 5.5, 3593 7.3 / 7.3 and 6200
+// 4.6 / 5.5.  Between 1600 and 4000 tasks it depends on the size of the ops (leaves of
+// 384^2: 3.5 / 3.9 ms), so that the line stays below them.
+constexpr int kUpdPipe = 1600;
 constexpr int kUpdSmallMinTasks = 4096;  // small update tasks needed for the team-per-task kernel
 constexpr float kTuneMargin = 0.95f;      // tensor cores chosen where at least 5 % faster
 
@@ -405,6 +412,56 @@ static int cluster_for(int ncols) {
   return 1;
 }
 
+// The items of the pipelined updates.  An op waits for the op before on its top
+// block (the ops of one interior follow one another) and for the last op before on
+// its lower block; items are sorted by the longest way to them, so that those taken
+// together are ready together.
+static void plan_update_items(const std::vector<UpdTask>& ut, const std::vector<UpdOp>& uo, std::vector<UpdItem>& out) {
+  struct Dep {
+    int in, inb, depth;  // positions in the op list
+  };
+  std::vector<Dep> dep(uo.size());
+  std::vector<char> seen(uo.size(), 0);
+  std::unordered_map<const double*, int> last;
+  int maxd = 0;
+  for (const UpdTask& t : ut) {
+    if (t.op_begin >= t.op_end || seen[t.op_begin]) continue;  // the chunks of a cluster share its ops
+    seen[t.op_begin] = 1;
+    last.clear();
+    for (int o = t.op_begin; o < t.op_end; ++o) {
+      Dep d{-1, -1, 0};
+      if (uo[o].kind == 1) {
+        d.in = o - 1;
+        auto it = last.find(uo[o].B);
+        if (it != last.end()) d.inb = it->second;
+        last[uo[o].B] = o;
+        d.depth = dep[d.in].depth + 1;
+        if (d.inb >= 0) d.depth = std::max(d.depth, dep[d.inb].depth + 1);
+      }
+      dep[o] = d;
+      maxd = std::max(maxd, d.depth);
+    }
+  }
+  std::vector<int> at(maxd + 2, 0);
+  size_t n = 0;
+  for (const UpdTask& t : ut)
+    for (int o = t.op_begin; o < t.op_end; ++o, ++n) ++at[dep[o].depth + 1];
+  for (int d = 0; d <= maxd; ++d) at[d + 1] += at[d];
+  out.resize(n);
+  std::vector<int> id;  // item of each of a task's ops
+  for (size_t k = 0; k < ut.size(); ++k) {
+    const UpdTask& t = ut[k];
+    id.resize(t.op_end - t.op_begin);
+    for (int o = t.op_begin; o < t.op_end; ++o) {
+      const Dep& d = dep[o];
+      const int me = id[o - t.op_begin] = at[d.depth]++;
+      const int nb = dev_nb();
+      out[me] = {(int)k, o, d.in < 0 ? -1 : id[d.in - t.op_begin], d.inb < 0 ? -1 : id[d.inb - t.op_begin],
+                 d.inb < 0 ? 0 : (uo[d.inb].k + nb - 1) / nb};
+    }
+  }
+}
+
 int Tree::factorize() {
   if (!assembled_) return fail(-4, "factorize called before assemble");
   set_factor_fp32(fp32_);
@@ -454,6 +511,7 @@ int Tree::factorize() {
       // scratch is reset every level: its chunks need only start with those the
       // recorded level ended with (checked below)
       key.sizes.assign(size_.begin() + Lv.first, size_.begin() + Lv.first + Lv.count);
+      key.sizes.push_back(update_pipe);
       key.flags = (fp32_ ? 1 : 0) | (rank_model_ ? 2 : 0) | (rank_log_ ? 4 : 0) | (verbose >= 2 ? 8 : 0);
       auto prefix = [](const std::vector<const char*>& have, const std::vector<const char*>& rec) {
         return have.size() >= rec.size() && std::equal(rec.begin(), rec.end(), have.begin());
@@ -667,8 +725,26 @@ int Tree::factorize() {
       if (!d_ut || !d_uo) return fail(-11, "out of device memory (update descriptors)");
       set_tensor_cores(use_tc(lvl, 0));
       lt_[lvl].kind_tc[0] = tensor_cores_on();
-      if (ck(launch_update_small(d_ut, d_uo, nut_small, stream_), "update kernel (small blocks)") ||
-          ck(launch_update(d_ut + nut_small, d_uo, (int)ut.size() - nut_small, stream_), "update kernel"))
+      // scratch is taken whichever kind of apply runs: a stored plan's addresses
+      // behind it stay valid when the choice changes
+      const int lim = update_pipe < 0 ? kUpdPipe : update_pipe;
+      const bool few = nut_small == 0 && !ut.empty() && ut.size() <= (size_t)lim, pipe = few && !tensor_cores_on();
+      UpdItem* d_ui = nullptr;
+      int* d_cnt = nullptr;
+      size_t cnt = 0;
+      if (few) {
+        if (P.ui.empty()) plan_update_items(ut, uo, P.ui);
+        cnt = sizeof(int) * (P.ui.size() + 1);
+        d_ui = static_cast<UpdItem*>(upload(pipe ? P.ui.data() : nullptr, sizeof(UpdItem) * P.ui.size()));
+        d_cnt = static_cast<int*>(scratch_.alloc(cnt));
+        if (!d_ui || !d_cnt) return fail(-11, "out of device memory (update descriptors)");
+      }
+      if (pipe) {
+        if (ck(cudaMemsetAsync(d_cnt, 0, cnt, stream_), "update counters") ||
+            ck(launch_update_pipe(d_ut, d_uo, d_ui, (int)P.ui.size(), d_cnt, d_cnt + 1, stream_), "update kernel"))
+          return -10;
+      } else if (ck(launch_update_small(d_ut, d_uo, nut_small, stream_), "update kernel (small blocks)") ||
+                 ck(launch_update(d_ut + nut_small, d_uo, (int)ut.size() - nut_small, stream_), "update kernel"))
         return -10;
     }
     cudaEventRecord(ev[1], stream_);
@@ -1395,7 +1471,7 @@ int Tree::factorize() {
     if (ck(cudaStreamSynchronize(stream_), "factorize level")) return -10;
     if (const int ds = h_status ? *h_status : device_status()) {
       clear_status();
-      if (ds & 16) return fail(-12, "elimination pipeline wait timed out on the device at level " + std::to_string(lvl));
+      if (ds & 16) return fail(-12, "elimination or update pipeline wait timed out on the device at level " + std::to_string(lvl));
       if (ds & 2) return fail(-12, "tensor-core MMA wait timed out on the device at level " + std::to_string(lvl));
       return fail(-13, std::string(ds & 4 ? "non-finite" : "zero") + " pivot in the QR factorizations of level " +
                            std::to_string(lvl));

@@ -73,6 +73,7 @@ struct LevelPlan {
   std::vector<const char*> abase_end, sbase_end;
   std::vector<UpdTask> ut;
   std::vector<UpdOp> uo;
+  std::vector<UpdItem> ui;  // the ops as items of the pipelined updates (empty: not planned)
   double fl_upd = 0, fl_sapp = 0;
   std::vector<EdgeChunk> rows_scale, cols_scale;
   std::vector<int> sp_w;
@@ -140,6 +141,8 @@ class Tree {
   // panels of more rows than this stay in global memory during the apply (0: as
   // shared memory allows; tests); takes effect at the next factorize
   int sweep_rows = 0;
+  // levels with at most this many update tasks run their ops as a pipeline (< 0: the engine's rule)
+  int update_pipe = -1;
   // host-side checks of the trailing-update, compression and merge
   // descriptors before each upload: every block address lies in the block
   // pool (failure: status -5, nothing launched)

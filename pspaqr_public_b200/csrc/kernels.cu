@@ -332,6 +332,43 @@ __global__ void __launch_bounds__(kThreads, 2) k_update(const UpdTask* __restric
   }
 }
 
+// The ops of a task as a pipeline of CTAs, for levels with few tasks: items are
+// taken by ticket, panel p of an op runs once the op before on the same top block has
+// finished its panel p, and an op starts once the last one before on its lower block
+// is done.  A level's longest task (three times the mean) and levels with fewer tasks
+// than CTA slots left the GPU waiting for single chains of up to 60 ops.
+// 64^3 FP64: updates 94.8 -> 64.7 ms; 45^3 FP32 30.5 -> 15.8 ms; 25^3 FP64 4.85 -> 2.32.
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 2) k_update_pipe(const UpdTask* __restrict__ tasks,
+                                                          const UpdOp* __restrict__ ops,
+                                                          const UpdItem* __restrict__ items, int* ticket, int* prog,
+                                                          int* status) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ int s_item;
+  T* sm = reinterpret_cast<T*>(smraw);
+  if (threadIdx.x == 0) s_item = atomicAdd(ticket, 1);
+  __syncthreads();
+  const UpdItem it = items[s_item];
+  const UpdTask t = tasks[it.task];
+  const UpdOp op = ops[it.op];
+  T* A = as<T>(op.A) + (size_t)t.col0 * op.lda;
+  T* B = op.kind == 0 ? nullptr : as<T>(op.B) + (size_t)t.col0 * op.ldb;
+  if (it.inb >= 0 && threadIdx.x == 0) chain_wait(prog + it.inb, it.inb_panels, status);
+  for (int j0 = 0; j0 < op.k; j0 += kNB) {
+    const int kb = min(kNB, op.k - j0), unit = op.kind == 0;
+    if (it.in >= 0 && threadIdx.x == 0) chain_wait(prog + it.in, j0 / kNB + 1, status);
+    __syncthreads();
+    dev::tile_left_qt<T>(as<T>(op.V) + (unit ? j0 : 0) + (size_t)j0 * op.ldv, op.ldv, as<T>(op.T) + (size_t)j0 * kNB, kNB,
+                         kb, unit, unit ? nullptr : A + j0, op.lda, unit ? A + j0 : B, unit ? op.lda : op.ldb,
+                         unit ? op.m - j0 : op.m, t.ncols, sm, 0, kApplyStages);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(prog + s_item), "r"(j0 / kNB + 1) : "memory");
+    }
+  }
+}
+
 // row scaling: columns [lo, lo+cnt) of A <- Qs^T A
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 2) k_edge_left(const EdgeChunk* __restrict__ tasks) {
@@ -1272,6 +1309,21 @@ cudaError_t launch_update(const UpdTask* t, const UpdOp* o, int ntasks, cudaStre
     k_update<double><<<ntasks, kThreads, b, st>>>(t, o);
   }
   return last();
+}
+
+cudaError_t launch_update_pipe(const UpdTask* t, const UpdOp* o, const UpdItem* items, int nitems, int* ticket,
+                               int* prog, cudaStream_t st) {
+  if (cudaError_t pre = begin("launch_update_pipe")) return pre;
+  if (nitems <= 0) return cudaSuccess;
+  if (!g_status) return cudaErrorInvalidValue;  // its waits read and set the status word
+  const size_t b = smem_bytes(kApplySmem);
+  counted();
+  auto go = [&](auto kern) {
+    if (cudaError_t e = prep(kern, b)) return e;
+    kern<<<nitems, kThreads, b, st>>>(t, o, items, ticket, prog, g_status);
+    return last();
+  };
+  return g_fp32 ? go(k_update_pipe<float>) : go(k_update_pipe<double>);
 }
 
 cudaError_t launch_edge(int kind, const EdgeChunk* t, int ntasks, cudaStream_t st) {

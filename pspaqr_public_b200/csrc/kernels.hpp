@@ -50,6 +50,10 @@ cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, in
                              cudaStream_t st);
 cudaError_t launch_scale(const ScaleTask* t, int ntasks, int cs, int nmax, cudaStream_t st);
 cudaError_t launch_update(const UpdTask* t, const UpdOp* o, int ntasks, cudaStream_t st);
+// The same updates with every op of a task an item of its own (CUDA cores and FP64
+// mma only); ticket and the items' progress counters must be zero.
+cudaError_t launch_update_pipe(const UpdTask* t, const UpdOp* o, const UpdItem* items, int nitems, int* ticket,
+                               int* prog, cudaStream_t st);
 // kind 0: left apply on column chunks, 1: right triangular solve on row chunks,
 // 2: right apply on row chunks
 cudaError_t launch_edge(int kind, const EdgeChunk* t, int ntasks, cudaStream_t st);

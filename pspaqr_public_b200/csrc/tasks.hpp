@@ -53,6 +53,14 @@ struct UpdOp {
   int kind, k, m, ldv, lda, ldb;
 };
 
+// One op of one task in the pipelined form of the trailing updates.  in: the item of
+// the op before on the same top block (followed panel by panel), inb: the last item
+// before on the same lower block (waited for as a whole, its `inb_panels` panels); -1:
+// none.  Items stand behind those that they wait for.
+struct UpdItem {
+  int task, op, in, inb, inb_panels;
+};
+
 // Distributed geqrt of one diagonal block (scaling QR, ptree.cpp:269-286).
 struct ScaleTask {
   double* S;
