@@ -339,10 +339,21 @@ __device__ void panel_qr(T* pan, int ldp, int pm, T* pr, int kb, T* lt, T* tg, d
 // ---------------------------------------------------------------- tiled matrix applies
 constexpr int kNC = 64;   // columns (rows for right applies) per pass
 constexpr int kRT = 32;   // rows (columns) per shared-memory tile
-constexpr int kLdV = 40;  // column stride of the V, T and left C tiles (8 mod 16: 16-byte fragment
-                          // loads of two columns a quarter-warp fall on distinct banks)
+constexpr int kLdC = 40;  // column stride of the left C tiles (8 mod 16: the 16-byte fragment loads of two
+                          // neighbouring columns a quarter-warp fall on distinct banks)
 constexpr int kLdR = 66;  // row stride of the right C tiles (2 mod 8: 8-byte fragments, likewise)
-constexpr int kTileV = kNB * kLdV, kTileC = kNC * kLdV;
+constexpr int kLdV = 36;  // column stride of the V and T tiles (4 mod 16, with frag_col)
+constexpr int kTileV = kNB * kLdV, kTileC = kNC * kLdC;
+// Column of a group of eight that fragment lane n of an mma's B operand takes, and so
+// accumulator n of a row: 0 2 1 3 6 4 7 5.  Lanes 2 l and 2 l + 1 stand two columns
+// apart (the 16-byte loads of a quarter-warp), accumulators 2 fk of the four lanes of
+// a row, and 2 fk + 1, hold columns that differ mod 4 (the 8-byte loads of the
+// second product): with kLdV both are free of bank conflicts.  With columns
+// 0 4 1 5 2 6 3 7 and kLdV = 40 both took two wavefronts for one, and shared memory
+// bounded the applies (L1 data pipe 77 % busy): 64^3 FP64 updates 64.7 -> 57.5 ms, scaling
+// applies 50.0 -> 41.6; FP32 factors updates 68 -> 59.5, scaling and compression applies
+// 87 -> 76 ms.
+__device__ __forceinline__ int frag_col(int n) { return (0x57463120 >> (4 * n)) & 15; }
 static_assert(kRT * kLdR <= kTileC, "right tiles");
 // Shared memory (doubles) of mma_apply with `stages` tiles of V and C.
 __host__ __device__ constexpr int tile_smem(int stages) { return stages * (kTileV + kTileC) + kTileV + 2; }
@@ -369,9 +380,8 @@ __device__ __forceinline__ T ld_v(const T* p) {
 // staged and rounded once when they are stored: more accurate than FP32 sums,
 // and faster than the FP32 pipes ran here).  Warp w owns vectors 8 w .. 8 w + 7
 // from start to end, so that w never leaves its registers: the accumulators of
-// one product are the A fragments of the next when fragment lane fn of the B
-// operand takes column (fn >> 1) + 4 (fn & 1) (`perm`), which makes accumulator
-// 2 fk + e column fk + 4 e.  Only tiles of V (and C) are shared, one barrier a
+// one product are the A fragments of the next, with the columns of a group of eight
+// in the order of frag_col.  Only tiles of V (and C) are shared, one barrier a
 // tile, `stages` tiles in shared memory; the second pass runs backwards, over the
 // tiles that are still there first.  Before, with W, the partial sums of the row
 // sets, T and W2 exchanged through shared memory on the FP64 (FP32) pipes, a
@@ -386,7 +396,8 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
   double* sV0 = sT + kTileV;
   double* sC0 = sV0 + stages * kTileV;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int fn = lane >> 2, fk = lane & 3, perm = (fn >> 1) + 4 * (fn & 1);
+  const int fn = lane >> 2, fk = lane & 3, perm = frag_col(fn);
+  const int fc[2] = {frag_col(2 * fk), frag_col(2 * fk + 1)};
   auto col = [&](int c) { return (size_t)(c + (c / kNB) * cgap); };
   // staging: V by (row = lane, four columns a warp); left C by (row = lane, the
   // warp's eight columns), right C by (vector = t % 64, columns t / 64 + 4 q): a
@@ -423,7 +434,7 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
 #pragma unroll
     for (int q = 0; q < kSC; ++q) {
       if (kRight) dc[(cr + 4 * q) * kLdR + cv] = (double)rc[q];
-      else dc[(warp * kSC + q) * kLdV + lane] = (double)rc[q];
+      else dc[(warp * kSC + q) * kLdC + lane] = (double)rc[q];
     }
   };
   const int ntile = (m + kRT - 1) / kRT;
@@ -446,7 +457,7 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
   for (int b = 0; b < 4; ++b)
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const int i = 8 * b + fk + 4 * e;
+      const int i = 8 * b + fc[e];
       a[b][e] = !unit && i < kb && have ? (double)ld_v<kCg>(A + i + col(c) * lda) : 0.0;
       w[b][e] = a[b][e];
     }
@@ -465,7 +476,7 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
         x.x = sC[(rr + 2 * fk) * kLdR + c];
         x.y = sC[(rr + 2 * fk + 1) * kLdR + c];
       } else {
-        x = *reinterpret_cast<const double2*>(sC + c * kLdV + rr + 2 * fk);
+        x = *reinterpret_cast<const double2*>(sC + c * kLdC + rr + 2 * fk);
       }
       double2 v[4];
 #pragma unroll
@@ -487,14 +498,14 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
 #pragma unroll
     for (int b = 0; b <= j; ++b)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) dmma(w2[j][0], w2[j][1], w[b][e], sT[(8 * j + perm) * kLdV + 8 * b + fk + 4 * e]);
+      for (int e = 0; e < 2; ++e) dmma(w2[j][0], w2[j][1], w[b][e], sT[(8 * j + perm) * kLdV + 8 * b + fc[e]]);
   }
   if (!unit)
 #pragma unroll
     for (int b = 0; b < 4; ++b)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int i = 8 * b + fk + 4 * e;
+        const int i = 8 * b + fc[e];
         if (i < kb && have) A[i + col(c) * lda] = (T)(a[b][e] - w2[b][e]);
       }
 #pragma unroll
@@ -517,7 +528,7 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
         x[u][0] = sC[(8 * u + 2 * fk) * kLdR + c];
         x[u][1] = sC[(8 * u + 2 * fk + 1) * kLdR + c];
       } else {
-        const double2 y = *reinterpret_cast<const double2*>(sC + c * kLdV + 8 * u + 2 * fk);
+        const double2 y = *reinterpret_cast<const double2*>(sC + c * kLdC + 8 * u + 2 * fk);
         x[u][0] = y.x;
         x[u][1] = y.y;
       }
@@ -528,7 +539,7 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
       for (int e = 0; e < 2; ++e)
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-          dmma(x[u][0], x[u][1], w2[b][e], sV[(8 * b + fk + 4 * e) * kLdV + 8 * u + fn]);
+          dmma(x[u][0], x[u][1], w2[b][e], sV[(8 * b + fc[e]) * kLdV + 8 * u + fn]);
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -594,7 +605,8 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
   double* sV0 = sT + kTileV;
   double* sC0 = sV0 + stages * kTileV;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int fn = lane >> 2, fk = lane & 3, perm = (fn >> 1) + 4 * (fn & 1);
+  const int fn = lane >> 2, fk = lane & 3, perm = frag_col(fn);
+  const int fc[2] = {frag_col(2 * fk), frag_col(2 * fk + 1)};
   constexpr int kSV = kNB / kWarps, kSC = kRT * kNC / kThreads;
   T rv[kSV], rc[kSC];
   const int cv = t % kNC, cr = t / kNC, c = 8 * warp + fn;
@@ -624,7 +636,7 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
     for (int b = 0; b < 4; ++b)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int j = 8 * b + fk + 4 * e;
+        const int j = 8 * b + fc[e];
         x[b][e] = j < jb && have ? (double)C[c + (size_t)(j0 + j) * ldc] : 0.0;
         w[b][e] = 0.0;
       }
@@ -662,13 +674,13 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
       for (int b = 0; b <= j; ++b)
 #pragma unroll
         for (int e = 0; e < 2; ++e)
-          dmma(y[j][0], y[j][1], x[b][e] - w[b][e], sT[(8 * j + perm) * kLdV + 8 * b + fk + 4 * e]);
+          dmma(y[j][0], y[j][1], x[b][e] - w[b][e], sT[(8 * j + perm) * kLdV + 8 * b + fc[e]]);
     }
 #pragma unroll
     for (int b = 0; b < 4; ++b)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int j = 8 * b + fk + 4 * e;
+        const int j = 8 * b + fc[e];
         if (j < jb && have) C[c + (size_t)(j0 + j) * ldc] = (T)y[b][e];
       }
     __syncthreads();  // X_J before it is read, T before it is overwritten
