@@ -461,6 +461,13 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
       a[b][e] = !unit && i < kb && have ? (double)ld_v<kCg>(A + i + col(c) * lda) : 0.0;
       w[b][e] = a[b][e];
     }
+  // Blocks of eight reflectors that meet the eight rows from r on: none past the last
+  // row or without vectors, none whose unit triangle starts below.  A tile that all of
+  // them meet takes the code without tests (and so does every tile of a distributed
+  // QR, whose blocks are large: its registers do not hold both).
+  const int nb = 8 * warp < nc ? (kb + 7) / 8 : 0;
+  auto blocks = [&](int r) { return r >= m ? 0 : unit ? min(nb, r / 8 + 1) : nb; };
+  auto full = [&](int tt) { return nb == 4 && (tt + 1) * kRT - 8 < m && !(unit && tt == 0); };
   // ---- w = c V (+ a)
   if (ntile > 0) stash(0);
   __syncthreads();
@@ -469,22 +476,42 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
     if (more) load(tt + 1);
     const double* sV = sV0 + (tt % stages) * kTileV;
     const double* sC = sC0 + (tt % stages) * kTileC;
+    if (kCg || full(tt)) {
 #pragma unroll
-    for (int rr = 0; rr < kRT; rr += 8) {
-      double2 x;
-      if (kRight) {
-        x.x = sC[(rr + 2 * fk) * kLdR + c];
-        x.y = sC[(rr + 2 * fk + 1) * kLdR + c];
-      } else {
-        x = *reinterpret_cast<const double2*>(sC + c * kLdC + rr + 2 * fk);
+      for (int rr = 0; rr < kRT; rr += 8) {
+        double2 x;
+        if (kRight) {
+          x.x = sC[(rr + 2 * fk) * kLdR + c];
+          x.y = sC[(rr + 2 * fk + 1) * kLdR + c];
+        } else {
+          x = *reinterpret_cast<const double2*>(sC + c * kLdC + rr + 2 * fk);
+        }
+        double2 v[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) v[b] = *reinterpret_cast<const double2*>(sV + (8 * b + perm) * kLdV + rr + 2 * fk);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], x.x, v[b].x);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], x.y, v[b].y);
       }
-      double2 v[4];
+    } else {
+#pragma unroll 1
+      for (int rr = 0, bl; rr < kRT && (bl = blocks(tt * kRT + rr)) > 0; rr += 8) {
+        double2 x;
+        if (kRight) {
+          x.x = sC[(rr + 2 * fk) * kLdR + c];
+          x.y = sC[(rr + 2 * fk + 1) * kLdR + c];
+        } else {
+          x = *reinterpret_cast<const double2*>(sC + c * kLdC + rr + 2 * fk);
+        }
 #pragma unroll
-      for (int b = 0; b < 4; ++b) v[b] = *reinterpret_cast<const double2*>(sV + (8 * b + perm) * kLdV + rr + 2 * fk);
-#pragma unroll
-      for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], x.x, v[b].x);
-#pragma unroll
-      for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], x.y, v[b].y);
+        for (int b = 0; b < 4; ++b)
+          if (b < bl) {
+            const double2 v = *reinterpret_cast<const double2*>(sV + (8 * b + perm) * kLdV + rr + 2 * fk);
+            dmma(w[b][0], w[b][1], x.x, v.x);
+            dmma(w[b][0], w[b][1], x.y, v.y);
+          }
+      }
     }
     // with two or more stages the next tile's buffer was last read a barrier ago
     if (more) stash(tt + 1);
@@ -497,6 +524,7 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
     w2[j][0] = w2[j][1] = 0.0;
 #pragma unroll
     for (int b = 0; b <= j; ++b)
+      if (kCg || j < nb)
 #pragma unroll
       for (int e = 0; e < 2; ++e) dmma(w2[j][0], w2[j][1], w[b][e], sT[(8 * j + perm) * kLdV + 8 * b + fc[e]]);
   }
@@ -533,13 +561,26 @@ __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int
         x[u][1] = y.y;
       }
     }
+    if (kCg || full(tt)) {
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
+      for (int b = 0; b < 4; ++b)
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
+        for (int e = 0; e < 2; ++e)
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          dmma(x[u][0], x[u][1], w2[b][e], sV[(8 * b + fc[e]) * kLdV + 8 * u + fn]);
+          for (int u = 0; u < 4; ++u)
+            dmma(x[u][0], x[u][1], w2[b][e], sV[(8 * b + fc[e]) * kLdV + 8 * u + fn]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int bl = blocks(tt * kRT + 8 * u);
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          if (b < bl)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              dmma(x[u][0], x[u][1], w2[b][e], sV[(8 * b + fc[e]) * kLdV + 8 * u + fn]);
+      }
+    }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -613,6 +654,7 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
   const bool have = c < m;
   for (int j0 = 0; j0 < n; j0 += kNB) {
     const int jb = min(kNB, n - j0), ntile = j0 / kRT;
+    const int nb = 8 * warp < m ? (jb + 7) / 8 : 0;  // blocks of eight columns
     auto load = [&](int tt) {
 #pragma unroll
       for (int q = 0; q < kSV; ++q) {
@@ -652,16 +694,30 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
       if (more) load(tt + 1);
       const double* sV = sV0 + (tt % stages) * kTileV;
       const double* sC = sC0 + (tt % stages) * kTileC;
+      if (nb == 4) {
 #pragma unroll
-      for (int rr = 0; rr < kRT; rr += 8) {
-        const double a0 = sC[(rr + 2 * fk) * kLdR + c], a1 = sC[(rr + 2 * fk + 1) * kLdR + c];
-        double2 v[4];
+        for (int rr = 0; rr < kRT; rr += 8) {
+          const double a0 = sC[(rr + 2 * fk) * kLdR + c], a1 = sC[(rr + 2 * fk + 1) * kLdR + c];
+          double2 v[4];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) v[b] = *reinterpret_cast<const double2*>(sV + (8 * b + perm) * kLdV + rr + 2 * fk);
+          for (int b = 0; b < 4; ++b) v[b] = *reinterpret_cast<const double2*>(sV + (8 * b + perm) * kLdV + rr + 2 * fk);
 #pragma unroll
-        for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], a0, v[b].x);
+          for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], a0, v[b].x);
 #pragma unroll
-        for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], a1, v[b].y);
+          for (int b = 0; b < 4; ++b) dmma(w[b][0], w[b][1], a1, v[b].y);
+        }
+      } else {
+#pragma unroll 1
+        for (int rr = 0; rr < kRT && nb > 0; rr += 8) {
+          const double a0 = sC[(rr + 2 * fk) * kLdR + c], a1 = sC[(rr + 2 * fk + 1) * kLdR + c];
+#pragma unroll
+          for (int b = 0; b < 4; ++b)
+            if (b < nb) {
+              const double2 v = *reinterpret_cast<const double2*>(sV + (8 * b + perm) * kLdV + rr + 2 * fk);
+              dmma(w[b][0], w[b][1], a0, v.x);
+              dmma(w[b][0], w[b][1], a1, v.y);
+            }
+        }
       }
       if (more) stash(tt + 1);
       __syncthreads();
@@ -672,9 +728,10 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
       y[j][0] = y[j][1] = 0.0;
 #pragma unroll
       for (int b = 0; b <= j; ++b)
+        if (j < nb)
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-          dmma(y[j][0], y[j][1], x[b][e] - w[b][e], sT[(8 * j + perm) * kLdV + 8 * b + fc[e]]);
+          for (int e = 0; e < 2; ++e)
+            dmma(y[j][0], y[j][1], x[b][e] - w[b][e], sT[(8 * j + perm) * kLdV + 8 * b + fc[e]]);
     }
 #pragma unroll
     for (int b = 0; b < 4; ++b)

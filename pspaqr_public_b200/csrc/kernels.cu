@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_edge_right_small(const EdgeChun
 
 // right compression: rows [lo, lo+cnt) of A <- A Q
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_edge_right(const EdgeChunk* __restrict__ tasks) {
+__global__ void __launch_bounds__(kThreads, 2) k_edge_right(const EdgeChunk* __restrict__ tasks) {
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);
   const EdgeChunk t = tasks[blockIdx.x];
