@@ -632,13 +632,38 @@ __device__ void mat_apply_q_right(const T* V, int ldv, const T* Tm, int k, T* C,
   }
 }
 
+// Inverse of an upper triangular kb x kb block (kb <= 32) by one warp with 32 x 33
+// doubles of scratch; lane j forms column j of `out` (32 x 32).  A zero on the diagonal
+// gives a zero row and column: the column that it belongs to drops out of the solve.
+__device__ inline void diag_inverse(const double* R, int ld, int kb, double* s, double* out) {
+  const int lane = threadIdx.x & 31;
+  for (int j = 0; j < kb; ++j)
+    if (lane <= j) s[lane * (kNB + 1) + j] = __ldcg(R + lane + (size_t)j * ld);
+  __syncwarp();
+  double x[32];
+#pragma unroll
+  for (int l = kNB - 1; l >= 0; --l) {
+    double v = l == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int q = l + 1; q < kNB; ++q)
+      if (q <= lane && q < kb) v -= s[l * (kNB + 1) + q] * x[q];
+    const double d = l <= lane && lane < kb ? s[l * (kNB + 1) + l] : 0.0;
+    x[l] = d != 0.0 ? v / d : 0.0;
+  }
+  if (lane < kb)
+#pragma unroll
+    for (int l = 0; l < 32; ++l) out[l + lane * 32] = x[l];
+  __syncwarp();
+}
+
 // C (m <= kNC rows x n) <- C R^{-1}, R upper triangular (n x n), left-looking by
 // blocks of 32 columns: X_J = (C_J - X(:, 0:j0) R(0:j0, J)) R_JJ^{-1} with the
 // inverses of R's diagonal blocks given (block b at Inv + 32 * 32 b, column-major,
 // FP64).  Both products on FP64 mma as in mma_apply: warp w owns rows 8 w ..
 // 8 w + 7, tiles of X and R are shared.  (Substitution inside the diagonal blocks,
-// one thread a row, took longer than the products.)
-template <typename T>
+// one thread a row, took longer than the products.)  kCg: R and the inverses are read
+// through L2.
+template <typename T, bool kCg = false>
 __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int ldc, int m, int n, double* sm,
                                int stages) {
   sm = reinterpret_cast<double*>((reinterpret_cast<size_t>(sm) + 15) & ~(size_t)15);
@@ -659,7 +684,7 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
 #pragma unroll
       for (int q = 0; q < kSV; ++q) {
         const int i = warp * kSV + q;
-        rv[q] = i < jb ? R[tt * kRT + lane + (size_t)(j0 + i) * ldr] : (T)0;
+        rv[q] = i < jb ? ld_v<kCg>(R + tt * kRT + lane + (size_t)(j0 + i) * ldr) : (T)0;
       }
 #pragma unroll
       for (int q = 0; q < kSC; ++q) rc[q] = cv < m ? C[cv + (size_t)(tt * kRT + cr + 4 * q) * ldc] : (T)0;
@@ -685,7 +710,7 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
 #pragma unroll
     for (int q = 0; q < kNB * kNB / kThreads; ++q) {
       const int j = warp + q * kWarps;
-      sT[j * kLdV + lane] = lane <= j && j < jb ? Inv[lane + (size_t)(j0 + j) * kNB] : 0.0;
+      sT[j * kLdV + lane] = lane <= j && j < jb ? ld_v<kCg>(Inv + lane + (size_t)(j0 + j) * kNB) : 0.0;
     }
     if (ntile > 0) stash(0);
     __syncthreads();

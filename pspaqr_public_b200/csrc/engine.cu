@@ -39,7 +39,11 @@ constexpr size_t kElimPipe = 160, kElimPipeMixed = 1024;
 // 4.6 / 5.5.  Between 1600 and 4000 tasks it depends on the size of the ops (leaves of
 // 384^2: 3.5 / 3.9 ms), so that the line stays below them.
 constexpr int kUpdPipe = 1600;
-constexpr int kUpdSmallMinTasks = 4096;  // small update tasks needed for the team-per-task kernel
+// Levels with at least kUpdSmallMinTasks update tasks whose ops all have at most
+// kUpdSmallOp reflectors and rows keep those off the tensor cores.  (FP64 mma with
+// FP32 factors: 64^3 level 0 6.2 ms; a 64-thread team a task on the FP32 pipes,
+// before: 13.1 ms.)
+constexpr int kUpdSmallMinTasks = 4096, kUpdSmallOp = 64;
 constexpr float kTuneMargin = 0.95f;      // tensor cores chosen where at least 5 % faster
 
 // Row scaling / left compression chunks of the FP32 factorization: those of
@@ -706,18 +710,16 @@ int Tree::factorize() {
                                   " addresses memory outside the block pool; nothing launched");
           }
       }
-      // FP32: tasks whose ops are all small first, for the team-per-task kernel
-      // (stable, so a stored plan stays partitioned)
+      // FP32: tasks whose ops are all small first (stable, so a stored plan stays
+      // partitioned)
       int nut_small = 0;
       if (fp32_) {
         const auto mid = std::stable_partition(ut.begin(), ut.end(), [&](const UpdTask& u) {
           for (int o = u.op_begin; o < u.op_end; ++o)
-            if (!update_op_small(uo[o].k, uo[o].m)) return false;
+            if (uo[o].k > kUpdSmallOp || uo[o].m > kUpdSmallOp) return false;
           return true;
         });
         nut_small = (int)(mid - ut.begin());
-        // a team runs one op chain slower than a CTA does: the team kernel pays
-        // only where there are enough small tasks to fill the GPU many times
         if (nut_small < kUpdSmallMinTasks) nut_small = 0;
       }
       auto* d_ut = static_cast<UpdTask*>(upload(ut.data(), sizeof(UpdTask) * ut.size()));
@@ -728,7 +730,7 @@ int Tree::factorize() {
       // scratch is taken whichever kind of apply runs: a stored plan's addresses
       // behind it stay valid when the choice changes
       const int lim = update_pipe < 0 ? kUpdPipe : update_pipe;
-      const bool few = nut_small == 0 && !ut.empty() && ut.size() <= (size_t)lim, pipe = few && !tensor_cores_on();
+      const bool few = !ut.empty() && ut.size() <= (size_t)lim, pipe = few && !tensor_cores_on();
       UpdItem* d_ui = nullptr;
       int* d_cnt = nullptr;
       size_t cnt = 0;
@@ -743,9 +745,14 @@ int Tree::factorize() {
         if (ck(cudaMemsetAsync(d_cnt, 0, cnt, stream_), "update counters") ||
             ck(launch_update_pipe(d_ut, d_uo, d_ui, (int)P.ui.size(), d_cnt, d_cnt + 1, stream_), "update kernel"))
           return -10;
-      } else if (ck(launch_update_small(d_ut, d_uo, nut_small, stream_), "update kernel (small blocks)") ||
-                 ck(launch_update(d_ut + nut_small, d_uo, (int)ut.size() - nut_small, stream_), "update kernel"))
-        return -10;
+      } else {
+        const bool tc = tensor_cores_on();
+        if (!tc) nut_small = 0;
+        set_tensor_cores(false);
+        if (ck(launch_update(d_ut, d_uo, nut_small, stream_), "update kernel (small blocks)")) return -10;
+        set_tensor_cores(tc);
+        if (ck(launch_update(d_ut + nut_small, d_uo, (int)ut.size() - nut_small, stream_), "update kernel")) return -10;
+      }
     }
     cudaEventRecord(ev[1], stream_);
     // ---------------- scaling + sparsification
@@ -1196,9 +1203,10 @@ int Tree::factorize() {
             r.V = spV[q];
             r.T = spT[q];
             r.tau = scratch_.dalloc(std::max(t.m, 1));
+            r.Rinv = scratch_.dalloc((size_t)NB * NB * ((l + NB - 1) / NB));
             r.colat = t.colat;
             r.rank = d_ell + q;
-            if (!t.G || !t.Lt || !t.colat || !r.tau) return fail(-11, "out of device memory (sketch)");
+            if (!t.G || !t.Lt || !t.colat || !r.tau || !r.Rinv) return fail(-11, "out of device memory (sketch)");
             for (int r0 = 0; r0 < ell[q]; r0 += 64)
               for (int c0 = r0; c0 < ell[q]; c0 += 64) gram_tiles.push_back({(int)q, r0, c0});
             const int cs = cluster_for(ell[q]);

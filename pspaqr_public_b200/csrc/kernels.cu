@@ -42,6 +42,7 @@ constexpr size_t pan_extra_bytes() {
 // Rows of a staged panel: 4 mod 16, so that the four rows x eight columns of an
 // mma fragment fall on distinct banks.
 inline int panel_rows(int m) { return (m + 11) / 16 * 16 + 4; }
+static_assert(kWarps * kNB * (kNB + 1) <= dev::kTileSmem, "k_selected_qr's diagonal blocks");
 constexpr int kWcap = dev::kTileSmem;  // shared scratch (doubles) of the tiled block applies of dist_qr
 constexpr int kApplyStages = 3;        // tiles staged by the chunked applies (two CTAs on an SM)
 constexpr int kApplySmem = dev::tile_smem(kApplyStages);
@@ -502,173 +503,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_edge_left_small(const EdgeChunk
   }
 }
 
-// Trailing updates of small column chunks (FP32 factors): one team of 64
-// threads per chunk, kTeams teams per 128-thread CTA, synchronised by their
-// own named barrier.  Every op of the chunk's chain has at most 64
-// reflectors and 64 rows.  The ops of one interior c (its geqrt apply, then
-// its tsqrt steps) all update the same block A(c, m): per 32-column half, the
-// team keeps that block in shared memory across the whole run of ops with
-// the same A and brings in only each step's neighbour block B(n, m) and the
-// reflector panels; every panel of an op is applied before B is written back.
-// Per panel: thread r stages row r of the panel of V (registers and shared
-// memory); thread t forms W(t mod 32, 16 columns) = V^T C (+ the top rows of
-// A for a tsqrt step), then W2 = T^T W; thread r updates its row.
-constexpr int kTeam = 64;
-constexpr int kTeams = 2;  // teams per CTA
-constexpr int kTeamThreads = kTeam * kTeams;
-constexpr int kSmallOp = 64;  // rows, reflectors and columns of an op on the small path
-// floats per team: A, B, V panel (64 x kSmallLd each), W (32 x kSmallLd), T (32 x 33)
-constexpr size_t kTeamSmem = (size_t)(3 * kSmallOp + kNB) * kSmallLd + kNB * (kNB + 1);
-constexpr size_t kUpdSmallSmem = kTeams * kTeamSmem * sizeof(float);
-
-__device__ __forceinline__ void team_sync(int team) {
-  asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(kTeam) : "memory");
-}
-
-// One panel (reflectors j0 .. j0 + kb) of an op on blocks in shared memory:
-// kind 0: C = sA rows [j0, m) <- Q^T C (V unit lower, rows j0 ..);
-// kind 1: [sA rows j0 .. j0 + kb; sB rows 0 .. m) <- Q^T [.] (V full, m rows).
-__device__ __forceinline__ void team_panel(const UpdOp& op, int j0, int kb, float* sA, float* sB, float* sV,
-                                           float* sW, float* sT, int team, int tl) {
-  const int r0 = op.kind ? 0 : j0;
-  const int nr = op.m - r0;
-  float* sC = op.kind ? sB : sA + (size_t)j0 * kSmallLd;  // rows r0 .. of the block V acts on
-  const float* V = as<float>(op.V);
-  const float* Tm = as<float>(op.T) + (size_t)j0 * kNB;
-  float vrow[kNB];
-#pragma unroll
-  for (int i = 0; i < kNB; ++i) {
-    float v = 0.0f;
-    if (tl < nr && i < kb) {
-      const int r = r0 + tl;
-      v = op.kind ? V[r + (size_t)(j0 + i) * op.ldv]
-                  : (tl == i ? 1.0f : (tl < i ? 0.0f : V[r + (size_t)(j0 + i) * op.ldv]));
-    }
-    vrow[i] = v;
-    sV[tl * kSmallLd + i] = v;
-  }
-  for (int e = tl; e < kNB * kNB; e += kTeam) {  // T transposed: sT[i * 33 + l] = T(l, i)
-    const int l = e % kNB, i = e / kNB;
-    sT[i * (kNB + 1) + l] = (l <= i && i < kb) ? Tm[l + (size_t)i * kNB] : 0.0f;
-  }
-  team_sync(team);
-  const int wi = tl & 31, jc = (tl >> 5) * 16;
-  float w[16];
-#pragma unroll
-  for (int u = 0; u < 16; ++u) w[u] = (op.kind && wi < kb) ? sA[(j0 + wi) * kSmallLd + jc + u] : 0.0f;
-  for (int r = 0; r < nr; ++r) {
-    const float vri = sV[r * kSmallLd + wi];
-    const float4* cr = reinterpret_cast<const float4*>(sC + r * kSmallLd + jc);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 x = cr[q];
-      w[4 * q] += vri * x.x;
-      w[4 * q + 1] += vri * x.y;
-      w[4 * q + 2] += vri * x.z;
-      w[4 * q + 3] += vri * x.w;
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < 16; ++u) sW[wi * kSmallLd + jc + u] = w[u];
-  team_sync(team);
-#pragma unroll
-  for (int u = 0; u < 16; ++u) w[u] = 0.0f;
-  for (int l = 0; l < kb; ++l) {
-    const float tlw = sT[wi * (kNB + 1) + l];  // T(l, wi); zero unless l <= wi < kb
-    const float4* wl = reinterpret_cast<const float4*>(sW + l * kSmallLd + jc);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 x = wl[q];
-      w[4 * q] += tlw * x.x;
-      w[4 * q + 1] += tlw * x.y;
-      w[4 * q + 2] += tlw * x.z;
-      w[4 * q + 3] += tlw * x.w;
-    }
-  }
-  team_sync(team);
-#pragma unroll
-  for (int u = 0; u < 16; ++u) sW[wi * kSmallLd + jc + u] = w[u];
-  team_sync(team);
-  if (op.kind)  // the top rows: A(j0 + i, .) -= W2(i, .)
-    for (int e = tl; e < kb * 32; e += kTeam) {
-      const int i = e >> 5, j = e & 31;
-      sA[(j0 + i) * kSmallLd + j] -= sW[i * kSmallLd + j];
-    }
-  if (tl < nr) {  // C(r, .) -= V(r, :) W2
-    float acc[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) acc[j] = 0.0f;
-#pragma unroll
-    for (int i = 0; i < kNB; ++i) {
-      if (i < kb) {
-        const float vi = vrow[i];
-        const float4* wr = reinterpret_cast<const float4*>(sW + i * kSmallLd);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 x = wr[q];
-          acc[4 * q] += vi * x.x;
-          acc[4 * q + 1] += vi * x.y;
-          acc[4 * q + 2] += vi * x.z;
-          acc[4 * q + 3] += vi * x.w;
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 32; ++j) sC[tl * kSmallLd + j] -= acc[j];
-  }
-  team_sync(team);
-}
-
-__global__ void __launch_bounds__(kTeamThreads, 3) k_update_small(const UpdTask* __restrict__ tasks,
-                                                              const UpdOp* __restrict__ ops, int ntasks) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int team = threadIdx.x / kTeam, tl = threadIdx.x % kTeam;
-  const int ti = blockIdx.x * kTeams + team;
-  if (ti >= ntasks) return;  // the whole team
-  float* sA = reinterpret_cast<float*>(smraw) + (size_t)team * kTeamSmem;  // sA[r * ld + j] = A(r, h + j)
-  float* sB = sA + kSmallOp * kSmallLd;                                    // sB[r * ld + j] = B(r, h + j)
-  float* sV = sB + kSmallOp * kSmallLd;
-  float* sW = sV + kSmallOp * kSmallLd;
-  float* sT = sW + kNB * kSmallLd;
-  const UpdTask t = tasks[ti];
-  for (int h = 0; h < t.ncols; h += 32) {
-    const int hc = min(32, t.ncols - h);
-    int o = t.op_begin;
-    while (o < t.op_end) {
-      const double* Aid = ops[o].A;
-      float* A = as<float>(ops[o].A) + (size_t)(t.col0 + h) * ops[o].lda;
-      const int lda = ops[o].lda;
-      const int arows = ops[o].kind ? ops[o].k : ops[o].m;
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        sA[tl * kSmallLd + j] = (tl < arows && j < hc) ? A[tl + (size_t)j * lda] : 0.0f;
-      team_sync(team);
-      for (; o < t.op_end && ops[o].A == Aid; ++o) {
-        const UpdOp op = ops[o];
-        float* B = nullptr;
-        if (op.kind) {
-          B = as<float>(op.B) + (size_t)(t.col0 + h) * op.ldb;
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            sB[tl * kSmallLd + j] = (tl < op.m && j < hc) ? B[tl + (size_t)j * op.ldb] : 0.0f;
-          // made visible by the barrier inside team_panel
-        }
-        for (int j0 = 0; j0 < op.k; j0 += kNB) team_panel(op, j0, min(kNB, op.k - j0), sA, sB, sV, sW, sT, team, tl);
-        if (op.kind && tl < op.m)
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j < hc) B[tl + (size_t)j * op.ldb] = sB[tl * kSmallLd + j];
-        team_sync(team);  // sB is reused by the next step
-      }
-      if (tl < arows)
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (j < hc) A[tl + (size_t)j * lda] = sA[tl * kSmallLd + j];
-      team_sync(team);  // sA is reused by the next group
-    }
-  }
-}
-
 // ------------------------------------------------------------ tensor-core applies (float factors)
 // The panel loops of dev::mat_apply_qt / mat_apply_tpqt on the tensor cores
 // (tc::left_qt, 3xTF32); chunks of at most 64 columns.
@@ -928,14 +762,15 @@ __global__ void __launch_bounds__(kThreads) k_rrqr_assemble(const RrqrSrc* __res
 
 // Householder QR of the selected columns C(:, colat[0:rank]) (the pivot order
 // fixed beforehand) into V / T / tau, then (where the task has a Qc) the
-// orthonormal basis Qc = C_sel R^{-1} (column-major, ld m) over the cluster's row blocks:
-// tiles of rt rows, 32-column blocks of R, a blocked update from the solved
-// columns and a triangular solve on the diagonal block.
+// orthonormal basis Qc = C_sel R^{-1} (column-major, ld m): the inverses of R's diagonal
+// blocks, a warp each, then mma_trsm_right on 64-row chunks dealt to the cluster's CTAs.
+// (Scalar sums and a substitution of one thread a row, before, took a quarter of the kernel: 64^3,
+// learned ranks: 34.1 -> 25.5 ms.)
 // kStage: the QR's panels are factored in shared memory (dist_qr's `pan`,
-// aliasing the basis tiles; mmax rows).
+// aliasing the basis' tiles; mmax rows).
 template <bool kStage>
 __global__ void __launch_bounds__(kThreads, 2) k_selected_qr(const RrqrTask* __restrict__ tasks, int cs, int mmax,
-                                                          int nmax, int rt, int pw) {
+                                                          int nmax, int pw) {
   extern __shared__ double sm[];
   const RrqrTask t = tasks[blockIdx.x / cs];
   const int rank = crank(cs);
@@ -946,9 +781,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_selected_qr(const RrqrTask* __r
   double* tmp = red + kRed;
   double* lt = tmp + kNB;
   double* vb = lt + nmax;
-  const int ldq = nmax + 1;
-  double* Qt = vb + mmax;      // rt x ldq: rows of the basis being solved (first the QR's tile scratch)
-  double* Rb = Qt + (size_t)rt * ldq;  // 32 x 33 block of R
+  double* tile = vb + mmax;
   const double* __restrict__ C = t.C;
   for (int l = warp; l < rk; l += kWarps) {
     if (!owns(l, rank, cs)) continue;
@@ -959,72 +792,25 @@ __global__ void __launch_bounds__(kThreads, 2) k_selected_qr(const RrqrTask* __r
       for (int r = lane; r < m; r += 32) t.V[r + (size_t)l * m] = __ldg(C + (size_t)r * ldw + c);
   }
   __syncthreads();
-  dist_qr<double>(t.V, m, nullptr, 0, m, rk, 1, t.T, t.tau, lt, vb, red, tmp, Qt, cs, nullptr,
-                  kStage ? Qt : nullptr, mmax, pw);
+  dist_qr<double>(t.V, m, nullptr, 0, m, rk, 1, t.T, t.tau, lt, vb, red, tmp, tile, cs, nullptr,
+                  kStage ? tile : nullptr, mmax, pw);
   if (!t.Qc) return;
   // R(l, j) = V[l + j m] for l <= j, written by the owners of column j
-  auto R = [&](int l, int j) { return __ldcg(t.V + l + (size_t)j * m); };
-  const int rc = (m + cs - 1) / cs;
-  const int ra = min(m, rank * rc), rb = min(m, ra + rc);
-  for (int r0 = ra; r0 < rb; r0 += rt) {
-    const int nr = min(rt, rb - r0);
+  for (int b = rank * kWarps + warp; b * kNB < rk; b += cs * kWarps)
+    dev::diag_inverse(t.V + (size_t)b * kNB * (m + 1), m, min(kNB, rk - b * kNB), tile + warp * kNB * (kNB + 1),
+                      t.Rinv + (size_t)b * kNB * kNB);
+  for (int r0 = rank * 64; r0 < m; r0 += cs * 64) {
+    const int nr = min(64, m - r0);
     for (int e = threadIdx.x; e < nr * rk; e += kThreads) {
-      const int rr = e / rk, l = e % rk;
+      const int rr = t.cm ? e % nr : e / rk, l = t.cm ? e / nr : e % rk;
       const int c = __ldg(t.colat + l);
-      Qt[rr * ldq + l] = __ldg(C + (t.cm ? (size_t)c * ldw + r0 + rr : (size_t)(r0 + rr) * ldw + c));
+      t.Qc[r0 + rr + (size_t)l * m] = __ldg(C + (t.cm ? (size_t)c * ldw + r0 + rr : (size_t)(r0 + rr) * ldw + c));
     }
-    __syncthreads();
-    for (int j0 = 0; j0 < rk; j0 += 32) {
-      const int jb = min(32, rk - j0);
-      // Q(:, j0:j0+jb) = X - Q(:, 0:j0) R(0:j0, j0:j0+jb), outputs (o / 32, o % 32)
-      double acc[(32 * 32 + kThreads - 1) / kThreads] = {};
-      for (int l0 = 0; l0 < j0; l0 += 32) {
-        for (int e = threadIdx.x; e < 32 * 32; e += kThreads) {
-          const int jj = e >> 5, ll = e & 31;
-          Rb[ll * 33 + jj] = jj < jb ? R(l0 + ll, j0 + jj) : 0.0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < (32 * 32 + kThreads - 1) / kThreads; ++u) {
-          const int o = threadIdx.x + u * kThreads, rr = o >> 5, jj = o & 31;
-          if (rr < nr) {
-            const double* q = Qt + rr * ldq + l0;
-            double a = 0.0;
-#pragma unroll 8
-            for (int ll = 0; ll < 32; ++ll) a += q[ll] * Rb[ll * 33 + jj];
-            acc[u] += a;
-          }
-        }
-        __syncthreads();
-      }
-#pragma unroll
-      for (int u = 0; u < (32 * 32 + kThreads - 1) / kThreads; ++u) {
-        const int o = threadIdx.x + u * kThreads, rr = o >> 5, jj = o & 31;
-        if (rr < nr && jj < jb) Qt[rr * ldq + j0 + jj] -= acc[u];
-      }
-      for (int e = threadIdx.x; e < 32 * 32; e += kThreads) {
-        const int jj = e >> 5, ll = e & 31;
-        Rb[ll * 33 + jj] = (jj < jb && ll <= jj) ? R(j0 + ll, j0 + jj) : 0.0;
-      }
-      __syncthreads();
-      // triangular solve on the diagonal block, one thread per row
-      for (int rr = threadIdx.x; rr < nr; rr += kThreads) {
-        double* q = Qt + rr * ldq + j0;
-        for (int jj = 0; jj < jb; ++jj) {
-          double x = q[jj];
-          for (int ll = 0; ll < jj; ++ll) x -= q[ll] * Rb[ll * 33 + jj];
-          const double dgn = Rb[jj * 33 + jj];
-          q[jj] = dgn != 0.0 ? x / dgn : 0.0;
-        }
-      }
-      __syncthreads();
-    }
-    for (int e = threadIdx.x; e < nr * rk; e += kThreads) {
-      const int l = e / nr, rr = e % nr;
-      t.Qc[(r0 + rr) + (size_t)l * m] = Qt[rr * ldq + l];
-    }
-    __syncthreads();
   }
+  __threadfence();
+  csync(cs);
+  for (int r0 = rank * 64; r0 < m; r0 += cs * 64)
+    dev::mma_trsm_right<double, true>(t.V, m, t.Rinv, t.Qc + r0, m, min(64, m - r0), rk, tile, 2);
 }
 
 // ------------------------------------------------------------ merge
@@ -1236,10 +1022,10 @@ struct StagePlan {
   int pw = kNB;
 };
 template <typename T>
-StagePlan staged_panel(size_t head, int rows, size_t other_bytes = 0) {
+StagePlan staged_panel(size_t head, int rows) {
   for (int pw = kNB; pw >= 8; pw /= 2) {
     const size_t panel = (size_t)rows * pw * sizeof(T) + pan_extra_bytes<T>();
-    const size_t region = std::max(std::max(smem_bytes(kWcap), panel), other_bytes);
+    const size_t region = std::max(smem_bytes(kWcap), panel);
     if (head + region + 1024 <= kSmemMax) return {head + region, pw};
   }
   return {};
@@ -1359,18 +1145,6 @@ cudaError_t launch_edge(int kind, const EdgeChunk* t, int ntasks, cudaStream_t s
                 : go(k_edge_left<double>, k_edge_trsm<double>, k_edge_right<double>);
 }
 
-cudaError_t launch_update_small(const UpdTask* t, const UpdOp* o, int ntasks, cudaStream_t st) {
-  if (cudaError_t pre = begin("launch_update_small")) return pre;
-  if (ntasks <= 0) return cudaSuccess;
-  if (!g_fp32) return cudaErrorInvalidValue;  // FP32 factors only
-  counted();
-  if (cudaError_t e = prep(k_update_small, kUpdSmallSmem)) return e;
-  k_update_small<<<(ntasks + kTeams - 1) / kTeams, kTeamThreads, kUpdSmallSmem, st>>>(t, o, ntasks);
-  return last();
-}
-
-bool update_op_small(int k, int m) { return k <= kSmallOp && m <= kSmallOp; }
-
 cudaError_t launch_edge_left_small(const EdgeChunk* t, int ntasks, cudaStream_t st) {
   if (cudaError_t pre = begin("launch_edge_left_small")) return pre;
   if (ntasks <= 0) return cudaSuccess;
@@ -1424,19 +1198,16 @@ cudaError_t launch_rrqr_assemble(const RrqrSrc* s, int nsrc, cudaStream_t st) {
   return last();
 }
 
-int selected_qr_rows(int nmax) { return std::max(1, std::min(32, 12288 / (std::max(nmax, 1) + 1))); }
-
 cudaError_t launch_selected_qr(const RrqrTask* t, int ntasks, int cs, int mmax, int nmax, cudaStream_t st) {
   if (cudaError_t pre = begin("launch_selected_qr")) return pre;
   if (ntasks <= 0) return cudaSuccess;
-  const int mm = panel_rows(std::max(mmax, 1)), nn = std::max(nmax, 1), rt = selected_qr_rows(nmax);
+  const int mm = panel_rows(std::max(mmax, 1)), nn = std::max(nmax, 1);
   const size_t head = smem_bytes(kRed + kNB + (size_t)nn + (size_t)mm);
-  const size_t basis = smem_bytes((size_t)rt * (nn + 1) + 32 * 33);
-  const StagePlan p = staged_panel<double>(head, mm, basis);
-  const size_t b = p.bytes ? p.bytes : head + std::max(basis, smem_bytes(kWcap));
+  const StagePlan p = staged_panel<double>(head, mm);
+  const size_t b = p.bytes ? p.bytes : head + smem_bytes(kWcap);
   auto go = [&](auto kern) {
     if (cudaError_t e = prep(kern, b)) return e;
-    return launch_clustered(kern, ntasks, cs, b, st, t, cs, mm, nn, rt, p.pw);
+    return launch_clustered(kern, ntasks, cs, b, st, t, cs, mm, nn, p.pw);
   };
   return p.bytes ? go(k_selected_qr<true>) : go(k_selected_qr<false>);
 }

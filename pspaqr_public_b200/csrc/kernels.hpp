@@ -89,11 +89,6 @@ bool edge_trsm_small(int ncols, int rows);
 // Right compression (launch_edge kind 2) of FP32 chunks with
 // edge_trsm_small(nc, cnt), one warp per chunk.
 cudaError_t launch_edge_right_small(const EdgeChunk* t, int ntasks, cudaStream_t st);
-// Trailing updates (FP32 factors) of tasks whose ops all satisfy
-// update_op_small(k, m) (at most 64 reflectors and 64 rows), a 64-thread team
-// per task.
-cudaError_t launch_update_small(const UpdTask* t, const UpdOp* o, int ntasks, cudaStream_t st);
-bool update_op_small(int k, int m);
 cudaError_t launch_spmv(int n, const int* rowptr, const int* col, const double* val, const double* x, double* y,
                         cudaStream_t st);
 int mgs_grid(int n);

@@ -103,6 +103,7 @@ struct RrqrTask {
   double* V;         // m x m output: reflector j below the diagonal of column j, R above (ld m)
   double* T;         // kNB x m output block factors
   double* tau;       // m
+  double* Rinv;      // with Qc: inverses of R's diagonal blocks (32 x 32 each)
   const int* colat;  // column at each pivot position
   int* rank;         // columns selected
   int m, w, ldw, cm;
