@@ -151,7 +151,11 @@ Tree::~Tree() {
   cudaFree(d_perm_);
   cudaFree(d_cval_);
   cudaFreeHost(h_cval_);
+  cudaFree(d_xwb_);
+  cudaFree(d_turnb_);
   cudaFree(d_krylov_);
+  cudaFreeHost(h_krylov_);
+  cudaFree(d_rhs_);
   scratch_.release();
   arena_.release();
   if (own_stream_ && stream_) cudaStreamDestroy(stream_);
@@ -1810,9 +1814,6 @@ void Tree::release_block_solve() {
   if (block_graph_) cudaGraphDestroy(block_graph_);
   block_exec_ = nullptr;
   block_graph_ = nullptr;
-  cudaFree(d_xwb_);
-  cudaFree(d_turnb_);
-  d_xwb_ = nullptr, d_turnb_ = nullptr;
   block_nrhs_ = 0;
   block_graph_kernels_ = 0;
 }
@@ -1820,16 +1821,28 @@ void Tree::release_block_solve() {
 // The preconditioner apply of nrhs vectors as one graph: groups of right-hand
 // sides that share their sweeps, as parallel branches with a workspace and
 // counters each, so that the GPU runs the groups concurrently.  Built on first
-// use per factorization and nrhs (it allocates), reused after.
+// use per factorization and nrhs, reused after; its workspaces only grow.
 int Tree::build_block_solve(int nrhs) {
   if (block_exec_ && block_nrhs_ == nrhs) return 0;
   release_block_solve();
   const int width = sweep_wide_ok_ ? kSweepWide : 1;
   const int groups = (nrhs + width - 1) / width;
   const size_t nc = sweep_counters();
-  if (check_cuda(cudaMalloc(&d_xwb_, sizeof(double) * (size_t)std::max<int64_t>(xw_size_, 1) * nrhs), "malloc") ||
-      check_cuda(cudaMalloc(&d_turnb_, sizeof(int) * nc * groups), "malloc"))
-    return -11;
+  const size_t nx = (size_t)std::max<int64_t>(xw_size_, 1) * nrhs, nt = nc * groups;
+  if (nx > xwb_cap_) {
+    cudaFree(d_xwb_);
+    d_xwb_ = nullptr;
+    xwb_cap_ = 0;
+    if (check_cuda(cudaMalloc(&d_xwb_, sizeof(double) * nx), "malloc")) return -11;
+    xwb_cap_ = nx;
+  }
+  if (nt > turnb_cap_) {
+    cudaFree(d_turnb_);
+    d_turnb_ = nullptr;
+    turnb_cap_ = 0;
+    if (check_cuda(cudaMalloc(&d_turnb_, sizeof(int) * nt), "malloc")) return -11;
+    turnb_cap_ = nt;
+  }
   if (check_cuda(cudaGraphCreate(&block_graph_, 0), "graph")) return -10;
   set_factor_fp32(fp32_);
   for (int q = 0, r = 0; q < groups; ++q) {
@@ -1856,42 +1869,27 @@ int Tree::build_block_solve(int nrhs) {
   return 0;
 }
 
-// M^{-1} x in place for the device vectors cols[0..nrhs) (permuted order), as
-// one block graph launch.
-int Tree::solve_block_cols(const std::vector<double*>& cols) {
+// Y = M^{-1} X for nrhs device vectors (column r of X at X + r * ldx, permuted
+// order; X == Y allowed), as one block graph launch.
+int Tree::solve_block_cols(const double* X, size_t ldx, double* Y, size_t ldy, int nrhs) {
   if (!factorized_) return fail(-4, "solve called before factorize");
-  const int nrhs = (int)cols.size();
   if (int rc = build_block_solve(nrhs)) return rc;
   const int n = st_.n;
   set_factor_fp32(fp32_);
-  for (int r = 0; r < nrhs; ++r) {
-    double* xw = elem(d_xwb_, (size_t)r * xw_size_);
-    if (fp32_) {
-      if (check_cuda(launch_to_f32(n, cols[r], xw, stream_), "block solve input")) return -10;
-    } else {
-      cudaMemcpyAsync(xw, cols[r], sizeof(double) * n, cudaMemcpyDeviceToDevice, stream_);
-    }
-  }
+  if (check_cuda(launch_copy_cols(n, nrhs, X, ldx, false, d_xwb_, xw_size_, fp32_, stream_), "block solve input"))
+    return -10;
   if (check_cuda(cudaGraphLaunch(block_exec_, stream_), "block solve graph")) return -10;
   add_kernel_launches(block_graph_kernels_);
-  for (int r = 0; r < nrhs; ++r) {
-    double* xw = elem(d_xwb_, (size_t)r * xw_size_);
-    if (fp32_) {
-      if (check_cuda(launch_to_f64(n, xw, cols[r], stream_), "block solve output")) return -10;
-    } else {
-      cudaMemcpyAsync(cols[r], xw, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream_);
-    }
-  }
+  if (check_cuda(launch_copy_cols(n, nrhs, d_xwb_, xw_size_, fp32_, Y, ldy, false, stream_), "block solve output"))
+    return -10;
   return 0;
 }
 
-// M^{-1} X for nrhs device vectors (column r at X + r * ldx, permuted order).
+// M^{-1} X in place.
 int Tree::solve_block_device(double* X, int nrhs, size_t ldx) {
   if (nrhs < 1 || ldx < (size_t)st_.n) return fail(-1, "solve_block: nrhs >= 1 and ldx >= n required");
   clear_status();
-  std::vector<double*> cols(nrhs);
-  for (int r = 0; r < nrhs; ++r) cols[r] = X + (size_t)r * ldx;
-  return solve_block_cols(cols);
+  return solve_block_cols(X, ldx, X, ldx, nrhs);
 }
 
 // Flexible GMRES for nrhs right-hand sides in lockstep: every iteration applies
@@ -1910,37 +1908,37 @@ int Tree::block_fgmres_device(double* B, int nrhs, size_t ldb, int maxit, double
   const size_t ldq = (size_t)n;
   const int grid = mgs_grid(n);
   // per right-hand side: V (n x maxit+1) | Z (n x maxit) | q | b | H column;
-  // then the shared partial sums and counter
+  // then the partial sums, a packed copy of the H columns and the counters
   const size_t hcap = (size_t)maxit + 3;
   const size_t per = ldq * (2 * (size_t)maxit + 1) + 2 * ldq + hcap;
-  if (int erc = ensure_krylov(per * nrhs + grid + 1)) return erc;
+  if (int erc = ensure_krylov((per + grid + hcap + 1) * nrhs, hcap * nrhs)) return erc;
   auto Vr = [&](int r) { return d_krylov_ + per * r; };
   auto Zr = [&](int r) { return Vr(r) + ldq * (maxit + 1); };
   auto qr = [&](int r) { return Zr(r) + ldq * maxit; };
   auto br = [&](int r) { return qr(r) + ldq; };
   auto hr = [&](int r) { return br(r) + ldq; };
   double* partial = d_krylov_ + per * nrhs;
-  unsigned int* done = reinterpret_cast<unsigned int*>(partial + grid);
+  double* packed = partial + (size_t)grid * nrhs;
+  unsigned int* done = reinterpret_cast<unsigned int*>(packed + hcap * nrhs);
   cudaError_t ge = cudaSuccess;
   auto g = [&](cudaError_t e) {
     if (!ge) ge = e;
   };
-  g(cudaMemsetAsync(done, 0, sizeof(unsigned int), stream_));
-  for (int r = 0; r < nrhs; ++r) {
-    g(cudaMemcpyAsync(br(r), B + (size_t)r * ldb, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream_));
-    g(cudaMemcpyAsync(qr(r), br(r), sizeof(double) * n, cudaMemcpyDeviceToDevice, stream_));
-    g(launch_mgs_step(n, qr(r), nullptr, nullptr, nullptr, partial, done, hr(r), 1, stream_));  // ||b||
-    g(launch_scale_copy(n, qr(r), hr(r), Vr(r), stream_));
-  }
-  std::vector<double> hk(hcap * nrhs, 0.0);
+  g(cudaMemsetAsync(done, 0, sizeof(unsigned int) * nrhs, stream_));
+  g(launch_copy_cols(n, nrhs, B, ldb, false, br(0), per, false, stream_));
+  g(launch_copy_cols(n, nrhs, B, ldb, false, qr(0), per, false, stream_));
+  g(launch_mgs_step(n, qr(0), nullptr, nullptr, nullptr, partial, done, hr(0), 1, stream_, nrhs, per));  // ||b||
+  g(launch_scale_copy(n, qr(0), hr(0), Vr(0), stream_, nrhs, per));
+  // the first cnt entries of every right-hand side's H column, in hk[cnt * r ..)
+  const double* hk = h_krylov_;
   auto readback = [&](int cnt) {
-    for (int r = 0; r < nrhs; ++r)
-      g(cudaMemcpyAsync(hk.data() + hcap * r, hr(r), sizeof(double) * cnt, cudaMemcpyDeviceToHost, stream_));
+    g(launch_copy_cols(cnt, nrhs, hr(0), per, false, packed, cnt, false, stream_));
+    g(cudaMemcpyAsync(h_krylov_, packed, sizeof(double) * cnt * nrhs, cudaMemcpyDeviceToHost, stream_));
     return check_cuda(ge ? ge : cudaStreamSynchronize(stream_), "block gmres");
   };
   int rc = readback(1);
   std::vector<double> rnorm(nrhs);
-  for (int r = 0; r < nrhs; ++r) rnorm[r] = hk[hcap * r];
+  for (int r = 0; r < nrhs; ++r) rnorm[r] = hk[r];
   const size_t hs = (size_t)(maxit + 1) * maxit;
   std::vector<double> H(hs * nrhs, 0.0), cs((size_t)maxit * nrhs, 0.0), sn((size_t)maxit * nrhs, 0.0),
       beta((size_t)(maxit + 1) * nrhs, 0.0);
@@ -1951,28 +1949,17 @@ int Tree::block_fgmres_device(double* B, int nrhs, size_t ldb, int maxit, double
   }
   int k = 0, active = nrhs;
   for (; !rc && k < maxit && active > 0; ++k) {
-    // Z(:, k) = M^{-1} V(:, k) for every right-hand side: the block apply works
-    // on the columns Z_r(:, k) in place
-    for (int r = 0; r < nrhs; ++r)
-      g(cudaMemcpyAsync(Zr(r) + (size_t)k * ldq, Vr(r) + (size_t)k * ldq, sizeof(double) * n,
-                        cudaMemcpyDeviceToDevice, stream_));
-    if (ge) break;
-    std::vector<double*> zk(nrhs);
-    for (int r = 0; r < nrhs; ++r) zk[r] = Zr(r) + (size_t)k * ldq;
-    if ((rc = solve_block_cols(zk))) break;
-    for (int r = 0; r < nrhs; ++r) {
-      double* zk = Zr(r) + (size_t)k * ldq;
-      double* Q = Vr(r);
-      double* q = qr(r);
-      double* hcol = hr(r);
-      if ((rc = spmv_device(zk, q))) break;
-      for (int i = 0; i <= k; ++i)
-        g(launch_mgs_step(n, q, i ? Q + (size_t)(i - 1) * ldq : nullptr, i ? hcol + (i - 1) : nullptr,
-                          Q + (size_t)i * ldq, partial, done, hcol + i, 0, stream_));
-      g(launch_mgs_step(n, q, Q + (size_t)k * ldq, hcol + k, nullptr, partial, done, hcol + k + 1, 1, stream_));
-      g(launch_scale_copy(n, q, hcol + k + 1, Q + (size_t)(k + 1) * ldq, stream_));
-    }
-    if (rc || (rc = readback(k + 2))) break;
+    // Z(:, k) = M^{-1} V(:, k), q = A Z(:, k), then the modified Gram-Schmidt steps
+    const size_t kc = (size_t)k * ldq;
+    double *Q = Vr(0), *q = qr(0), *hcol = hr(0);
+    if ((rc = solve_block_cols(Q + kc, per, Zr(0) + kc, per, nrhs))) break;
+    g(launch_spmv(n, d_rowptr_, d_col_, d_val_, Zr(0) + kc, q, stream_, nrhs, per, per));
+    for (int i = 0; i <= k; ++i)
+      g(launch_mgs_step(n, q, i ? Q + (size_t)(i - 1) * ldq : nullptr, i ? hcol + (i - 1) : nullptr,
+                        Q + (size_t)i * ldq, partial, done, hcol + i, 0, stream_, nrhs, per));
+    g(launch_mgs_step(n, q, Q + kc, hcol + k, nullptr, partial, done, hcol + k + 1, 1, stream_, nrhs, per));
+    g(launch_scale_copy(n, q, hcol + k + 1, Q + kc + ldq, stream_, nrhs, per));
+    if ((rc = readback(k + 2))) break;
     for (int r = 0; r < nrhs; ++r) {
       if (kfin[r] >= 0) continue;
       double* Hr = H.data() + hs * r;
@@ -1980,7 +1967,7 @@ int Tree::block_fgmres_device(double* B, int nrhs, size_t ldb, int maxit, double
       double* s2 = sn.data() + (size_t)maxit * r;
       double* be = beta.data() + (size_t)(maxit + 1) * r;
       auto Hc = [&](int i, int j) -> double& { return Hr[(size_t)j * (maxit + 1) + i]; };
-      for (int i = 0; i <= k + 1; ++i) Hc(i, k) = hk[hcap * r + i];
+      for (int i = 0; i <= k + 1; ++i) Hc(i, k) = hk[(size_t)(k + 2) * r + i];
       for (int i = 0; i < k; ++i) {
         const double temp = c[i] * Hc(i, k) + s2[i] * Hc(i + 1, k);
         Hc(i + 1, k) = -s2[i] * Hc(i, k) + c[i] * Hc(i + 1, k);
@@ -2008,33 +1995,30 @@ int Tree::block_fgmres_device(double* B, int nrhs, size_t ldb, int maxit, double
   }
   if (!rc && device_status() != 0) rc = fail(-12, "forward sweep wait timed out on the device");
   if (!rc) {
-    std::vector<double> nr(2 * nrhs, 1.0);
+    // x = Z y for each right-hand side (y through the packed columns), then all
+    // true residuals
     for (int r = 0; r < nrhs; ++r) {
       const int kr = kfin[r] >= 0 ? kfin[r] : std::min(k, maxit) - 1;
       double* Hr = H.data() + hs * r;
       double* be = beta.data() + (size_t)(maxit + 1) * r;
       auto Hc = [&](int i, int j) -> double& { return Hr[(size_t)j * (maxit + 1) + i]; };
-      std::vector<double> y(kr + 1, 0.0);
+      double* y = h_krylov_ + hcap * r;
       for (int i = kr; i >= 0; --i) {
         y[i] = be[i];
         for (int j = i + 1; j < kr + 1; ++j) y[i] -= Hc(i, j) * y[j];
         y[i] /= Hc(i, i);
       }
-      double* x = B + (size_t)r * ldb;
-      double* q = qr(r);
-      double* hcol = hr(r);
-      g(cudaMemcpyAsync(hcol, y.data(), sizeof(double) * (kr + 1), cudaMemcpyHostToDevice, stream_));
-      g(launch_combine(n, kr + 1, Zr(r), ldq, hcol, x, stream_));
-      g(spmv_device(x, q) ? cudaErrorUnknown : cudaSuccess);
-      g(launch_sub(n, br(r), q, q, stream_));
-      g(launch_mgs_step(n, q, nullptr, nullptr, nullptr, partial, done, hcol, 1, stream_));
-      g(launch_mgs_step(n, br(r), nullptr, nullptr, nullptr, partial, done, hcol + 1, 1, stream_));
-      g(cudaMemcpyAsync(nr.data() + 2 * r, hcol, sizeof(double) * 2, cudaMemcpyDeviceToHost, stream_));
-      // the host copy of y must stay alive until the copy has run
-      if ((rc = check_cuda(ge ? ge : cudaStreamSynchronize(stream_), "block gmres finish"))) break;
       iters[r] = kr;
     }
-    for (int r = 0; !rc && r < nrhs; ++r) relres[r] = nr[2 * r] / nr[2 * r + 1];
+    g(cudaMemcpyAsync(packed, h_krylov_, sizeof(double) * hcap * nrhs, cudaMemcpyHostToDevice, stream_));
+    for (int r = 0; r < nrhs; ++r)
+      g(launch_combine(n, iters[r] + 1, Zr(r), ldq, packed + hcap * r, B + (size_t)r * ldb, stream_));
+    g(launch_spmv(n, d_rowptr_, d_col_, d_val_, B, qr(0), stream_, nrhs, ldb, per));
+    g(launch_sub(n, br(0), qr(0), qr(0), stream_, nrhs, per));
+    g(launch_mgs_step(n, qr(0), nullptr, nullptr, nullptr, partial, done, hr(0), 1, stream_, nrhs, per));
+    g(launch_mgs_step(n, br(0), nullptr, nullptr, nullptr, partial, done, hr(0) + 1, 1, stream_, nrhs, per));
+    rc = readback(2);
+    for (int r = 0; !rc && r < nrhs; ++r) relres[r] = hk[2 * r] / hk[2 * r + 1];
   }
   t_gmres = wall() - t0;
   return rc;
@@ -2046,14 +2030,14 @@ int Tree::solve_device(double* x) {
   set_factor_fp32(fp32_);
   if (fp32_) {
     // the preconditioner applies in the factors' precision
-    if (check_cuda(launch_to_f32(n, x, d_xw_, stream_), "solve input")) return -10;
+    if (check_cuda(launch_copy_cols(n, 1, x, 0, false, d_xw_, 0, true, stream_), "solve input")) return -10;
   } else {
     cudaMemcpyAsync(d_xw_, x, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream_);
   }
   if (check_cuda(cudaGraphLaunch(solve_exec_, stream_), "solve graph")) return -10;
   add_kernel_launches(solve_graph_kernels_);
   if (fp32_) {
-    if (check_cuda(launch_to_f64(n, d_xw_, x, stream_), "solve output")) return -10;
+    if (check_cuda(launch_copy_cols(n, 1, d_xw_, 0, true, x, 0, false, stream_), "solve output")) return -10;
   } else {
     cudaMemcpyAsync(x, d_xw_, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream_);
   }
@@ -2143,7 +2127,7 @@ int Tree::gmres_device(double* b, int maxit, double gtol, int* iters, double* re
   const int grid = mgs_grid(n);
   // workspace: basis (n x maxit+1) | q | b | H column | partial sums | counter
   const size_t need = ldq * (maxit + 1) + 2 * (size_t)n + (maxit + 3) + grid + 1;
-  if (int erc = ensure_krylov(need)) return erc;
+  if (int erc = ensure_krylov(need, maxit + 3)) return erc;
   double* Q = d_krylov_;
   double* q = Q + ldq * (maxit + 1);
   double* bsave = q + n;
@@ -2167,7 +2151,7 @@ int Tree::gmres_device(double* b, int maxit, double gtol, int* iters, double* re
   auto Hc = [&](int i, int j) -> double& { return H[(size_t)j * (maxit + 1) + i]; };
   beta[0] = r_norm;
   int k = 0;
-  std::vector<double> hk(maxit + 2);
+  double* hk = h_krylov_;
   int nh = 0;
   if (!rc && (std::isnan(r_norm) || device_status() != 0)) rc = fail(-12, "preconditioner apply failed");
   for (; !rc && k < maxit; ++k) {
@@ -2177,7 +2161,7 @@ int Tree::gmres_device(double* b, int maxit, double gtol, int* iters, double* re
                         Q + (size_t)i * ldq, partial, done, hcol + i, 0, stream_));
     g(launch_mgs_step(n, q, Q + (size_t)k * ldq, hcol + k, nullptr, partial, done, hcol + k + 1, 1, stream_));
     g(launch_scale_copy(n, q, hcol + k + 1, Q + (size_t)(k + 1) * ldq, stream_));
-    cudaMemcpyAsync(hk.data(), hcol, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, stream_);
+    cudaMemcpyAsync(hk, hcol, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, stream_);
     if ((rc = check_cuda(ge ? ge : cudaStreamSynchronize(stream_), "gmres iteration"))) break;
     for (int i = 0; i <= k + 1; ++i) Hc(i, k) = hk[i];
     for (int i = 0; i < k; ++i) {
@@ -2372,7 +2356,7 @@ int Tree::fgmres_device(double* b, int maxit, double gtol, int* iters, double* r
   const int grid = mgs_grid(n);
   // workspace: V (n x maxit+1) | Z (n x maxit) | q | b | H column | partial sums | counter
   const size_t need = ldq * (2 * (size_t)maxit + 1) + 2 * (size_t)n + (maxit + 3) + grid + 1;
-  if (int erc = ensure_krylov(need)) return erc;
+  if (int erc = ensure_krylov(need, maxit + 3)) return erc;
   double* Q = d_krylov_;
   double* Z = Q + ldq * (maxit + 1);
   double* q = Z + ldq * maxit;
@@ -2396,7 +2380,7 @@ int Tree::fgmres_device(double* b, int maxit, double gtol, int* iters, double* r
   auto Hc = [&](int i, int j) -> double& { return H[(size_t)j * (maxit + 1) + i]; };
   beta[0] = r_norm;
   int k = 0, nh = 0;
-  std::vector<double> hk(maxit + 2);
+  double* hk = h_krylov_;
   if (!rc && !(r_norm > 0)) rc = fail(-1, "zero or invalid right-hand side");
   for (; !rc && k < maxit; ++k) {
     double* zk = Z + (size_t)k * ldq;
@@ -2407,7 +2391,7 @@ int Tree::fgmres_device(double* b, int maxit, double gtol, int* iters, double* r
                         Q + (size_t)i * ldq, partial, done, hcol + i, 0, stream_));
     g(launch_mgs_step(n, q, Q + (size_t)k * ldq, hcol + k, nullptr, partial, done, hcol + k + 1, 1, stream_));
     g(launch_scale_copy(n, q, hcol + k + 1, Q + (size_t)(k + 1) * ldq, stream_));
-    g(cudaMemcpyAsync(hk.data(), hcol, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, stream_));
+    g(cudaMemcpyAsync(hk, hcol, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, stream_));
     if ((rc = check_cuda(ge ? ge : cudaStreamSynchronize(stream_), "gmres iteration"))) break;
     for (int i = 0; i <= k + 1; ++i) Hc(i, k) = hk[i];
     for (int i = 0; i < k; ++i) {
@@ -2465,8 +2449,8 @@ int Tree::block_gmres_host(double* B, int nrhs, size_t ldb, int maxit, double gt
   if (!factorized_) return fail(-4, "gmres called before factorize");
   if (nrhs < 1 || ldb < (size_t)st_.n) return fail(-1, "block gmres: nrhs >= 1, ldb >= n");
   const size_t n = st_.n;
-  double* d = nullptr;
-  if (check_cuda(cudaMalloc(&d, sizeof(double) * n * nrhs), "malloc block right-hand sides")) return -11;
+  if (int rc = ensure_rhs(n * nrhs)) return rc;
+  double* d = d_rhs_;
   for (int r = 0; r < nrhs; ++r)
     cudaMemcpyAsync(d + n * r, B + ldb * r, sizeof(double) * n, cudaMemcpyHostToDevice, stream_);
   int rc = block_fgmres_device(d, nrhs, n, maxit, gtol, iters, relres);
@@ -2475,32 +2459,52 @@ int Tree::block_gmres_host(double* B, int nrhs, size_t ldb, int maxit, double gt
       cudaMemcpyAsync(B + ldb * r, d + n * r, sizeof(double) * n, cudaMemcpyDeviceToHost, stream_);
     rc = check_cuda(cudaStreamSynchronize(stream_), "block gmres download");
   }
-  cudaFree(d);
   return rc;
 }
 
-int Tree::ensure_krylov(size_t doubles) {
-  if (doubles <= krylov_doubles_) return 0;
-  cudaFree(d_krylov_);
-  d_krylov_ = nullptr;
-  krylov_doubles_ = 0;
-  if (check_cuda(cudaMalloc(&d_krylov_, sizeof(double) * doubles), "malloc Krylov workspace")) return -11;
-  krylov_doubles_ = doubles;
+// Device workspace and pinned host array of the Krylov methods; both only grow.
+int Tree::ensure_krylov(size_t doubles, size_t host_doubles) {
+  if (doubles > krylov_doubles_) {
+    cudaFree(d_krylov_);
+    d_krylov_ = nullptr;
+    krylov_doubles_ = 0;
+    if (check_cuda(cudaMalloc(&d_krylov_, sizeof(double) * doubles), "malloc Krylov workspace")) return -11;
+    krylov_doubles_ = doubles;
+  }
+  if (host_doubles > krylov_host_) {
+    cudaFreeHost(h_krylov_);
+    h_krylov_ = nullptr;
+    krylov_host_ = 0;
+    if (check_cuda(cudaHostAlloc(&h_krylov_, sizeof(double) * host_doubles, cudaHostAllocDefault), "host alloc"))
+      return -11;
+    krylov_host_ = host_doubles;
+  }
+  return 0;
+}
+
+// Device copy of a caller's host vectors, kept between calls (an allocation and a
+// release for each solve took 0.3 ms, and at times hundreds).
+int Tree::ensure_rhs(size_t doubles) {
+  if (doubles <= rhs_doubles_) return 0;
+  cudaFree(d_rhs_);
+  d_rhs_ = nullptr;
+  rhs_doubles_ = 0;
+  if (check_cuda(cudaMalloc(&d_rhs_, sizeof(double) * doubles), "malloc right-hand sides")) return -11;
+  rhs_doubles_ = doubles;
   return 0;
 }
 
 int Tree::gmres_host(double* b, int maxit, double gtol, int* iters, double* relres, double* hist, int hist_cap) {
   const int n = st_.n;
   if (!factorized_) return fail(-4, "gmres called before factorize");
-  double* d = nullptr;
-  if (check_cuda(cudaMalloc(&d, sizeof(double) * n), "malloc")) return -10;
+  if (ensure_rhs(n)) return -10;
+  double* d = d_rhs_;
   cudaMemcpyAsync(d, b, sizeof(double) * n, cudaMemcpyHostToDevice, stream_);
   int rc = gmres_device(d, maxit, gtol, iters, relres, hist, hist_cap);
   if (!rc) {
     cudaMemcpyAsync(b, d, sizeof(double) * n, cudaMemcpyDeviceToHost, stream_);
     rc = check_cuda(cudaStreamSynchronize(stream_), "gmres copy-out");
   }
-  cudaFree(d);
   return rc;
 }
 

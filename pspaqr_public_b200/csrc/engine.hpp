@@ -281,7 +281,7 @@ class Tree {
   size_t xw_cap_ = 0, counter_cap_ = 0;  // allocated elements of d_xw_ / d_turn_
   int build_block_solve(int nrhs);
   void release_block_solve();
-  int solve_block_cols(const std::vector<double*>& cols);
+  int solve_block_cols(const double* X, size_t ldx, double* Y, size_t ldy, int nrhs);
   // one zeroed region for the blocks of `edges`; sets ptr_/ld_ (rows_/cols_ must be set)
   int alloc_level_blocks(const std::vector<int>& edges);
 
@@ -340,7 +340,13 @@ class Tree {
   // Krylov workspace kept across GMRES calls
   double* d_krylov_ = nullptr;
   size_t krylov_doubles_ = 0;
-  int ensure_krylov(size_t doubles);
+  size_t xwb_cap_ = 0, turnb_cap_ = 0;
+  int ensure_krylov(size_t doubles, size_t host_doubles);
+  double* h_krylov_ = nullptr;  // pinned
+  size_t krylov_host_ = 0;
+  double* d_rhs_ = nullptr;
+  size_t rhs_doubles_ = 0;
+  int ensure_rhs(size_t doubles);
   std::vector<LevelTiming> lt_;
   std::vector<LevelPlan> plans_;  // per level, cleared by partition
   // tuning of the float applies (tensor_cores == 2): per level and kind, the

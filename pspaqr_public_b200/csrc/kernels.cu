@@ -832,8 +832,15 @@ __global__ void k_permute(int n, const int* __restrict__ perm, const double* __r
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[perm[i]] = src[i];
 }
 
+// The vector kernels of the Krylov methods: blockIdx.y is the right-hand side, whose
+// arrays lie a fixed stride behind those of the one before.  (One launch for each of 16
+// right-hand sides and step was half of a block method's time: 16 right-hand sides of
+// 384^2 BLKFIG.)
 __global__ void k_spmv(int n, const int* __restrict__ rowptr, const int* __restrict__ col,
-                       const double* __restrict__ val, const double* __restrict__ x, double* __restrict__ y) {
+                       const double* __restrict__ val, const double* __restrict__ x, size_t ldx,
+                       double* __restrict__ y, size_t ldy) {
+  x += blockIdx.y * ldx;
+  y += blockIdx.y * ldy;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     double s = 0.0;
     for (int k = rowptr[r]; k < rowptr[r + 1]; ++k) s += val[k] * x[col[k]];
@@ -847,7 +854,14 @@ __global__ void k_spmv(int n, const int* __restrict__ rowptr, const int* __restr
 __global__ void __launch_bounds__(kThreads) k_mgs_step(int n, double* __restrict__ q, const double* __restrict__ Qprev,
                                                        const double* hprev, const double* __restrict__ Qi,
                                                        double* partial, unsigned int* done, double* out,
-                                                       int take_sqrt) {
+                                                       int take_sqrt, size_t stride) {
+  const size_t off = blockIdx.y * stride;
+  q += off;
+  out += off;
+  if (Qprev) Qprev += off, hprev += off;
+  if (Qi) Qi += off;
+  partial += blockIdx.y * gridDim.x;
+  done += blockIdx.y;
   __shared__ double red[kRed];
   __shared__ bool last;
   const double h = Qprev ? *hprev : 0.0;
@@ -880,8 +894,11 @@ __global__ void __launch_bounds__(kThreads) k_mgs_step(int n, double* __restrict
   }
 }
 
-__global__ void k_scale_copy(int n, const double* __restrict__ src, const double* s, double* __restrict__ dst) {
-  const double inv = 1.0 / *s;
+__global__ void k_scale_copy(int n, const double* __restrict__ src, const double* s, double* __restrict__ dst,
+                             size_t stride) {
+  src += blockIdx.y * stride;
+  dst += blockIdx.y * stride;
+  const double inv = 1.0 / s[blockIdx.y * stride];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i] * inv;
 }
 
@@ -895,8 +912,11 @@ __global__ void k_combine(int n, int k, const double* __restrict__ Q, size_t ldq
   }
 }
 
-__global__ void k_sub(int n, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ c) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) c[i] = a[i] - b[i];
+__global__ void k_sub(int n, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ c,
+                      size_t stride) {
+  const size_t off = blockIdx.y * stride;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    c[off + i] = a[off + i] - b[off + i];
 }
 
 
@@ -911,13 +931,12 @@ inline size_t smem_bytes(size_t doubles) { return doubles * sizeof(double); }
 
 // ------------------------------------------------------------ precision conversion
 // dst (float) <- src (double), n elements
-__global__ void k_to_f32(long long n, const double* __restrict__ src, float* __restrict__ dst) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = (float)src[i];
-}
-__global__ void k_to_f64(long long n, const float* __restrict__ src, double* __restrict__ dst) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = (double)src[i];
+// columns of n elements between (and of) the two precisions
+template <typename S, typename D>
+__global__ void k_copy_cols(int n, const S* __restrict__ src, size_t lds, D* __restrict__ dst, size_t ldd) {
+  src += blockIdx.y * lds;
+  dst += blockIdx.y * ldd;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = (D)src[i];
 }
 // batched: one CTA per array
 __global__ void k_to_f32_batch(const ConvTask* __restrict__ tasks) {
@@ -1221,21 +1240,29 @@ cudaError_t launch_merge(const MergeTask* t, int ntasks, cudaStream_t st) {
   return last();
 }
 
-cudaError_t launch_to_f32(long long n, const double* src, double* dst, cudaStream_t st) {
-  if (cudaError_t pre = begin("launch_to_f32")) return pre;
-  if (n <= 0) return cudaSuccess;
-  counted();
-  k_to_f32<<<grid_for((int)std::min<long long>(n, 1 << 30)), 256, 0, st>>>(n, src, reinterpret_cast<float*>(dst));
+// f(first right-hand side, right-hand sides) for as many as a grid's y dimension holds
+template <typename F>
+cudaError_t by_rhs(int nrhs, F f) {
+  for (int r = 0; r < nrhs; r += 65535) {
+    counted();
+    f(r, std::min(65535, nrhs - r));
+  }
   return last();
 }
 
-cudaError_t launch_to_f64(long long n, const double* src, double* dst, cudaStream_t st) {
-  if (cudaError_t pre = begin("launch_to_f64")) return pre;
+cudaError_t launch_copy_cols(int n, int nrhs, const double* src, size_t lds, bool src32, double* dst, size_t ldd,
+                             bool dst32, cudaStream_t st) {
+  if (cudaError_t pre = begin("launch_copy_cols")) return pre;
   if (n <= 0) return cudaSuccess;
-  counted();
-  k_to_f64<<<grid_for((int)std::min<long long>(n, 1 << 30)), 256, 0, st>>>(n, reinterpret_cast<const float*>(src),
-                                                                           dst);
-  return last();
+  auto go = [&](auto* s, auto* d) {
+    return by_rhs(nrhs, [&](int r, int cnt) {
+      k_copy_cols<<<dim3(grid_for(n), cnt), 256, 0, st>>>(n, s + r * lds, lds, d + r * ldd, ldd);
+    });
+  };
+  const float* s32 = reinterpret_cast<const float*>(src);
+  float* d32 = reinterpret_cast<float*>(dst);
+  if (src32) return dst32 ? go(s32, d32) : go(s32, dst);
+  return dst32 ? go(src, d32) : go(src, dst);
 }
 
 cudaError_t launch_to_f32_batch(const ConvTask* t, int ntasks, cudaStream_t st) {
@@ -1247,28 +1274,34 @@ cudaError_t launch_to_f32_batch(const ConvTask* t, int ntasks, cudaStream_t st) 
 }
 
 cudaError_t launch_spmv(int n, const int* rowptr, const int* col, const double* val, const double* x, double* y,
-                        cudaStream_t st) {
+                        cudaStream_t st, int nrhs, size_t ldx, size_t ldy) {
   if (cudaError_t pre = begin("launch_spmv")) return pre;
-  counted();
-  k_spmv<<<grid_for(n), 256, 0, st>>>(n, rowptr, col, val, x, y);
-  return last();
+  return by_rhs(nrhs, [&](int r, int cnt) {
+    k_spmv<<<dim3(grid_for(n), cnt), 256, 0, st>>>(n, rowptr, col, val, x + r * ldx, ldx, y + r * ldy, ldy);
+  });
 }
 
 int mgs_grid(int n) { return grid_for(n, kThreads * 4, 148 * 4); }
 
 cudaError_t launch_mgs_step(int n, double* q, const double* Qprev, const double* hprev, const double* Qi,
-                            double* partial, unsigned int* done, double* out, int take_sqrt, cudaStream_t st) {
+                            double* partial, unsigned int* done, double* out, int take_sqrt, cudaStream_t st, int nrhs,
+                            size_t stride) {
   if (cudaError_t pre = begin("launch_mgs_step")) return pre;
-  counted();
-  k_mgs_step<<<mgs_grid(n), kThreads, 0, st>>>(n, q, Qprev, hprev, Qi, partial, done, out, take_sqrt);
-  return last();
+  const int grid = mgs_grid(n);
+  return by_rhs(nrhs, [&](int r, int cnt) {
+    const size_t off = r * stride;
+    k_mgs_step<<<dim3(grid, cnt), kThreads, 0, st>>>(n, q + off, Qprev ? Qprev + off : nullptr,
+                                                     Qprev ? hprev + off : nullptr, Qi ? Qi + off : nullptr,
+                                                     partial + (size_t)r * grid, done + r, out + off, take_sqrt, stride);
+  });
 }
 
-cudaError_t launch_scale_copy(int n, const double* src, const double* s, double* dst, cudaStream_t st) {
+cudaError_t launch_scale_copy(int n, const double* src, const double* s, double* dst, cudaStream_t st, int nrhs,
+                              size_t stride) {
   if (cudaError_t pre = begin("launch_scale_copy")) return pre;
-  counted();
-  k_scale_copy<<<grid_for(n), 256, 0, st>>>(n, src, s, dst);
-  return last();
+  return by_rhs(nrhs, [&](int r, int cnt) {
+    k_scale_copy<<<dim3(grid_for(n), cnt), 256, 0, st>>>(n, src + r * stride, s + r * stride, dst + r * stride, stride);
+  });
 }
 
 cudaError_t launch_combine(int n, int k, const double* Q, size_t ldq, const double* y, double* x, cudaStream_t st) {
@@ -1278,11 +1311,11 @@ cudaError_t launch_combine(int n, int k, const double* Q, size_t ldq, const doub
   return last();
 }
 
-cudaError_t launch_sub(int n, const double* a, const double* b, double* c, cudaStream_t st) {
+cudaError_t launch_sub(int n, const double* a, const double* b, double* c, cudaStream_t st, int nrhs, size_t stride) {
   if (cudaError_t pre = begin("launch_sub")) return pre;
-  counted();
-  k_sub<<<grid_for(n), 256, 0, st>>>(n, a, b, c);
-  return last();
+  return by_rhs(nrhs, [&](int r, int cnt) {
+    k_sub<<<dim3(grid_for(n), cnt), 256, 0, st>>>(n, a + r * stride, b + r * stride, c + r * stride, stride);
+  });
 }
 
 }  // namespace spq

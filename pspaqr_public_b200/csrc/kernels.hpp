@@ -34,8 +34,10 @@ void set_status_word(int* status);
 cudaError_t launch_tc_probe(const float* C, const float* V, const float* W2, int m, int flags, float* out1,
                             float* out2, int* status, cudaStream_t st);
 // n doubles -> n floats stored at dst, and back (vectors, factors)
-cudaError_t launch_to_f32(long long n, const double* src, double* dst, cudaStream_t st);
-cudaError_t launch_to_f64(long long n, const double* src, double* dst, cudaStream_t st);
+// nrhs columns of n elements, float arrays (their addresses carried as double*) where
+// src32 / dst32
+cudaError_t launch_copy_cols(int n, int nrhs, const double* src, size_t lds, bool src32, double* dst, size_t ldd,
+                             bool dst32, cudaStream_t st);
 cudaError_t launch_to_f32_batch(const ConvTask* t, int ntasks, cudaStream_t st);
 void add_kernel_launches(long long n);
 
@@ -89,13 +91,18 @@ bool edge_trsm_small(int ncols, int rows);
 // Right compression (launch_edge kind 2) of FP32 chunks with
 // edge_trsm_small(nc, cnt), one warp per chunk.
 cudaError_t launch_edge_right_small(const EdgeChunk* t, int ntasks, cudaStream_t st);
+// The vector kernels below work on nrhs right-hand sides whose arrays lie `stride` (ldx,
+// ldy) doubles apart; partial sums and counters are mgs_grid(n) and one each.
 cudaError_t launch_spmv(int n, const int* rowptr, const int* col, const double* val, const double* x, double* y,
-                        cudaStream_t st);
+                        cudaStream_t st, int nrhs = 1, size_t ldx = 0, size_t ldy = 0);
 int mgs_grid(int n);
 cudaError_t launch_mgs_step(int n, double* q, const double* Qprev, const double* hprev, const double* Qi,
-                            double* partial, unsigned int* done, double* out, int take_sqrt, cudaStream_t st);
-cudaError_t launch_scale_copy(int n, const double* src, const double* s, double* dst, cudaStream_t st);
+                            double* partial, unsigned int* done, double* out, int take_sqrt, cudaStream_t st,
+                            int nrhs = 1, size_t stride = 0);
+cudaError_t launch_scale_copy(int n, const double* src, const double* s, double* dst, cudaStream_t st, int nrhs = 1,
+                              size_t stride = 0);
 cudaError_t launch_combine(int n, int k, const double* Q, size_t ldq, const double* y, double* x, cudaStream_t st);
-cudaError_t launch_sub(int n, const double* a, const double* b, double* c, cudaStream_t st);
+cudaError_t launch_sub(int n, const double* a, const double* b, double* c, cudaStream_t st, int nrhs = 1,
+                       size_t stride = 0);
 
 }  // namespace spq
