@@ -24,7 +24,6 @@ double wall() {
 }
 constexpr size_t kAlign = 256;
 constexpr size_t kArenaChunk = size_t(1) << 30;
-// bounded wait of the forward sweep: ~1 s at 2 GHz
 constexpr int kChunk = 64;        // columns (rows) per CTA of the chunked applies
 // Levels with at most kElimPipe interiors pipeline their chains: about 1.6 times
 // the work of a chain on one CTA (waits, no reuse between steps), so that it pays
@@ -940,6 +939,9 @@ int Tree::factorize() {
                npan >= (2 << lg))
           ++lg;
         PivotShape sh = pivot_shape(mp, w, 1 << lg);
+        // however many matrices there are, a CTA's share of the columns has to fit: their bounds
+        // and positions alone pass its shared memory at 15,000 columns
+        while (lg < 4 && !sh.ok) sh = pivot_shape(mp, w, 1 << ++lg);
         if (lg == 4 && !pivots_cluster_fit(16, sh.smem, sh.big)) sh = pivot_shape(mp, w, 1 << --lg);
         if (w > kPivotMaxCols || !sh.ok) {
           fail(-12, "interface too wide for the pivoted QR kernel");
