@@ -15,8 +15,9 @@ learned-rank method (float factors whose left block-reflector applies are
           better.
   e2e   : the same step through the C ABI with host buffers: assemble (matrix
           upload) + factorize + spq_gmres(host b -> host x).
-  roofline : the tensor-core trailing updates of the headline step (k_update_tc)
-          against the 3xTF32 ceiling derived from the measured bf16 peak;
+  roofline : the trailing updates of the headline step against cuBLAS DGEMM
+          measured in the run (FP64 mma), or, where most of their flops ran on
+          the tcgen05 path, against the 3xTF32 ceiling from the measured bf16 peak;
           roofline_fp64_rrqr: the plain method's pivoted QR against the measured
           HBM peak.
   backward_error : ||A z - u|| / ||u|| with z = M^-1 u for seeded probes, per
@@ -53,10 +54,6 @@ WORKLOAD = {
     "n": 64, "d": 3, "nlevels": 12, "tol": 1e-2, "skip": 0, "gmres_tol": 1e-10, "maxit": 300, "rhs_seed": 2,
 }
 METRIC = "time to 1e-10 rel. residual (factor+GMRES), 64^3 diffusion: mixed+learned vs FP64"
-# DRAM bytes per algorithmic byte of the pivoted-QR launches, from an ncu
-# capture of the 48^3 member of the workload family
-# (profiles/k_rrqr_diff3d_48_traffic.md)
-RRQR_DRAM_PER_ALGO_BYTE = 0.78
 # DRAM bytes per nominal flop of the tensor-core trailing-update launches
 # (k_update_tc), from an ncu capture of the 32^3 member of the workload family,
 # scaled by flops to the 64^3 step (None: not captured for this kernel yet)
@@ -155,28 +152,6 @@ def fp64_gemm_peak(torch) -> float:
         e1.record()
         torch.cuda.synchronize()
         best = min(best, e0.elapsed_time(e1) / 1e3)
-    del a, b
-    return 2.0 * n ** 3 / best / 1e12
-
-
-def fp32_simt_peak(torch) -> float:
-    """cuBLAS SGEMM 8192^3 with TF32 off (FP32 on the CUDA cores), TFLOP/s: the
-    roofline denominator of the FP32 factor kernels (MEASURED_PEAKS.json carries
-    HBM and bf16 tensor figures only)."""
-    n = 8192
-    prev = torch.backends.cuda.matmul.allow_tf32
-    torch.backends.cuda.matmul.allow_tf32 = False
-    a = torch.randn(n, n, dtype=torch.float32, device="cuda")
-    b = torch.randn(n, n, dtype=torch.float32, device="cuda")
-    best = 1e30
-    for _ in range(4):
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-        torch.matmul(a, b)
-        e1.record()
-        torch.cuda.synchronize()
-        best = min(best, e0.elapsed_time(e1) / 1e3)
-    torch.backends.cuda.matmul.allow_tf32 = prev
     del a, b
     return 2.0 * n ** 3 / best / 1e12
 
@@ -314,10 +289,9 @@ def run_ours(args):
         e2e = float(np.mean(e2e_times))
     peaks = measured_peaks()
     fp64_peak = fp64_gemm_peak(torch) if rank == 0 else 0.0
-    fp32_peak = fp32_simt_peak(torch) if rank == 0 else 0.0
-    # dominant kernel of the headline step: the FP32 trailing updates (k_update,
-    # one launch per level), compute-bound on the CUDA cores; nominal flops of
-    # the updates phase over its event-timed duration (same stream)
+    # trailing updates of the headline step (k_update / k_update_pipe, one launch
+    # per level): FP64 mma on blocks widened from FP32; nominal flops of the
+    # updates phase over its event-timed duration (same stream)
     ui = ParTree.LEVEL_PHASES.index("updates")
     upd_s = float(head["level_ms"][:, ui].sum()) / 1e3
     upd_flops = float(head["level_flops"][:, ui].sum())
@@ -325,8 +299,10 @@ def run_ours(args):
     upd_tflops = upd_flops / upd_s / 1e12 if upd_s > 0 else 0.0
     fact = float(np.mean(head["ftimes"]))
     # dominant kernel of the plain factorization: the pivoted QR
-    # (k_rrqr_assemble + k_rrqr launches of every level), HBM-bound;
-    # algorithmic bytes over its event-timed duration
+    # (k_rrqr_assemble, k_pivots, k_selected_qr of every level).  Bytes it cannot
+    # do without (the gather and one pass for the norms) over its event-timed
+    # duration: a small share of HBM's rate, since the catch-up products and the
+    # latency of the pivot steps bound it
     plt = res["fp64"]["level_ms"]
     rrqr_s = float(plt[:, ParTree.LEVEL_PHASES.index("rrqr")].sum()) / 1e3
     rrqr_bytes = res["fp64"]["rrqr_bytes"]
@@ -340,11 +316,10 @@ def run_ours(args):
     nint = max(cnt["accepted"] + cnt["fallback"], 1)
     nfact = args.warmup + args.steps
     dr = head["ranks"] - res["fp64"]["ranks"]
-    # the trailing updates run per level on the tensor cores (3xTF32) or the
-    # CUDA cores, whichever the tuning measured faster; the roofline's ceiling
-    # is that of the kind that ran most of the update flops: three kind::tf32
-    # MMAs per product at half the measured bf16 tensor rate, or cuBLAS SGEMM
-    # (TF32 off) measured in this run
+    # the trailing updates run per level on tcgen05 (3xTF32) or on FP64 mma,
+    # whichever the tuning measured faster; the roofline's ceiling is that of the
+    # kind that ran most of the update flops: three kind::tf32 MMAs per product at
+    # half the measured bf16 tensor rate, or cuBLAS DGEMM measured in this run
     tune = head["tune"]
     on_tc = tune[:, :, 2] == 1
     lf = head["level_flops"][:, ui]
@@ -357,10 +332,10 @@ def run_ours(args):
                    if bf16 else "fallback 1590 TFLOP/s bf16 / 2 / 3, of fallback")
         upd_kernel = "k_update_tc: 3xTF32 tcgen05 trailing updates (the levels tuned to the tensor cores)"
     else:
-        upd_bound = "fp32"
-        upd_peak = fp32_peak
-        upd_src = "cuBLAS SGEMM 8192^3, TF32 off, measured in this run (MEASURED_PEAKS.json has no FP32 figure)"
-        upd_kernel = "k_update<float>: FP32 trailing updates on the CUDA cores (the levels tuned to them)"
+        upd_bound = "fp64"
+        upd_peak = fp64_peak
+        upd_src = "cuBLAS DGEMM, measured in this run (MEASURED_PEAKS.json has no FP64 figure)"
+        upd_kernel = "k_update / k_update_pipe<float>: trailing updates on FP64 mma (the levels tuned to them)"
     out = {
         "metric": METRIC,
         "value": step,
@@ -405,8 +380,7 @@ def run_ours(args):
                      "per_launch_flops": upd_flops / max(upd_launches, 1), "peak_source": upd_src},
         "tensor_core_levels": {k: int(on_tc[:, i].sum()) for i, k in enumerate(("updates", "left", "right"))},
         "roofline_fp64_rrqr": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
-                               "frac": achieved / hbm_peak,
-                               "traffic": RRQR_DRAM_PER_ALGO_BYTE * rrqr_bytes if RRQR_DRAM_PER_ALGO_BYTE else None,
+                               "frac": achieved / hbm_peak, "traffic": None,
                                "duration_s": rrqr_s},
         "factor_fp64_tflops": res["fp64"]["flops"] / float(np.mean(res["fp64"]["ftimes"])) / 1e12,
         "dgemm_peak_tflops": fp64_peak,
