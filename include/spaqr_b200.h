@@ -64,16 +64,17 @@ int spq_set_precision(spq_tree* t, int bits);
  * The block-reflector applies of float factors -- the trailing updates (the
  * reference's larfb / tpmqrt, ptree.cpp:216-266), the row scaling and left
  * compression applies and the right compression applies (ptree.cpp:1613-1659,
- * 1860-1903) -- run either as 3xTF32 tcgen05 MMAs with FP32 accumulation or in
- * FP32 on the CUDA cores.  mode 0 = CUDA cores, 1 = tensor cores, 2 (default) =
+ * 1860-1903) -- run either as 3xTF32 tcgen05 MMAs with FP32 accumulation or
+ * on FP64 mma.sync, float blocks widened in shared memory ("FP64 mma").
+ * mode 0 = FP64 mma, 1 = tensor cores, 2 (default) =
  * tuned: the first float factorization of a partition runs every apply on the
- * tensor cores, the second on the CUDA cores, and later ones run, per level and
+ * tensor cores, the second on FP64 mma, and later ones run, per level and
  * kind of apply, the tensor cores where they measured at least 5 % faster, else
- * the CUDA cores (so the first two factorizations of a partition differ from
+ * FP64 mma (so the first two factorizations of a partition differ from
  * later ones in rounding; the margin keeps near-ties from flipping between
  * runs).  No effect on FP64 factors.  Takes effect at the next factorize.
  * spq_tune_table: per level 9 floats -- for updates, left applies, right
- * applies: tensor-core ms, CUDA-core ms, choice (1 tensor, 0 CUDA, -1 not
+ * applies: tensor-core ms, FP64 mma ms, choice (1 tensor, 0 FP64 mma, -1 not
  * tuned yet). */
 int spq_set_tensor_cores(spq_tree* t, int mode);
 int spq_tune_table(spq_tree* t, float* out);

@@ -127,7 +127,7 @@ void Arena::release() {
 // ---------------------------------------------------------------- Tree
 Tree::Tree(int L, int s) : nlevels(L), skip(s) {
   // SPQ_TENSOR_CORES=0 / 1 / 2 in the environment sets the starting mode of
-  // spq_set_tensor_cores (CUDA cores / tensor cores / tuned per level)
+  // spq_set_tensor_cores (FP64 mma / tensor cores / tuned per level)
   if (const char* e = std::getenv("SPQ_TENSOR_CORES")) tensor_cores = std::min(std::max(std::atoi(e), 0), 2);
 }
 
@@ -1526,7 +1526,7 @@ int Tree::factorize() {
   for (const LevelTiming& t : lt_)
     for (double f : t.flops) flops_ += f;
   // tuning of the float applies: the first two factorizations measure each
-  // level's applies on the tensor cores, then on the CUDA cores
+  // level's applies on the tensor cores, then on FP64 mma
   if (fp32_ && tensor_cores == 2 && tune_runs_ < 2) {
     tune_ms_[tune_runs_].assign(L, {0.f, 0.f, 0.f});
     for (int l = 0; l < L; ++l)
@@ -1547,7 +1547,7 @@ int Tree::factorize() {
 bool Tree::use_tc(int lvl, int kind) const {
   if (!fp32_ || tensor_cores == 0) return false;
   if (tensor_cores == 1) return true;
-  if (tune_runs_ < 2) return tune_runs_ == 0;  // measuring: tensor cores first, then CUDA cores
+  if (tune_runs_ < 2) return tune_runs_ == 0;  // measuring: tensor cores first, then FP64 mma
   // the tensor cores only where they were clearly faster: near-ties (a level
   // whose two timings differ by a few microseconds) would otherwise flip from
   // run to run and with them the rounding of the factor

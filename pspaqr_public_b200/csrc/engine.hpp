@@ -129,10 +129,10 @@ class Tree {
   // when the factors are float
   int krylov = -1;
   // float factors: where the block-reflector applies (trailing updates, row
-  // scaling and left compression, right compression) run: 0 = CUDA cores,
+  // scaling and left compression, right compression) run: 0 = FP64 mma,
   // 1 = tensor cores (3xTF32), 2 = tuned per level and kind of apply from the
   // measured times of the first two float factorizations of a partition (the
-  // first on the tensor cores, the second on the CUDA cores)
+  // first on the tensor cores, the second on FP64 mma)
   int tensor_cores = 2;
   // cycle budget of every bounded spin wait of the preconditioner apply's
   // forward sweep (takes effect at the next factorize, which captures the
@@ -155,7 +155,7 @@ class Tree {
   // same sizes and allocator states (LevelPlan)
   bool plan_cache = true;
   long long plan_hits() const { return plan_hits_; }
-  // per level: 3 kinds x (tensor-core ms, CUDA-core ms, chosen: 1 tensor, 0 CUDA,
+  // per level: 3 kinds x (tensor-core ms, FP64 mma ms, chosen: 1 tensor, 0 FP64 mma,
   // -1 not tuned yet)
   void tune_table(std::vector<float>& out) const;
   // learned ranks: the sketch's pivoted QR stops at sketch_tol * tol (the
@@ -350,7 +350,7 @@ class Tree {
   std::vector<LevelTiming> lt_;
   std::vector<LevelPlan> plans_;  // per level, cleared by partition
   // tuning of the float applies (tensor_cores == 2): per level and kind, the
-  // measured milliseconds on the tensor cores [0] and on the CUDA cores [1]
+  // measured milliseconds on the tensor cores [0] and on FP64 mma [1]
   std::vector<std::array<float, 3>> tune_ms_[2];
   int tune_runs_ = 0;  // float factorizations of this partition measured so far
   bool use_tc(int lvl, int kind) const;

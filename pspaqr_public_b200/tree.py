@@ -245,14 +245,14 @@ class ParTree:
         self._chk(lib().spq_set_precision(self._h, bits), "set_precision")
 
     def set_tensor_cores(self, mode):
-        """Float factors' block-reflector applies: 0 / False = CUDA cores, 1 / True =
+        """Float factors' block-reflector applies: 0 / False = FP64 mma, 1 / True =
         3xTF32 tcgen05 MMAs, 2 = tuned per level from the first two factorizations (the
         tensor cores where at least 5 % faster)."""
         self._chk(lib().spq_set_tensor_cores(self._h, int(mode)), "set_tensor_cores")
 
     def tune_table(self) -> np.ndarray:
         """(nlevels, 3, 3): for updates / left applies / right applies: tensor-core ms,
-        CUDA-core ms, choice (1 tensor, 0 CUDA, -1 not tuned yet)."""
+        FP64 mma ms, choice (1 tensor, 0 FP64 mma, -1 not tuned yet)."""
         out = np.zeros(9 * self.nlevels, np.float32)
         lib().spq_tune_table(self._h, _pf(out))
         return out.reshape(self.nlevels, 3, 3)
