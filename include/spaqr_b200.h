@@ -100,6 +100,10 @@ int spq_debug_pivots(const double* C, int m, int w, int cm, int cs, long long sm
  * reflector tails; T (32 x n for each of the nout + 1 steps) the panels' block factors.  bits 64 or 32: the factors'
  * type. */
 int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int cs, int pipe, int bits, double* T);
+/* A triangular solve of the preconditioner apply on its own, for tests: X <- R^{-1} X for the k <= 8 columns of X
+ * (n x k, column-major) and the upper triangle of R (n x n, column-major).  bits 64 or 32: the factors' type; panels
+ * of more than `rows` rows from global memory (0: as shared memory allows). */
+int spq_debug_upper(const double* R, int n, double* X, int k, int bits, int rows);
 /* Diagnostic of the preconditioner apply (no reference counterpart): from the
  * next factorize on, reflector panels of more than `rows` rows are read from
  * global memory where they are used, as panels too long for shared memory are

@@ -262,6 +262,56 @@ int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int 
   return 0;
 }
 
+int spq_debug_upper(const double* R, int n, double* X, int k, int bits, int rows) {
+  if (!R || !X || n < 1 || k < 1 || k > spq::kSweepWide || (bits != 64 && bits != 32) || rows < 0) return -1;
+  const bool f32 = bits == 32;
+  const size_t es = f32 ? 4 : 8, nr = ((size_t)n * n + 63) / 64 * 64, nx = ((size_t)n + 63) / 64 * 64;
+  const int nb = (n + 31) / 32;
+  // R, the vectors, the inverses (32 x 32 doubles a block), the descriptors, the rank (no reflectors)
+  const size_t inv0 = (nr + nx * k) * es, task0 = inv0 + sizeof(double) * 1024 * nb;
+  std::vector<char> h(task0 + sizeof(spq::InvTask) * nb + sizeof(spq::SparsItem) + 2 * sizeof(int), 0);
+  auto put = [&](size_t at, const double* x, size_t cnt) {
+    for (size_t i = 0; i < cnt; ++i)
+      if (f32) reinterpret_cast<float*>(h.data())[at + i] = (float)x[i];
+      else reinterpret_cast<double*>(h.data())[at + i] = x[i];
+  };
+  char* d = nullptr;
+  if (cudaMalloc(&d, h.size()) != cudaSuccess) return -11;
+  put(0, R, (size_t)n * n);
+  for (int r = 0; r < k; ++r) put(nr + nx * r, X + (size_t)n * r, n);
+  auto* dR = reinterpret_cast<double*>(d);
+  auto* dinv = reinterpret_cast<double*>(d + inv0);
+  auto* it = reinterpret_cast<spq::InvTask*>(h.data() + task0);
+  for (int b = 0; b < nb; ++b) it[b] = {dR, dinv, nullptr, n, b};
+  auto* si = reinterpret_cast<spq::SparsItem*>(it + nb);
+  auto* dit = reinterpret_cast<spq::InvTask*>(d + task0);
+  auto* dsi = reinterpret_cast<spq::SparsItem*>(dit + nb);
+  auto* dint = reinterpret_cast<int*>(dsi + 1);  // rank 0, status
+  *si = {dR, dR, dR, dR, dinv, dint, 0, n};
+  spq::SweepRun run{};
+  run.xw = reinterpret_cast<double*>(d + nr * es);
+  run.stride = (long long)nx;
+  run.nrhs = k;
+  run.wide = k > 1;
+  run.status = dint + 1;
+  run.rows_limit = rows;
+  cudaError_t e = cudaMemcpy(d, h.data(), h.size(), cudaMemcpyHostToDevice);
+  const bool was = spq::factor_fp32();
+  spq::set_factor_fp32(f32);
+  if (!e) e = spq::launch_diag_inverse(dit, nb, nullptr);
+  if (!e) e = spq::launch_sweep_spars(false, dsi, 1, n, run, nullptr);
+  spq::set_factor_fp32(was);
+  if (!e) e = cudaDeviceSynchronize();
+  if (!e) e = cudaMemcpy(h.data(), d, inv0, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e) return -10;
+  for (int r = 0; r < k; ++r)
+    for (int i = 0; i < n; ++i)
+      X[(size_t)n * r + i] = f32 ? (double)reinterpret_cast<float*>(h.data())[nr + nx * r + i]
+                                 : reinterpret_cast<double*>(h.data())[nr + nx * r + i];
+  return 0;
+}
+
 int spq_set_tensor_cores(spq_tree* h, int mode) {
   if (!h || mode < 0 || mode > 2) return -1;
   h->t->tensor_cores = mode;

@@ -632,15 +632,31 @@ __device__ void mat_apply_q_right(const T* V, int ldv, const T* Tm, int k, T* C,
   }
 }
 
+// How a solve with an upper triangular diagonal block may use its inverse X, from the
+// Frobenius norms |R| |X| (at least the block's size; they bound every product of the
+// entries' magnitudes).  Solving by X alone leaves a residual of up to u |R| |X| times
+// that of a substitution: kInvPlain where that is the size of the sums around it.  Up to
+// 2^24 one step of refinement with R brings it back to u (its square, times u, is below
+// one), and a float solve with X in FP64 leaves less than a float's rounding
+// (kInvRefine).  Above, or not finite: kInvSubstitute.
+enum InvRule { kInvPlain = 0, kInvRefine = 1, kInvSubstitute = 2 };
+constexpr double kInvPlainMax = 256.0, kInvRefineMax = 16777216.0;
+
 // Inverse of an upper triangular kb x kb block (kb <= 32) by one warp with 32 x 33
-// doubles of scratch; lane j forms column j of `out` (32 x 32).  A zero on the diagonal
-// gives a zero row and column: the column that it belongs to drops out of the solve.
-__device__ inline void diag_inverse(const double* R, int ld, int kb, double* s, double* out) {
+// doubles of scratch; lane j forms column j in x and all return the rule.  A zero on the
+// diagonal gives a zero row and column: the column that it belongs to drops out of the
+// solve (the QR factorizations report it through the status word).
+template <typename T>
+__device__ inline int diag_inverse(const T* R, int ld, int kb, double* s, double (&x)[kNB]) {
   const int lane = threadIdx.x & 31;
+  double nr = 0.0, nx = 0.0;
   for (int j = 0; j < kb; ++j)
-    if (lane <= j) s[lane * (kNB + 1) + j] = __ldcg(R + lane + (size_t)j * ld);
+    if (lane <= j) {
+      const double r = (double)__ldcg(R + lane + (size_t)j * ld);
+      s[lane * (kNB + 1) + j] = r;
+      nr += r * r;
+    }
   __syncwarp();
-  double x[32];
 #pragma unroll
   for (int l = kNB - 1; l >= 0; --l) {
     double v = l == lane ? 1.0 : 0.0;
@@ -649,10 +665,17 @@ __device__ inline void diag_inverse(const double* R, int ld, int kb, double* s, 
       if (q <= lane && q < kb) v -= s[l * (kNB + 1) + q] * x[q];
     const double d = l <= lane && lane < kb ? s[l * (kNB + 1) + l] : 0.0;
     x[l] = d != 0.0 ? v / d : 0.0;
+    nx += x[l] * x[l];
   }
+  const double k = sqrt(warp_sum(nr)) * sqrt(warp_sum(nx));
+  return k <= kInvPlainMax ? kInvPlain : k <= kInvRefineMax ? kInvRefine : kInvSubstitute;
+}
+// Column-major, ld 32; the rule below the first diagonal entry.
+__device__ inline void store_inverse(const double (&x)[kNB], int kb, int rule, double* out) {
+  const int lane = threadIdx.x & 31;
   if (lane < kb)
 #pragma unroll
-    for (int l = 0; l < 32; ++l) out[l + lane * 32] = x[l];
+    for (int l = 0; l < kNB; ++l) out[l + lane * kNB] = lane == 0 && l == 1 ? (double)rule : x[l];
   __syncwarp();
 }
 

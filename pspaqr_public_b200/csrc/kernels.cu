@@ -796,9 +796,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_selected_qr(const RrqrTask* __r
                   kStage ? tile : nullptr, mmax, pw);
   if (!t.Qc) return;
   // R(l, j) = V[l + j m] for l <= j, written by the owners of column j
-  for (int b = rank * kWarps + warp; b * kNB < rk; b += cs * kWarps)
-    dev::diag_inverse(t.V + (size_t)b * kNB * (m + 1), m, min(kNB, rk - b * kNB), tile + warp * kNB * (kNB + 1),
-                      t.Rinv + (size_t)b * kNB * kNB);
+  for (int b = rank * kWarps + warp; b * kNB < rk; b += cs * kWarps) {
+    const int kb = min(kNB, rk - b * kNB);
+    double x[kNB];
+    const int rule = dev::diag_inverse(t.V + (size_t)b * kNB * (m + 1), m, kb, tile + warp * kNB * (kNB + 1), x);
+    dev::store_inverse(x, kb, rule, t.Rinv + (size_t)b * kNB * kNB);
+  }
   for (int r0 = rank * 64; r0 < m; r0 += cs * 64) {
     const int nr = min(64, m - r0);
     for (int e = threadIdx.x; e < nr * rk; e += kThreads) {

@@ -44,9 +44,11 @@ struct BwdEdge {
   long long x;
   int ldr, s;
 };
-// Inverses of the 32 x 32 diagonal blocks of an upper-triangular R (n x n, ld n),
-// block b at out + 32 * 32 * b (column-major, ld 32), computed in FP64 and stored
-// in the factors' precision; out64: also unrounded, or null.
+// Inverses of the 32 x 32 diagonal blocks of an upper-triangular R (n x n, ld n) in
+// FP64, block b at out + 32 * 32 * b (column-major, ld 32), the rule for its use below
+// its first diagonal entry (dense.cuh InvRule).  Float factors: that in out64 (or null),
+// and in `out` the blocks as the sweeps take them (solve.cu kInvBlock32), fewer floats
+// than 32 * 32 doubles a block.
 struct InvTask {
   const double* R;
   double* out;
