@@ -104,6 +104,8 @@ int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int 
  * (n x k, column-major) and the upper triangle of R (n x n, column-major).  bits 64 or 32: the factors' type; panels
  * of more than `rows` rows from global memory (0: as shared memory allows). */
 int spq_debug_upper(const double* R, int n, double* X, int k, int bits, int rows);
+/* The column scaling on its own, for tests: A <- A R^{-1} for A (m x n, column-major). */
+int spq_debug_scale_cols(const double* R, int n, double* A, int m, int bits);
 /* Diagnostic of the preconditioner apply (no reference counterpart): from the
  * next factorize on, reflector panels of more than `rows` rows are read from
  * global memory where they are used, as panels too long for shared memory are

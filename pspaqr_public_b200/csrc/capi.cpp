@@ -312,6 +312,56 @@ int spq_debug_upper(const double* R, int n, double* X, int k, int bits, int rows
   return 0;
 }
 
+int spq_debug_scale_cols(const double* R, int n, double* A, int m, int bits) {
+  if (!R || !A || n < 1 || m < 1 || (bits != 64 && bits != 32)) return -1;
+  const bool f32 = bits == 32;
+  const size_t es = f32 ? 4 : 8, nr = ((size_t)n * n + 63) / 64 * 64, na = ((size_t)m * n + 63) / 64 * 64;
+  const int nb = (n + 31) / 32, nc = (m + 63) / 64;
+  // R, A, the inverses in the factors' precision and in FP64 (32 x 32 doubles a block), the descriptors
+  const size_t inv0 = (nr + na) * es, task0 = inv0 + 2 * sizeof(double) * 1024 * nb;
+  std::vector<char> h(task0 + sizeof(spq::InvTask) * nb + sizeof(spq::EdgeChunk) * nc, 0);
+  auto put = [&](size_t at, const double* x, size_t cnt) {
+    for (size_t i = 0; i < cnt; ++i)
+      if (f32) reinterpret_cast<float*>(h.data())[at + i] = (float)x[i];
+      else reinterpret_cast<double*>(h.data())[at + i] = x[i];
+  };
+  char* d = nullptr;
+  if (cudaMalloc(&d, h.size()) != cudaSuccess) return -11;
+  put(0, R, (size_t)n * n);
+  put(nr, A, (size_t)m * n);
+  auto* dR = reinterpret_cast<double*>(d);
+  auto* dinv = reinterpret_cast<double*>(d + inv0);
+  double* dinv64 = f32 ? dinv + 1024 * nb : dinv;
+  auto* it = reinterpret_cast<spq::InvTask*>(h.data() + task0);
+  for (int b = 0; b < nb; ++b) it[b] = {dR, dinv, f32 ? dinv64 : nullptr, n, b};
+  auto* ch = reinterpret_cast<spq::EdgeChunk*>(it + nb);
+  for (int k = 0; k < nc; ++k) {
+    spq::EdgeChunk c{};
+    c.A = reinterpret_cast<double*>(d + nr * es);
+    c.V = dR;
+    c.T = dinv64;
+    c.lda = c.m = m;
+    c.nc = c.ldv = n;
+    c.lo = 64 * k;
+    c.cnt = std::min(64, m - 64 * k);
+    ch[k] = c;
+  }
+  auto* dit = reinterpret_cast<spq::InvTask*>(d + task0);
+  cudaError_t e = cudaMemcpy(d, h.data(), h.size(), cudaMemcpyHostToDevice);
+  const bool was = spq::factor_fp32();
+  spq::set_factor_fp32(f32);
+  if (!e) e = spq::launch_diag_inverse(dit, nb, nullptr);
+  if (!e) e = spq::launch_edge(1, reinterpret_cast<spq::EdgeChunk*>(dit + nb), nc, nullptr);
+  spq::set_factor_fp32(was);
+  if (!e) e = cudaDeviceSynchronize();
+  if (!e) e = cudaMemcpy(h.data(), d, inv0, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e) return -10;
+  for (size_t i = 0; i < (size_t)m * n; ++i)
+    A[i] = f32 ? (double)reinterpret_cast<float*>(h.data())[nr + i] : reinterpret_cast<double*>(h.data())[nr + i];
+  return 0;
+}
+
 int spq_set_tensor_cores(spq_tree* h, int mode) {
   if (!h || mode < 0 || mode > 2) return -1;
   h->t->tensor_cores = mode;

@@ -684,8 +684,9 @@ __device__ inline void store_inverse(const double (&x)[kNB], int kb, int rule, d
 // inverses of R's diagonal blocks given (block b at Inv + 32 * 32 b, column-major,
 // FP64).  Both products on FP64 mma as in mma_apply: warp w owns rows 8 w ..
 // 8 w + 7, tiles of X and R are shared.  (Substitution inside the diagonal blocks,
-// one thread a row, took longer than the products.)  kCg: R and the inverses are read
-// through L2.
+// one thread a row, took longer than the products.)  Ill-conditioned diagonal blocks
+// follow their InvRule: a step of refinement (FP64 only, a float result is rounded by
+// more), or that substitution.  kCg: R and the inverses are read through L2.
 template <typename T, bool kCg = false>
 __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int ldc, int m, int n, double* sm,
                                int stages) {
@@ -703,6 +704,7 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
   for (int j0 = 0; j0 < n; j0 += kNB) {
     const int jb = min(kNB, n - j0), ntile = j0 / kRT;
     const int nb = 8 * warp < m ? (jb + 7) / 8 : 0;  // blocks of eight columns
+    const int rule = (int)ld_v<kCg>(Inv + (size_t)j0 * kNB + 1);
     auto load = [&](int tt) {
 #pragma unroll
       for (int q = 0; q < kSV; ++q) {
@@ -770,16 +772,65 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
       if (more) stash(tt + 1);
       __syncthreads();
     }
+    // y = v times an upper triangular block of 32 columns in shared memory
+    auto times = [&](const double (&v)[4][2], const double* tri, double (&y)[4][2]) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        y[j][0] = y[j][1] = 0.0;
+#pragma unroll
+        for (int b = 0; b <= j; ++b)
+          if (j < nb)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) dmma(y[j][0], y[j][1], v[b][e], tri[(8 * j + perm) * kLdV + 8 * b + fc[e]]);
+      }
+    };
     double y[4][2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      y[j][0] = y[j][1] = 0.0;
+    for (int b = 0; b < 4; ++b)
 #pragma unroll
-      for (int b = 0; b <= j; ++b)
-        if (j < nb)
+      for (int e = 0; e < 2; ++e) x[b][e] -= w[b][e];
+    const bool refine = sizeof(T) == 8 && rule == kInvRefine, substitute = rule == kInvSubstitute;
+    if (refine || substitute) {  // R_JJ (no tile is read any more)
 #pragma unroll
-          for (int e = 0; e < 2; ++e)
-            dmma(y[j][0], y[j][1], x[b][e] - w[b][e], sT[(8 * j + perm) * kLdV + 8 * b + fc[e]]);
+      for (int q = 0; q < kNB * kNB / kThreads; ++q) {
+        const int j = warp + q * kWarps;
+        sV0[j * kLdV + lane] = lane <= j && j < jb ? (double)ld_v<kCg>(R + j0 + lane + (size_t)(j0 + j) * ldr) : 0.0;
+      }
+      if (substitute)
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) sC0[(8 * b + fc[e]) * kLdR + c] = x[b][e];
+      __syncthreads();
+    }
+    if (substitute) {
+      if (t < kNC)
+        for (int j = 0; j < jb; ++j) {
+          double v = sC0[j * kLdR + t];
+          for (int i = 0; i < j; ++i) v -= sC0[i * kLdR + t] * sV0[j * kLdV + i];
+          const double d = sV0[j * kLdV + j];
+          sC0[j * kLdR + t] = d != 0.0 ? v / d : 0.0;
+        }
+      __syncthreads();
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) y[b][e] = sC0[(8 * b + fc[e]) * kLdR + c];
+    } else {
+      times(x, sT, y);
+      if (refine) {
+        double r[4][2];
+        times(y, sV0, r);
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) x[b][e] -= r[b][e];
+        times(x, sT, r);
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) y[b][e] += r[b][e];
+      }
     }
 #pragma unroll
     for (int b = 0; b < 4; ++b)

@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_edge_right_tc(const EdgeChunk* 
 
 // column scaling: rows [lo, lo+cnt) of A <- A R^{-1}
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_edge_trsm(const EdgeChunk* __restrict__ tasks) {
+__global__ void __launch_bounds__(kThreads, 2) k_edge_trsm(const EdgeChunk* __restrict__ tasks) {
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);
   const EdgeChunk t = tasks[blockIdx.x];

@@ -62,6 +62,7 @@ def lib():
             "spq_debug_update_pipe": (i32, [vp, i32]),
             "spq_debug_sweep_rows": (i32, [vp, i32]),
             "spq_debug_upper": (i32, [pd, i32, pd, i32, i32, i32]),
+            "spq_debug_scale_cols": (i32, [pd, i32, pd, i32, i32]),
             "spq_debug_chain": (i32, [pd, i32, pd, pi, i32, i32, i32, i32, pd]),
             "spq_debug_pivots": (i32, [pd, i32, i32, i32, i32, C.c_longlong, f64, f64, pi, pi]),
             "spq_get_factor": (i32, [vp, i32, i32, pd, pi]),

@@ -27,12 +27,12 @@ def upper(n, kind, seed, f):
     return (R + np.diag(rng.choice([-1.0, 1.0], n))).astype(f).astype(np.float64)
 
 
-def check(R, x, b, u):
-    """Residuals of R x = b (columns), block row by block row."""
+def check(R, x, b, u, first=0):
+    """Residuals of R x = b (columns), block row by block row; the first block has NB - first rows."""
     n = len(R)
     res = (R.astype(np.longdouble) @ x.astype(np.longdouble) - b).astype(np.float64)
-    for c in range(0, n, NB):
-        e = min(n, c + NB)
+    for c in range(-first, n, NB):
+        c, e = max(c, 0), min(n, c + NB)
         D = R[c:e, c:e]
         k = np.linalg.norm(D) * np.linalg.norm(np.linalg.inv(D))
         factor = max(2.0, k) if k <= 256.0 else 2.0
@@ -62,3 +62,20 @@ def test_sweep_solve_is_backward_stable(n, rows, kind, bits):
         x = np.array(b, order="F")
         assert lib().spq_debug_upper(p(np.asfortranarray(R)), n, p(x), k, bits, rows) == 0
         check(R, x, b, np.finfo(f).eps / 2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits", [64, 32])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n,m", [(1, 1), (31, 5), (32, 64), (33, 65), (100, 130), (300, 70)])
+def test_column_scaling_is_backward_stable(n, m, kind, bits):
+    from pspaqr_public_b200.tree import lib
+
+    f = np.float64 if bits == 64 else np.float32
+    R = upper(n, kind, n, f)
+    p = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))
+    b = (np.random.default_rng(m).standard_normal((m, n)) @ R).astype(f).astype(np.float64)
+    x = np.array(b, order="F")
+    assert lib().spq_debug_scale_cols(p(np.asfortranarray(R)), n, p(x), m, bits) == 0
+    # X R = B is the transposed system with the order of the blocks reversed
+    check(R[::-1, ::-1].T, x.T[::-1], b.T[::-1], np.finfo(f).eps / 2, NB - 1 - (n - 1) % NB)
