@@ -115,6 +115,9 @@ int spq_debug_sweep_rows(spq_tree* t, int rows);
 /* For tests: levels with at most `tasks` update tasks run their trailing updates as a pipeline of ops (negative:
  * the library's own rule).  The results are the same bit for bit. */
 int spq_debug_update_pipe(spq_tree* t, int tasks);
+/* For tests: cycles without any progress after which a wait of the elimination chains' and of the trailing updates'
+ * pipelines runs out (default 2e9 each, about a second; 0: at once).  factorize then returns -12. */
+int spq_debug_factor_spin(spq_tree* t, long long chains, long long updates);
 /* Reuse of descriptor lists across factorizations of one partition (no
  * reference counterpart; the reference rebuilds its task graph every time,
  * ptree.cpp:885-2123).  A level's lists depend only on its cluster sizes and on

@@ -95,6 +95,13 @@ int spq_debug_update_pipe(spq_tree* h, int tasks) {
   return 0;
 }
 
+int spq_debug_factor_spin(spq_tree* h, long long chains, long long updates) {
+  if (!h || chains < 0 || updates < 0) return -1;
+  h->t->chain_spin = chains;
+  h->t->update_spin = updates;
+  return 0;
+}
+
 int spq_debug_sweep_rows(spq_tree* h, int rows) {
   if (!h || rows < 0) return -1;
   h->t->sweep_rows = rows;
@@ -203,7 +210,7 @@ int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int 
   const bool f32 = bits == 32;
   const size_t es = f32 ? 4 : 8;
   const size_t nd = sizeof(spq::ElimStep) * (nout + 1) + sizeof(spq::ElimTask) + sizeof(spq::ElimOut) * nout;
-  const size_t cnt = (size_t)nout + 2;  // ticket, status, progress
+  const size_t cnt = (size_t)nout + 3;  // status, ticket, work finished, progress
   char* d = nullptr;
   if (cudaMalloc(&d, tot * es + nd + sizeof(int) * cnt) != cudaSuccess) return -11;
   auto at = [&](size_t i) { return reinterpret_cast<double*>(d + i * es); };
@@ -241,15 +248,15 @@ int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int 
   if (!e) e = cudaMemset(d_cnt, 0, sizeof(int) * cnt);
   const bool was = spq::factor_fp32();
   spq::set_factor_fp32(f32);
-  spq::set_status_word(d_cnt + 1);
+  spq::set_status_word(d_cnt);
   if (!e)
-    e = pipe ? spq::launch_elim_pipe(d_st, nout + 1, cs, n, vm, d_cnt, d_cnt + 2, nullptr)
+    e = pipe ? spq::launch_elim_pipe(d_st, nout + 1, cs, n, vm, d_cnt + 1, 2000000000LL, nullptr)
              : spq::launch_elim(d_et, d_eo, 1, cs, n, vm, nullptr);
   spq::set_factor_fp32(was);
   spq::set_status_word(nullptr);  // a factorization sets its own
   if (!e) e = cudaDeviceSynchronize();
   int status = 0;
-  if (!e) e = cudaMemcpy(&status, d_cnt + 1, sizeof(int), cudaMemcpyDeviceToHost);
+  if (!e) e = cudaMemcpy(&status, d_cnt, sizeof(int), cudaMemcpyDeviceToHost);
   if (!e) e = cudaMemcpy(hv, d, tot * es, cudaMemcpyDeviceToHost);
   cudaFree(d);
   if (e || status & 16) return e ? -10 : -12;

@@ -598,10 +598,10 @@ int Tree::factorize() {
         int cs = cluster_for(nm);
         while (cs > 1 && st.size() * cs > (size_t)num_sms()) cs = cs == kBigCluster ? 4 : 1;
         auto* d_st = static_cast<ElimStep*>(upload(st.data(), sizeof(ElimStep) * st.size()));
-        auto* d_cnt = static_cast<int*>(scratch_.alloc(sizeof(int) * (size_t)(nprog + 1)));
+        auto* d_cnt = static_cast<int*>(scratch_.alloc(sizeof(int) * (size_t)(nprog + 2)));
         if (!d_st || !d_cnt) return fail(-11, "out of device memory (elimination descriptors)");
-        if (ck(cudaMemsetAsync(d_cnt, 0, sizeof(int) * (size_t)(nprog + 1), stream_), "elimination counters") ||
-            ck(launch_elim_pipe(d_st, (int)st.size(), cs, nm, vm, d_cnt, d_cnt + 1, stream_), "elimination kernel"))
+        if (ck(cudaMemsetAsync(d_cnt, 0, sizeof(int) * (size_t)(nprog + 2), stream_), "elimination counters") ||
+            ck(launch_elim_pipe(d_st, (int)st.size(), cs, nm, vm, d_cnt, chain_spin, stream_), "elimination kernel"))
           return -10;
       } else {
         auto* d_eo = static_cast<ElimOut*>(upload(eo.data(), sizeof(ElimOut) * eo.size()));
@@ -739,14 +739,14 @@ int Tree::factorize() {
       size_t cnt = 0;
       if (few) {
         if (P.ui.empty()) plan_update_items(ut, uo, P.ui);
-        cnt = sizeof(int) * (P.ui.size() + 1);
+        cnt = sizeof(int) * (P.ui.size() + 2);
         d_ui = static_cast<UpdItem*>(upload(pipe ? P.ui.data() : nullptr, sizeof(UpdItem) * P.ui.size()));
         d_cnt = static_cast<int*>(scratch_.alloc(cnt));
         if (!d_ui || !d_cnt) return fail(-11, "out of device memory (update descriptors)");
       }
       if (pipe) {
         if (ck(cudaMemsetAsync(d_cnt, 0, cnt, stream_), "update counters") ||
-            ck(launch_update_pipe(d_ut, d_uo, d_ui, (int)P.ui.size(), d_cnt, d_cnt + 1, stream_), "update kernel"))
+            ck(launch_update_pipe(d_ut, d_uo, d_ui, (int)P.ui.size(), d_cnt, update_spin, stream_), "update kernel"))
           return -10;
       } else {
         const bool tc = tensor_cores_on();

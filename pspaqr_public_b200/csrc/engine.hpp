@@ -138,6 +138,9 @@ class Tree {
   // forward sweep (takes effect at the next factorize, which captures the
   // apply); a wait that runs out fails the apply with status -12
   long long spin_limit = 2000000000LL;
+  // cycles without progress after which a wait of the elimination's and the updates'
+  // pipelines runs out (about a second): the factorization fails with status -12
+  long long chain_spin = 2000000000LL, update_spin = 2000000000LL;
   // panels of more rows than this stay in global memory during the apply (0: as
   // shared memory allows; tests); takes effect at the next factorize
   int sweep_rows = 0;

@@ -92,25 +92,37 @@ __global__ void k_scatter(int nnz, const double* __restrict__ val, double* const
 // 32 columns or 16 or 8 where a whole panel does not fit; may alias `tile`), the
 // owner copies the panel into shared memory, factors it there (dev::panel_qr) and
 // writes it back once.
+//
+// A pipeline's waits are bounded by lack of progress: `ticks` counts the panels and
+// block applies that its CTAs have finished, and a wait runs out after `limit` cycles
+// without another one (0: at its first look).  A wait itself may take most of the
+// level's time: the last of a chain of 60 updates waits for all before it.  One that
+// runs out sets the status word's bit 4 (value 16) and the step goes on without
+// waiting.
 struct ChainLink {
   const int* in = nullptr;  // panels of R finished by the step before
   int* out = nullptr;       // panels finished here
+  int* ticks = nullptr;
+  long long limit = 0;
 };
-// Cycle limit of a pipeline's waits (about a second); a wait that runs out sets
-// the status word's bit 4 (value 16) and the step goes on without waiting.
-constexpr long long kChainSpin = 2000000000LL;
 __device__ __forceinline__ int chain_acquire(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void chain_wait(const int* p, int v, int* status) {
-  const long long t0 = clock64();
+__device__ __forceinline__ void chain_wait(const int* p, int v, int* status, const int* ticks, long long limit) {
+  long long t0 = clock64();
+  int seen = -1;
   while (chain_acquire(p) < v) {
     if (chain_acquire(status) & 16) break;
-    if (clock64() - t0 > kChainSpin) {
-      atomicOr(status, 16);
-      break;
+    if (clock64() - t0 > limit) {
+      const int now = chain_acquire(ticks);
+      if (limit <= 0 || now == seen) {
+        atomicOr(status, 16);
+        break;
+      }
+      seen = now;
+      t0 = clock64();
     }
   }
   __threadfence();
@@ -123,6 +135,9 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
   const int rank = crank(cs);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gap = (cs - 1) * kNB;  // columns between two panels of one CTA
+  auto tick = [&]() {
+    if (chain.ticks && threadIdx.x == 0) atomicAdd(chain.ticks, 1);
+  };
   // one panel's (or part's) block reflector on nc columns: Rc their rows of R from
   // j0 on, Bc their columns of B
   auto apply = [&](T* Rc, T* Bc, const T* Tm, int j0, int kb, int nc, int cgap) {
@@ -134,7 +149,7 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
     const int kb = (n - j0) < kNB ? (n - j0) : kNB;
     const int pend = j0 + kb;
     if (chain.in) {
-      if (threadIdx.x == 0) chain_wait(chain.in, j0 / kNB + 1, status);
+      if (threadIdx.x == 0) chain_wait(chain.in, j0 / kNB + 1, status, chain.ticks, chain.limit);
       __syncthreads();
     }
     if (owns(j0, rank, cs) && pan) {
@@ -226,6 +241,7 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
         dev::panel_t(B + (size_t)j0 * ldb, ldb, m, kb, 0, lt + j0, Tout + (size_t)j0 * kNB, kNB, tmp);
       __threadfence();
     }
+    tick();
     csync(cs);
     // the panel's block reflector on own later panels, two per pass
     const T* Tm = Tout + (size_t)j0 * kNB;
@@ -235,6 +251,7 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
       const int second = q0 + cs * kNB;
       const int nc = (q0 + kNB < n ? kNB : n - q0) + (second < n ? ((second + kNB < n ? kNB : n - second)) : 0);
       apply(R + j0 + (size_t)q0 * ldr, B + (size_t)q0 * ldb, Tm, j0, kb, nc, gap);
+      tick();
     }
     if (chain.out) {
       csync(cs);
@@ -274,11 +291,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_elim(const ElimTask* __restrict
 // that the step a cluster waits for is held by a running one.
 template <typename T, bool kStage>
 __global__ void __launch_bounds__(kThreads, 2) k_elim_pipe(const ElimStep* __restrict__ steps, int cs, int nmax,
-                                                        int vmax, int pw, int* ticket, int* prog, int* status) {
+                                                        int vmax, int pw, int* counters, long long limit,
+                                                        int* status) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int s_step;
   T* sm = reinterpret_cast<T*>(smraw);
-  if (threadIdx.x == 0 && crank(cs) == 0) s_step = atomicAdd(ticket, 1);
+  if (threadIdx.x == 0 && crank(cs) == 0) s_step = atomicAdd(counters, 1);
   csync(cs);
   if (cs > 1) {
     const int v = *cg::this_cluster().map_shared_rank(&s_step, 0);
@@ -293,8 +311,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_elim_pipe(const ElimStep* __res
   T* vb = lt + nmax;
   T* tile = vb + vmax;
   ChainLink link;
-  if (t.in >= 0) link.in = prog + t.in;
-  if (t.out >= 0) link.out = prog + t.out;
+  if (t.in >= 0) link.in = counters + 2 + t.in;
+  if (t.out >= 0) link.out = counters + 2 + t.out;
+  link.ticks = counters + 1;
+  link.limit = limit;
   T* B = as<T>(t.B);
   dist_qr<T>(as<T>(t.S), t.n, B, t.m, B ? t.m : t.n, t.n, B ? 0 : 1, as<T>(t.T), as<T>(t.tau), lt, vb, red, tmp, tile,
              cs, status, kStage ? tile : nullptr, vmax, pw, link);
@@ -342,22 +362,23 @@ __global__ void __launch_bounds__(kThreads, 2) k_update(const UpdTask* __restric
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 2) k_update_pipe(const UpdTask* __restrict__ tasks,
                                                           const UpdOp* __restrict__ ops,
-                                                          const UpdItem* __restrict__ items, int* ticket, int* prog,
-                                                          int* status) {
+                                                          const UpdItem* __restrict__ items, int* counters,
+                                                          long long limit, int* status) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int s_item;
   T* sm = reinterpret_cast<T*>(smraw);
-  if (threadIdx.x == 0) s_item = atomicAdd(ticket, 1);
+  if (threadIdx.x == 0) s_item = atomicAdd(counters, 1);
   __syncthreads();
+  int *ticks = counters + 1, *prog = counters + 2;
   const UpdItem it = items[s_item];
   const UpdTask t = tasks[it.task];
   const UpdOp op = ops[it.op];
   T* A = as<T>(op.A) + (size_t)t.col0 * op.lda;
   T* B = op.kind == 0 ? nullptr : as<T>(op.B) + (size_t)t.col0 * op.ldb;
-  if (it.inb >= 0 && threadIdx.x == 0) chain_wait(prog + it.inb, it.inb_panels, status);
+  if (it.inb >= 0 && threadIdx.x == 0) chain_wait(prog + it.inb, it.inb_panels, status, ticks, limit);
   for (int j0 = 0; j0 < op.k; j0 += kNB) {
     const int kb = min(kNB, op.k - j0), unit = op.kind == 0;
-    if (it.in >= 0 && threadIdx.x == 0) chain_wait(prog + it.in, j0 / kNB + 1, status);
+    if (it.in >= 0 && threadIdx.x == 0) chain_wait(prog + it.in, j0 / kNB + 1, status, ticks, limit);
     __syncthreads();
     dev::tile_left_qt<T>(as<T>(op.V) + (unit ? j0 : 0) + (size_t)j0 * op.ldv, op.ldv, as<T>(op.T) + (size_t)j0 * kNB, kNB,
                          kb, unit, unit ? nullptr : A + j0, op.lda, unit ? A + j0 : B, unit ? op.lda : op.ldb,
@@ -366,6 +387,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_update_pipe(const UpdTask* __re
     if (threadIdx.x == 0) {
       __threadfence();
       asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(prog + s_item), "r"(j0 / kNB + 1) : "memory");
+      atomicAdd(ticks, 1);
     }
   }
 }
@@ -1069,8 +1091,8 @@ cudaError_t launch_elim(const ElimTask* t, const ElimOut* o, int ntasks, int cs,
   return p.bytes ? go(k_elim<double, true>) : go(k_elim<double, false>);
 }
 
-cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, int vmax, int* ticket, int* prog,
-                             cudaStream_t st) {
+cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, int vmax, int* counters,
+                             long long limit, cudaStream_t st) {
   if (cudaError_t pre = begin("launch_elim_pipe")) return pre;
   if (nsteps <= 0) return cudaSuccess;
   if (!g_status) return cudaErrorInvalidValue;  // its waits read and set the status word
@@ -1080,7 +1102,7 @@ cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, in
   const size_t b = p.bytes ? p.bytes : head + smem_bytes(kWcap);
   auto go = [&](auto kern) {
     if (cudaError_t e = prep(kern, b)) return e;
-    return launch_clustered(kern, nsteps, cs, b, st, t, cs, nmax, vmax, p.pw, ticket, prog, g_status);
+    return launch_clustered(kern, nsteps, cs, b, st, t, cs, nmax, vmax, p.pw, counters, limit, g_status);
   };
   if (g_fp32) return p.bytes ? go(k_elim_pipe<float, true>) : go(k_elim_pipe<float, false>);
   return p.bytes ? go(k_elim_pipe<double, true>) : go(k_elim_pipe<double, false>);
@@ -1119,8 +1141,8 @@ cudaError_t launch_update(const UpdTask* t, const UpdOp* o, int ntasks, cudaStre
   return last();
 }
 
-cudaError_t launch_update_pipe(const UpdTask* t, const UpdOp* o, const UpdItem* items, int nitems, int* ticket,
-                               int* prog, cudaStream_t st) {
+cudaError_t launch_update_pipe(const UpdTask* t, const UpdOp* o, const UpdItem* items, int nitems, int* counters,
+                               long long limit, cudaStream_t st) {
   if (cudaError_t pre = begin("launch_update_pipe")) return pre;
   if (nitems <= 0) return cudaSuccess;
   if (!g_status) return cudaErrorInvalidValue;  // its waits read and set the status word
@@ -1128,7 +1150,7 @@ cudaError_t launch_update_pipe(const UpdTask* t, const UpdOp* o, const UpdItem* 
   counted();
   auto go = [&](auto kern) {
     if (cudaError_t e = prep(kern, b)) return e;
-    kern<<<nitems, kThreads, b, st>>>(t, o, items, ticket, prog, g_status);
+    kern<<<nitems, kThreads, b, st>>>(t, o, items, counters, limit, g_status);
     return last();
   };
   return g_fp32 ? go(k_update_pipe<float>) : go(k_update_pipe<double>);

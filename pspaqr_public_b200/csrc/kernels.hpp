@@ -28,7 +28,7 @@ bool tensor_cores_on();
 // Device status word of the factorization kernels launched by this thread:
 // bit 2 (value 2) a tensor-core wait ran out, 4 a non-finite pivot, 8 a zero
 // pivot in a QR factorization (elimination chains, scaling QR), 16 a wait of the
-// elimination pipeline ran out.
+// elimination or the update pipeline ran out.
 void set_status_word(int* status);
 // Diagnostic of the tensor-core operand layouts (tc_apply.cuh tc::probe).
 cudaError_t launch_tc_probe(const float* C, const float* V, const float* W2, int m, int flags, float* out1,
@@ -47,15 +47,16 @@ cudaError_t launch_permute(int n, const int* perm, const double* src, double* ds
 // cs = CTAs per task (thread-block cluster size); vmax = longest reflector tail
 cudaError_t launch_elim(const ElimTask* t, const ElimOut* o, int ntasks, int cs, int nmax, int vmax, cudaStream_t st);
 // The same chains with every step a cluster of its own, panel by panel behind
-// the step before; ticket and the progress counters must be zero.
-cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, int vmax, int* ticket, int* prog,
-                             cudaStream_t st);
+// the step before.  counters (zero): the ticket, the work finished, the steps'
+// progress; waits run out after `limit` cycles without progress (0: at once).
+cudaError_t launch_elim_pipe(const ElimStep* t, int nsteps, int cs, int nmax, int vmax, int* counters,
+                             long long limit, cudaStream_t st);
 cudaError_t launch_scale(const ScaleTask* t, int ntasks, int cs, int nmax, cudaStream_t st);
 cudaError_t launch_update(const UpdTask* t, const UpdOp* o, int ntasks, cudaStream_t st);
-// The same updates with every op of a task an item of its own (CUDA cores and FP64
-// mma only); ticket and the items' progress counters must be zero.
-cudaError_t launch_update_pipe(const UpdTask* t, const UpdOp* o, const UpdItem* items, int nitems, int* ticket,
-                               int* prog, cudaStream_t st);
+// The same updates with every op of a task an item of its own (not on the tensor
+// cores); counters and limit as above, a progress counter an item.
+cudaError_t launch_update_pipe(const UpdTask* t, const UpdOp* o, const UpdItem* items, int nitems, int* counters,
+                               long long limit, cudaStream_t st);
 // kind 0: left apply on column chunks, 1: right triangular solve on row chunks,
 // 2: right apply on row chunks
 cudaError_t launch_edge(int kind, const EdgeChunk* t, int ntasks, cudaStream_t st);

@@ -60,6 +60,7 @@ def lib():
             "spq_plan_hits": (C.c_longlong, [vp]),
             "spq_debug_corrupt_descriptor": (i32, [vp]),
             "spq_debug_update_pipe": (i32, [vp, i32]),
+            "spq_debug_factor_spin": (i32, [vp, C.c_longlong, C.c_longlong]),
             "spq_debug_sweep_rows": (i32, [vp, i32]),
             "spq_debug_upper": (i32, [pd, i32, pd, i32, i32, i32]),
             "spq_debug_scale_cols": (i32, [pd, i32, pd, i32, i32]),
