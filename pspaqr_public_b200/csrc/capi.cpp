@@ -274,8 +274,8 @@ int spq_debug_upper(const double* R, int n, double* X, int k, int bits, int rows
   const bool f32 = bits == 32;
   const size_t es = f32 ? 4 : 8, nr = ((size_t)n * n + 63) / 64 * 64, nx = ((size_t)n + 63) / 64 * 64;
   const int nb = (n + 31) / 32;
-  // R, the vectors, the inverses (32 x 32 doubles a block), the descriptors, the rank (no reflectors)
-  const size_t inv0 = (nr + nx * k) * es, task0 = inv0 + sizeof(double) * 1024 * nb;
+  // R, the vectors, the inverses, the descriptors, the rank (no reflectors)
+  const size_t inv0 = (nr + nx * k) * es, task0 = inv0 + es * ((spq::sweep_inverse_elems(n) + 63) / 64 * 64);
   std::vector<char> h(task0 + sizeof(spq::InvTask) * nb + sizeof(spq::SparsItem) + 2 * sizeof(int), 0);
   auto put = [&](size_t at, const double* x, size_t cnt) {
     for (size_t i = 0; i < cnt; ++i)
@@ -324,8 +324,9 @@ int spq_debug_scale_cols(const double* R, int n, double* A, int m, int bits) {
   const bool f32 = bits == 32;
   const size_t es = f32 ? 4 : 8, nr = ((size_t)n * n + 63) / 64 * 64, na = ((size_t)m * n + 63) / 64 * 64;
   const int nb = (n + 31) / 32, nc = (m + 63) / 64;
-  // R, A, the inverses in the factors' precision and in FP64 (32 x 32 doubles a block), the descriptors
-  const size_t inv0 = (nr + na) * es, task0 = inv0 + 2 * sizeof(double) * 1024 * nb;
+  // R, A, the inverses of the apply and those in FP64 (32 x 32 doubles a block), the descriptors
+  const size_t inv0 = (nr + na) * es, inv1 = inv0 + es * ((spq::sweep_inverse_elems(n) + 63) / 64 * 64);
+  const size_t task0 = inv1 + sizeof(double) * 1024 * nb;
   std::vector<char> h(task0 + sizeof(spq::InvTask) * nb + sizeof(spq::EdgeChunk) * nc, 0);
   auto put = [&](size_t at, const double* x, size_t cnt) {
     for (size_t i = 0; i < cnt; ++i)
@@ -338,9 +339,9 @@ int spq_debug_scale_cols(const double* R, int n, double* A, int m, int bits) {
   put(nr, A, (size_t)m * n);
   auto* dR = reinterpret_cast<double*>(d);
   auto* dinv = reinterpret_cast<double*>(d + inv0);
-  double* dinv64 = f32 ? dinv + 1024 * nb : dinv;
+  auto* dinv64 = reinterpret_cast<double*>(d + inv1);
   auto* it = reinterpret_cast<spq::InvTask*>(h.data() + task0);
-  for (int b = 0; b < nb; ++b) it[b] = {dR, dinv, f32 ? dinv64 : nullptr, n, b};
+  for (int b = 0; b < nb; ++b) it[b] = {dR, dinv, dinv64, n, b};
   auto* ch = reinterpret_cast<spq::EdgeChunk*>(it + nb);
   for (int k = 0; k < nc; ++k) {
     spq::EdgeChunk c{};

@@ -773,11 +773,10 @@ int Tree::factorize() {
         t.T = Ts_[p];
         t.tau = scratch_.dalloc(std::max(np, 1));
         t.n = np;
-        const size_t ninv = (size_t)NB * NB * std::max(1, (np + NB - 1) / NB);
-        Rinv_[p] = arena_.dalloc(ninv);
-        inv64[p] = fp32_ ? scratch_.dalloc(ninv) : Rinv_[p];
+        Rinv_[p] = alloc_inverses(np);
+        inv64[p] = scratch_.dalloc((size_t)NB * NB * std::max(1, (np + NB - 1) / NB));
         if (!t.T || !t.tau || !Rinv_[p] || !inv64[p]) return fail(-11, "out of device memory (scaling)");
-        for (int b = 0; b * NB < np; ++b) inv.push_back({t.S, Rinv_[p], fp32_ ? inv64[p] : nullptr, np, b});
+        for (int b = 0; b * NB < np; ++b) inv.push_back({t.S, Rinv_[p], inv64[p], np, b});
         const int cs = cluster_for(np);
         const int g = cs == 1 ? 0 : (cs == 4 ? 1 : 2);
         sc[g].push_back(t);
@@ -1586,6 +1585,11 @@ int Tree::alloc_level_blocks(const std::vector<int>& edges) {
   return 0;
 }
 
+double* Tree::alloc_inverses(int n) {
+  const size_t e = sweep_inverse_elems(n);
+  return arena_.dalloc(fp32_ ? (e + 1) / 2 : e);
+}
+
 // Levels with at most this many interiors run the apply's forward elimination as a
 // pipeline of one CTA per chain step; more interiors fill the GPU by themselves
 // (384^2 float, 1024 leaves: 0.98 ms an apply at 256, 1.19 ms with the leaves
@@ -1610,7 +1614,7 @@ int Tree::plan_sweep() {
   std::vector<InvTask> inv;
   InvTask* d_inv = nullptr;
   auto inverses = [&](const double* R, int n) {
-    double* out = arena_.dalloc((size_t)NB * NB * std::max(1, (n + NB - 1) / NB));
+    double* out = alloc_inverses(n);
     for (int b = 0; b * NB < n; ++b) inv.push_back({R, out, nullptr, n, b});
     return out;
   };

@@ -278,6 +278,7 @@ class Tree {
   bool sweep_wide_ok_ = false;  // kSweepWide right-hand sides fit the kernels at every level
   int nprog_ = 0, ndone_ = 0;  // pipeline progress and completion counters of one apply
   int plan_sweep();
+  double* alloc_inverses(int n);  // of the diagonal blocks of an n x n triangle
   // counters of one apply: turns, tickets, progress, completions
   size_t sweep_counters() const;
   int capture_sweep(SweepRun run, int* counters, cudaGraph_t* g, long long* kernels);

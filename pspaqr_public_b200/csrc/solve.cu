@@ -23,8 +23,9 @@
 // Diffusion on 128^2 with coefficients of 10^-3 and 10^3, FP32 factors, tolerance
 // 1e-2: GMRES took 34 iterations with the inverses alone, 21 with this rule (and with
 // substitutions everywhere).  Coefficients of 10^-4 .. 10^4 at random on 100^2, FP64,
-// tolerance 1e-9: GMRES left a residual of 5.1e-10, now 1.1e-11.  The rule costs an
-// apply of 64^2 (FP64) 2 us of 98, one of 48^3 2 us of 1654.
+// tolerance 1e-9: GMRES left a residual of 5.1e-10, now 1.1e-11.  With the
+// inverses alone, in T's layout, an FP64 apply of 64^2 took 96.9 us, of 48^3 1640 us;
+// now 97.1 and 1555.
 //
 // Forward elimination, levels with few interiors: the steps of one interior (its
 // own reflectors, then one per out-edge) run as separate CTAs in a pipeline.
@@ -61,6 +62,11 @@ template <typename T>
 __device__ __forceinline__ void cp_async_el(T* dst, const T* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"((int)sizeof(T)) : "memory");
+}
+template <typename T>
+__device__ __forceinline__ void cp_async_16(T* dst, const T* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // all but the newest `pending` groups have arrived
@@ -104,9 +110,11 @@ __host__ __device__ constexpr size_t fixed_elems() {
 // diagonal, the inverse's entries above its diagonal mirrored below, its diagonal in
 // the last row; FP32, the inverse rounded to float above, what the rounding left out
 // mirrored below (where the rule calls for a substitution: R above).  Then the rule.
+// The inverses lie in global memory as the buffers of 32 columns, one after the other,
+// so that a block is one copy of 16-byte pieces (gathered from R and a plain inverse by
+// elements, an apply of 64^2 took 100.4 us instead of 97.1, one of 48^3 1656 instead of 1555).
 __host__ __device__ constexpr int tri_elems(int KB) { return KB * (KB + 1) + 8; }
-// FP32 inverses in global memory: the same layout, a block after the other
-constexpr int kInvBlock32 = kNB * (kNB + 1) + 2;
+constexpr int kInvBlock = tri_elems(kNB);
 constexpr int kMaxStages = 4;
 
 // One CTA's view of a chain of panels.  NW compute warps, panels of KB columns,
@@ -172,25 +180,21 @@ struct Chain {
       if (l <= j) cp_async_el(td + j * (KB + 1) + l, tp + l + (size_t)j * kNB);
     }
   }
-  // The diagonal block of R (ld n) at c0 and its inverse, as tri_elems says.
-  __device__ void stage_diag(int buf, const T* R, int n, const T* inv, int c0, int kb) {
+  // The inverse of the diagonal block at c0, as tri_elems says.
+  __device__ void stage_diag(int buf, const T* inv, int c0, int kb) {
     T* td = sT + buf * kTri;
-    const int o = c0 % kNB;
-    const T* rp = R + c0 + (size_t)c0 * n;
-    const T* ip = inv + (size_t)(c0 / kNB) * (sizeof(T) == 8 ? kNB * kNB : kInvBlock32);
-    for (int e = threadIdx.x; e < KB * kb; e += kThreads) {
-      const int l = e % KB, j = e / KB;
-      if (l > j) continue;
-      T* low = l < j ? td + l * (KB + 1) + j : td + j * (KB + 1) + KB;
-      if (sizeof(T) == 8) {
-        cp_async_el(td + j * (KB + 1) + l, rp + l + (size_t)j * n);
-        cp_async_el(low, ip + (o + l) + (o + j) * kNB);
-      } else {
-        cp_async_el(td + j * (KB + 1) + l, ip + (o + j) * (kNB + 1) + (o + l));
-        cp_async_el(low, l < j ? ip + (o + l) * (kNB + 1) + (o + j) : ip + (o + j) * (kNB + 1) + kNB);
+    const T* ip = inv + (size_t)(c0 / kNB) * kInvBlock;
+    if (KB == kNB) {
+      constexpr int kPer = 16 / sizeof(T);
+      for (int e = threadIdx.x * kPer; e <= KB * (KB + 1); e += kThreads * kPer) cp_async_16(td + e, ip + e);
+    } else {
+      const T* sp = ip + (size_t)(c0 % kNB) * (kNB + 1);
+      for (int e = threadIdx.x; e < (KB + 1) * kb; e += kThreads) {
+        const int l = e % (KB + 1), j = e / (KB + 1);
+        cp_async_el(td + e, sp + j * (kNB + 1) + (l < KB ? c0 % kNB + l : kNB));
       }
+      if (threadIdx.x == 0) cp_async_el(td + KB * (KB + 1), ip + kNB * (kNB + 1));
     }
-    if (threadIdx.x == 0) cp_async_el(td + KB * (KB + 1), sizeof(T) == 8 ? ip + 1 : ip + kNB * (kNB + 1));
   }
   __device__ T el(int buf, int i, int r) const {  // row r of the panel's column i
     if (!kDirect) return sV[(size_t)buf * KB * lds + (size_t)i * lds + r];
@@ -451,7 +455,7 @@ struct Chain {
       if (ahead < np) {
         const int c = (np - 1 - ahead) * KB;
         stage_panel(pb, R + (size_t)c * n, n, min(KB, n - c), 0, c, false);
-        stage_diag(pb, R, n, inv, c, min(KB, n - c));
+        stage_diag(pb, inv, c, min(KB, n - c));
         pb = next(pb);
         ++ahead;
       }
@@ -786,20 +790,18 @@ __global__ void __launch_bounds__(128) k_diag_inverse(const InvTask* __restrict_
   const T* R = as<T>(t.R) + c + (size_t)c * t.n;
   double x[kNB];
   const int rule = dev::diag_inverse(R, t.n, kb, sR[warp], x);
-  double* out64 = sizeof(T) == 8 ? t.out : t.out64;
-  if (out64) dev::store_inverse(x, kb, rule, out64 + (size_t)t.block * kNB * kNB);
-  if (sizeof(T) == 4) {
-    float* p = reinterpret_cast<float*>(t.out) + (size_t)t.block * kInvBlock32;
-    if (lane < kb)
+  if (t.out64) dev::store_inverse(x, kb, rule, t.out64 + (size_t)t.block * kNB * kNB);
+  T* p = reinterpret_cast<T*>(t.out) + (size_t)t.block * kInvBlock;
+  if (lane < kb)
 #pragma unroll
-      for (int l = 0; l < kNB; ++l)
-        if (l <= lane) {
-          const float hi = (float)x[l];
-          p[lane * (kNB + 1) + l] = rule == dev::kInvSubstitute ? (float)R[l + (size_t)lane * t.n] : hi;
-          p[l < lane ? l * (kNB + 1) + lane : lane * (kNB + 1) + kNB] = (float)(x[l] - (double)hi);
-        }
-    if (lane == 0) p[kNB * (kNB + 1)] = (float)rule;
-  }
+    for (int l = 0; l < kNB; ++l)
+      if (l <= lane) {
+        const T hi = (T)x[l];
+        const bool whole = sizeof(T) == 8 || rule == dev::kInvSubstitute;
+        p[lane * (kNB + 1) + l] = whole ? R[l + (size_t)lane * t.n] : hi;
+        p[l < lane ? l * (kNB + 1) + lane : lane * (kNB + 1) + kNB] = sizeof(T) == 8 ? hi : (T)(x[l] - (double)hi);
+      }
+  if (lane == 0) p[kNB * (kNB + 1)] = (T)rule;
 }
 
 // ---------------------------------------------------------------- launchers
@@ -861,6 +863,7 @@ cudaError_t begin(const char* name) {
 }  // namespace
 
 int sweep_bwd_rows() { return kBwdRows; }
+size_t sweep_inverse_elems(int n) { return (size_t)kInvBlock * std::max(1, (n + kNB - 1) / kNB); }
 
 bool sweep_wide_fits(int rows, int nmax) {
   bool ok = false;

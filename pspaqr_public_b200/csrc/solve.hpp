@@ -44,11 +44,10 @@ struct BwdEdge {
   long long x;
   int ldr, s;
 };
-// Inverses of the 32 x 32 diagonal blocks of an upper-triangular R (n x n, ld n) in
-// FP64, block b at out + 32 * 32 * b (column-major, ld 32), the rule for its use below
-// its first diagonal entry (dense.cuh InvRule).  Float factors: that in out64 (or null),
-// and in `out` the blocks as the sweeps take them (solve.cu kInvBlock32), fewer floats
-// than 32 * 32 doubles a block.
+// Inverses of the 32 x 32 diagonal blocks of an upper-triangular R (n x n, ld n): in
+// `out` as the sweeps take them (sweep_inverse_elems(n) factor elements for all blocks);
+// out64 (or null): in FP64, block b at out64 + 32 * 32 * b (column-major, ld 32), the
+// rule for its use below its first diagonal entry (dense.cuh InvRule).
 struct InvTask {
   const double* R;
   double* out;
@@ -75,6 +74,7 @@ constexpr int kSweepWide = 8;
 // longest x_c) fit in the launchers' current precision.
 bool sweep_wide_fits(int rows, int nmax);
 int sweep_bwd_rows();  // rows of one backward item
+size_t sweep_inverse_elems(int n);
 
 cudaError_t launch_diag_inverse(const InvTask* t, int ntasks, cudaStream_t st);
 cudaError_t launch_sweep_fwd(const FwdItem* t, const FwdEdge* e, int ntasks, bool pipe, int nmax, int mmax, int* ticket,
