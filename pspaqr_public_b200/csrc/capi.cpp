@@ -189,7 +189,7 @@ int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int 
   if (!S || !T || n < 1 || nout < 0 || (nout && (!B || !rows)) || cs < 1 || cs > 8 || (cs & (cs - 1)) || pipe < 0 ||
       pipe > 1 || (bits != 64 && bits != 32))
     return -1;
-  // arrays on 64-element boundaries, as the engine's pools place them: S, the blocks, T of each step, tau
+  // arrays on 64-element boundaries, as the engine's pools place them: S, the blocks, T of each step
   auto pad = [](size_t k) { return (k + 63) / 64 * 64; };
   std::vector<size_t> ob(nout), ot(nout + 1);
   size_t tot = pad((size_t)n * n);
@@ -205,8 +205,6 @@ int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int 
     ot[i] = tot;
     tot += pad(nt);
   }
-  const size_t otau = tot;
-  tot += pad(n);
   const bool f32 = bits == 32;
   const size_t es = f32 ? 4 : 8;
   const size_t nd = sizeof(spq::ElimStep) * (nout + 1) + sizeof(spq::ElimTask) + sizeof(spq::ElimOut) * nout;
@@ -226,12 +224,12 @@ int spq_debug_chain(double* S, int n, double* B, const int* rows, int nout, int 
   };
   std::vector<spq::ElimStep> st;
   std::vector<spq::ElimOut> eo;
-  const spq::ElimTask et{at(0), at(ot[0]), at(otau), n, 0, nout};
-  st.push_back({at(0), nullptr, at(ot[0]), at(otau), n, n, -1, nout ? 0 : -1});
+  const spq::ElimTask et{at(0), at(ot[0]), n, 0, nout};
+  st.push_back({at(0), nullptr, at(ot[0]), n, n, -1, nout ? 0 : -1});
   put(0, S, (size_t)n * n);
   const double* src = B;
   for (int i = 0; i < nout; ++i) {
-    st.push_back({at(0), at(ob[i]), at(ot[i + 1]), at(otau), n, rows[i], i, i + 1 < nout ? i + 1 : -1});
+    st.push_back({at(0), at(ob[i]), at(ot[i + 1]), n, rows[i], i, i + 1 < nout ? i + 1 : -1});
     eo.push_back({at(ob[i]), at(ot[i + 1]), rows[i]});
     put(ob[i], src, (size_t)rows[i] * n);
     src += (size_t)rows[i] * n;

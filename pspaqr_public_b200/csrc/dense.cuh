@@ -138,7 +138,7 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 // Householder QR of one panel of kb <= 32 columns in shared memory: a geqrt of
 // pan (pm rows, column-major, ld ldp; pr = null) or the tpqrt of [pr; pan] (pr kb x
 // kb upper triangular, ld kNB).  Writes the reflectors and R in place, tau to
-// lt[0:kb] and tg[0:kb], T (kNB x kb layout) to global Tout.
+// lt[0:kb], T (kNB x kb layout) to global Tout.
 //
 // A panel is latency: 32 reflectors one after the other.  Reflectors are built and
 // applied within parts of eight columns, one column a warp and one barrier a
@@ -152,8 +152,7 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 // 3.4 -> 2.6 ms.
 constexpr int kPanelScratch = kWarps * 256 + 2 * 256 + kNB * (kNB + 1);
 template <typename T>
-__device__ void panel_qr(T* pan, int ldp, int pm, T* pr, int kb, T* lt, T* tg, double* sc, T* red, int* status,
-                         T* Tout) {
+__device__ void panel_qr(T* pan, int ldp, int pm, T* pr, int kb, T* lt, double* sc, T* red, int* status, T* Tout) {
   __shared__ T s_nrm2[2];
   constexpr int kL = kNB + 1;
   const bool unit = pr == nullptr;
@@ -191,7 +190,6 @@ __device__ void panel_qr(T* pan, int ldp, int pm, T* pr, int kb, T* lt, T* tg, d
       if (t == 0) {
         if (prev_ajj) *prev_ajj = prev_beta;
         lt[jj] = tj;
-        tg[jj] = tj;
         // R(j, j) = 0 or not finite: the triangular solves would break down
         if (status && !(isfinite(beta) && beta != (T)0)) atomicOr(status, isfinite(beta) ? 8 : 4);
       }

@@ -544,7 +544,6 @@ int Tree::factorize() {
       ElimTask t;
       t.S = ptr_[se];
       t.T = T_[c];
-      t.tau = scratch_.dalloc(std::max(nc, 1));
       t.n = nc;
       t.out_begin = (int)eo.size();
       lt_[lvl].flops[0] += 2.0 * nc * nc * (nc - nc / 3.0);
@@ -561,7 +560,7 @@ int Tree::factorize() {
         lt_[lvl].flops[0] += 2.0 * rows_[e] * nc * nc;
       }
       t.out_end = (int)eo.size();
-      if (!t.T || !t.tau) return fail(-11, "out of device memory (elimination)");
+      if (!t.T) return fail(-11, "out of device memory (elimination)");
       const int cs = cluster_for(nc);
       const int g = cs == 1 ? 0 : (cs == 4 ? 1 : 2);
       et[g].push_back(t);
@@ -588,11 +587,11 @@ int Tree::factorize() {
         std::sort(all.begin(), all.end(), [](const ElimTask* x, const ElimTask* y) { return x->out_begin < y->out_begin; });
         for (const ElimTask* t : all) {
           const int nout = t->out_end - t->out_begin;
-          st.push_back({t->S, nullptr, t->T, t->tau, t->n, t->n, -1, nout ? nprog++ : -1});
+          st.push_back({t->S, nullptr, t->T, t->n, t->n, -1, nout ? nprog++ : -1});
           for (int k = 0; k < nout; ++k) {
             const ElimOut& o = eo[t->out_begin + k];
             const int in = nprog - 1;
-            st.push_back({t->S, o.B, o.T, t->tau, t->n, o.m, in, k + 1 < nout ? nprog++ : -1});
+            st.push_back({t->S, o.B, o.T, t->n, o.m, in, k + 1 < nout ? nprog++ : -1});
           }
         }
         int cs = cluster_for(nm);
@@ -771,11 +770,10 @@ int Tree::factorize() {
         ScaleTask t;
         t.S = ptr_[Lv.self_edge_of[p - Lv.first]];
         t.T = Ts_[p];
-        t.tau = scratch_.dalloc(std::max(np, 1));
         t.n = np;
         Rinv_[p] = alloc_inverses(np);
         inv64[p] = scratch_.dalloc((size_t)NB * NB * std::max(1, (np + NB - 1) / NB));
-        if (!t.T || !t.tau || !Rinv_[p] || !inv64[p]) return fail(-11, "out of device memory (scaling)");
+        if (!t.T || !Rinv_[p] || !inv64[p]) return fail(-11, "out of device memory (scaling)");
         for (int b = 0; b * NB < np; ++b) inv.push_back({t.S, Rinv_[p], inv64[p], np, b});
         const int cs = cluster_for(np);
         const int g = cs == 1 ? 0 : (cs == 4 ? 1 : 2);
@@ -965,14 +963,13 @@ int Tree::factorize() {
         r.C = C;
         r.V = spV[sp_q[p]];
         r.T = spT[sp_q[p]];
-        r.tau = scratch_.dalloc(std::max(mp, 1));
         r.colat = t.colat;
         r.rank = rank;
         r.m = mp;
         r.w = w;
         r.ldw = ldc;
         r.cm = t.cm;
-        if (!t.Q || (sh.panel && !t.panel) || !t.colat || !r.tau) {
+        if (!t.Q || (sh.panel && !t.panel) || !t.colat) {
           fail(-11, "out of device memory (rrqr)");
           return 0;
         }
@@ -1207,11 +1204,10 @@ int Tree::factorize() {
             r.Qc = Qc;
             r.V = spV[q];
             r.T = spT[q];
-            r.tau = scratch_.dalloc(std::max(t.m, 1));
             r.Rinv = scratch_.dalloc((size_t)NB * NB * ((l + NB - 1) / NB));
             r.colat = t.colat;
             r.rank = d_ell + q;
-            if (!t.G || !t.Lt || !t.colat || !r.tau || !r.Rinv) return fail(-11, "out of device memory (sketch)");
+            if (!t.G || !t.Lt || !t.colat || !r.Rinv) return fail(-11, "out of device memory (sketch)");
             for (int r0 = 0; r0 < ell[q]; r0 += 64)
               for (int c0 = r0; c0 < ell[q]; c0 += 64) gram_tiles.push_back({(int)q, r0, c0});
             const int cs = cluster_for(ell[q]);

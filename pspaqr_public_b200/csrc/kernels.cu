@@ -79,8 +79,8 @@ __global__ void k_scatter(int nnz, const double* __restrict__ val, double* const
 // panel its owner builds the kb reflectors, applying each only inside the
 // panel, and the panel's T factor; after one cluster barrier every CTA
 // applies the block reflector to its own later panels with the tiled apply
-// (two of its panels per pass).  `lt` holds the owner's tau values, `tg`
-// the global copy, `vb` a reflector tail, `tile` dev::kTileSmem elements.
+// (two of its panels per pass).  `lt` holds the owner's tau values, `vb`
+// a reflector tail, `tile` dev::kTileSmem elements.
 //
 // Steps of a chain on the same R (a tpqrt per out-edge, after the geqrt of R
 // itself) can run as a pipeline of CTAs: panel p of a step needs the rows of
@@ -129,8 +129,8 @@ __device__ __forceinline__ void chain_wait(const int* p, int v, int* status, con
 }
 
 template <typename T>
-__device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T* Tout, T* tg,
-                        T* lt, T* vb, T* red, T* tmp, T* tile, int cs, int* status = nullptr, T* pan = nullptr,
+__device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T* Tout, T* lt, T* vb, T* red, T* tmp,
+                        T* tile, int cs, int* status = nullptr, T* pan = nullptr,
                         int ldp = 0, int pw = kNB, ChainLink chain = ChainLink()) {
   const int rank = crank(cs);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -171,7 +171,7 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
           if (r <= c) pr[r + c * kNB] = __ldcg(R + (j0 + r) + (size_t)(j0 + c) * ldr);
         }
       __syncthreads();
-      dev::panel_qr(pan, ldp, pm, unit ? nullptr : pr, kb, lt + j0, tg + j0, sc, red, status,
+      dev::panel_qr(pan, ldp, pm, unit ? nullptr : pr, kb, lt + j0, sc, red, status,
                     Tout + (size_t)j0 * kNB + (j0 - pstart));
       for (int c = warp; c < kb; c += kWarps) {
         T* dst = unit ? (R + j0 + (size_t)(j0 + c) * ldr) : (B + (size_t)(j0 + c) * ldb);
@@ -217,7 +217,6 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
         if (threadIdx.x == 0) {
           R[j + (size_t)j * ldr] = beta;
           lt[j] = tj;
-          tg[j] = tj;
           // R(j, j) = 0 or not finite: the triangular solves would break down
           if (status && !(isfinite(beta) && beta != (T)0)) atomicOr(status, isfinite(beta) ? 8 : 4);
         }
@@ -278,12 +277,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_elim(const ElimTask* __restrict
   T* vb = lt + t.n;
   T* tile = vb + vmax;
   T* pan = kStage ? tile : nullptr;
-  dist_qr<T>(as<T>(t.S), t.n, nullptr, 0, t.n, t.n, 1, as<T>(t.T), as<T>(t.tau), lt, vb, red, tmp, tile, cs, status,
-             pan, vmax, pw);
+  dist_qr<T>(as<T>(t.S), t.n, nullptr, 0, t.n, t.n, 1, as<T>(t.T), lt, vb, red, tmp, tile, cs, status, pan, vmax, pw);
   for (int o = t.out_begin; o < t.out_end; ++o) {
     const ElimOut e = outs[o];
-    dist_qr<T>(as<T>(t.S), t.n, as<T>(e.B), e.m, e.m, t.n, 0, as<T>(e.T), as<T>(t.tau), lt, vb, red, tmp, tile,
-               cs, status, pan, vmax, pw);
+    dist_qr<T>(as<T>(t.S), t.n, as<T>(e.B), e.m, e.m, t.n, 0, as<T>(e.T), lt, vb, red, tmp, tile, cs, status,
+               pan, vmax, pw);
   }
 }
 
@@ -316,8 +314,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_elim_pipe(const ElimStep* __res
   link.ticks = counters + 1;
   link.limit = limit;
   T* B = as<T>(t.B);
-  dist_qr<T>(as<T>(t.S), t.n, B, t.m, B ? t.m : t.n, t.n, B ? 0 : 1, as<T>(t.T), as<T>(t.tau), lt, vb, red, tmp, tile,
-             cs, status, kStage ? tile : nullptr, vmax, pw, link);
+  dist_qr<T>(as<T>(t.S), t.n, B, t.m, B ? t.m : t.n, t.n, B ? 0 : 1, as<T>(t.T), lt, vb, red, tmp, tile, cs, status,
+             kStage ? tile : nullptr, vmax, pw, link);
 }
 
 // kStage: panels factored in shared memory (nmax rows), as in k_elim.
@@ -332,8 +330,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_scale(const ScaleTask* __restri
   T* lt = tmp + kNB;
   T* vb = lt + nmax;
   T* tile = vb + nmax;
-  dist_qr<T>(as<T>(t.S), t.n, nullptr, 0, t.n, t.n, 1, as<T>(t.T), as<T>(t.tau), lt, vb, red, tmp, tile, cs,
-             status, kStage ? tile : nullptr, nmax, pw);
+  dist_qr<T>(as<T>(t.S), t.n, nullptr, 0, t.n, t.n, 1, as<T>(t.T), lt, vb, red, tmp, tile, cs, status,
+             kStage ? tile : nullptr, nmax, pw);
 }
 
 // ------------------------------------------------------------ chunked applies
@@ -783,7 +781,7 @@ __global__ void __launch_bounds__(kThreads) k_rrqr_assemble(const RrqrSrc* __res
 }
 
 // Householder QR of the selected columns C(:, colat[0:rank]) (the pivot order
-// fixed beforehand) into V / T / tau, then (where the task has a Qc) the
+// fixed beforehand) into V / T, then (where the task has a Qc) the
 // orthonormal basis Qc = C_sel R^{-1} (column-major, ld m): the inverses of R's diagonal
 // blocks, a warp each, then mma_trsm_right on 64-row chunks dealt to the cluster's CTAs.
 // (Scalar sums and a substitution of one thread a row, before, took a quarter of the kernel: 64^3,
@@ -814,7 +812,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_selected_qr(const RrqrTask* __r
       for (int r = lane; r < m; r += 32) t.V[r + (size_t)l * m] = __ldg(C + (size_t)r * ldw + c);
   }
   __syncthreads();
-  dist_qr<double>(t.V, m, nullptr, 0, m, rk, 1, t.T, t.tau, lt, vb, red, tmp, tile, cs, nullptr,
+  dist_qr<double>(t.V, m, nullptr, 0, m, rk, 1, t.T, lt, vb, red, tmp, tile, cs, nullptr,
                   kStage ? tile : nullptr, mmax, pw);
   if (!t.Qc) return;
   // R(l, j) = V[l + j m] for l <= j, written by the owners of column j

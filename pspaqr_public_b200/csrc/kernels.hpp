@@ -76,7 +76,7 @@ bool pivots_cluster_fit(int cs, size_t smem, bool big);
 cudaError_t launch_pivots(const PivotTask* t, int ntasks, int cs, size_t smem, bool big, double tol,
                           double pivot_rtol, cudaStream_t st);
 // Householder QR of the columns C(:, colat[0:*rank]) (pivot order given) into
-// V / T / tau and (where the task has a Qc) the orthonormal basis
+// V / T and (where the task has a Qc) the orthonormal basis
 // Qc = C_sel R^{-1}; cs-CTA clusters, tasks of at most mmax rows and nmax
 // selected columns.
 cudaError_t launch_selected_qr(const RrqrTask* t, int ntasks, int cs, int mmax, int nmax, cudaStream_t st);

@@ -17,7 +17,6 @@ namespace spq {
 struct ElimTask {
   double* S;      // n x n diagonal block (ld = n)
   double* T;      // kNB x n block factors of the diagonal QR
-  double* tau;    // n doubles of scratch (reflector broadcast)
   int n;
   int out_begin, out_end;  // range in ElimOut
 };
@@ -33,7 +32,6 @@ struct ElimStep {
   double* S;
   double* B;
   double* T;
-  double* tau;
   int n, m, in, out;
 };
 
@@ -65,7 +63,6 @@ struct UpdItem {
 struct ScaleTask {
   double* S;
   double* T;
-  double* tau;
   int n;
 };
 
@@ -102,7 +99,6 @@ struct RrqrTask {
   double* Qc;        // m x *rank output: the orthonormal basis C_sel R^{-1}, or null
   double* V;         // m x m output: reflector j below the diagonal of column j, R above (ld m)
   double* T;         // kNB x m output block factors
-  double* tau;       // m
   double* Rinv;      // with Qc: inverses of R's diagonal blocks (32 x 32 each)
   const int* colat;  // column at each pivot position
   int* rank;         // columns selected
