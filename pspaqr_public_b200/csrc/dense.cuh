@@ -388,6 +388,7 @@ template <typename T, bool kCg, bool kRight>
 __device__ void mma_apply(const T* V, int ldv, const T* Tm, int ldt, int kb, int unit, T* A, int lda, T* C, int ldc,
                           int m, int nc, double* sm, int stages, int cgap) {
   static_assert(kThreads == 256 && kNB == 32 && kNC == 64 && kRT == 32, "tile shapes");
+  if (m <= 0) return;  // no barrier would part this call's reads of T from the next one's writes
   // 16-byte fragments; a float caller's scratch starts on any 4 bytes
   sm = reinterpret_cast<double*>((reinterpret_cast<size_t>(sm) + 15) & ~(size_t)15);
   double* sT = sm;

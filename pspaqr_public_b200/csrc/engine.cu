@@ -421,7 +421,8 @@ static int cluster_for(int ncols) {
 
 // The items of the pipelined updates.  An op waits for the op before on its top
 // block (the ops of one interior follow one another) and for the last op before on
-// its lower block; items are sorted by the longest way to them, so that those taken
+// its lower block (every op has panels and rows, so that one that is done has waited for
+// those before it); items are sorted by the longest way to them, so that those taken
 // together are ready together.
 static void plan_update_items(const std::vector<UpdTask>& ut, const std::vector<UpdOp>& uo, std::vector<UpdItem>& out) {
   struct Dep {
@@ -625,6 +626,7 @@ int Tree::factorize() {
         const int c = Lv.col_c[q];
         const int ecm = Lv.col_ecm[q];
         const int nc = size_[c];
+        if (nc == 0) continue;  // no reflectors
         const int se = Lv.self_edge_of[c - Lv.first];
         UpdOp a;
         a.kind = 0;
@@ -644,6 +646,7 @@ int Tree::factorize() {
         for (int r = Lv.out_begin[ii]; r < Lv.out_end[ii]; ++r, ++j) {
           const int ecn = Lv.out_edges[r];
           const int emn = Lv.col_emn[j];
+          if (rows_[ecn] == 0) continue;  // no rows: the reflectors are the identity
           UpdOp b;
           b.kind = 1;
           b.V = ptr_[ecn];
@@ -660,7 +663,7 @@ int Tree::factorize() {
         }
       }
       const int op_end = (int)uo.size();
-      for (int c0 = 0; c0 < ncol; c0 += kChunk) ut.push_back({op_begin, op_end, c0, std::min(kChunk, ncol - c0)});
+      for (int c0 = 0; op_end > op_begin && c0 < ncol; c0 += kChunk) ut.push_back({op_begin, op_end, c0, std::min(kChunk, ncol - c0)});
     }
     lt_[lvl].flops[1] += P.fl_upd;
     lt_[lvl].ntasks_elim = (int)Lv.interiors.size();
@@ -1766,7 +1769,6 @@ int Tree::capture_sweep(SweepRun run, int* counters, cudaGraph_t* g, long long* 
 
 int Tree::build_solve_graph() {
   set_factor_fp32(fp32_);
-  const int L = st_.nlevels;
   const int ncl = (int)st_.clusters.size();
   xoff_.assign(ncl, 0);
   int64_t off = st_.n;
