@@ -281,7 +281,10 @@ __global__ void __launch_bounds__(kT, 512 / kT) k_pivots(const PivotTask* __rest
   lap(0);
 
   const double f2 = (1.0 - pivot_rtol) * (1.0 - pivot_rtol);
-  const double tol2 = tol * tol;
+  // the stop on squares: |R(i,i)|^2 >= tol2 |R(0,0)|^2; a zero |R(i,i)| stops at every
+  // positive tolerance, those whose square underflows among them
+  const double tol2 = tol > 0.0 ? tol * tol : 0.0;
+  auto keep = [&](double v2, double r2) { return v2 >= tol2 * r2 && (v2 > 0.0 || !(tol > 0.0)); };
   int par = 0, rk = kmin, nrebuild = 0, npan = 0, pub = 0;
   int base = 0;        // steps contained in the panel's residuals
   double ref2 = 0.0;   // largest squared norm when they were last brought up to date
@@ -659,7 +662,7 @@ __global__ void __launch_bounds__(kT, 512 / kT) k_pivots(const PivotTask* __rest
         if (i == base) ref2 = gmx2;
         int act = 0;
         double thr2 = gmx2 * f2;
-        if (i > 0 && !(r002 > 0.0 && M2 >= tol2 * r002)) {
+        if (i > 0 && !(r002 > 0.0 && keep(M2, r002))) {
           act = 2;
         } else if (i > base && (i - base == kLag || gmx2 < 1e-3 * ref2)) {
           act = 4;
@@ -801,7 +804,7 @@ __global__ void __launch_bounds__(kT, 512 / kT) k_pivots(const PivotTask* __rest
     if (cs > 1 && rank == powner) __threadfence();
     if (i == 0) {
       r002 = nrm2;
-    } else if (!(nrm2 >= tol2 * r002) || isinf(nrm2)) {
+    } else if (!keep(nrm2, r002) || isinf(nrm2)) {
       rk = i;
       break;
     }
