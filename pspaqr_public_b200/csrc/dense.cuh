@@ -329,7 +329,7 @@ __device__ void panel_qr(T* pan, int ldp, int pm, T* pr, int kb, T* lt, double* 
   }
   for (int e = t; e < kb * kb; e += kThreads) {
     const int l = e % kb, j = e / kb;
-    if (l <= j) Tout[l + (size_t)j * kNB] = (T)sT[l + j * kL];
+    Tout[l + (size_t)j * kNB] = l <= j ? (T)sT[l + j * kL] : (T)0;
   }
 }
 
