@@ -430,8 +430,9 @@ __global__ void __launch_bounds__(kT, 512 / kT) k_pivots(const PivotTask* __rest
       }
     for (int b = tid; b < kBins; b += kT) S.hist[b] = 0;
     if (tid < 4) s_cnt[tid] = 0;
-    // columns below the stop threshold can no longer become pivots
-    const double dead = i > 0 ? tol2 * r002 : 0.0;
+    // columns further below the stop threshold than pivot_rtol can no longer become
+    // pivots (one within it can, as the first position, and then stops the selection)
+    const double dead = i > 0 ? tol2 * r002 * f2 : 0.0;
     __syncthreads();
     const double cthr = M2 * f2;
     const int top = __double2hiint(M2);
