@@ -62,10 +62,9 @@ int spq_set_rank_margin(spq_tree* h, float margin) {
   return 0;
 }
 
-int spq_set_sketch_tuning(spq_tree* h, double sketch_tol, int smem) {
+int spq_set_sketch_tuning(spq_tree* h, double sketch_tol, int /*smem*/) {
   if (!h || !(sketch_tol > 0 && sketch_tol <= 1)) return -1;
   h->t->sketch_tol = sketch_tol;
-  h->t->sketch_smem = smem != 0;
   return 0;
 }
 

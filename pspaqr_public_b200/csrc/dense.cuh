@@ -127,6 +127,16 @@ __device__ void panel_t(const T* V, int ldv, int m, int kb, int unit, const T* t
   larft_from_gram(Tm, ldt, kb, tau, tmp);
 }
 
+// Counters that CTAs of one launch wait on.
+__device__ __forceinline__ int ld_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(int* p, int v) {
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 // D (8 x 8) += A (8 x 4) B (4 x 8) in FP64, one warp.  Lane = 4 n + k holds
 // A(n, k) and B(k, n), and D(n, 2 k), D(n, 2 k + 1).
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
@@ -841,17 +851,6 @@ __device__ void mma_trsm_right(const T* R, int ldr, const double* Inv, T* C, int
     __syncthreads();  // X_J before it is read, T before it is overwritten
   }
 }
-
-// ---------------------------------------------------------------- asynchronous copies
-template <typename T>
-__device__ __forceinline__ void cp_async_elem(T* sdst, const T* gsrc) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
-  if (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 }  // namespace dev
 }  // namespace spq

@@ -519,7 +519,7 @@ int Tree::factorize() {
       // scratch is reset every level: its chunks need only start with those the
       // recorded level ended with (checked below)
       key.sizes.assign(size_.begin() + Lv.first, size_.begin() + Lv.first + Lv.count);
-      key.sizes.push_back(update_pipe);
+      key.update_pipe = update_pipe;
       key.flags = (fp32_ ? 1 : 0) | (rank_model_ ? 2 : 0) | (rank_log_ ? 4 : 0) | (verbose >= 2 ? 8 : 0);
       auto prefix = [](const std::vector<const char*>& have, const std::vector<const char*>& rec) {
         return have.size() >= rec.size() && std::equal(rec.begin(), rec.end(), have.begin());

