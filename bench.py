@@ -18,8 +18,8 @@ learned-rank method (float factors whose left block-reflector applies are
   roofline : the trailing updates of the headline step against cuBLAS DGEMM
           measured in the run (FP64 mma), or, where most of their flops ran on
           the tcgen05 path, against the 3xTF32 ceiling from the measured bf16 peak;
-          roofline_fp64_rrqr: the plain method's pivoted QR against the measured
-          HBM peak.
+          fp64_rrqr: time of the plain method's pivoted QR, bound by latency and
+          shared memory, beside the time of the bytes it cannot do without.
   backward_error : ||A z - u|| / ||u|| with z = M^-1 u for seeded probes, per
           variant (the factorization's relative backward error).
   cpu_baseline : the CPU oracle (LAPACK restatement of the reference path,
@@ -27,7 +27,7 @@ learned-rank method (float factors whose left block-reflector applies are
 
 ``--impl reference`` times that CPU oracle as the reference arm (the reference
 itself cannot be built here: no Eigen, MPI, TaskTorrent or LAPACKE headers).
-``--config5`` runs BASELINE config 5 (1024^2 convection-diffusion, 16
+``--config5`` runs the block workload (1024^2 convection-diffusion, 16
 right-hand sides solved together) and prints its own line.  With torchrun
 (N > 1) every rank solves its own replica (the subtree sharding plan is in
 pspaqr_public_b200.shard; the factorization itself is not sharded yet).
@@ -299,15 +299,14 @@ def run_ours(args):
     upd_tflops = upd_flops / upd_s / 1e12 if upd_s > 0 else 0.0
     fact = float(np.mean(head["ftimes"]))
     # dominant kernel of the plain factorization: the pivoted QR
-    # (k_rrqr_assemble, k_pivots, k_selected_qr of every level).  Bytes it cannot
-    # do without (the gather and one pass for the norms) over its event-timed
-    # duration: a small share of HBM's rate, since the catch-up products and the
-    # latency of the pivot steps bound it
+    # (k_rrqr_assemble, k_pivots, k_selected_qr of every level): event-timed duration,
+    # and the bytes it cannot do without (the gather and one pass for the norms).  No
+    # share of HBM's rate: the catch-up products (shared memory) and the latency of the
+    # pivot steps and panels bound it
     plt = res["fp64"]["level_ms"]
     rrqr_s = float(plt[:, ParTree.LEVEL_PHASES.index("rrqr")].sum()) / 1e3
     rrqr_bytes = res["fp64"]["rrqr_bytes"]
     hbm_peak = peaks.get("hbm_gbs") or 6650.0
-    achieved = rrqr_bytes / rrqr_s / 1e9
     nnz = len(ri)
     # per step: the matrix values (the sparsity maps are built once per partition)
     # and b host->device, x device->host
@@ -379,9 +378,8 @@ def run_ours(args):
                      "algorithmic_flops": upd_flops, "launches": upd_launches, "duration_s": upd_s,
                      "per_launch_flops": upd_flops / max(upd_launches, 1), "peak_source": upd_src},
         "tensor_core_levels": {k: int(on_tc[:, i].sum()) for i, k in enumerate(("updates", "left", "right"))},
-        "roofline_fp64_rrqr": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
-                               "frac": achieved / hbm_peak, "traffic": None,
-                               "duration_s": rrqr_s},
+        "fp64_rrqr": {"bound": "latency and shared memory", "duration_s": rrqr_s, "floor_bytes": rrqr_bytes,
+                      "floor_s": rrqr_bytes / hbm_peak / 1e9},
         "factor_fp64_tflops": res["fp64"]["flops"] / float(np.mean(res["fp64"]["ftimes"])) / 1e12,
         "dgemm_peak_tflops": fp64_peak,
         "clocks": clk.summary(),
@@ -476,7 +474,7 @@ def run_reference(args):
 
 
 def run_config5(args):
-    """2D upwinded convection-diffusion on 1024^2 (n = 1,048,576),
+    """Block workload: 2D upwinded convection-diffusion on 1024^2 (n = 1,048,576),
     rotating unit vortex, eps 1e-2, 14 levels, tol 1e-2; mixed-precision factor with
     learned ranks; 16 right-hand sides b_j ~ N(0,1) (seed 4) solved together by
     lockstep flexible GMRES in FP64 to 1e-10.  A step is factorize + the block
