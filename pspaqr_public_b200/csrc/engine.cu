@@ -30,7 +30,11 @@ constexpr int kChunk = 64;        // columns (rows) per CTA of the chunked appli
 // while whole chains would leave a third of the GPU idle (64^3 FP64: 256 interiors
 // 2.7 ms whole, 4.3 ms pipelined; 128 interiors 10.4 and 5.3 ms).  With up to
 // kElimPipeMixed interiors of different cluster sizes, which as whole chains run
-// one size after the other, it pays too (1024 leaves of 384^2: 15.5 and 9.8 ms).
+// one size after the other, it pays too where at least a quarter take clusters of
+// several CTAs.  Share of those, FP64 chains whole / pipelined: 512 leaves of 240^2 7 %
+// 2.83 / 2.80 ms, 256^2 28 % 4.03 / 3.18, 272^2 51 % 5.39 / 3.45; about 1000 of 48^3 1 % 3.24 /
+// 4.09, 56^3 6 % 4.59 / 6.51, 360^2 26 % 5.54 / 4.82, 384^2 71 % 10.6 / 5.57; 2048 of 480^2
+// 7 % 7.47 / 10.9, 512^2 24 % 12.3 / 12.2 (FP32 10.3 / 11.3), 544^2 51 % 19.1 / 13.4.
 constexpr size_t kElimPipe = 160, kElimPipeMixed = 1024;
 // Levels with at most kUpdPipe update tasks run the ops of a task as a pipeline of
 // CTAs.  64^3 FP64, tasks whole / pipelined: 1372 tasks 11.5 / 9.2 ms, 794 13.2 / 9.1,
@@ -573,7 +577,9 @@ int Tree::factorize() {
       // few interiors: a pipeline of one cluster per chain step, in clusters as
       // wide as the steps leave SMs for
       const size_t ni = Lv.interiors.size(), sizes = !et[0].empty() + !et[1].empty() + !et[2].empty();
-      const bool pipe = !eo.empty() && (ni <= kElimPipe || (sizes > 1 && ni <= kElimPipeMixed));
+      const size_t wide = et[1].size() + et[2].size();
+      const bool pipe =
+          !eo.empty() && (ni <= kElimPipe || (sizes > 1 && ni <= kElimPipeMixed && 4 * wide >= ni));
       if (pipe) {
         std::vector<ElimStep> st;
         int nprog = 0, nm = 1, vm = 1;
