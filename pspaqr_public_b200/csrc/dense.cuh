@@ -357,10 +357,12 @@ constexpr int kTileV = kNB * kLdV, kTileC = kNC * kLdC;
 // apart (the 16-byte loads of a quarter-warp), accumulators 2 fk of the four lanes of
 // a row, and 2 fk + 1, hold columns that differ mod 4 (the 8-byte loads of the
 // second product): with kLdV both are free of bank conflicts.  With columns
-// 0 4 1 5 2 6 3 7 and kLdV = 40 both took two wavefronts for one, and shared memory
-// bounded the applies (L1 data pipe 77 % busy): 64^3 FP64 updates 64.7 -> 57.5 ms, scaling
-// applies 50.0 -> 41.6; FP32 factors updates 68 -> 59.5, scaling and compression applies
-// 87 -> 76 ms.
+// 0 4 1 5 2 6 3 7 and kLdV = 40 both took two wavefronts for one: 64^3 FP64 updates
+// 64.7 -> 57.5 ms, scaling applies 50.0 -> 41.6; FP32 factors updates 68 -> 59.5, scaling and
+// compression applies 87 -> 76 ms.  What bounds them now is the latency of the mma chains,
+// loads and barriers at two CTAs an SM (ncu, 48^3 FP64: k_edge_left and k_update_pipe issue
+// with a quarter of the warps, stalls on fixed latencies first, the shared-memory data
+// pipe 45 and 53 % busy, DRAM 8 %).
 __device__ __forceinline__ int frag_col(int n) { return (0x57463120 >> (4 * n)) & 15; }
 static_assert(kRT * kLdR <= kTileC, "right tiles");
 // Shared memory (doubles) of mma_apply with `stages` tiles of V and C.

@@ -14,8 +14,7 @@
 // rebuilt from the largest bounds and its new columns are caught up with all
 // basis vectors found so far, a matrix product (FP64 mma.sync, 8 columns x 8
 // basis vectors per warp and tile).  On the 3D diffusion interfaces a column
-// enters a panel 0.3-0.5 times on average and five times fewer column updates
-// are made than by dlaqp2 (48^3, tolerance 1e-2).
+// enters a panel 0.2-0.4 times on average (48^3, tolerance 1e-2).
 //
 // A pivot step reads the panel once: r_j = q_i^T c_j for its columns, whose
 // squared norms lose r_j^2; the residuals themselves are brought up to date
@@ -32,9 +31,11 @@
 // selection and QR of the selected columns, bound by L2 and HBM traffic), 104 ms
 // now (52 ms selection, 36 ms QR of the selected columns, 8 ms gather).
 //
-// What bounds it: on wide interfaces the catch-up (shared memory bandwidth: 24
-// wavefronts per 8 rows x 8 columns x 8 vectors against 16 cycles of FP64
-// mma), on small ones the latency of the pivot steps.
+// What bounds it: latency.  The steps take half to two thirds of the time (48^3:
+// 2.7 of 3.1 million cycles at the top, 0.8 of 2.8 where the rebuilds take most), four to
+// five barriers each; ncu at 144 interfaces of 176 x 3225: barrier stalls first, the
+// shared-memory pipe 29 % busy with the catch-up (24 wavefronts per 8 rows x 8 columns x 8
+// vectors against 16 cycles of FP64 mma), FP64 pipe and DRAM below 5 %.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
